@@ -305,6 +305,19 @@ int b200_gdn_chunked_prefill_fused(const void* q, int64_t q_stride_t, int64_t q_
                                    void* out, int64_t out_stride_t, int64_t out_stride_h, int32_t num_heads,
                                    int32_t key_dim, int32_t value_dim, b200_stream_t stream);
 
+/* The same packed chunk-64 prefill in two launches: the chunks' own matrices, all at once, then a walk over every sequence's
+ * chunks with the state in registers.  Same arguments and rules, plus `workspace`:
+ * b200_gdn_chunked_prefill_walk_workspace_bytes(batch, total_tokens, num_heads) bytes of caller-owned device memory, 16-byte
+ * aligned (contents undefined afterwards). */
+int64_t b200_gdn_chunked_prefill_walk_workspace_bytes(int32_t batch, int32_t total_tokens, int32_t num_heads);
+int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k,
+                                  int64_t k_stride_t, int64_t k_stride_h, const void* v, int64_t v_stride_t,
+                                  int64_t v_stride_h, const float* beta, int64_t beta_stride_t,
+                                  int64_t beta_stride_h, const float* g, int64_t g_stride_t, int64_t g_stride_h,
+                                  const int32_t* cu_seqlens, int32_t batch, int32_t total_tokens, void* workspace,
+                                  float* state, void* out, int64_t out_stride_t, int64_t out_stride_h, int32_t num_heads,
+                                  int32_t key_dim, int32_t value_dim, b200_stream_t stream);
+
 /* ------------------------------------------------------------------------------------------------------------------
  * Row-wise layer operators around the projections (one launch each).  bf16 tensors, fp32 math, one rounding at the
  * reference's rounding points.

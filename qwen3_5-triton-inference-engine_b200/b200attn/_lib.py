@@ -64,6 +64,8 @@ SIGNATURES: dict[str, list] = {
     "b200_swiglu_pair": [P, I64, P, I64, P, I32, I32, P],
     "b200_gdn_chunked_prefill_fused": [P, I64, I64, P, I64, I64, P, I64, I64, P, I64, I64, P, I64, I64, P, I32, I32,
                                        P, P, I64, I64, I32, I32, I32, P],
+    "b200_gdn_chunked_prefill_walk": [P, I64, I64, P, I64, I64, P, I64, I64, P, I64, I64, P, I64, I64, P, I32, I32,
+                                      P, P, P, I64, I64, I32, I32, I32, P],
     "b200_hyper_connect": [P, I32, P, P, P, I32, P, P, P, I32, I32, I32, I32, c_float, I32, I32, P],
     "b200_swiglu_f32": [P, I64, P, I32, I32, P],
     "b200_mingru_prefill": [P, I64, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, P],
@@ -107,6 +109,7 @@ OTHER = {
     "b200_fused_decode_workspace_bytes": ([], c_int64),
     "b200_argmax_rows_workspace_bytes": ([], c_int64),
     "b200_gdn_chunked_prefill_packed_workspace_bytes": ([I32, I32, I32], c_int64),
+    "b200_gdn_chunked_prefill_walk_workspace_bytes": ([I32, I32, I32], c_int64),
 }
 
 _lib = None

@@ -622,18 +622,12 @@ def _(q, k, delta, g_cumsum, chunk_state):
 _ONE_SEQUENCE_CU: dict = {}
 
 
-# One sequence walks its chunks serially: the single kernel spends ~9 us per chunk on 16 CTAs, the three stages ~3.3 us
-# per chunk in the state stage plus two chunk-parallel stages, which is the shorter way from about 16 chunks on.
-CHUNKED_THREE_STAGE_FROM = 1024
-
-
 def call_gdn_recurrent_prefill_chunked_triton(q, k, v, beta, g):
     """Chunk-64 prefill of ONE sequence; returns (out [T,H,DV] bf16, final_state [H,DK,DV] fp32).
     triton_kernels/gdn_recurrent_prefill.py:1026-1047 (name kept for drop-in use; no Triton is involved).  The caller
-    wants only the output and the final state, so up to CHUNKED_THREE_STAGE_FROM tokens the three stages run as the
-    single tcgen05 kernel with cu_seqlens = [0, T] whenever its layout rules hold (128-dim heads, 16-byte aligned
-    q/k/v with strides that are multiples of 8); longer sequences, and inputs outside those rules, take the three
-    reference-shaped stages (tensor-core products, HBM intermediates in one workspace) in one call."""
+    wants only the output and the final state, so the packed form runs with cu_seqlens = [0, T] whenever its layout rules
+    hold (128-dim heads, 16-byte aligned q/k/v with strides that are multiples of 8; 2048 tokens: 80 us against 180 us in
+    three stages); other inputs take the three reference-shaped stages (HBM intermediates in one workspace) in one call."""
     token_num = q.shape[0]
     fusable = (q.shape[-1] == GDN_DIM and v.shape[-1] == GDN_DIM
                and all(t.stride(-1) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
@@ -643,7 +637,7 @@ def call_gdn_recurrent_prefill_chunked_triton(q, k, v, beta, g):
         if len(_ONE_SEQUENCE_CU) > 4096:
             _ONE_SEQUENCE_CU.clear()
         _ONE_SEQUENCE_CU[key] = torch.tensor([0, token_num], dtype=torch.int32, device=q.device)
-    if fusable and token_num < CHUNKED_THREE_STAGE_FROM:
+    if fusable:
         out, state = gdn_chunked_prefill_packed(q, k, v, beta, g, _ONE_SEQUENCE_CU[key])
     else:
         out, state = gdn_chunked_prefill_packed(q, k, v, beta, g, _ONE_SEQUENCE_CU[key], max_seqlen=token_num,
@@ -656,8 +650,9 @@ def gdn_chunked_prefill_packed(q, k, v, beta, g, cu_seqlens, max_seqlen=None, fu
     sequence start).  Returns (out [T,H,DV] bf16, state [B,H,DK,DV] fp32).  The reference's chunk path is
     single-sequence only (engine/runner.py:263-267); this is its packed form, equal to
     gdn_recurrent_prefill_sequential(..., cu_seqlens) up to fp32 rounding.
-    fused=True: one tcgen05 kernel, state resident in tensor memory, no workspace (q/k/v need token and head strides
-    that are multiples of 8 elements).  fused=False: the three reference-shaped stages through a workspace;
+    fused=True: what the chunks need of themselves, all at once, then a walk over each sequence's chunks with the state in
+    registers (q/k/v need token and head strides that are multiples of 8 elements).  fused=False: the three
+    reference-shaped stages through a workspace;
     `max_seqlen` (host int) sizes their grid.  `state_out` (contiguous fp32 [B,H,DK,DV]) receives the final states in
     place of a fresh tensor, e.g. a cache's own state buffer."""
     _check_gdn(q, k, v, beta, g)
@@ -675,9 +670,11 @@ def gdn_chunked_prefill_packed(q, k, v, beta, g, cu_seqlens, max_seqlen=None, fu
     out = torch.empty((token_num, num_heads, value_dim), dtype=q.dtype, device=q.device)
     if fused:
         cu_seqlens = cu_seqlens.contiguous()  # kept alive until the launch is enqueued
-        _lib.call("b200_gdn_chunked_prefill_fused", _ptr(q), q.stride(0), q.stride(1), _ptr(k), k.stride(0), k.stride(1),
+        nbytes = _lib.load().b200_gdn_chunked_prefill_walk_workspace_bytes(batch, token_num, num_heads)
+        workspace = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        _lib.call("b200_gdn_chunked_prefill_walk", _ptr(q), q.stride(0), q.stride(1), _ptr(k), k.stride(0), k.stride(1),
                   _ptr(v), v.stride(0), v.stride(1), _ptr(beta), beta.stride(0), beta.stride(1), _ptr(g), g.stride(0),
-                  g.stride(1), _ptr(cu_seqlens), batch, token_num, _ptr(state), _ptr(out), out.stride(0),
+                  g.stride(1), _ptr(cu_seqlens), batch, token_num, _ptr(workspace), _ptr(state), _ptr(out), out.stride(0),
                   out.stride(1), num_heads, key_dim, value_dim, _stream())
         return out, state
     assert max_seqlen is not None, "the three-stage path needs max_seqlen"

@@ -132,3 +132,41 @@ def test_chunk_stages_on_unaligned_views(ops, token_num):
     w, u, gcs = ops.gdn_chunk_prepare_wy(kd, vd, beta.to(DEV), g.to(DEV))
     w2, u2, gcs2 = ops.gdn_chunk_prepare_wy(k.to(DEV), v.to(DEV), beta.to(DEV), g.to(DEV))
     assert torch.equal(w, w2) and torch.equal(u, u2) and torch.equal(gcs, gcs2)
+
+
+@pytest.mark.parametrize("heads,lengths", [(2, [0, 1, 16, 17, 33, 63, 64, 65, 300]), (3, [0, 1, 16, 17, 33, 63, 64, 65, 300, 129, 32, 48]),
+                                           (8, [0, 1, 16, 17, 33, 63, 64, 65, 300]), (16, [0, 1, 16, 17, 33, 63, 64, 65, 300])])
+def test_walk_forms(ops, heads, lengths):
+    """Every form of the chunk walk (the number of heads in the call chooses: teams, two teams, half and whole heads per CTA) at the
+    edges of its 16-token tiles and 64-token chunks, against the token-serial kernel; and a sequence full of NaN changes nothing
+    in its neighbours, whose last chunks end in the middle of a tile.  Bars as above."""
+    gen = torch.Generator().manual_seed(31 * heads)
+    total = sum(lengths)
+    q, k, v, beta, g = (x.to(DEV) for x in gdn_inputs(total, heads, gen))
+    ends = torch.tensor(lengths).cumsum(0).tolist()
+    cu = torch.tensor([0] + ends, dtype=torch.int32, device=DEV)
+    out, state = ops.gdn_chunked_prefill_packed(q, k, v, beta, g, cu)
+    ref_out, ref_state = ops.gdn_recurrent_prefill_sequential(q, k, v, beta, g, cu)
+    assert maxabs(out, ref_out) <= 1e-2 and maxabs(state, ref_state) <= 5e-4
+    assert float(state[0].abs().max()) == 0.0
+    lo, hi = ends[3], ends[4]
+    q[lo:hi], k[lo:hi], v[lo:hi], beta[lo:hi], g[lo:hi] = (float("nan"),) * 5
+    out2, state2 = ops.gdn_chunked_prefill_packed(q, k, v, beta, g, cu)
+    assert torch.equal(out2[:lo], out[:lo]) and torch.equal(out2[hi:], out[hi:])
+    others = [i for i in range(len(lengths)) if i != 4]
+    assert torch.equal(state2[others], state[others])
+
+
+def test_one_launch_entry(ops):
+    """The entry point without a workspace (tcgen05, one CTA per head) gives what the walk gives."""
+    from b200attn import _lib
+    gen, lengths, heads = torch.Generator().manual_seed(8), [5, 64, 65, 1, 200], 16
+    total = sum(lengths)
+    q, k, v, beta, g = (x.to(DEV) for x in gdn_inputs(total, heads, gen))
+    cu = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    out, state = torch.empty_like(v), torch.empty(len(lengths), heads, 128, 128, device=DEV)
+    _lib.call("b200_gdn_chunked_prefill_fused", *(a for t in (q, k, v, beta, g) for a in (t.data_ptr(), t.stride(0), t.stride(1))), cu.data_ptr(),
+              len(lengths), total, state.data_ptr(), out.data_ptr(), out.stride(0), out.stride(1), heads, 128, 128,
+              torch.cuda.current_stream().cuda_stream)
+    ref_out, ref_state = ops.gdn_chunked_prefill_packed(q, k, v, beta, g, cu)
+    assert maxabs(out, ref_out) <= 1e-2 and maxabs(state, ref_state) <= 5e-4
