@@ -504,6 +504,15 @@ int b200_hgrn2_prefill(const void* qfv, int64_t stride, const float* lower, cons
                        int32_t batch, int32_t tokens, int32_t heads, int32_t dim, int32_t vdim, int32_t true_vdim, float eps,
                        int32_t f32, int32_t serial, int32_t segment, int32_t segments, float* workspace,
                        b200_stream_t stream);
+/* b200_hgrn2_prefill (b200_gla_prefill) with a workspace of b200_outer_walk_workspace_bytes() for what every chunk needs of
+ * itself: computed for all chunks at once, then walked (64 < dim <= 128; other shapes do not use it).  The size is 0 where
+ * the shape does not, or where it would be more than 1 GiB; a NULL workspace is the form without. */
+int64_t b200_outer_walk_workspace_bytes(int32_t tokens, int32_t batch, int32_t heads, int32_t dim, int32_t vdim);
+int b200_hgrn2_prefill_walk(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm, float* state,
+                            const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start, float* o_scratch, void* out,
+                            int32_t batch, int32_t tokens, int32_t heads, int32_t dim, int32_t vdim, int32_t true_vdim, float eps,
+                            int32_t f32, int32_t serial, int32_t segment, int32_t segments, float* workspace, void* chunks,
+                            b200_stream_t stream);
 int b200_hgrn2_decode(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm, float* state,
                       const int64_t* pos, const int64_t* active, void* out, int32_t batch, int32_t heads, int32_t dim,
                       int32_t vdim, int32_t true_vdim, float eps, int32_t f32, int32_t overlap, b200_stream_t stream);
@@ -519,6 +528,12 @@ int b200_gla_prefill(const void* qkv, int64_t stride, const float* z, int64_t z_
                      const int32_t* start, float* o_scratch, void* out, int64_t out_stride, int32_t batch, int32_t tokens,
                      int32_t heads, int32_t dim, int32_t vdim, int32_t true_vdim, float q_scale, float inv_tau, float eps,
                      int32_t f32, int32_t serial, int32_t segment, int32_t segments, float* workspace, b200_stream_t stream);
+int b200_gla_prefill_walk(const void* qkv, int64_t stride, const float* z, int64_t z_stride, const float* bias, const float* norm,
+                          const void* gate, int64_t gate_stride, float* state, const int32_t* cu_seqlens, const int32_t* slots,
+                          const int32_t* start, float* o_scratch, void* out, int64_t out_stride, int32_t batch, int32_t tokens,
+                          int32_t heads, int32_t dim, int32_t vdim, int32_t true_vdim, float q_scale, float inv_tau, float eps,
+                          int32_t f32, int32_t serial, int32_t segment, int32_t segments, float* workspace, void* chunks,
+                          b200_stream_t stream);
 int b200_gla_decode(const void* qkv, int64_t stride, const void* low, const void* w_low, int32_t rank, const float* bias,
                     const float* norm, const void* gate, int64_t gate_stride, float* state, const int64_t* pos,
                     const int64_t* active, void* out, int64_t out_stride, int32_t batch, int32_t heads, int32_t dim,

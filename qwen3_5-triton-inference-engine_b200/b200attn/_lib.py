@@ -72,6 +72,8 @@ SIGNATURES: dict[str, list] = {
     "b200_mingru_decode": [P, I64, P, P, P, P, P, I32, I32, I32, I32, P],
     "b200_hgrn2_prefill": [P, I64, P, P, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, I32, c_float, I32, I32, I32, I32, P,
                            P],
+    "b200_hgrn2_prefill_walk": [P, I64, P, P, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, I32, c_float, I32, I32, I32, I32, P,
+                                P, P],
     "b200_hgrn2_decode": [P, I64, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, c_float, I32, I32, P],
     "b200_latent_prep": [P, I64, P, P, P, I32, P, P, P, I64, P, P, P, I32, I32, I32, I32, I32, I32, I32, c_float, I32, I32,
                          P],
@@ -96,6 +98,8 @@ SIGNATURES: dict[str, list] = {
     "b200_window_merge": [P, P, P, I64, P, I64, I32, I32, I32, I32, c_float, I32, I32, P],
     "b200_gla_prefill": [P, I64, P, I64, P, P, P, I64, P, P, P, P, P, P, I64, I32, I32, I32, I32, I32, I32, c_float, c_float,
                          c_float, I32, I32, I32, I32, P, P],
+    "b200_gla_prefill_walk": [P, I64, P, I64, P, P, P, I64, P, P, P, P, P, P, I64, I32, I32, I32, I32, I32, I32, c_float, c_float,
+                              c_float, I32, I32, I32, I32, P, P, P],
     "b200_gla_decode": [P, I64, P, P, I32, P, P, P, I64, P, P, P, P, I64, I32, I32, I32, I32, I32, c_float, c_float, c_float, I32,
                         I32, P],
 }
@@ -103,6 +107,7 @@ OTHER = {
     "b200_ssd_chunked": ([I32, I32], c_int32),
     "b200_mingru_workspace_bytes": ([I32, I32, I32], c_int64),
     "b200_hgrn2_workspace_bytes": ([I32, I32, I32, I32, I32], c_int64),
+    "b200_outer_walk_workspace_bytes": ([I32, I32, I32, I32, I32], c_int64),
     "b200_last_error": ([], c_char_p),
     "b200_abi_version": ([], c_int),
     "b200_wait_timed_out": ([], c_int),

@@ -122,6 +122,18 @@ def hgrn2_segments(max_len: int, groups: int, sm_count: int) -> tuple[int, int]:
     return segment, -(-max_len // segment)
 
 
+OUTER_WALK_FROM = 33
+
+
+def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool):
+    """Workspace of the form that prepares all chunks at once, or None where the shape does not take it.  Two launches pay
+    from the third chunk of 16 tokens on: 32 sequences of 16 tokens take 31 us without it and 39 with it, one of 64 tokens
+    28.7 and 26.6, 8 of 256 to 1024 tokens 336 and 162 (16 heads of 128 x 128)."""
+    takes = chunked and batch.max_len >= OUTER_WALK_FROM
+    nbytes = _lib.load().b200_outer_walk_workspace_bytes(x.shape[0], batch.count, heads, dim, vdim) if takes else 0
+    return torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+
+
 def hgrn2_prefill(qfv, lower, bias, norm, state, batch, true_vdim: int, eps: float, serial: bool = False, segments=None):
     """qfv [tokens, 2*heads*dim + heads*vdim]; state [slots, heads, dim, vdim] fp32, in place.  segments: (length, count) to
     pin how sequences are cut."""
@@ -136,9 +148,10 @@ def hgrn2_prefill(qfv, lower, bias, norm, state, batch, true_vdim: int, eps: flo
         ws = torch.empty(nbytes // 4, dtype=torch.float32, device=qfv.device)
     scratch = None if chunked and vdim <= 128 else torch.empty((tokens, heads * vdim), dtype=torch.float32, device=qfv.device)
     out = torch.empty((tokens, heads * vdim), dtype=qfv.dtype, device=qfv.device)
-    _lib.call("b200_hgrn2_prefill", _ptr(qfv), qfv.stride(0), _ptr(lower), _ptr(bias), _ptr(norm), _ptr(state), _ptr(batch.cu),
+    chunks = _outer_chunks(qfv, batch, heads, dim, vdim, chunked)
+    _lib.call("b200_hgrn2_prefill_walk", _ptr(qfv), qfv.stride(0), _ptr(lower), _ptr(bias), _ptr(norm), _ptr(state), _ptr(batch.cu),
               _ptr(batch.slots), _ptr(batch.start), _ptr(scratch), _ptr(out), batch.count, tokens, heads, dim, vdim, true_vdim,
-              float(eps), _f32(qfv), int(serial), segment, count, _ptr(ws), _stream())
+              float(eps), _f32(qfv), int(serial), segment, count, _ptr(ws), _ptr(chunks), _stream())
     return out
 
 
@@ -482,10 +495,11 @@ def gla_prefill(qkv, z, bias, norm, gate, state, out, batch, true_vdim: int, q_s
         ws = torch.empty(_lib.load().b200_hgrn2_workspace_bytes(batch.count, count, heads, dim, vdim) // 4, dtype=torch.float32,
                          device=qkv.device)
     scratch = None if chunked and vdim <= 128 else torch.empty((tokens, heads * vdim), dtype=torch.float32, device=qkv.device)
-    _lib.call("b200_gla_prefill", _ptr(qkv), qkv.stride(0), _ptr(z), z.stride(0), _ptr(bias), _ptr(norm), _ptr(gate), gate.stride(0),
+    chunks = _outer_chunks(qkv, batch, heads, dim, vdim, chunked)
+    _lib.call("b200_gla_prefill_walk", _ptr(qkv), qkv.stride(0), _ptr(z), z.stride(0), _ptr(bias), _ptr(norm), _ptr(gate), gate.stride(0),
               _ptr(state), _ptr(batch.cu), _ptr(batch.slots), _ptr(batch.start), _ptr(scratch), _ptr(out), out.stride(0), batch.count,
               tokens, heads, dim, vdim, true_vdim, float(q_scale), 1.0 / float(tau), float(eps), _f32(qkv), int(serial), segment, count,
-              _ptr(ws), _stream())
+              _ptr(ws), _ptr(chunks), _stream())
     return out
 
 

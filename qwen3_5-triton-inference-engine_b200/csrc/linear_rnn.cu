@@ -600,10 +600,12 @@ static int outer_rnn_prefill(OuterRnnParams p, RnnKind kind, bool f32, bool seri
   const bool chunked = !f32 && !serial && outer_rnn_chunk_supports(p.dim, p.vdim) && p.stride % 8 == 0 && p.q_off % 8 == 0 &&
                        p.k_off % 8 == 0 && p.v_off % 8 == 0 && p.z_stride % 4 == 0 && aligned16(p.x);
   void* const out = p.out;
-  if (chunked && p.vdim <= 128) return outer_rnn_chunk_launch(p, kind, n, st);  // the head norm inside: one launch
+  const bool walk = chunked && outer_rnn_walk_supports(p);
+  auto chunks = [&] { return walk ? outer_rnn_walk_launch(p, kind, n, tokens, st) : outer_rnn_chunk_launch(p, kind, n, st); };
+  if (chunked && p.vdim <= 128) return chunks();  // the head norm inside
   B200_REQUIRE(scratch, "outer_rnn: this shape needs a scratch tensor");
   p.out = nullptr;
-  const int rc = chunked ? outer_rnn_chunk_launch(p, kind, n, st) : outer_rnn_serial_launch(p, kind, f32, n, st);
+  const int rc = chunked ? chunks() : outer_rnn_serial_launch(p, kind, f32, n, st);
   if (rc != OK) return rc;
   p.out = out;
   const int64_t rows = static_cast<int64_t>(tokens) * p.heads;
@@ -665,11 +667,12 @@ extern "C" int64_t b200_hgrn2_workspace_bytes(int32_t batch, int32_t segments, i
   return static_cast<int64_t>(batch) * segments * heads * dim * (vdim + 1) * 4;
 }
 
-extern "C" int b200_hgrn2_prefill(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm,
+extern "C" int b200_hgrn2_prefill_walk(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm,
                                   float* state, const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start,
                                   float* o_scratch, void* out, int32_t batch, int32_t tokens, int32_t heads, int32_t dim,
                                   int32_t vdim, int32_t true_vdim, float eps, int32_t f32, int32_t serial,
-                                  int32_t segment, int32_t segments, float* workspace, b200_stream_t stream) {
+                                  int32_t segment, int32_t segments, float* workspace, void* chunks,
+                                       b200_stream_t stream) {
   if (batch <= 0 || tokens <= 0) return OK;
   B200_REQUIRE(segment > 0 && segments > 0 && (segments == 1 || (segment % 16 == 0 && workspace && aligned16(workspace))),
                "hgrn2_prefill: segments must be multiples of 16 tokens and have a workspace");
@@ -677,14 +680,23 @@ extern "C" int b200_hgrn2_prefill(const void* qfv, int64_t stride, const float* 
   B200_REQUIRE(dim > 0 && dim <= 256 && vdim > 0 && vdim % 4 == 0 && vdim <= OD_MAX_VDIM && true_vdim <= vdim,
                "hgrn2_prefill: dim at most 256, vdim a multiple of 4 and at most %d (got %d, %d)", OD_MAX_VDIM, dim, vdim);
   B200_REQUIRE(heads > 0 && heads <= 65535 && batch <= 65535, "hgrn2_prefill: at most 65535 heads and sequences");
-  B200_REQUIRE(aligned16(o_scratch) && aligned16(out) && aligned16(norm), "hgrn2_prefill: unaligned tensor");
+  B200_REQUIRE(aligned16(chunks) && aligned16(o_scratch) && aligned16(out) && aligned16(norm), "hgrn2_prefill: unaligned tensor");
   OuterRnnParams p = {};
   p.x = qfv, p.stride = stride, p.q_off = 0, p.k_off = heads * dim, p.v_off = 2 * heads * dim, p.per_group = 1;
   p.lower = lower, p.bias = bias, p.state = state, p.cu = cu_seqlens, p.slots = slots, p.start = start, p.o = o_scratch;
   p.heads = heads, p.dim = dim, p.vdim = vdim, p.norm = norm, p.out = out, p.out_stride = static_cast<int64_t>(heads) * vdim;
-  p.true_vdim = true_vdim, p.eps = eps, p.segment = segment, p.segments = segments, p.seg_state = workspace;
+  p.true_vdim = true_vdim, p.eps = eps, p.segment = segment, p.segments = segments, p.seg_state = workspace, p.chunks = chunks;
   p.seg_decay = workspace ? workspace + static_cast<int64_t>(batch) * segments * heads * dim * vdim : nullptr;
   return outer_rnn_prefill(p, RNN_FORGET, f32 != 0, serial != 0, batch, tokens, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int b200_hgrn2_prefill(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm,
+                                  float* state, const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start,
+                                  float* o_scratch, void* out, int32_t batch, int32_t tokens, int32_t heads, int32_t dim,
+                                  int32_t vdim, int32_t true_vdim, float eps, int32_t f32, int32_t serial,
+                                  int32_t segment, int32_t segments, float* workspace, b200_stream_t stream) {
+  return b200_hgrn2_prefill_walk(qfv, stride, lower, bias, norm, state, cu_seqlens, slots, start, o_scratch, out, batch, tokens, heads,
+                                 dim, vdim, true_vdim, eps, f32, serial, segment, segments, workspace, nullptr, stream);
 }
 
 extern "C" int b200_hgrn2_decode(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm,
@@ -700,19 +712,20 @@ extern "C" int b200_hgrn2_decode(const void* qfv, int64_t stride, const float* l
   return outer_rnn_decode_launch(p, RNN_FORGET, f32 != 0, batch, "hgrn2_decode", reinterpret_cast<cudaStream_t>(stream));
 }
 
-extern "C" int b200_gla_prefill(const void* qkv, int64_t stride, const float* z, int64_t z_stride, const float* bias,
+extern "C" int b200_gla_prefill_walk(const void* qkv, int64_t stride, const float* z, int64_t z_stride, const float* bias,
                                 const float* norm, const void* gate, int64_t gate_stride, float* state,
                                 const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start, float* o_scratch,
                                 void* out, int64_t out_stride, int32_t batch, int32_t tokens, int32_t heads, int32_t dim,
                                 int32_t vdim, int32_t true_vdim, float q_scale, float inv_tau, float eps, int32_t f32,
-                                int32_t serial, int32_t segment, int32_t segments, float* workspace, b200_stream_t stream) {
+                                int32_t serial, int32_t segment, int32_t segments, float* workspace, void* chunks,
+                                     b200_stream_t stream) {
   if (batch <= 0 || tokens <= 0) return OK;
   B200_REQUIRE(segment > 0 && segments > 0 && (segments == 1 || (segment % 16 == 0 && workspace && aligned16(workspace))),
                "gla_prefill: segments must be multiples of 16 tokens and have a workspace");
   B200_REQUIRE(dim > 0 && dim <= 256 && vdim > 0 && vdim % 4 == 0 && vdim <= OD_MAX_VDIM && true_vdim <= vdim,
                "gla_prefill: dim at most 256, vdim a multiple of 4 and at most %d (got %d, %d)", OD_MAX_VDIM, dim, vdim);
   B200_REQUIRE(heads > 0 && heads <= 65535 && static_cast<int64_t>(batch) * segments <= 65535, "gla_prefill: too many heads or segments");
-  B200_REQUIRE(aligned16(z) && aligned16(gate) && aligned16(o_scratch) && aligned16(out) && aligned16(norm) &&
+  B200_REQUIRE(aligned16(chunks) && aligned16(z) && aligned16(gate) && aligned16(o_scratch) && aligned16(out) && aligned16(norm) &&
                    gate_stride % 8 == 0 && out_stride % 8 == 0,
                "gla_prefill: unaligned tensor");
   OuterRnnParams p = {};
@@ -721,9 +734,20 @@ extern "C" int b200_gla_prefill(const void* qkv, int64_t stride, const float* z,
   p.state = state, p.cu = cu_seqlens, p.slots = slots, p.start = start, p.o = o_scratch;
   p.heads = heads, p.dim = dim, p.vdim = vdim, p.norm = norm, p.gate = gate, p.gate_stride = gate_stride;
   p.out = out, p.out_stride = out_stride, p.true_vdim = true_vdim, p.eps = eps;
-  p.segment = segment, p.segments = segments, p.seg_state = workspace;
+  p.segment = segment, p.segments = segments, p.seg_state = workspace, p.chunks = chunks;
   p.seg_decay = workspace ? workspace + static_cast<int64_t>(batch) * segments * heads * dim * vdim : nullptr;
   return outer_rnn_prefill(p, RNN_KEYED, f32 != 0, serial != 0, batch, tokens, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int b200_gla_prefill(const void* qkv, int64_t stride, const float* z, int64_t z_stride, const float* bias,
+                                const float* norm, const void* gate, int64_t gate_stride, float* state,
+                                const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start, float* o_scratch,
+                                void* out, int64_t out_stride, int32_t batch, int32_t tokens, int32_t heads, int32_t dim,
+                                int32_t vdim, int32_t true_vdim, float q_scale, float inv_tau, float eps, int32_t f32,
+                                int32_t serial, int32_t segment, int32_t segments, float* workspace, b200_stream_t stream) {
+  return b200_gla_prefill_walk(qkv, stride, z, z_stride, bias, norm, gate, gate_stride, state, cu_seqlens, slots, start, o_scratch, out,
+                               out_stride, batch, tokens, heads, dim, vdim, true_vdim, q_scale, inv_tau, eps, f32, serial, segment,
+                               segments, workspace, nullptr, stream);
 }
 
 extern "C" int b200_gla_decode(const void* qkv, int64_t stride, const void* low, const void* w_low, int32_t rank,

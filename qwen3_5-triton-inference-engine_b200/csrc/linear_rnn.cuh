@@ -52,6 +52,7 @@ struct OuterRnnParams {
   int segment, segments;
   float* seg_state;        // [sequences, segments, heads, dim, vdim]
   float* seg_decay;        // [sequences, segments, heads, dim]
+  void* chunks;            // fragments of all chunks (linear_rnn_walk.cu), or NULL
   // decode step
   const int64_t *pos, *active;
   int lanes_per_row, overlap;
@@ -59,6 +60,8 @@ struct OuterRnnParams {
 
 bool outer_rnn_chunk_supports(int dim, int vdim);
 int outer_rnn_chunk_launch(const OuterRnnParams& p, RnnKind kind, int n, cudaStream_t st);   // FORGET, KEYED
+bool outer_rnn_walk_supports(const OuterRnnParams& p);
+int outer_rnn_walk_launch(const OuterRnnParams& p, RnnKind kind, int n, int tokens, cudaStream_t st);   // FORGET, KEYED
 void outer_rnn_fold_launch(const OuterRnnParams& p, int n, cudaStream_t st);
 int outer_rnn_serial_launch(const OuterRnnParams& p, RnnKind kind, bool f32, int n, cudaStream_t st);
 int outer_rnn_decode_launch(OuterRnnParams p, RnnKind kind, bool f32, int batch, const char* name, cudaStream_t st);

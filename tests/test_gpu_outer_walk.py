@@ -1,0 +1,55 @@
+"""Chunk preparation and walk of HGRN2 and gated linear attention (64 < dim <= 128) at the edges of its 16-token chunks and
+four-slot ring, against the token-by-token restatement, with bars of the one-launch form's tests."""
+import pytest
+import torch
+
+from test_gpu_core_ops import gla_inputs, gla_want
+from test_gpu_hybrid_ops import DEV, Batch, _hgrn2_inputs, _hgrn2_want, close, hops, rnd  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(5, 128, 128), (2, 72, 8), (3, 96, 136)])
+@pytest.mark.parametrize("lengths", [[33], [64, 1, 65, 16], [49] + [1, 2, 17] * 44])
+def test_hgrn2_walk(hops, heads, dim, vdim, lengths):  # noqa: F811
+    """One sequence, several, and more of them than a CTA looks through at once; states carried in every second one."""
+    n, eps = len(lengths), 1e-5
+    qfv, lower, bias, norm = _hgrn2_inputs(sum(lengths), heads, dim, vdim, torch.bfloat16, 51)
+    before, starts = rnd(n, heads, dim, vdim, seed=52), [i % 2 for i in range(n)]
+    slots, state = list(range(n))[::-1], before.to(DEV)
+    batch = Batch(slots, starts, lengths)
+    out = hops.hgrn2_prefill(*[t.to(DEV) for t in (qfv, lower, bias, norm)], state, batch, vdim, eps)
+    row = 0
+    for i, (slot, start, length) in enumerate(zip(slots, starts, lengths)):
+        if i < 6:
+            want, last = _hgrn2_want(qfv[row: row + length], lower, bias, norm, heads, dim, vdim,
+                                     before[slot] if start else torch.zeros(heads, dim, vdim), eps, vdim)
+            close(out[row: row + length], want, torch.bfloat16, f"length {length}", 2.0)
+            close(state[slot], last, torch.float32, f"state after {length}", 4.0)
+        row += length
+    assert torch.isfinite(out).all() and torch.isfinite(state).all()
+
+
+@pytest.mark.parametrize("segments", [None, (32, 9), (16, 17)])
+@pytest.mark.parametrize("heads,dim,vdim,true", [(3, 128, 128, 100), (2, 80, 136, 136)])
+def test_gla_walk(hops, heads, dim, vdim, true, segments):  # noqa: F811
+    """A sequence full of NaN changes nothing in its neighbours."""
+    lengths, slots, starts, eps = [257, 15, 48, 33], [0, 3, 2, 1], [0, 4, 0, 9], 1e-5
+    qkv, z, gate = gla_inputs(heads, dim, vdim, sum(lengths), torch.bfloat16, seed=61)
+    z[:, ::9] = -90.0
+    qkv[:, 2 * heads * dim:].view(-1, heads, vdim)[..., true:] = 0
+    qkv[257:272] = float("nan")
+    bias, norm, before = rnd(heads * dim, seed=62) + 1.0, rnd(vdim, seed=63), rnd(4, heads, dim, vdim, seed=64)
+    before[..., true:] = 0
+    state, out = before.to(DEV), torch.empty(sum(lengths), heads * vdim, dtype=torch.bfloat16, device=DEV)
+    hops.gla_prefill(qkv.to(DEV), z.to(DEV), bias.to(DEV), norm.to(DEV), gate.to(DEV), state, out, Batch(slots, starts, lengths), true,
+                     dim ** -0.5, 8.0, eps, segments=segments)
+    row = 0
+    for slot, start, n in zip(slots, starts, lengths):
+        if slot != 3:
+            first = before[slot] if start else torch.zeros(heads, dim, vdim)
+            want, last = gla_want(qkv[row: row + n], z[row: row + n], gate[row: row + n], bias, norm, heads, dim, vdim, true, dim ** -0.5,
+                                  8.0, eps, first)
+            close(out[row: row + n], want, torch.bfloat16, f"length {n}", 2.0)
+            close(state[slot], last, torch.float32, f"state after {n}", 20.0)
+        row += n
