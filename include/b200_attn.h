@@ -560,6 +560,15 @@ int b200_ssd_prefill(const void* xbc, int64_t stride, const void* dt, int64_t dt
                      const float* skip, float* state, const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start,
                      void* y, int32_t batch, int32_t heads, int32_t groups, int32_t dim, int32_t vdim, int32_t f32,
                      int32_t serial, int32_t segment, int32_t segments, float* workspace, b200_stream_t stream);
+/* b200_ssd_prefill with a workspace of b200_ssd_walk_workspace_bytes() for the chunks' own matrices, computed for all chunks at
+ * once, then walked; tokens: rows of the packed batch.  As b200_hgrn2_prefill_walk: size 0 where the shape does not take it or
+ * would need more than 1 GiB, a NULL workspace is the form without. */
+int64_t b200_ssd_walk_workspace_bytes(int32_t tokens, int32_t batch, int32_t heads, int32_t dim, int32_t vdim);
+int b200_ssd_prefill_walk(const void* xbc, int64_t stride, const void* dt, int64_t dt_stride, const float* dt_bias,
+                          const float* a_log, const float* skip, float* state, const int32_t* cu_seqlens, const int32_t* slots,
+                          const int32_t* start, void* y, int32_t batch, int32_t heads, int32_t groups, int32_t dim, int32_t vdim,
+                          int32_t f32, int32_t serial, int32_t segment, int32_t segments, float* workspace, int32_t tokens,
+                          void* chunks, b200_stream_t stream);
 int b200_ssd_decode(const void* xbc, int64_t stride, const void* dt, int64_t dt_stride, const float* dt_bias, const float* a_log,
                     const float* skip, const float* conv_weight, const float* conv_bias, float* ring, int32_t taps, float* state,
                     const int64_t* pos, const int64_t* active, float* y, int32_t batch, int32_t heads, int32_t groups,

@@ -87,6 +87,7 @@ SIGNATURES: dict[str, list] = {
     "b200_latent_value": [P, P, P, P, P, I32, I32, I32, I32, I32, I32, I32, P],
     "b200_conv_prefill": [P, I64, P, P, P, P, P, P, P, I64, I32, I32, I32, I32, I32, P],
     "b200_ssd_prefill": [P, I64, P, I64, P, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, I32, I32, I32, I32, P, P],
+    "b200_ssd_prefill_walk": [P, I64, P, I64, P, P, P, P, P, P, P, P, I32, I32, I32, I32, I32, I32, I32, I32, I32, P, I32, P, P],
     "b200_ssd_decode": [P, I64, P, I64, P, P, P, P, P, P, I32, P, P, P, P, I32, I32, I32, I32, I32, I32, I32, P],
     "b200_gated_group_norm": [P, I64, P, I64, P, P, I64, I32, I32, I32, I32, I32, c_float, I32, I32, I32, P],
     "b200_gated_act": [P, I64, I32, P, I64, I32, I32, I32, I32, I32, P],
@@ -108,6 +109,7 @@ OTHER = {
     "b200_mingru_workspace_bytes": ([I32, I32, I32], c_int64),
     "b200_hgrn2_workspace_bytes": ([I32, I32, I32, I32, I32], c_int64),
     "b200_outer_walk_workspace_bytes": ([I32, I32, I32, I32, I32], c_int64),
+    "b200_ssd_walk_workspace_bytes": ([I32, I32, I32, I32, I32], c_int64),
     "b200_last_error": ([], c_char_p),
     "b200_abi_version": ([], c_int),
     "b200_wait_timed_out": ([], c_int),

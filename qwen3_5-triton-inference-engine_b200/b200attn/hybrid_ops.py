@@ -125,13 +125,16 @@ def hgrn2_segments(max_len: int, groups: int, sm_count: int) -> tuple[int, int]:
 OUTER_WALK_FROM = 33
 
 
-def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool):
-    """Workspace of the form that prepares all chunks at once, or None where the shape does not take it.  Two launches pay
-    from the third chunk of 16 tokens on: 32 sequences of 16 tokens take 31 us without it and 39 with it, one of 64 tokens
-    28.7 and 26.6, 8 of 256 to 1024 tokens 336 and 162 (16 heads of 128 x 128)."""
-    takes = chunked and batch.max_len >= OUTER_WALK_FROM
-    nbytes = _lib.load().b200_outer_walk_workspace_bytes(x.shape[0], batch.count, heads, dim, vdim) if takes else 0
+def _chunk_workspace(size: str, x, batch, heads: int, dim: int, vdim: int, takes: bool):
+    """Workspace of a form that prepares all chunks at once, or None where the call does not take it."""
+    nbytes = getattr(_lib.load(), size)(x.shape[0], batch.count, heads, dim, vdim) if takes else 0
     return torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
+
+
+def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool):
+    """Two launches pay from the third chunk of 16 tokens on: 32 sequences of 16 tokens take 31 us in one launch and 39 in two,
+    one of 64 tokens 28.7 and 26.6, 8 of 256 to 1024 tokens 336 and 162 (16 heads of 128 x 128)."""
+    return _chunk_workspace("b200_outer_walk_workspace_bytes", x, batch, heads, dim, vdim, chunked and batch.max_len >= OUTER_WALK_FROM)
 
 
 def hgrn2_prefill(qfv, lower, bias, norm, state, batch, true_vdim: int, eps: float, serial: bool = False, segments=None):
@@ -413,6 +416,9 @@ def conv_prefill(x, weight, bias, ring, batch):
     return out
 
 
+SSD_WALK_FROM = 33      # a second chunk: one of 64 tokens takes 18.4 us in one launch and 14.3 in two, 32 of 16 tokens 26.6 in one
+
+
 def ssd_segments(max_len: int, groups: int, sm_count: int) -> tuple[int, int]:
     """(segment length, segments of the longest sequence) of the chunked state-space prefill, as `hgrn2_segments`."""
     parts = min(2 * sm_count // groups, max_len // 128)
@@ -440,9 +446,10 @@ def ssd_prefill(xbc, dt, dt_bias, a_log, skip, state, groups: int, batch, serial
         ws = torch.empty(_lib.load().b200_hgrn2_workspace_bytes(batch.count, count, heads, dim, vdim) // 4, dtype=torch.float32,
                          device=xbc.device)
     y = torch.empty((tokens, heads * vdim), dtype=torch.bfloat16 if chunked else torch.float32, device=xbc.device)
-    _lib.call("b200_ssd_prefill", _ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state),
+    chunks = _chunk_workspace("b200_ssd_walk_workspace_bytes", xbc, batch, heads, dim, vdim, chunked and batch.max_len >= SSD_WALK_FROM)
+    _lib.call("b200_ssd_prefill_walk", _ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state),
               _ptr(batch.cu), _ptr(batch.slots), _ptr(batch.start), _ptr(y), batch.count, heads, groups, dim, vdim, _f32(xbc),
-              int(not chunked), segment, count, _ptr(ws), _stream())
+              int(not chunked), segment, count, _ptr(ws), tokens, _ptr(chunks), _stream())
     return y
 
 

@@ -62,6 +62,8 @@ bool outer_rnn_chunk_supports(int dim, int vdim);
 int outer_rnn_chunk_launch(const OuterRnnParams& p, RnnKind kind, int n, cudaStream_t st);   // FORGET, KEYED
 bool outer_rnn_walk_supports(const OuterRnnParams& p);
 int outer_rnn_walk_launch(const OuterRnnParams& p, RnnKind kind, int n, int tokens, cudaStream_t st);   // FORGET, KEYED
+bool ssd_walk_supports(const OuterRnnParams& p);
+int ssd_walk_launch(const OuterRnnParams& p, int n, int tokens, cudaStream_t st);
 void outer_rnn_fold_launch(const OuterRnnParams& p, int n, cudaStream_t st);
 int outer_rnn_serial_launch(const OuterRnnParams& p, RnnKind kind, bool f32, int n, cudaStream_t st);
 int outer_rnn_decode_launch(OuterRnnParams p, RnnKind kind, bool f32, int batch, const char* name, cudaStream_t st);

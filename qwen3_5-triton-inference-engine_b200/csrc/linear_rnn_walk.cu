@@ -188,6 +188,11 @@ __global__ void __launch_bounds__(32 * OW_PREP_WARPS, 4) outer_prep_kernel(const
   *reinterpret_cast<uint4*>(ws + OW_A + 512 + lane * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
 }
 
+template <bool V>
+struct Flag {
+  static constexpr bool value = V;
+};
+
 struct WalkSmem {
   uint8_t slot[OW_STAGES][OW_SLOT];
   __nv_bfloat16 v[OW_STAGES][OW_WARPS][OW_C * OW_VP];
@@ -342,42 +347,46 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
       const int flip = ((lane >> 2) & 1) * 4;
       // the update's tile (m, a), slot lane / 4 = channel 16 m + (slot / 2) * 4 + 2 a + slot % 2
       const int slot = lane >> 2, row = (slot & 1) * 4 + (lane & 3);
+      auto products = [&](auto enters) {          // whether a state enters the chunk
 #pragma unroll
-      for (int m = 0; m < OW_D / 16; ++m) {
-        float(&a)[4] = S[2 * m];
-        float(&b)[4] = S[2 * m + 1];
-        const float4 d = *reinterpret_cast<const float4*>(at + OW_B + (4 * m + (lane & 3)) * 16);
-        const uint8_t* kr = at + OW_K + ((4 * m + (slot >> 1)) ^ row) * 16 + row * 512;
-        const uint4 k0 = *reinterpret_cast<const uint4*>(kr), k1 = *reinterpret_cast<const uint4*>(kr + 8 * 512);
-        if (!LOCAL) {
-          const int unit = ((4 * m + (lane & 3)) ^ flip) * 16;
-          const uint4 r0 = *reinterpret_cast<const uint4*>(q0 + unit), r1 = *reinterpret_cast<const uint4*>(q0 + 8 * 512 + unit);
-          const uint32_t qh[4] = {r0.x, r1.x, r0.y, r1.y}, ql[4] = {r0.z, r1.z, r0.w, r1.w};
-          uint32_t h[2][2], l[2][2];
+        for (int m = 0; m < OW_D / 16; ++m) {
+          float(&a)[4] = S[2 * m];
+          float(&b)[4] = S[2 * m + 1];
+          const float4 d = *reinterpret_cast<const float4*>(at + OW_B + (4 * m + (lane & 3)) * 16);
+          const uint8_t* kr = at + OW_K + ((4 * m + (slot >> 1)) ^ row) * 16 + row * 512;
+          const uint4 k0 = *reinterpret_cast<const uint4*>(kr), k1 = *reinterpret_cast<const uint4*>(kr + 8 * 512);
+          if (enters.value) {
+            const int unit = ((4 * m + (lane & 3)) ^ flip) * 16;
+            const uint4 r0 = *reinterpret_cast<const uint4*>(q0 + unit), r1 = *reinterpret_cast<const uint4*>(q0 + 8 * 512 + unit);
+            const uint32_t qh[4] = {r0.x, r1.x, r0.y, r1.y}, ql[4] = {r0.z, r1.z, r0.w, r1.w};
+            uint32_t h[2][2], l[2][2];
 #pragma unroll
-          for (int n = 0; n < 2; ++n) {           // value columns 0-7 and 8-15 of the warp
-            split_pair(a[2 * n], a[2 * n + 1], h[n][0], l[n][0]);
-            split_pair(b[2 * n], b[2 * n + 1], h[n][1], l[n][1]);
+            for (int n = 0; n < 2; ++n) {           // value columns 0-7 and 8-15 of the warp
+              split_pair(a[2 * n], a[2 * n + 1], h[n][0], l[n][0]);
+              split_pair(b[2 * n], b[2 * n + 1], h[n][1], l[n][1]);
+            }
+            a[0] *= d.x, a[1] *= d.y, a[2] *= d.x, a[3] *= d.y;
+            b[0] *= d.z, b[1] *= d.w, b[2] *= d.z, b[3] *= d.w;
+            mma_bf16_16816(x[0], qh, l[0][0], l[0][1]);
+            mma_bf16_16816(x[1], qh, l[1][0], l[1][1]);
+            mma_bf16_16816(a, vm, k0.x, k0.y);
+            mma_bf16_16816(b, vm, k1.x, k1.y);
+            mma_bf16_16816(o[0], qh, h[0][0], h[0][1]);
+            mma_bf16_16816(o[1], qh, h[1][0], h[1][1]);
+            mma_bf16_16816(x[0], ql, h[0][0], h[0][1]);
+            mma_bf16_16816(x[1], ql, h[1][0], h[1][1]);
+          } else {
+            a[0] *= d.x, a[1] *= d.y, a[2] *= d.x, a[3] *= d.y;
+            b[0] *= d.z, b[1] *= d.w, b[2] *= d.z, b[3] *= d.w;
+            mma_bf16_16816(a, vm, k0.x, k0.y);
+            mma_bf16_16816(b, vm, k1.x, k1.y);
           }
-          a[0] *= d.x, a[1] *= d.y, a[2] *= d.x, a[3] *= d.y;
-          b[0] *= d.z, b[1] *= d.w, b[2] *= d.z, b[3] *= d.w;
-          mma_bf16_16816(x[0], qh, l[0][0], l[0][1]);
-          mma_bf16_16816(x[1], qh, l[1][0], l[1][1]);
-          mma_bf16_16816(a, vm, k0.x, k0.y);
-          mma_bf16_16816(b, vm, k1.x, k1.y);
-          mma_bf16_16816(o[0], qh, h[0][0], h[0][1]);
-          mma_bf16_16816(o[1], qh, h[1][0], h[1][1]);
-          mma_bf16_16816(x[0], ql, h[0][0], h[0][1]);
-          mma_bf16_16816(x[1], ql, h[1][0], h[1][1]);
-        } else {
-          a[0] *= d.x, a[1] *= d.y, a[2] *= d.x, a[3] *= d.y;
-          b[0] *= d.z, b[1] *= d.w, b[2] *= d.z, b[3] *= d.w;
-          mma_bf16_16816(a, vm, k0.x, k0.y);
-          mma_bf16_16816(b, vm, k1.x, k1.y);
+          mma_bf16_16816(a, vm, k0.z, k0.w);
+          mma_bf16_16816(b, vm, k1.z, k1.w);
         }
-        mma_bf16_16816(a, vm, k0.z, k0.w);
-        mma_bf16_16816(b, vm, k1.z, k1.w);
-      }
+      };
+      if (!LOCAL && (carry || i > 0)) products(Flag<true>());
+      else products(Flag<false>());
     }
     if (LOCAL && tid < OW_D) total *= *reinterpret_cast<const float*>(at + OW_B + tid * 4);
     fetch_values(i + OW_STAGES);                  // the warp has read its stage of values

@@ -522,11 +522,12 @@ extern "C" int b200_conv_prefill(const void* x, int64_t stride, const float* wei
 
 extern "C" int32_t b200_ssd_chunked(int32_t dim, int32_t vdim) { return dim % 8 == 0 && dim <= 128 && vdim % 16 == 0; }
 
-extern "C" int b200_ssd_prefill(const void* xbc, int64_t stride, const void* dt, int64_t dt_stride, const float* dt_bias,
+extern "C" int b200_ssd_prefill_walk(const void* xbc, int64_t stride, const void* dt, int64_t dt_stride, const float* dt_bias,
                                 const float* a_log, const float* skip, float* state, const int32_t* cu_seqlens,
                                 const int32_t* slots, const int32_t* start, void* y, int32_t batch, int32_t heads,
                                 int32_t groups, int32_t dim, int32_t vdim, int32_t f32, int32_t serial, int32_t segment,
-                                int32_t segments, float* workspace, b200_stream_t stream) {
+                                int32_t segments, float* workspace, int32_t tokens,
+                                     void* chunks, b200_stream_t stream) {
   if (batch <= 0) return OK;
   B200_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0 && heads <= 65535 && static_cast<int64_t>(batch) * segments <= 65535,
                "ssd_prefill: heads must be a multiple of the groups, at most 65535 heads and segments");
@@ -537,18 +538,28 @@ extern "C" int b200_ssd_prefill(const void* xbc, int64_t stride, const void* dt,
   p.x = xbc, p.stride = stride, p.v_off = 0, p.k_off = heads * vdim, p.q_off = p.k_off + groups * dim, p.per_group = heads / groups;
   p.dt = dt, p.dt_stride = dt_stride, p.bias = dt_bias, p.a_log = a_log, p.skip = skip;
   p.state = state, p.cu = cu_seqlens, p.slots = slots, p.start = start, p.heads = heads, p.dim = dim, p.vdim = vdim;
-  p.segment = segment, p.segments = segments, p.seg_state = workspace;
+  p.segment = segment, p.segments = segments, p.seg_state = workspace, p.chunks = chunks;
   p.seg_decay = workspace ? workspace + static_cast<int64_t>(batch) * segments * heads * dim * vdim : nullptr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (f32 || serial || !b200_ssd_chunked(dim, vdim)) {
     p.o = static_cast<float*>(y);
     return outer_rnn_serial_launch(p, RNN_SSD, f32 != 0, batch, st);
   }
-  B200_REQUIRE(aligned16(xbc) && aligned16(y) && stride % 8 == 0, "ssd_prefill: unaligned tensor");
+  B200_REQUIRE(aligned16(xbc) && aligned16(y) && aligned16(chunks) && stride % 8 == 0, "ssd_prefill: unaligned tensor");
   p.out = y, p.out_stride = static_cast<int64_t>(heads) * vdim;
+  if (ssd_walk_supports(p)) return ssd_walk_launch(p, batch, tokens, st);
   if (dim <= 32) return launch_ssd<32>(p, batch, st);
   if (dim <= 64) return launch_ssd<64>(p, batch, st);
   return launch_ssd<128>(p, batch, st);
+}
+
+extern "C" int b200_ssd_prefill(const void* xbc, int64_t stride, const void* dt, int64_t dt_stride, const float* dt_bias,
+                                const float* a_log, const float* skip, float* state, const int32_t* cu_seqlens,
+                                const int32_t* slots, const int32_t* start, void* y, int32_t batch, int32_t heads,
+                                int32_t groups, int32_t dim, int32_t vdim, int32_t f32, int32_t serial, int32_t segment,
+                                int32_t segments, float* workspace, b200_stream_t stream) {
+  return b200_ssd_prefill_walk(xbc, stride, dt, dt_stride, dt_bias, a_log, skip, state, cu_seqlens, slots, start, y, batch, heads, groups,
+                               dim, vdim, f32, serial, segment, segments, workspace, 0, nullptr, stream);
 }
 
 extern "C" int b200_ssd_decode(const void* xbc, int64_t stride, const void* dt, int64_t dt_stride, const float* dt_bias,

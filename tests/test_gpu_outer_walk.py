@@ -1,9 +1,9 @@
-"""Chunk preparation and walk of HGRN2 and gated linear attention (64 < dim <= 128) at the edges of its 16-token chunks and
-four-slot ring, against the token-by-token restatement, with bars of the one-launch form's tests."""
+"""Chunk preparation and walk of HGRN2, gated linear attention and the state-space recurrence (64 < dim <= 128) at the edges of
+their chunks (16 and 32 tokens) and rings of slots, against the token-by-token restatement, with bars of the one-launch forms' tests."""
 import pytest
 import torch
 
-from test_gpu_core_ops import gla_inputs, gla_want
+from test_gpu_core_ops import gla_inputs, gla_want, ssd_inputs, ssd_want
 from test_gpu_hybrid_ops import DEV, Batch, _hgrn2_inputs, _hgrn2_want, close, hops, rnd  # noqa: F401
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +53,25 @@ def test_gla_walk(hops, heads, dim, vdim, true, segments):  # noqa: F811
             close(out[row: row + n], want, torch.bfloat16, f"length {n}", 2.0)
             close(state[slot], last, torch.float32, f"state after {n}", 20.0)
         row += n
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(9, 1, 128, 64), (18, 2, 72, 48), (2, 2, 96, 112)])
+@pytest.mark.parametrize("lengths,segments", [([33], None), ([64, 31, 65, 128, 1], None), ([100] + [1, 32, 40] * 90, None), ([257, 32, 200], (64, 5))])
+def test_state_space_walk(hops, heads, groups, dim, vdim, lengths, segments):  # noqa: F811
+    """Groups of more heads than a prep CTA takes, whole and part columns, more sequences than a CTA looks through at once."""
+    n = len(lengths)
+    xbc, step, dt_bias, a_log, skip = ssd_inputs(heads, groups, dim, vdim, sum(lengths), torch.bfloat16, seed=71)
+    a_log = a_log - 3.0
+    before, starts, slots = rnd(n, heads, dim, vdim, seed=72), [i % 2 for i in range(n)], list(range(n))[::-1]
+    state = before.to(DEV)
+    y = hops.ssd_prefill(xbc.to(DEV), step.to(DEV), *(t.to(DEV) for t in (dt_bias, a_log, skip)), state, groups, Batch(slots, starts, lengths),
+                         segments=segments)
+    row = 0
+    for i, (slot, start, length) in enumerate(zip(slots, starts, lengths)):
+        if i < 5:
+            first = before[slot] if start else torch.zeros(heads, dim, vdim)
+            want, last = ssd_want(xbc[row: row + length], step[row: row + length], dt_bias, a_log, skip, heads, groups, dim, vdim, first)
+            close(y[row: row + length], want, torch.bfloat16, f"length {length}")
+            close(state[slot], last, torch.float32, f"state after {length}", 20.0)
+        row += length
+    assert torch.isfinite(y).all() and torch.isfinite(state).all()
