@@ -881,15 +881,18 @@ static int fused_decode_impl(const void* q, int64_t q_stride_b, int64_t q_stride
   p.gap = FD_GAP;
   p.cluster_size = csize;
   cudaError_t launched;
+  // Also a call without flags is launched with the attribute: the kernel then waits for its predecessor before it reads
+  // anything, but its launch does not.  Six layers of one sequence 63.8 -> 61.8 us, of 32 sequences 198 -> 194 (graph replays).
+  const bool early = (overlap & OVERLAP_START) != 0 || chain_overlap();
   if (csize > 1) {
     // every CTA of the launch must be resident together with its cluster mates; the other forms work with any grid
     int cgrid = cluster_limit(csize);
     if (cgrid > grid / csize * csize) cgrid = grid / csize * csize;
-    launched = launch_pdl_cluster((overlap & OVERLAP_START) != 0, static_cast<unsigned>(csize), fused_decode_kernel,
+    launched = launch_pdl_cluster(early, static_cast<unsigned>(csize), fused_decode_kernel,
                                   dim3(cgrid), dim3(FD_THREADS), FD_SMEM_TOTAL, reinterpret_cast<cudaStream_t>(stream), p,
                                   map_k, map_v);
   } else {
-    launched = launch_pdl((overlap & OVERLAP_START) != 0, fused_decode_kernel, dim3(grid), dim3(FD_THREADS), FD_SMEM_TOTAL,
+    launched = launch_pdl(early, fused_decode_kernel, dim3(grid), dim3(FD_THREADS), FD_SMEM_TOTAL,
                           reinterpret_cast<cudaStream_t>(stream), p, map_k, map_v);
   }
   if (launched != cudaSuccess)

@@ -845,6 +845,9 @@ extern "C" int b200_gdn_decode_fused(const void* fused, int64_t fused_stride, vo
   const int64_t heads_total = static_cast<int64_t>(batch) * num_heads;
   const int form = g_gdn_decode_form.load();
   const bool ring_ok = aligned16(state) && heads_total * GDN_D < (1LL << 31);
+  // A call without flags too: the kernel waits for its predecessor before it reads anything, its launch does not (18 layers of
+  // 32 sequences 289 -> 283 us, of 4 sequences 105 -> 93).
+  const bool early = (overlap & OVERLAP_START) != 0 || chain_overlap();
   if (ring_ok && (form == 3 || (form != 1 && heads_total > 2 * sm_count()))) {
     constexpr int SMEM = MX_STAGES * MX_BOX * 4 + 128;
     static bool configured[64] = {false};
@@ -875,12 +878,12 @@ extern "C" int b200_gdn_decode_fused(const void* fused, int64_t fused_stride, vo
     p.overlap = overlap;
     const int slots = MX_CTAS * sm_count();
     const int grid = heads_total < slots ? static_cast<int>(heads_total) : slots;
-    if (launch_pdl((overlap & OVERLAP_START) != 0, gdn_mixer_ring_kernel<MX_STAGES, MX_CTAS>, dim3(grid),
+    if (launch_pdl(early, gdn_mixer_ring_kernel<MX_STAGES, MX_CTAS>, dim3(grid),
                    dim3(MX_THREADS + 32), SMEM, reinterpret_cast<cudaStream_t>(stream), p, map) != cudaSuccess)
       return fail(ERR_LAUNCH, "gdn_decode_fused: %s", cudaGetErrorString(cudaGetLastError()));
     return check_launch("gdn_decode_fused");
   }
-  if (launch_pdl((overlap & OVERLAP_START) != 0, gdn_decode_fused_kernel, dim3(static_cast<unsigned>(batch) * num_heads), dim3(GDN_THREADS), 0,
+  if (launch_pdl(early, gdn_decode_fused_kernel, dim3(static_cast<unsigned>(batch) * num_heads), dim3(GDN_THREADS), 0,
                  reinterpret_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(fused), fused_stride,
                  static_cast<__nv_bfloat16*>(conv_state), static_cast<const __nv_bfloat16*>(weight4), a_log,
                  static_cast<const __nv_bfloat16*>(dt_bias), norm_weight, state, static_cast<__nv_bfloat16*>(out),
