@@ -442,6 +442,12 @@ int b200_conv4_decode(const void* x, int64_t x_stride_b, void* state, const void
                       int64_t out_stride_b, int32_t batch, int32_t channels, b200_stream_t stream);
 int b200_conv_state_from_packed_prefill(void* state, const void* x, int64_t x_stride_t, const int32_t* cu_seqlens,
                                         int32_t batch, int32_t channels, b200_stream_t stream);
+/* b200_conv4_prefill and b200_gdn_qk_norm_gates in one pass over rows [q | k | v | ...] of num_heads * 128 channels each: weight
+ * contiguous [3 * num_heads * 128, 4]; q_out, k_out (normed) and v_out [tokens, num_heads, 128]. */
+int b200_gdn_conv_norm_gates(const void* x, int64_t x_stride_t, const void* weight, const int32_t* seq_start, const void* a,
+                             int64_t a_stride_t, const void* b, int64_t b_stride_t, const float* a_log, const void* dt_bias,
+                             void* q_out, void* k_out, void* v_out, float* beta, float* g, int32_t tokens, int32_t num_heads,
+                             int32_t head_dim, b200_stream_t stream);
 int b200_gdn_qk_norm_gates(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k, int64_t k_stride_t,
                            int64_t k_stride_h, const void* a, int64_t a_stride_t, const void* b, int64_t b_stride_t,
                            const float* a_log, const void* dt_bias, void* q_out, void* k_out, float* beta, float* g,

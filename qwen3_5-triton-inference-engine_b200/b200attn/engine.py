@@ -193,12 +193,12 @@ class Engine(SlotEngine):
                 x, h = ops.add_rmsnorm(pending, layer["ln1"], cfg.eps, residual=x)
             if layer["kind"] == "gdn":
                 qkv, z, a, b = self._split_gdn(glue.gemm_2d(h, layer["in_proj"]))
-                conv = _conv4_prefill(qkv, layer["conv"], seq_start)
-                kd = cfg.gdn_width
-                q = conv[:, :kd].view(total, heads, dim)
-                k = conv[:, kd: 2 * kd].view(total, heads, dim)
-                v = conv[:, 2 * kd:].view(total, heads, dim)
-                q_n, k_n, beta, g = _qk_norm_gates(q, k, a, b, layer["a_log"], layer["dt_bias"])
+                ready = ops.gdn_conv_norm_gates(qkv, layer["conv"], seq_start, a, b, layer["a_log"], layer["dt_bias"])
+                if ready is None:                        # rows that are no whole vectors
+                    q, k, v = _conv4_prefill(qkv, layer["conv"], seq_start).view(total, 3, heads, dim).unbind(1)
+                    q_n, k_n, beta, g = _qk_norm_gates(q, k, a, b, layer["a_log"], layer["dt_bias"])
+                else:
+                    q_n, k_n, v, beta, g = ready
                 if slots is None:                        # every slot: the kernel writes the cache's own states
                     core, _ = ops.gdn_chunked_prefill_packed(q_n, k_n, v, beta, g, cu, state_out=self.rec_state[i])
                     _conv_state_pack(self.conv_state[i], qkv, cu)

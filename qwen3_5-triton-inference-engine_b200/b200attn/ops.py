@@ -788,6 +788,26 @@ def gdn_gated_rmsnorm_fused(x, z, weight):
     return out
 
 
+def gdn_conv_norm_gates(qkv, weight, seq_start, a, b, a_log, dt_bias):
+    """Convolution + SiLU, q/k norms and gates of a packed prompt in one pass (the operators depthwise_causal_conv4_prefill and
+    gdn_qk_norm_gates, engine/runner.py:255-292): rows [q | k | v], any of them a column range of the projection's ->
+    q_n, k_n, v bf16 [tokens, heads, 128], beta, g fp32 [tokens, heads].  None where rows or taps are not 16-byte vectors."""
+    tokens, heads = a.shape
+    assert qkv.shape == (tokens, 3 * heads * GDN_DIM) and weight.numel() == 4 * qkv.shape[1] and b.shape == a.shape
+    assert all(t.dtype == torch.bfloat16 for t in (qkv, weight, a, b, dt_bias)) and a_log.dtype == torch.float32
+    assert seq_start.dtype == torch.int32 and seq_start.shape == (tokens,) and seq_start.is_contiguous()
+    if (qkv.stride(1) != 1 or qkv.stride(0) % 8 or qkv.data_ptr() % 16 or not weight.is_contiguous() or weight.data_ptr() % 16
+            or a.stride(1) != 1 or b.stride(1) != 1):
+        return None
+    _require_cuda(qkv, weight, seq_start, a, b, a_log, dt_bias)
+    q, k, v = (torch.empty((tokens, heads, GDN_DIM), dtype=torch.bfloat16, device=qkv.device) for _ in range(3))
+    beta, g = (torch.empty((tokens, heads), dtype=torch.float32, device=qkv.device) for _ in range(2))
+    a_log, dt_bias = a_log.contiguous(), dt_bias.contiguous()
+    _lib.call("b200_gdn_conv_norm_gates", _ptr(qkv), qkv.stride(0), _ptr(weight), _ptr(seq_start), _ptr(a), a.stride(0), _ptr(b), b.stride(0),
+              _ptr(a_log), _ptr(dt_bias), _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(g), tokens, heads, GDN_DIM, _stream())
+    return q, k, v, beta, g
+
+
 def gdn_decode_fused(fused, conv_state, weight4, a_log, dt_bias, norm_weight, state, num_heads: int, overlap: int = 0):
     """The Gated-DeltaNet mixer of one decode token per sequence between its projections in ONE launch: conv + SiLU,
     q/k norms, gates, delta-rule step and gated RMSNorm (engine/runner.py:431-441).  fused [B, 4*H*128 + 2*H] is the
