@@ -137,13 +137,27 @@ def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool):
     return _chunk_workspace("b200_outer_walk_workspace_bytes", x, batch, heads, dim, vdim, chunked and batch.max_len >= OUTER_WALK_FROM)
 
 
+def outer_walk_segments(max_len: int, groups: int, sm_count: int, chunk: int = 16) -> tuple[int, int]:
+    """`hgrn2_segments` and `ssd_segments` for the walks (chunks of 16 and 32 tokens), whose tensor pipes are busy with 128 value
+    columns per SM: as many segments, of at least 128 tokens, as leave an SM to each.  16 heads, microseconds: one sequence of
+    4096 tokens in 1 segment 457, 4 195, 8 127, 16 137; 4 of 1024 tokens in 1 147, 2 129, 4 135.  State space, 32 heads of 64
+    columns: one of 4096 tokens in 4 segments 105, 8 80, 16 88; one of 1024 in 4 38, 8 35."""
+    parts = min(sm_count // max(groups, 1), max_len // 128)
+    if parts < 2:
+        return max_len, 1
+    segment = -(-max_len // (parts * chunk)) * chunk
+    return segment, -(-max_len // segment)
+
+
 def hgrn2_prefill(qfv, lower, bias, norm, state, batch, true_vdim: int, eps: float, serial: bool = False, segments=None):
     """qfv [tokens, 2*heads*dim + heads*vdim]; state [slots, heads, dim, vdim] fp32, in place.  segments: (length, count) to
     pin how sequences are cut."""
     heads, dim, vdim = _check_hgrn2(qfv, lower, bias, norm, state)
     tokens = qfv.shape[0]
     chunked = qfv.dtype == torch.bfloat16 and dim <= 128 and not serial
-    segment, count = (batch.max_len, 1) if not chunked else segments or hgrn2_segments(
+    chunks = _outer_chunks(qfv, batch, heads, dim, vdim, chunked)
+    rule = hgrn2_segments if chunks is None else outer_walk_segments
+    segment, count = (batch.max_len, 1) if not chunked else segments or rule(
         batch.max_len, batch.count * heads * -(-vdim // 128), sm_count(qfv.device))
     ws = None
     if count > 1:
@@ -151,7 +165,6 @@ def hgrn2_prefill(qfv, lower, bias, norm, state, batch, true_vdim: int, eps: flo
         ws = torch.empty(nbytes // 4, dtype=torch.float32, device=qfv.device)
     scratch = None if chunked and vdim <= 128 else torch.empty((tokens, heads * vdim), dtype=torch.float32, device=qfv.device)
     out = torch.empty((tokens, heads * vdim), dtype=qfv.dtype, device=qfv.device)
-    chunks = _outer_chunks(qfv, batch, heads, dim, vdim, chunked)
     _lib.call("b200_hgrn2_prefill_walk", _ptr(qfv), qfv.stride(0), _ptr(lower), _ptr(bias), _ptr(norm), _ptr(state), _ptr(batch.cu),
               _ptr(batch.slots), _ptr(batch.start), _ptr(scratch), _ptr(out), batch.count, tokens, heads, dim, vdim, true_vdim,
               float(eps), _f32(qfv), int(serial), segment, count, _ptr(ws), _ptr(chunks), _stream())
@@ -439,14 +452,14 @@ def ssd_prefill(xbc, dt, dt_bias, a_log, skip, state, groups: int, batch, serial
     _require_cuda(xbc, dt, dt_bias, a_log, skip, state)
     tokens = xbc.shape[0]
     chunked = xbc.dtype == torch.bfloat16 and not serial and bool(_lib.load().b200_ssd_chunked(dim, vdim))
-    segment, count = (batch.max_len, 1) if not chunked else segments or ssd_segments(
-        batch.max_len, batch.count * max(1, heads * vdim // 128), sm_count(xbc.device))
+    chunks = _chunk_workspace("b200_ssd_walk_workspace_bytes", xbc, batch, heads, dim, vdim, chunked and batch.max_len >= SSD_WALK_FROM)
+    size = (batch.max_len, batch.count * max(1, heads * vdim // 128), sm_count(xbc.device))
+    segment, count = (batch.max_len, 1) if not chunked else segments or (ssd_segments(*size) if chunks is None else outer_walk_segments(*size, 32))
     ws = None
     if count > 1:
         ws = torch.empty(_lib.load().b200_hgrn2_workspace_bytes(batch.count, count, heads, dim, vdim) // 4, dtype=torch.float32,
                          device=xbc.device)
     y = torch.empty((tokens, heads * vdim), dtype=torch.bfloat16 if chunked else torch.float32, device=xbc.device)
-    chunks = _chunk_workspace("b200_ssd_walk_workspace_bytes", xbc, batch, heads, dim, vdim, chunked and batch.max_len >= SSD_WALK_FROM)
     _lib.call("b200_ssd_prefill_walk", _ptr(xbc), xbc.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state),
               _ptr(batch.cu), _ptr(batch.slots), _ptr(batch.start), _ptr(y), batch.count, heads, groups, dim, vdim, _f32(xbc),
               int(not chunked), segment, count, _ptr(ws), tokens, _ptr(chunks), _stream())
@@ -495,14 +508,15 @@ def gla_prefill(qkv, z, bias, norm, gate, state, out, batch, true_vdim: int, q_s
     tokens = qkv.shape[0]
     assert z.dtype == torch.float32 and _rows(z) and z.shape == (tokens, heads * dim)
     chunked = qkv.dtype == torch.bfloat16 and dim <= 128 and not serial
-    segment, count = (batch.max_len, 1) if not chunked else segments or hgrn2_segments(
+    chunks = _outer_chunks(qkv, batch, heads, dim, vdim, chunked)
+    rule = hgrn2_segments if chunks is None else outer_walk_segments
+    segment, count = (batch.max_len, 1) if not chunked else segments or rule(
         batch.max_len, batch.count * heads * -(-vdim // 128), sm_count(qkv.device))
     ws = None
     if count > 1:
         ws = torch.empty(_lib.load().b200_hgrn2_workspace_bytes(batch.count, count, heads, dim, vdim) // 4, dtype=torch.float32,
                          device=qkv.device)
     scratch = None if chunked and vdim <= 128 else torch.empty((tokens, heads * vdim), dtype=torch.float32, device=qkv.device)
-    chunks = _outer_chunks(qkv, batch, heads, dim, vdim, chunked)
     _lib.call("b200_gla_prefill_walk", _ptr(qkv), qkv.stride(0), _ptr(z), z.stride(0), _ptr(bias), _ptr(norm), _ptr(gate), gate.stride(0),
               _ptr(state), _ptr(batch.cu), _ptr(batch.slots), _ptr(batch.start), _ptr(scratch), _ptr(out), out.stride(0), batch.count,
               tokens, heads, dim, vdim, true_vdim, float(q_scale), 1.0 / float(tau), float(eps), _f32(qkv), int(serial), segment, count,

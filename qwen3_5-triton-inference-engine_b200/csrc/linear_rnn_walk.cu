@@ -193,6 +193,8 @@ struct Flag {
   static constexpr bool value = V;
 };
 
+__device__ __forceinline__ bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }   // a warp gives up as a whole
+
 struct WalkSmem {
   uint8_t slot[OW_STAGES][OW_SLOT];
   __nv_bfloat16 v[OW_STAGES][OW_WARPS][OW_C * OW_VP];
@@ -205,9 +207,12 @@ struct WalkSmem {
 // shared memory, a chunk behind: head norm, gate, stores.  Slots come by one bulk copy each, OW_STAGES ahead.
 // What bounds it: the tensor pipe, 84 products per warp and chunk (16 cycles each and scheduler, two warps per scheduler).  The
 // state's update stands between the products of q and S, so that consecutive ones do not depend on one another, and nothing
-// else is left to the multiplying warps (with norm, gate and stores in their own loop a chunk took 2.2 to 3.0 us, now 1.9).
-// 8 sequences of 256 to 1024 tokens, 16 heads of 128 x 128, both launches: HGRN2 336 -> 162 us, gated linear attention 461 -> 178
-// against linear_rnn_chunk.cu, whose CTAs go through gates, decays, scores and products of every chunk in turn.  grid (vdim / 128, heads, sequences * segments)
+// else is left to the multiplying warps (with norm, gate and stores in their own loop a chunk took 2.2 to 3.0 us, now 1.7; the
+// pipe alone 1.4).  Half heads per CTA, two to a cluster that exchanges the norm's sums, gained on one long sequence and lost on
+// batches: the exchange made the output warps the bound.
+// 8 sequences of 256 to 1024 tokens, 16 heads of 128 x 128, both launches: HGRN2 336 -> 158 us, gated linear attention 461 -> 176
+// against linear_rnn_chunk.cu, whose CTAs go through gates, decays, scores and products of every chunk in turn.
+// grid (vdim / 128, heads, sequences * segments)
 template <bool LOCAL>
 __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_constant__ OuterRnnParams p, int* err) {
   extern __shared__ __align__(128) uint8_t ow_smem[];
@@ -244,19 +249,18 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
     if (!LOCAL && fused_norm && on) w = load4(p.norm + c);
     constexpr int ROWS = OW_C / OW_OUT_WARPS;
     const __nv_bfloat16* gate = p.gate ? static_cast<const __nv_bfloat16*>(p.gate) + row0 * p.gate_stride + head * p.vdim + c : nullptr;
-#pragma unroll 1
-    for (int i = 0; i < chunks; ++i) {
-      const int t0 = out_warp * ROWS, first = i * OW_C + t0;
-      uint2 raw[ROWS];                            // silu's inputs, requested while the products run
-      if (!LOCAL && gate) {
+    static_assert(ROWS == 4, "a warp's rows are dealt to its lanes by two bits");
+    const int t0 = out_warp * ROWS;
+    uint2 raw[2][ROWS] = {};                      // silu's inputs, requested a chunk ahead
+    auto request = [&](int i, uint2 (&to)[ROWS]) {
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r)
-          if (on && first + r < len) raw[r] = *reinterpret_cast<const uint2*>(gate + (first + r) * p.gate_stride);
-      }
-      if (!mbar_wait_bounded(&sm.done[i & 1], (i >> 1) & 1)) {
-        atomicExch(err, 1);
-        return;
-      }
+      for (int r = 0; r < ROWS; ++r)
+        if (on && i * OW_C + t0 + r < len) to[r] = *reinterpret_cast<const uint2*>(gate + (i * OW_C + t0 + r) * p.gate_stride);
+    };
+    auto take = [&](int i, const uint2 (&silu_in)[ROWS], uint2 (&next)[ROWS]) {
+      const int first = i * OW_C + t0;
+      if (!LOCAL && gate && i + 1 < chunks) request(i + 1, next);
+      if (!all_lanes(mbar_wait_bounded(&sm.done[i & 1], (i >> 1) & 1))) return false;
       if (copies && i + OW_STAGES < chunks) fetch_slot(i + OW_STAGES);
       float4 y[ROWS];
       if (!LOCAL) {
@@ -265,28 +269,46 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.taken[i & 1]);
-      if (!LOCAL) {
-        if (fused_norm) {
-          float sq[ROWS];
+      if (LOCAL) return true;
+      if (fused_norm) {
+        // Sums over the warp by halves: lane bits 4 and 3 are left with the row, and a lane sees to one row's scale.  (Four sums and
+        // four scales in every lane made this loop, not the products, the bound: 1.9 us a chunk.)
+        float v[ROWS];
 #pragma unroll
-          for (int r = 0; r < ROWS; ++r) sq[r] = warp_sum(y[r].x * y[r].x + y[r].y * y[r].y + y[r].z * y[r].z + y[r].w * y[r].w);
+        for (int r = 0; r < ROWS; ++r) v[r] = y[r].x * y[r].x + y[r].y * y[r].y + y[r].z * y[r].z + y[r].w * y[r].w;
+        const bool up16 = lane & 16, up8 = lane & 8;
+        float a = (up16 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up16 ? v[0] : v[2], 16);
+        const float b = (up16 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up16 ? v[1] : v[3], 16);
+        a = (up8 ? b : a) + __shfl_xor_sync(0xffffffffu, up8 ? a : b, 8);
+        a += __shfl_xor_sync(0xffffffffu, a, 4);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        const float my_scale = 1.0f / sqrtf(a / static_cast<float>(p.true_vdim) + p.eps);
 #pragma unroll
-          for (int r = 0; r < ROWS; ++r) {
-            const float scale = 1.0f / sqrtf(sq[r] / static_cast<float>(p.true_vdim) + p.eps);
-            float4 z = make_float4(y[r].x * scale * w.x, y[r].y * scale * w.y, y[r].z * scale * w.z, y[r].w * scale * w.w);
-            if (gate) {
-              z.x *= silu_f<__nv_bfloat16>(bf16_lo(raw[r].x)), z.y *= silu_f<__nv_bfloat16>(bf16_hi(raw[r].x));
-              z.z *= silu_f<__nv_bfloat16>(bf16_lo(raw[r].y)), z.w *= silu_f<__nv_bfloat16>(bf16_hi(raw[r].y));
-            }
-            if (on && first + r < len) store4(static_cast<__nv_bfloat16*>(p.out) + (row0 + first + r) * p.out_stride + head * p.vdim + c, z);
+        for (int r = 0; r < ROWS; ++r) {
+          const float scale = __shfl_sync(0xffffffffu, my_scale, r * 8);
+          float4 z = make_float4(y[r].x * scale * w.x, y[r].y * scale * w.y, y[r].z * scale * w.z, y[r].w * scale * w.w);
+          if (gate) {
+            z.x *= silu_f<__nv_bfloat16>(bf16_lo(silu_in[r].x)), z.y *= silu_f<__nv_bfloat16>(bf16_hi(silu_in[r].x));
+            z.z *= silu_f<__nv_bfloat16>(bf16_lo(silu_in[r].y)), z.w *= silu_f<__nv_bfloat16>(bf16_hi(silu_in[r].y));
           }
-        } else {
-#pragma unroll
-          for (int r = 0; r < ROWS; ++r)
-            if (on && first + r < len) store4(p.o + (static_cast<int64_t>(row0 + first + r) * p.heads + head) * p.vdim + c, y[r]);
+          if (on && first + r < len) store4(static_cast<__nv_bfloat16*>(p.out) + (row0 + first + r) * p.out_stride + head * p.vdim + c, z);
         }
+      } else {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+          if (on && first + r < len) store4(p.o + (static_cast<int64_t>(row0 + first + r) * p.heads + head) * p.vdim + c, y[r]);
       }
+      return true;
+    };
+    if (!LOCAL && gate) request(0, raw[0]);
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i < chunks && ok; i += 2) {
+      ok = take(i, raw[0], raw[1]);
+      if (ok && i + 1 < chunks) ok = take(i + 1, raw[1], raw[0]);
     }
+    if (!ok) atomicExch(err, 1);
     return;
   }
   // ---------------------------------------------------------------------------------------------------------- products
@@ -326,7 +348,7 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
     asm volatile("cp.async.wait_group %0;" ::"n"(OW_STAGES - 1) : "memory");
     __syncwarp();
     // the slot is here, and the buffer of o that chunk i - 2 used is free (so the barriers are never two phases ahead)
-    if (!mbar_wait_bounded(&sm.full[st], (i / OW_STAGES) & 1) || (i >= 2 && !mbar_wait_bounded(&sm.taken[i & 1], ((i >> 1) - 1) & 1))) {
+    if (!all_lanes(mbar_wait_bounded(&sm.full[st], (i / OW_STAGES) & 1) && (i < 2 || mbar_wait_bounded(&sm.taken[i & 1], ((i >> 1) - 1) & 1)))) {
       atomicExch(err, 1);
       return;
     }
