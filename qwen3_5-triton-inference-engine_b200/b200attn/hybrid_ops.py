@@ -133,7 +133,7 @@ def _chunk_workspace(size: str, x, batch, heads: int, dim: int, vdim: int, takes
 
 def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool):
     """Two launches pay from the third chunk of 16 tokens on: 32 sequences of 16 tokens take 31 us in one launch and 39 in two,
-    one of 64 tokens 28.7 and 26.6, 8 of 256 to 1024 tokens 336 and 162 (16 heads of 128 x 128)."""
+    one of 64 tokens 28.7 and 24.6, 8 of 256 to 1024 tokens 336 and 158 (16 heads of 128 x 128)."""
     return _chunk_workspace("b200_outer_walk_workspace_bytes", x, batch, heads, dim, vdim, chunked and batch.max_len >= OUTER_WALK_FROM)
 
 

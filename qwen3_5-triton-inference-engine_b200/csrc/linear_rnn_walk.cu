@@ -483,7 +483,7 @@ int outer_rnn_walk_launch(const OuterRnnParams& p, RnnKind kind, int n, int toke
 
 using namespace b200;
 
-// A walk pays where the chunks' fragments (35 bytes a token and value) stay a small part of the card's memory.
+// 1120 bytes per token and head: at most 1 GiB, a small part of the card's memory.
 extern "C" int64_t b200_outer_walk_workspace_bytes(int32_t tokens, int32_t batch, int32_t heads, int32_t dim, int32_t vdim) {
   if (tokens <= 0 || batch <= 0 || dim <= 64 || dim > OW_D || dim % 8 != 0 || vdim % 8 != 0) return 0;
   const int64_t bytes = slots_of(tokens, batch) * heads * OW_SLOT;

@@ -6,7 +6,7 @@
 // a warp owns 16 value columns of S^T as accumulators and weights its own x in registers; two copy warps bring the chunks, and
 // multiplying warps wait for nothing but the copies.
 // One launch (ssd.cu) went through decays, scores, weights and products in turn, 4.7 us a chunk.  32 heads of 64 columns, one
-// group, before -> now: 8 sequences of 256 to 1024 tokens 153 -> 84 us, 32 of 128 64 -> 57, one of 4096 100 -> 88 (in segments),
+// group, before -> now: 8 sequences of 256 to 1024 tokens 153 -> 84 us, 32 of 128 64 -> 57, one of 4096 100 -> 78 (in segments),
 // one of 512 45 -> 29, 32 of 48 39 -> 35; heads of 128 columns, 8 groups, ragged 139 -> 88.  Sequences of one chunk stay there.
 #include "linear_rnn.cuh"
 
