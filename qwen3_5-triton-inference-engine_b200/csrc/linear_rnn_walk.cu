@@ -221,7 +221,10 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int all = p.cu[seq + 1] - p.cu[seq], seg0 = seg * p.segment;
   const int row0 = p.cu[seq] + seg0, len = min(all - seg0, p.segment);
-  if (len <= 0 || (LOCAL && seg0 + len == all)) return;  // nothing follows a sequence's last segment
+  if (len <= 0 || (LOCAL && seg0 + len == all)) {   // nothing follows a sequence's last segment
+    pdl_wait();                                   // an idle CTA still orders the grid after the preparation
+    return;
+  }
   const int chunks = (len + OW_C - 1) / OW_C;
   if (tid == 0) {
 #pragma unroll

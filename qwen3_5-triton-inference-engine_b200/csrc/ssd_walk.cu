@@ -136,7 +136,10 @@ __global__ void __launch_bounds__(SW_THREADS, 2) ssd_walk_kernel(const __grid_co
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int all = p.cu[seq + 1] - p.cu[seq], seg0 = seg * p.segment;
   const int row0 = p.cu[seq] + seg0, len = min(all - seg0, p.segment);
-  if (len <= 0 || (LOCAL && seg0 + len == all)) return;  // nothing follows a sequence's last segment
+  if (len <= 0 || (LOCAL && seg0 + len == all)) {   // nothing follows a sequence's last segment
+    pdl_wait();                                   // an idle CTA still orders the grid after the preparation
+    return;
+  }
   const int chunks = (len + SW_Q - 1) / SW_Q, cols = min(SW_COLS, p.vdim - col0);
   const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(p.x) + static_cast<int64_t>(row0) * p.stride;
   if (tid == 0) {

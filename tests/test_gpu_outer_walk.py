@@ -75,3 +75,41 @@ def test_state_space_walk(hops, heads, groups, dim, vdim, lengths, segments):  #
             close(state[slot], last, torch.float32, f"state after {length}", 20.0)
         row += length
     assert torch.isfinite(y).all() and torch.isfinite(state).all()
+
+
+@pytest.mark.parametrize("lengths", [[300, 40], [60] * 6])
+@pytest.mark.parametrize("kind", ["hgrn2", "gla", "ssd"])
+def test_segments_to_spare(hops, kind, lengths):  # noqa: F811
+    """More segments asked for than any sequence has: no CTA of the first pass has work, and what follows it still comes after the
+    preparation.  Twice over the same memory, so that slots which were not written again would hold other values' fragments."""
+    heads, dim, vdim, eps, n, total = 3, 128, 64, 1e-5, len(lengths), sum(lengths)
+    batch, zero = Batch(list(range(n)), [0] * n, lengths), torch.zeros(heads, dim, vdim)
+    for seed in (81, 91):
+        state = torch.zeros(n, heads, dim, vdim, device=DEV)
+        if kind == "hgrn2":
+            qfv, lower, bias, norm = _hgrn2_inputs(total, heads, dim, vdim, torch.bfloat16, seed)
+            out = hops.hgrn2_prefill(*[t.to(DEV) for t in (qfv, lower, bias, norm)], state, batch, vdim, eps, segments=(512, 2))
+
+            def want(a, b):
+                return _hgrn2_want(qfv[a:b], lower, bias, norm, heads, dim, vdim, zero, eps, vdim)
+        elif kind == "gla":
+            qkv, z, gate = gla_inputs(heads, dim, vdim, total, torch.bfloat16, seed=seed)
+            bias, norm = rnd(heads * dim, seed=seed + 3) + 1.0, rnd(vdim, seed=seed + 4)
+            out = torch.empty(total, heads * vdim, dtype=torch.bfloat16, device=DEV)
+            hops.gla_prefill(*[t.to(DEV) for t in (qkv, z, bias, norm, gate)], state, out, batch, vdim, dim ** -0.5, 8.0, eps, segments=(512, 2))
+
+            def want(a, b):
+                return gla_want(qkv[a:b], z[a:b], gate[a:b], bias, norm, heads, dim, vdim, vdim, dim ** -0.5, 8.0, eps, zero)
+        else:
+            xbc, step, dt_bias, a_log, skip = ssd_inputs(heads, 1, dim, vdim, total, torch.bfloat16, seed=seed)
+            a_log = a_log - 3.0
+            out = hops.ssd_prefill(*[t.to(DEV) for t in (xbc, step, dt_bias, a_log, skip)], state, 1, batch, segments=(512, 2))
+
+            def want(a, b):
+                return ssd_want(xbc[a:b], step[a:b], dt_bias, a_log, skip, heads, 1, dim, vdim, zero)
+        row = 0
+        for i, length in enumerate(lengths):
+            y, last = want(row, row + length)
+            close(out[row: row + length], y, torch.bfloat16, f"length {length}", 2.0)
+            close(state[i], last, torch.float32, f"state after {length}", 20.0)
+            row += length
