@@ -126,6 +126,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
   return false;
 }
+// The same for all 32 lanes of a warp, which go on or give up as one (matrix instructions and shuffles need every lane); a lane
+// that has given up before says so with `ok`.
+__device__ __forceinline__ bool warp_wait_bounded(uint64_t* bar, uint32_t parity, bool ok = true) {
+  return __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar, parity)) != 0;
+}
 // 1-D bulk async copy global -> shared, completion counted in bytes on an mbarrier.  dst, src and
 // bytes must all be multiples of 16.  No cluster multicast is used anywhere in this library.
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
@@ -146,6 +151,19 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 // Barrier among `count` threads (a multiple of 32) that all name the same id (1..15; 0 is __syncthreads).
 __device__ __forceinline__ void named_barrier(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+// The same barrier; true where `ok` held in every one of them.
+__device__ __forceinline__ bool named_barrier_all(int id, int count, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "bar.red.and.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(id), "r"(count), "r"(ok ? 1u : 0u)
+      : "memory");
+  return all != 0;
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

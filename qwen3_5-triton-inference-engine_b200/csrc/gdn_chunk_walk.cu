@@ -213,9 +213,8 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
   constexpr int SPLIT = GDN_D / COLS, THREADS = 32 * GW_COPY_WARPS;
   uint64_t *full = reinterpret_cast<uint64_t*>(smem + L::BARS), *empty = full + GW_STAGES;
   int* handover = reinterpret_cast<int*>(smem + L::HANDOVER);
-  int stage = 0;
-  uint32_t parity = 1;
-  bool waited = false;
+  int fills = 0;                                        // chunks asked for so far, also those that hold nothing
+  bool waited = false, ok = true;
   for (int item = blockIdx.x;;) {
     int h = 0, col = 0, start = 0, len = 0, slot0 = 0;
     const bool more = item < p.items;
@@ -225,10 +224,9 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
       start = p.cu[b], len = p.cu[b + 1] - start, slot0 = first_slot(p.cu, b);
     }
     for (int t0 = 0; t0 == 0 || t0 < len; t0 += CHUNK) {       // an empty sequence passes once: its state is zero
-      if (!mbar_wait_bounded(&empty[stage], parity)) {
-        atomicExch(p.err, 1);
-        return;
-      }
+      const int stage = fills % GW_STAGES;
+      ok = warp_wait_bounded(&empty[stage], (fills / GW_STAGES & 1) ^ 1);
+      if (!ok) break;                                   // ... and the other warps hear of it where they meet, below
       uint8_t* to = smem + stage * L::STAGE;
       const int rows = min(CHUNK, len - t0);
       if (rows > 0) {
@@ -250,15 +248,22 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
         }
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[stage])) : "memory");
-      if (++stage == GW_STAGES) stage = 0, parity ^= 1;
+      ++fills;
     }
     if (!more) break;
-    if (ct == 0) *handover = gridDim.x + atomicAdd(p.next, 1);
-    named_barrier(1, THREADS);
+    if (ct == 0 && ok) *handover = gridDim.x + atomicAdd(p.next, 1);
+    ok = named_barrier_all(1, THREADS, ok);             // they go on or give up as one
+    if (!ok) break;
     item = *handover;
     named_barrier(1, THREADS);
   }
   cp_async_wait_all();
+  if (!ok) {
+    atomicExch(p.err, 1);
+    // bulk copies that nobody waits for any more may still be landing in this CTA's shared memory
+    if (ct == 0)
+      for (int i = max(fills - GW_STAGES, 0); i < fills; ++i) mbar_wait_bounded(&full[i % GW_STAGES], i / GW_STAGES & 1, 1u << 12);
+  }
 }
 template <int COLS>
 __device__ __forceinline__ void init_stages(uint8_t* smem, int consumers) {
@@ -437,7 +442,7 @@ __global__ void __launch_bounds__(32 * (WARPS + GW_COPY_WARPS), 1) gdn_walk_kern
   int stage = 0;
   uint32_t parity = 0;
   for (;;) {
-    if (!mbar_wait_bounded(&full[stage], parity)) {
+    if (!warp_wait_bounded(&full[stage], parity)) {
       if (lane == 0) atomicExch(p.err, 1);
       return;
     }
@@ -510,7 +515,8 @@ __device__ __forceinline__ void pair_products(float (&s)[2][3][4], const uint32_
   mma_bf16_16816(s[1][2], hi, b.z, b.w);
 }
 
-// Wait among the warps of a team, which are a few hundred cycles apart at most: polls that do not put the warp to sleep
+// Wait among the warps of a team, which are a few hundred cycles apart at most: polls that do not put the warp to sleep.  Lanes
+// that give up stay with their warp, which leaves as one before the next chunk.
 __device__ __forceinline__ bool team_wait(uint64_t* bar, uint32_t parity) {
   for (int i = 0; i < (1 << 22); ++i) {
     uint32_t ok;
@@ -560,7 +566,7 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
   int stage = 0, bh = 0, h = 0, col = 0;
   bool ok = true;
   for (;;) {
-    if (!mbar_wait_bounded(&full[stage], full_parity)) ok = false;
+    ok = warp_wait_bounded(&full[stage], full_parity, ok);
     if (!ok) break;
     const int4 info = *reinterpret_cast<const int4*>(smem + L::INFO + stage * 16);
     if (info.x < 0) return;

@@ -193,8 +193,6 @@ struct Flag {
   static constexpr bool value = V;
 };
 
-__device__ __forceinline__ bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }   // a warp gives up as a whole
-
 struct WalkSmem {
   uint8_t slot[OW_STAGES][OW_SLOT];
   __nv_bfloat16 v[OW_STAGES][OW_WARPS][OW_C * OW_VP];
@@ -263,7 +261,7 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
     auto take = [&](int i, const uint2 (&silu_in)[ROWS], uint2 (&next)[ROWS]) {
       const int first = i * OW_C + t0;
       if (!LOCAL && gate && i + 1 < chunks) request(i + 1, next);
-      if (!all_lanes(mbar_wait_bounded(&sm.done[i & 1], (i >> 1) & 1))) return false;
+      if (!warp_wait_bounded(&sm.done[i & 1], (i >> 1) & 1)) return false;
       if (copies && i + OW_STAGES < chunks) fetch_slot(i + OW_STAGES);
       float4 y[ROWS];
       if (!LOCAL) {
@@ -306,12 +304,18 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
     };
     if (!LOCAL && gate) request(0, raw[0]);
     bool ok = true;
+    int at = 0;                                   // the chunk waited for last
 #pragma unroll 1
     for (int i = 0; i < chunks && ok; i += 2) {
-      ok = take(i, raw[0], raw[1]);
-      if (ok && i + 1 < chunks) ok = take(i + 1, raw[1], raw[0]);
+      ok = take(at = i, raw[0], raw[1]);
+      if (ok && i + 1 < chunks) ok = take(at = i + 1, raw[1], raw[0]);
     }
-    if (!ok) atomicExch(err, 1);
+    if (!ok) {
+      atomicExch(err, 1);
+      // bulk copies that nobody waits for any more may still be landing in this CTA's shared memory
+      if (copies)
+        for (int i = at; i < at + OW_STAGES && i < chunks; ++i) mbar_wait_bounded(&sm.full[i % OW_STAGES], i / OW_STAGES & 1, 1u << 12);
+    }
     return;
   }
   // ---------------------------------------------------------------------------------------------------------- products
@@ -351,8 +355,10 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
     asm volatile("cp.async.wait_group %0;" ::"n"(OW_STAGES - 1) : "memory");
     __syncwarp();
     // the slot is here, and the buffer of o that chunk i - 2 used is free (so the barriers are never two phases ahead)
-    if (!all_lanes(mbar_wait_bounded(&sm.full[st], (i / OW_STAGES) & 1) && (i < 2 || mbar_wait_bounded(&sm.taken[i & 1], ((i >> 1) - 1) & 1)))) {
+    const bool taken = i < 2 || mbar_wait_bounded(&sm.taken[i & 1], ((i >> 1) - 1) & 1);
+    if (!warp_wait_bounded(&sm.full[st], (i / OW_STAGES) & 1, taken)) {
       atomicExch(err, 1);
+      asm volatile("cp.async.wait_all;" ::: "memory");
       return;
     }
     const uint8_t* at = sm.slot[st];

@@ -152,12 +152,10 @@ __global__ void __launch_bounds__(SW_THREADS, 2) ssd_walk_kernel(const __grid_co
     // ------------------------------------------------------------------------------------------------------- copies
     const uint8_t* slots = static_cast<const uint8_t*>(p.chunks) + ((first_slot(p.cu, seq) + seg0 / SW_Q) * p.heads + head) * SW_SLOT;
     const int ct = tid - 32 * SW_WARPS, bc_col = (head / p.per_group) * p.dim, x_col = p.v_off + head * p.vdim + col0;
-    for (int i = 0; i < chunks; ++i) {
+    int i = 0;
+    for (; i < chunks; ++i) {
       const int st = i % SW_STAGES, t0 = i * SW_Q;
-      if (i >= SW_STAGES && !mbar_wait_bounded(&sm.empty[st], (i / SW_STAGES - 1) & 1)) {
-        atomicExch(err, 1);
-        break;
-      }
+      if (i >= SW_STAGES && !warp_wait_bounded(&sm.empty[st], (i / SW_STAGES - 1) & 1)) break;
 #pragma unroll 8
       for (int k = ct; k < SW_Q * (SW_N / 8); k += SW_COPY) {
         const int t = k / (SW_N / 8), d = (k % (SW_N / 8)) * 8;
@@ -181,6 +179,12 @@ __global__ void __launch_bounds__(SW_THREADS, 2) ssd_walk_kernel(const __grid_co
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&sm.full[st])) : "memory");
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    if (i < chunks) {                             // the other warp runs out as well: no chunk is complete without this one's part
+      atomicExch(err, 1);
+      // bulk copies that nobody waits for any more may still be landing in this CTA's shared memory
+      if (ct == 0)
+        for (int k = max(i - SW_STAGES, 0); k < i; ++k) mbar_wait_bounded(&sm.full[k % SW_STAGES], k / SW_STAGES & 1, 1u << 12);
+    }
     return;
   }
   // ---------------------------------------------------------------------------------------------------------- products
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(SW_THREADS, 2) ssd_walk_kernel(const __grid_co
 #pragma unroll 1
   for (int i = 0; i < chunks; ++i) {
     const int st = i % SW_STAGES;
-    if (!mbar_wait_bounded(&sm.full[st], (i / SW_STAGES) & 1)) {
+    if (!warp_wait_bounded(&sm.full[st], (i / SW_STAGES) & 1)) {
       atomicExch(err, 1);
       return;
     }

@@ -26,3 +26,28 @@ def test_every_cta_orders_the_grid(name):
     text = body(name, EARLY[name])
     assert "pdl_wait()" in text
     assert "return" not in text[: text.index("pdl_wait()")]
+
+
+@pytest.mark.parametrize("name", ["gdn_chunk_walk", "linear_rnn_walk", "ssd_walk"])
+def test_warps_give_up_whole(name):
+    """A wait that runs out must not leave some lanes of a warp to matrix instructions, or some threads to a barrier, that the others
+    have left: what a wait says decides nothing before the warp has voted.  Single threads wait for copies that nobody waits for any
+    more, and go nowhere afterwards."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / f"{name}.cu").read_text())
+    assert not re.findall(r"if \([^\n]*(?:mbar_wait_bounded|team_wait)\(", text)
+    assert "warp_wait_bounded(" in text
+
+
+def test_copy_warps_give_up_together():
+    """The copy warps of a Gated-DeltaNet walk meet between items: none leaves before it has said so there."""
+    text = body("gdn_chunk_walk", "copy_chunks")
+    assert "return" not in text
+    assert text.index("named_barrier_all(") < text.index("item = *handover")
+
+
+def test_team_lanes_stay():
+    """Lanes whose wait among the warps of a team ran out stay until the vote that opens a chunk, and store nothing."""
+    text = body("gdn_chunk_walk", "gdn_walk_team_kernel")
+    assert text.index("warp_wait_bounded(&full[stage], full_parity, ok)") < text.index("team_wait(")
+    assert len(re.findall(r"ok = ok && team_wait\(", text)) == text.count("team_wait(")
+    assert text.count("return;") == 2                   # the copy warps, and the end of the items
