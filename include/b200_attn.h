@@ -48,9 +48,11 @@ int b200_wait_timed_out(void);
  * microseconds long and are called one after the other; they are launched for programmatic dependent launch: every such
  * kernel lets its successor in the stream be scheduled at once and itself touches global memory only after its
  * predecessor has completed, so the launch latencies overlap instead of adding up (a kernel of another library in
- * between is unaffected: it starts when its predecessor has finished, as always).  b200_set_chain_overlap(0) launches
- * them plainly again, process-wide (for comparisons, or under tools that do not model such launches).  No counterpart
- * in the reference. */
+ * between is unaffected: it starts when its predecessor has finished, as always).  fused_decode_attention and
+ * gdn_decode_fused called without overlap flags are launched for it as well; they wait in the same way and do not let
+ * their successor start.  b200_set_chain_overlap(0) launches all of these plainly again, process-wide (for comparisons,
+ * or under tools that do not model such launches); calls with B200_OVERLAP_START are not its concern.  No counterpart in
+ * the reference. */
 int b200_set_chain_overlap(int32_t enabled);
 
 /* Diagnostic: one CTA multiplies two bf16 tiles loaded by tensor-map TMA with tcgen05.mma (accumulator in tensor
@@ -337,13 +339,13 @@ int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, int64_t q_s
  * x and out contiguous [rows, 128], z row (n, head) at z + n * z_stride + head * 128
  * (triton_kernels/gdn_gated_rmsnorm.py:95-140). */
 /* Overlap flags (programmatic dependent launch) of b200_(norm_)skinny_gemm, b200_add_rmsnorm, b200_swiglu and
- * b200_gdn_decode_fused; 0 = plain stream order.
+ * b200_gdn_decode_fused; 0 = nothing is read or written before the kernel in front has completed.
  *   START    the kernel may begin while the kernel in front of it in the stream still runs; it reads that kernel's
  *            output, and writes anything, only after that kernel has completed.
  *   TRIGGER  the kernel lets the NEXT kernel in the stream begin early in the same way.  Pass it only when that next
  *            kernel is one of these four launched with START: a kernel that does not itself wait for its predecessor
  *            before finishing (some library initialisation kernels) would break the ordering of everything after it.
- *   PREFETCH b200_gdn_decode_fused only, see there. */
+ *   PREFETCH b200_gdn_decode_fused (and b200_fused_decode_attention_ex), see there; it takes effect together with START. */
 #define B200_OVERLAP_START 1
 #define B200_OVERLAP_TRIGGER 2
 #define B200_OVERLAP_PREFETCH 4

@@ -882,8 +882,9 @@ static int fused_decode_impl(const void* q, int64_t q_stride_b, int64_t q_stride
   p.cluster_size = csize;
   cudaError_t launched;
   // Also a call without flags is launched with the attribute: the kernel then waits for its predecessor before it reads
-  // anything, but its launch does not.  Six layers of one sequence 63.8 -> 61.8 us, of 32 sequences 198 -> 194 (graph replays).
-  const bool early = (overlap & OVERLAP_START) != 0 || chain_overlap();
+  // anything, but its launch does not.  Six layers of 32 sequences 198.7 -> 195.1 us, of one 64.6 -> 64.2 (graph replays).
+  // PREFETCH alone reads before it waits: launched plainly.
+  const bool early = (overlap & OVERLAP_START) != 0 || (chain_overlap() && !(overlap & OVERLAP_PREFETCH));
   if (csize > 1) {
     // every CTA of the launch must be resident together with its cluster mates; the other forms work with any grid
     int cgrid = cluster_limit(csize);

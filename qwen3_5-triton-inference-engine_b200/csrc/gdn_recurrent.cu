@@ -136,11 +136,10 @@ gdn_decode_slice_kernel(const __nv_bfloat16* q, int64_t q_b, int64_t q_h, const 
 // k, v and z slices and value column t of the state; every intermediate keeps the reference's rounding point (conv
 // output, q_n, k_n and the recurrence output are bf16 tensors there).
 __global__ void __launch_bounds__(GDN_THREADS)
-gdn_decode_fused_kernel(const __nv_bfloat16* fused, int64_t fused_stride,  // no __restrict__: see pdl_wait()
-                        __nv_bfloat16* __restrict__ conv_state, const __nv_bfloat16* __restrict__ w4,
-                        const float* __restrict__ a_log, const __nv_bfloat16* __restrict__ dt_bias,
-                        const float* __restrict__ norm_w, float* __restrict__ state, __nv_bfloat16* __restrict__ out,
-                        int heads, int overlap) {
+gdn_decode_fused_kernel(const __nv_bfloat16* fused, int64_t fused_stride,  // no __restrict__: see pdl_wait(); any of
+                        __nv_bfloat16* conv_state, const __nv_bfloat16* w4, const float* a_log,  // these may be the output
+                        const __nv_bfloat16* dt_bias, const float* norm_w, float* state,         // of the kernel in front
+                        __nv_bfloat16* out, int heads, int overlap) {
   __shared__ __align__(16) float kf[GDN_D];
   __shared__ __align__(16) float qf[GDN_D];
   __shared__ float red[3][4];
@@ -846,8 +845,8 @@ extern "C" int b200_gdn_decode_fused(const void* fused, int64_t fused_stride, vo
   const int form = g_gdn_decode_form.load();
   const bool ring_ok = aligned16(state) && heads_total * GDN_D < (1LL << 31);
   // A call without flags too: the kernel waits for its predecessor before it reads anything, its launch does not (18 layers of
-  // 32 sequences 289 -> 283 us, of 4 sequences 105 -> 93).
-  const bool early = (overlap & OVERLAP_START) != 0 || chain_overlap();
+  // 32 sequences 288.2 -> 286.3 us, of 4 sequences 105 -> 93).  PREFETCH alone reads before it waits: launched plainly.
+  const bool early = (overlap & OVERLAP_START) != 0 || (chain_overlap() && !(overlap & OVERLAP_PREFETCH));
   if (ring_ok && (form == 3 || (form != 1 && heads_total > 2 * sm_count()))) {
     constexpr int SMEM = MX_STAGES * MX_BOX * 4 + 128;
     static bool configured[64] = {false};

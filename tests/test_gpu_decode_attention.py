@@ -360,11 +360,68 @@ def test_overlapped_decode_attention_in_graph_equals_plain(ops):
         torch.cuda.synchronize()
         return outs, kc, vc, pos
 
-    plain, fast = run(False), run(True)
+    ops.set_chain_overlap(False)             # without it a call without flags is launched early as well
+    try:
+        plain = run(False)
+    finally:
+        ops.set_chain_overlap(True)
+    fast = run(True)
     no_timeouts()
     for x, y in zip(plain[0], fast[0]):
         assert torch.equal(x, y)
     assert torch.equal(plain[1], fast[1]) and torch.equal(plain[2], fast[2]) and torch.equal(plain[3], fast[3])
+
+
+@pytest.mark.parametrize("lengths", [[700], [30, 3, 200, 1025], [50 + 37 * i for i in range(40)]])
+def test_decode_attention_without_flags_in_a_row(ops, lengths):
+    """Calls without overlap flags, early launches by default, against plain ones: back to back on one cache, behind kernels that
+    write the positions and the projections, and (inside a capture) behind a kernel of another stream."""
+    c = make_paged_case(lengths, seed=79, slack_tokens=12)
+    d, inv, b = to_dev(c), rope_inv_freq().to(DEV), len(lengths)
+    gen = torch.Generator().manual_seed(3)
+    rows = torch.stack([torch.stack([bf16_randn(b, 20 * 256, gen=gen) for _ in range(3)]) for _ in range(3)]).to(DEV)
+
+    def run(early: bool):
+        x, here = rows[0].clone(), torch.zeros_like(rows[0][0])
+        kc, vc, pos, ws = d["k_cache"].clone(), d["v_cache"].clone(), d["pos"].clone(), ops.fused_decode_workspace(DEV)
+
+        def call(r):
+            return ops.fused_decode_attention(r[:, :2048].view(b, 8, 256), r[:, 4096:4608].view(b, 2, 256), r[:, 4608:].view(b, 2, 256),
+                                              r[:, 2048:4096], kc, vc, d["block_table"], pos, inv, 64, ws)
+
+        def step():
+            got = [call(x[0]), call(x[1])]
+            pos.add_(1)
+            got.append(call(x[0]))
+            main, other = torch.cuda.current_stream(), torch.cuda.Stream()
+            other.wait_stream(main)
+            with torch.cuda.stream(other):
+                here.copy_(x[2])
+            pos.add_(1)
+            main.wait_stream(other)
+            return got + [call(here)]
+
+        ops.set_chain_overlap(early)
+        try:
+            outs = [o.clone() for o in step()]           # eagerly
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = step()
+        finally:
+            ops.set_chain_overlap(True)
+        for nxt in rows[1:]:
+            x.copy_(nxt)
+            graph.replay()
+            outs += [o.clone() for o in got]
+        torch.cuda.synchronize()
+        return outs, kc, vc, pos
+
+    plain, early = run(False), run(True)
+    no_timeouts()
+    for p, q in zip(plain[0], early[0]):
+        assert torch.equal(p, q)
+    assert torch.equal(plain[1], early[1]) and torch.equal(plain[2], early[2]) and torch.equal(plain[3], early[3])
 
 
 @pytest.mark.parametrize("one_launch", [False, True])

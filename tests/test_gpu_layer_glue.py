@@ -328,10 +328,72 @@ def test_overlapped_chain_in_graph_equals_plain(mods):
         torch.cuda.synchronize()
         return outs, state, conv
 
-    plain, fast = run(False), run(True)
+    ops.set_chain_overlap(False)                 # without it a call without flags is launched early as well
+    try:
+        plain = run(False)
+    finally:
+        ops.set_chain_overlap(True)
+    fast = run(True)
     for a, b in zip(plain[0], fast[0]):
         assert torch.equal(a, b)
     assert torch.equal(plain[1], fast[1]) and torch.equal(plain[2], fast[2])
+
+
+@pytest.mark.parametrize("batch", [4, 40])       # a head's state in registers; a ring of boxes
+def test_mixers_without_flags_in_a_row(mods, batch):
+    """Calls without overlap flags, early launches by default, against plain ones: back to back on one state, behind kernels that
+    write the gates' weights and the convolution's state, and (inside a capture) behind a kernel of another stream."""
+    ops, _ = mods
+    gen = torch.Generator().manual_seed(23)
+    heads, kd, calls = 16, 2048, 4
+    w4 = (torch.randn(4, 3 * kd, generator=gen) * 0.5).to(torch.bfloat16).to(DEV)
+    a_log = (torch.rand(heads, generator=gen) * 2.7).to(DEV)
+    dts = (torch.randn(calls, heads, generator=gen) * 0.5).to(torch.bfloat16).to(DEV)
+    norm_w = (1 + 0.1 * torch.randn(128, generator=gen)).to(DEV)
+    conv0 = torch.randn(batch, 4, 3 * kd, generator=gen).to(torch.bfloat16).to(DEV)
+    state0 = (torch.randn(batch, heads, 128, 128, generator=gen) * 0.1).to(DEV)
+    rows = torch.randn(3, calls, batch, 4 * kd + 2 * heads, generator=gen).to(torch.bfloat16).to(DEV)
+
+    def run(early: bool):
+        conv, state, x, here = conv0.clone(), state0.clone(), rows[0].clone(), torch.zeros_like(rows[0][0])
+        dt_bias, outs = dts[0].clone(), []
+
+        def step():
+            got = [ops.gdn_decode_fused(x[0], conv, w4, a_log, dt_bias, norm_w, state, heads),
+                   ops.gdn_decode_fused(x[1], conv, w4, a_log, dt_bias, norm_w, state, heads)]
+            dt_bias.copy_(dts[1])
+            conv.mul_(0.5)
+            got.append(ops.gdn_decode_fused(x[2], conv, w4, a_log, dt_bias, norm_w, state, heads))
+            main, other = torch.cuda.current_stream(), torch.cuda.Stream()
+            other.wait_stream(main)
+            with torch.cuda.stream(other):
+                here.copy_(x[3])
+            state.mul_(0.9)
+            main.wait_stream(other)
+            got.append(ops.gdn_decode_fused(here, conv, w4, a_log, dt_bias, norm_w, state, heads))
+            dt_bias.copy_(dts[0])
+            return got
+
+        ops.set_chain_overlap(early)
+        try:
+            outs += [o.clone() for o in step()]          # eagerly
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = step()
+        finally:
+            ops.set_chain_overlap(True)
+        for nxt in rows[1:]:
+            x.copy_(nxt)
+            graph.replay()
+            outs += [o.clone() for o in got]
+        torch.cuda.synchronize()
+        return outs, state, conv
+
+    plain, early = run(False), run(True)
+    for a, b in zip(plain[0], early[0]):
+        assert torch.equal(a, b)
+    assert torch.equal(plain[1], early[1]) and torch.equal(plain[2], early[2])
 
 
 @pytest.mark.parametrize("m,k,inter", [(32, 1024, 3584), (4, 256, 512), (17, 1280, 1000), (1, 128, 8), (32, 1024, 40)])

@@ -1,4 +1,4 @@
-"""Rules of the chunk walks that no run can show without a race or a lost copy, read from their sources."""
+"""Rules of early launches and bounded waits that no run can show without a race or a lost copy, read from the sources."""
 import re
 from pathlib import Path
 
@@ -26,6 +26,14 @@ def test_every_cta_orders_the_grid(name):
     text = body(name, EARLY[name])
     assert "pdl_wait()" in text
     assert "return" not in text[: text.index("pdl_wait()")]
+
+
+def test_early_mixer_reads_plain_pointers():
+    """Loads through `const __restrict__` may be moved above the wait for the kernel in front; its calls without flags are launched
+    early too, so that anything it reads may be that kernel's output."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "gdn_recurrent.cu").read_text())
+    at = text.index("gdn_decode_fused_kernel(const")
+    assert "__restrict__" not in text[at: text.index("{", at)]
 
 
 @pytest.mark.parametrize("name", ["gdn_chunk_walk", "linear_rnn_walk", "ssd_walk"])
