@@ -40,7 +40,8 @@ typedef void* b200_stream_t; /* cudaStream_t */
 const char* b200_last_error(void); /* host string describing the last non-zero return */
 int b200_abi_version(void);
 /* host-synchronous: 1 if a kernel on the current device gave up a bounded wait on a staged copy since the
- * last call (the flag is cleared), 0 if not, -1 on a runtime error.  For tests and debugging. */
+ * last call (the flag is cleared), or found a packed prefill batch to hold more tokens than its call named; 0 if not, -1
+ * on a runtime error.  For tests and debugging. */
 int b200_wait_timed_out(void);
 
 /* The small operators of a decode step (partial_rope, attention_gate_pack, paged_kv_append, the split / combine pair,

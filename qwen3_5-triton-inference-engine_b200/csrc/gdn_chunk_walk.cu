@@ -37,7 +37,7 @@ struct GdnWalkParams {
   float* state;           // [batch, heads, 128, 128]
   __nv_bfloat16* out;
   int64_t o_t, o_h;
-  int heads, batch, items;
+  int heads, batch, items, slots;
   int *next, *err;        // counter of the walk's items, behind the slots; the flag of waits that ran out
 };
 template <int N>
@@ -218,12 +218,15 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
   for (int item = blockIdx.x;;) {
     int h = 0, col = 0, start = 0, len = 0, slot0 = 0;
     const bool more = item < p.items;
+    bool fits = true;
     if (more) {
       const int bh = item / SPLIT, b = bh / p.heads;
       h = bh % p.heads, col = item % SPLIT * COLS;
       start = p.cu[b], len = p.cu[b + 1] - start, slot0 = first_slot(p.cu, b);
+      fits = slot0 + (len + CHUNK - 1) / CHUNK <= p.slots;      // else more tokens than the call named: nobody prepared the end
+      if (!fits && ct == 0) atomicExch(p.err, 1);
     }
-    for (int t0 = 0; t0 == 0 || t0 < len; t0 += CHUNK) {       // an empty sequence passes once: its state is zero
+    for (int t0 = 0; fits && (t0 == 0 || t0 < len); t0 += CHUNK) {   // an empty sequence passes once: its state is zero
       const int stage = fills % GW_STAGES;
       ok = warp_wait_bounded(&empty[stage], (fills / GW_STAGES & 1) ^ 1);
       if (!ok) break;                                   // ... and the other warps hear of it where they meet, below
@@ -251,6 +254,8 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
       ++fills;
     }
     if (!more) break;
+    if (!waited) pdl_wait();                            // the counter is complete, also where the first item was left alone
+    waited = true;
     if (ct == 0 && ok) *handover = gridDim.x + atomicAdd(p.next, 1);
     ok = named_barrier_all(1, THREADS, ok);             // they go on or give up as one
     if (!ok) break;
@@ -785,7 +790,7 @@ extern "C" int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, 
   p.g = g, p.g_t = g_stride_t, p.g_h = g_stride_h;
   p.cu = cu_seqlens, p.ws = static_cast<uint8_t*>(workspace), p.state = state;
   p.out = static_cast<__nv_bfloat16*>(out), p.o_t = out_stride_t, p.o_h = out_stride_h;
-  p.heads = num_heads, p.batch = batch;
+  p.heads = num_heads, p.batch = batch, p.slots = static_cast<int>(walk_slots(batch, total_tokens));
   p.next = reinterpret_cast<int*>(p.ws + walk_slots(batch, total_tokens) * num_heads * GW_SLOT_BYTES);
   p.err = wait_timeout_flag();
   if (!p.err) return fail(ERR_RUNTIME, "gdn_chunked_prefill_walk: no error flag");

@@ -53,6 +53,7 @@ struct OuterRnnParams {
   float* seg_state;        // [sequences, segments, heads, dim, vdim]
   float* seg_decay;        // [sequences, segments, heads, dim]
   void* chunks;            // fragments of all chunks (linear_rnn_walk.cu), or NULL
+  int chunk_slots;         // how many there are, by the number of tokens the call names
   // decode step
   const int64_t *pos, *active;
   int lanes_per_row, overlap;
@@ -63,7 +64,7 @@ int outer_rnn_chunk_launch(const OuterRnnParams& p, RnnKind kind, int n, cudaStr
 bool outer_rnn_walk_supports(const OuterRnnParams& p);
 int outer_rnn_walk_launch(const OuterRnnParams& p, RnnKind kind, int n, int tokens, cudaStream_t st);   // FORGET, KEYED
 bool ssd_walk_supports(const OuterRnnParams& p);
-int ssd_walk_launch(const OuterRnnParams& p, int n, int tokens, cudaStream_t st);
+int ssd_walk_launch(OuterRnnParams p, int n, int tokens, cudaStream_t st);
 void outer_rnn_fold_launch(const OuterRnnParams& p, int n, cudaStream_t st);
 int outer_rnn_serial_launch(const OuterRnnParams& p, RnnKind kind, bool f32, int n, cudaStream_t st);
 int outer_rnn_decode_launch(OuterRnnParams p, RnnKind kind, bool f32, int batch, const char* name, cudaStream_t st);

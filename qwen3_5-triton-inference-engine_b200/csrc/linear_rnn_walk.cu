@@ -223,6 +223,11 @@ __global__ void __launch_bounds__(OW_THREADS, 1) outer_walk_kernel(const __grid_
     pdl_wait();                                   // an idle CTA still orders the grid after the preparation
     return;
   }
+  if (first_slot(p.cu, seq) + (all + OW_C - 1) / OW_C > p.chunk_slots) {   // more tokens than the call named: nobody prepared the end
+    pdl_wait();
+    if (tid == 0) atomicExch(err, 1);
+    return;
+  }
   const int chunks = (len + OW_C - 1) / OW_C;
   if (tid == 0) {
 #pragma unroll
@@ -464,10 +469,11 @@ int launch_pass(const OuterRnnParams& p, dim3 grid, bool early, int* err, cudaSt
 }
 
 template <bool KEYED>
-int launch_walk(const OuterRnnParams& p, int n, int tokens, cudaStream_t st) {
+int launch_walk(OuterRnnParams p, int n, int tokens, cudaStream_t st) {
   int* err = wait_timeout_flag();
   if (!err) return fail(ERR_RUNTIME, "outer_rnn: no error flag");
-  const dim3 prep(static_cast<unsigned>(slots_of(tokens, n)), (p.heads + OW_PREP_WARPS - 1) / OW_PREP_WARPS);
+  p.chunk_slots = static_cast<int>(slots_of(tokens, n));
+  const dim3 prep(static_cast<unsigned>(p.chunk_slots), (p.heads + OW_PREP_WARPS - 1) / OW_PREP_WARPS);
   outer_prep_kernel<KEYED><<<prep, 32 * OW_PREP_WARPS, 0, st>>>(p, n);
   const dim3 grid((p.vdim + OW_COLS - 1) / OW_COLS, p.heads, n * p.segments);
   if (p.segments > 1) {

@@ -549,6 +549,7 @@ extern "C" int b200_ssd_prefill_walk(const void* xbc, int64_t stride, const void
     return outer_rnn_serial_launch(p, RNN_SSD, f32 != 0, batch, st);
   }
   B200_REQUIRE(aligned16(xbc) && aligned16(y) && aligned16(chunks) && stride % 8 == 0, "ssd_prefill: unaligned tensor");
+  B200_REQUIRE(!chunks || tokens > 0, "ssd_prefill: a workspace for the chunks goes with the number of tokens");
   p.out = y, p.out_stride = static_cast<int64_t>(heads) * vdim;
   if (ssd_walk_supports(p)) return ssd_walk_launch(p, batch, tokens, st);
   if (dim <= 32) return launch_ssd<32>(p, batch, st);

@@ -140,6 +140,11 @@ __global__ void __launch_bounds__(SW_THREADS, 2) ssd_walk_kernel(const __grid_co
     pdl_wait();                                   // an idle CTA still orders the grid after the preparation
     return;
   }
+  if (first_slot(p.cu, seq) + (all + SW_Q - 1) / SW_Q > p.chunk_slots) {   // more tokens than the call named: nobody prepared the end
+    pdl_wait();
+    if (tid == 0) atomicExch(err, 1);
+    return;
+  }
   const int chunks = (len + SW_Q - 1) / SW_Q, cols = min(SW_COLS, p.vdim - col0);
   const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(p.x) + static_cast<int64_t>(row0) * p.stride;
   if (tid == 0) {
@@ -353,11 +358,12 @@ bool shape_walks(int dim, int vdim) { return dim > 64 && dim <= SW_N && dim % 8 
 
 bool ssd_walk_supports(const OuterRnnParams& p) { return p.chunks && shape_walks(p.dim, p.vdim); }
 
-int ssd_walk_launch(const OuterRnnParams& p, int n, int tokens, cudaStream_t st) {
+int ssd_walk_launch(OuterRnnParams p, int n, int tokens, cudaStream_t st) {
   int* err = wait_timeout_flag();
   if (!err) return fail(ERR_RUNTIME, "ssd_prefill: no error flag");
   const int groups = p.heads / p.per_group * ((p.per_group + SW_PREP_WARPS - 1) / SW_PREP_WARPS);   // at most heads
-  ssd_prep_kernel<<<dim3(static_cast<unsigned>(slots_of(tokens, n)), groups), 32 * SW_PREP_WARPS, 0, st>>>(p, n);
+  p.chunk_slots = static_cast<int>(slots_of(tokens, n));
+  ssd_prep_kernel<<<dim3(static_cast<unsigned>(p.chunk_slots), groups), 32 * SW_PREP_WARPS, 0, st>>>(p, n);
   const dim3 grid((p.vdim + SW_COLS - 1) / SW_COLS, p.heads, n * p.segments);
   if (p.segments > 1) {
     const int rc = launch_pass<true>(p, grid, true, err, st);

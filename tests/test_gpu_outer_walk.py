@@ -113,3 +113,44 @@ def test_segments_to_spare(hops, kind, lengths):  # noqa: F811
             close(out[row: row + length], y, torch.bfloat16, f"length {length}", 2.0)
             close(state[i], last, torch.float32, f"state after {length}", 20.0)
             row += length
+
+
+@pytest.mark.parametrize("kind,arg", [("hgrn2", 12), ("gla", 16), ("ssd", -3), ("gdn", 17)])
+def test_batch_longer_than_named(hops, kind, arg, monkeypatch):  # noqa: F811
+    """A call that names fewer tokens than its sequences hold: those within what was named are right, the others are left alone, and
+    the flag that a kernel gave up is raised."""
+    from b200attn import _lib, ops
+    from helpers import gdn_inputs
+    heads, dim, vdim, eps, lengths = 16, 128, 64, 1e-5, [70, 40, 200]
+    n, total, batch = len(lengths), sum(lengths), Batch([0, 1, 2], [0] * 3, lengths)
+    call = _lib.call
+
+    def short(name, *args):
+        args = list(args)
+        args[arg] = 112                       # two sequences and a bit of the third
+        return call(name, *args)
+
+    def run():
+        if kind == "gdn":
+            out, state = ops.gdn_chunked_prefill_packed(*(t.to(DEV) for t in gdn_inputs(total, heads, torch.Generator().manual_seed(5))), batch.cu,
+                                                        state_out=torch.full((n, heads, 128, 128), 7.0, device=DEV))
+            return out, state
+        state = torch.full((n, heads, dim, vdim), 7.0, device=DEV)
+        if kind == "hgrn2":
+            return hops.hgrn2_prefill(*[t.to(DEV) for t in _hgrn2_inputs(total, heads, dim, vdim, torch.bfloat16, 5)], state, batch, vdim, eps), state
+        if kind == "gla":
+            qkv, z, gate = (t.to(DEV) for t in gla_inputs(heads, dim, vdim, total, torch.bfloat16, seed=5))
+            out = torch.empty(total, heads * vdim, dtype=torch.bfloat16, device=DEV)
+            hops.gla_prefill(qkv, z, torch.ones(heads * dim, device=DEV), torch.ones(vdim, device=DEV), gate, state, out, batch, vdim, 0.1, 8.0, eps)
+            return out, state
+        return hops.ssd_prefill(*[t.to(DEV) for t in ssd_inputs(heads, 1, dim, vdim, total, torch.bfloat16, seed=5)], state, 1, batch), state
+
+    want = run()
+    torch.cuda.synchronize()
+    assert _lib.load().b200_wait_timed_out() == 0
+    monkeypatch.setattr(_lib, "call", short)
+    got = run()
+    torch.cuda.synchronize()
+    assert _lib.load().b200_wait_timed_out() == 1
+    assert torch.equal(got[0][:110], want[0][:110]) and torch.equal(got[1][:2], want[1][:2])
+    assert torch.equal(got[1][2], torch.full_like(got[1][2], 7.0))
