@@ -85,7 +85,10 @@ __global__ void __launch_bounds__(GP_THREADS, 4) gdn_walk_prep_kernel(const __gr
   const int slot = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int b = -1;             // the last sequence whose slots start at or before this one
   for (int i0 = 0; i0 < p.batch; i0 += GP_THREADS) b += __syncthreads_count(i0 + tid < p.batch && first_slot(p.cu, i0 + tid) <= slot);
-  if (slot == 0 && h == 0 && tid == 0) *p.next = 0;
+  if (slot == 0 && h == 0 && tid == 0) {
+    *p.next = 0;
+    if (first_slot(p.cu, p.batch) > p.slots) atomicExch(p.err, 1);   // more tokens than the call named
+  }
   if (b < 0) return;
   const int t0 = p.cu[b] + (slot - first_slot(p.cu, b)) * CHUNK, rows = min(CHUNK, p.cu[b + 1] - t0);
   if (rows <= 0) return;
@@ -213,25 +216,21 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
   constexpr int SPLIT = GDN_D / COLS, THREADS = 32 * GW_COPY_WARPS;
   uint64_t *full = reinterpret_cast<uint64_t*>(smem + L::BARS), *empty = full + GW_STAGES;
   int* handover = reinterpret_cast<int*>(smem + L::HANDOVER);
-  int fills = 0;                                        // chunks asked for so far, also those that hold nothing
-  bool waited = false, ok = true;
+  int stage = 0;
+  uint32_t parity = 1;
+  bool waited = false, ok = true;                       // a thread whose wait ran out copies nothing more, and completes no stage
   for (int item = blockIdx.x;;) {
     int h = 0, col = 0, start = 0, len = 0, slot0 = 0;
     const bool more = item < p.items;
-    bool fits = true;
     if (more) {
       const int bh = item / SPLIT, b = bh / p.heads;
       h = bh % p.heads, col = item % SPLIT * COLS;
       start = p.cu[b], len = p.cu[b + 1] - start, slot0 = first_slot(p.cu, b);
-      fits = slot0 + (len + CHUNK - 1) / CHUNK <= p.slots;      // else more tokens than the call named: nobody prepared the end
-      if (!fits && ct == 0) atomicExch(p.err, 1);
     }
-    for (int t0 = 0; fits && (t0 == 0 || t0 < len); t0 += CHUNK) {   // an empty sequence passes once: its state is zero
-      const int stage = fills % GW_STAGES;
-      ok = warp_wait_bounded(&empty[stage], (fills / GW_STAGES & 1) ^ 1);
-      if (!ok) break;                                   // ... and the other warps hear of it where they meet, below
+    for (int t0 = 0; t0 == 0 || t0 < len; t0 += CHUNK) {   // an empty sequence passes once: its state is zero
+      ok = ok && mbar_wait_bounded(&empty[stage], parity);
       uint8_t* to = smem + stage * L::STAGE;
-      const int rows = min(CHUNK, len - t0);
+      const int rows = ok ? min(CHUNK, len - t0) : 0;
       if (rows > 0) {
         const int64_t t = start + t0;
         fetch_rows<THREADS>(smem_u32(to) + L::K, GW_PITCH, p.k + t * p.k_t + h * p.k_h, p.k_t, rows, GDN_D, ct);
@@ -240,22 +239,23 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
       }
       if (!waited) pdl_wait();                          // the prepared matrices and the counter are complete
       waited = true;
-      if (ct == 0) {
+      if (ct == 0 && ok) {
+        // a batch of more tokens than the call named: nobody prepared this sequence's end, and its state and output stay as they are
+        const bool fits = !more || slot0 + (len + CHUNK - 1) / CHUNK <= p.slots;
         *reinterpret_cast<int4*>(smem + L::INFO + stage * 16) =
-            make_int4(more ? item : -1, start + t0, rows, (t0 + CHUNK >= len ? 1 : 0) | (t0 == 0 ? 2 : 0));
-        if (rows > 0) {
+            make_int4(more ? item : -1, start + t0, fits ? rows : 0, fits ? (t0 + CHUNK >= len ? 1 : 0) | (t0 == 0 ? 2 : 0) : 0);
+        if (fits && rows > 0) {
           mbar_expect_tx(&full[stage], GW_SLOT_BYTES);
           bulk_g2s(to + L::P, p.ws + (static_cast<int64_t>(slot0 + t0 / CHUNK) * p.heads + h) * GW_SLOT_BYTES, GW_SLOT_BYTES, &full[stage]);
         } else {
           mbar_arrive(&full[stage]);
         }
       }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[stage])) : "memory");
-      ++fills;
+      if (ok) asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[stage])) : "memory");
+      if (++stage == GW_STAGES) stage = 0, parity ^= 1;
     }
     if (!more) break;
-    if (!waited) pdl_wait();                            // the counter is complete, also where the first item was left alone
-    waited = true;
+    __syncwarp();
     if (ct == 0 && ok) *handover = gridDim.x + atomicAdd(p.next, 1);
     ok = named_barrier_all(1, THREADS, ok);             // they go on or give up as one
     if (!ok) break;
@@ -265,9 +265,9 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
   cp_async_wait_all();
   if (!ok) {
     atomicExch(p.err, 1);
-    // bulk copies that nobody waits for any more may still be landing in this CTA's shared memory
+    // bulk copies that nobody waits for any more may still be landing in this CTA's shared memory: either phase of a stage
     if (ct == 0)
-      for (int i = max(fills - GW_STAGES, 0); i < fills; ++i) mbar_wait_bounded(&full[i % GW_STAGES], i / GW_STAGES & 1, 1u << 12);
+      for (int i = 0; i < 2 * GW_STAGES; ++i) mbar_wait_bounded(&full[i >> 1], i & 1, 1u << 12);
   }
 }
 template <int COLS>
