@@ -7,6 +7,8 @@
 // and an accumulator pair of one product is the left operand of the next (S -> k S, q S; R -> delta; delta -> A delta, S), so
 // no value leaves the registers between products and warps never wait for one another inside a chunk.  P and A arrive as
 // right-operand fragments: a lane's two registers of an 8 x 16 tile, high and low parts, are 16 consecutive bytes.
+// The workspace is at most 1 GiB: where all slots would take more, the two launches go through a window of them at a time, and
+// the states wait in device memory in between (fp32, so that the results are the same bits).
 // Precision: q, k, v are exact bf16 operands; fp32 operands (S, R, delta, P, A) are bf16 pairs hi + lo with the products
 // hi hi + hi lo + lo hi (hi + lo against an exact one).
 #include "b200_attn.h"
@@ -33,11 +35,12 @@ struct GdnWalkParams {
   const float *beta, *g;
   int64_t be_t, be_h, g_t, g_h;
   const int32_t* cu;
-  uint8_t* ws;            // [slots, heads, GW_SLOT_BYTES]
+  uint8_t* ws;            // [slots of a window, heads, GW_SLOT_BYTES]
   float* state;           // [batch, heads, 128, 128]
   __nv_bfloat16* out;
   int64_t o_t, o_h;
   int heads, batch, items, slots;
+  int from, to;           // the window's slots
   int *next, *err;        // counter of the walk's items, behind the slots; the flag of waits that ran out
 };
 template <int N>
@@ -82,10 +85,10 @@ static_assert(CHUNK * INV_LP * 4 <= GW_TILE * 2, "L and P lie over the q and k t
 __global__ void __launch_bounds__(GP_THREADS, 4) gdn_walk_prep_kernel(const __grid_constant__ GdnWalkParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   pdl_trigger();          // the walk may take over SMs as the last CTAs of this grid finish
-  const int slot = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int slot = p.from + blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int b = -1;             // the last sequence whose slots start at or before this one
   for (int i0 = 0; i0 < p.batch; i0 += GP_THREADS) b += __syncthreads_count(i0 + tid < p.batch && first_slot(p.cu, i0 + tid) <= slot);
-  if (slot == 0 && h == 0 && tid == 0) {
+  if (blockIdx.x == 0 && h == 0 && tid == 0) {
     *p.next = 0;
     if (first_slot(p.cu, p.batch) > p.slots) atomicExch(p.err, 1);   // more tokens than the call named
   }
@@ -122,7 +125,7 @@ __global__ void __launch_bounds__(GP_THREADS, 4) gdn_walk_prep_kernel(const __gr
     const float hi = static_cast<float>(G);
     gs[tid] = make_float2(hi, static_cast<float>(G - hi));
   }
-  uint8_t* ws = p.ws + (static_cast<int64_t>(slot) * p.heads + h) * GW_SLOT_BYTES;
+  uint8_t* ws = p.ws + (static_cast<int64_t>(blockIdx.x) * p.heads + h) * GW_SLOT_BYTES;
   // ---- scores: warp = (16 rows, 32 columns); columns past the diagonal block are skipped
   const int mt = warp & 3, nh = warp >> 2, gr = lane >> 2, c2 = (lane & 3) * 2;
   float sk[4][4] = {}, sq[4][4] = {};
@@ -200,7 +203,7 @@ constexpr int GW_STAGES = 2;
 constexpr int GW_COPY_WARPS = 4;                        // a whole warpgroup, so that it can hand registers over
 
 // Shared memory of a CTA with COLS value columns: stages of k | q | v tiles and a slot of the workspace, then what a stage holds
-// (item or -1, first token, rows, last (1) and first (2) chunk of a sequence), its barriers, and a word between the copy warps.
+// (item or -1, first token, rows, flags: last (1) and first (2) chunk of a sequence; of a window 1 and 4), its barriers, and a word between the copy warps.
 template <int COLS>
 struct WalkSmem {
   static constexpr int VP = COLS + 8;                   // bf16 pitch of the value tile
@@ -209,8 +212,8 @@ struct WalkSmem {
 };
 
 // The copy warps: items = (sequence, head, COLS value columns), the first by block index, the others from a counter; chunks go
-// into the next stage that `empty` releases, across items.
-template <int COLS>
+// into the next stage that `empty` releases, across items.  WINDOWS: only the chunks of this launch's window.
+template <int COLS, bool WINDOWS>
 __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* smem, int ct) {
   using L = WalkSmem<COLS>;
   constexpr int SPLIT = GDN_D / COLS, THREADS = 32 * GW_COPY_WARPS;
@@ -227,7 +230,14 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
       h = bh % p.heads, col = item % SPLIT * COLS;
       start = p.cu[b], len = p.cu[b + 1] - start, slot0 = first_slot(p.cu, b);
     }
-    for (int t0 = 0; t0 == 0 || t0 < len; t0 += CHUNK) {   // an empty sequence passes once: its state is zero
+    int begin = 0, end = len;
+    bool some = true;
+    if (WINDOWS && more) {
+      const int chunks = (len + CHUNK - 1) / CHUNK;
+      begin = min(max(p.from - slot0, 0), chunks) * CHUNK, end = min(len, min(p.to - slot0, chunks) * CHUNK);
+      some = len > 0 ? begin < end : p.from <= slot0 && slot0 < p.to;
+    }
+    for (int t0 = begin; some && (t0 == begin || t0 < end); t0 += CHUNK) {   // an empty sequence passes once: its state is zero
       ok = ok && mbar_wait_bounded(&empty[stage], parity);
       uint8_t* to = smem + stage * L::STAGE;
       const int rows = ok ? min(CHUNK, len - t0) : 0;
@@ -243,10 +253,11 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
         // a batch of more tokens than the call named: nobody prepared this sequence's end, and its state and output stay as they are
         const bool fits = !more || slot0 + (len + CHUNK - 1) / CHUNK <= p.slots;
         *reinterpret_cast<int4*>(smem + L::INFO + stage * 16) =
-            make_int4(more ? item : -1, start + t0, fits ? rows : 0, fits ? (t0 + CHUNK >= len ? 1 : 0) | (t0 == 0 ? 2 : 0) : 0);
+            make_int4(more ? item : -1, start + t0, fits ? rows : 0,
+                      fits ? (t0 + CHUNK >= end ? 1 : 0) | (t0 == 0 ? 2 : 0) | (WINDOWS && t0 > 0 && t0 == begin ? 4 : 0) : 0);
         if (fits && rows > 0) {
           mbar_expect_tx(&full[stage], GW_SLOT_BYTES);
-          bulk_g2s(to + L::P, p.ws + (static_cast<int64_t>(slot0 + t0 / CHUNK) * p.heads + h) * GW_SLOT_BYTES, GW_SLOT_BYTES, &full[stage]);
+          bulk_g2s(to + L::P, p.ws + (static_cast<int64_t>(slot0 + t0 / CHUNK - (WINDOWS ? p.from : 0)) * p.heads + h) * GW_SLOT_BYTES, GW_SLOT_BYTES, &full[stage]);
         } else {
           mbar_arrive(&full[stage]);
         }
@@ -255,6 +266,8 @@ __device__ __forceinline__ void copy_chunks(const GdnWalkParams& p, uint8_t* sme
       if (++stage == GW_STAGES) stage = 0, parity ^= 1;
     }
     if (!more) break;
+    if (WINDOWS && !waited) pdl_wait();                 // the counter is complete, also where the first item has nothing here
+    if (WINDOWS) waited = true;
     __syncwarp();
     if (ct == 0 && ok) *handover = gridDim.x + atomicAdd(p.next, 1);
     ok = named_barrier_all(1, THREADS, ok);             // they go on or give up as one
@@ -420,7 +433,7 @@ __device__ __forceinline__ void walk_chunk(float (&S)[GDN_D / 8][4], const uint8
 
 // A warp = 16 value columns of one head, alone with its 16 x 128 state; the tensor pipe bounds it (504 products of 2048
 // multiply-adds per full chunk; two warps per scheduler keep the pipe 84 % busy).
-template <int WARPS>
+template <int WARPS, bool WINDOWS>
 __global__ void __launch_bounds__(32 * (WARPS + GW_COPY_WARPS), 1) gdn_walk_kernel(const __grid_constant__ GdnWalkParams p) {
   using L = WalkSmem<16 * WARPS>;
   constexpr int SPLIT = 8 / WARPS;
@@ -435,7 +448,7 @@ __global__ void __launch_bounds__(32 * (WARPS + GW_COPY_WARPS), 1) gdn_walk_kern
   if (warp >= WARPS) {
     // 8 + 4 warps start with 168 registers each (3 x 168 = 504 per column of warpgroups): 40 + 2 x 232 of them
     if constexpr (WARPS == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    copy_chunks<16 * WARPS>(p, smem, tid - 32 * WARPS);
+    copy_chunks<16 * WARPS, WINDOWS>(p, smem, tid - 32 * WARPS);
     return;
   }
   if constexpr (WARPS == 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
@@ -454,6 +467,13 @@ __global__ void __launch_bounds__(32 * (WARPS + GW_COPY_WARPS), 1) gdn_walk_kern
     const int4 info = *reinterpret_cast<const int4*>(smem + L::INFO + stage * 16);
     if (info.x < 0) return;
     const int bh = info.x / SPLIT, h = bh % p.heads, col = info.x % SPLIT * 16 * WARPS + warp * 16;
+    if (WINDOWS && (info.w & 4)) {                      // what the window before left
+      const float* from = p.state + static_cast<int64_t>(bh) * GDN_D * GDN_D + col;
+#pragma unroll
+      for (int n = 0; n < GDN_D / 8; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[n][j] = from[(n * 8 + c2 + (j & 1)) * GDN_D + gr + (j >> 1) * 8];
+    }
     if (info.z > 0) {
       const uint8_t* st = smem + stage * L::STAGE;
       const bool carry = !(info.w & 2);
@@ -537,7 +557,7 @@ __device__ __forceinline__ bool team_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
-template <int TEAMS>
+template <int TEAMS, bool WINDOWS>
 __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_team_kernel(const __grid_constant__ GdnWalkParams p) {
   using L = WalkSmem<16 * TEAMS>;
   using T = TeamSmem<TEAMS>;
@@ -552,7 +572,7 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
   }
   __syncthreads();
   if (team == TEAMS) {
-    copy_chunks<16 * TEAMS>(p, smem, tid - 128 * TEAMS);
+    copy_chunks<16 * TEAMS, WINDOWS>(p, smem, tid - 128 * TEAMS);
     return;
   }
   uint8_t* ex = smem + T::EX + team * GT_BYTES;
@@ -575,7 +595,20 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
     if (!ok) break;
     const int4 info = *reinterpret_cast<const int4*>(smem + L::INFO + stage * 16);
     if (info.x < 0) return;
-    if (info.w & 2) bh = info.x / SPLIT, h = bh % p.heads, col = info.x % SPLIT * 16 * TEAMS + team * 16;
+    if (info.w & (WINDOWS ? 6 : 2)) bh = info.x / SPLIT, h = bh % p.heads, col = info.x % SPLIT * 16 * TEAMS + team * 16;
+    if (WINDOWS && (info.w & 4)) {                      // what the window before left
+      const float* from = p.state + static_cast<int64_t>(bh) * GDN_D * GDN_D + w * 32 * GDN_D + col;
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[n][j] = from[(n * 8 + c2 + (j & 1)) * GDN_D + gr + (j >> 1) * 8];
+      uint32_t hi[4], lo[4];
+      split_frag(S[0], S[1], hi, lo);
+      put_frag(ex + GT_S + 2 * w * 1024, hi, lo, lane);
+      split_frag(S[2], S[3], hi, lo);
+      put_frag(ex + GT_S + (2 * w + 1) * 1024, hi, lo, lane);
+      arrive(0);
+    }
     if (info.z > 0) {
       const uint8_t* st = smem + stage * L::STAGE;
       const uint32_t at = smem_u32(st);
@@ -745,6 +778,11 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
 }
 
 int64_t walk_slots(int batch, int total_tokens) { return static_cast<int64_t>(total_tokens) / CHUNK + batch; }
+// Slots of a window: at most 1 GiB of them, as in the other walks (51 thousand chunks of a head, 3.3 million tokens).
+int64_t window_slots(int batch, int total_tokens, int heads) {
+  const int64_t slots = walk_slots(batch, total_tokens), most = (int64_t{1} << 30) / (static_cast<int64_t>(heads) * GW_SLOT_BYTES);
+  return slots <= most ? slots : most > 0 ? most : 1;
+}
 
 // `items_per_head` CTAs' worth of work per head and sequence, at most one CTA per SM
 int launch_walk(void (*kernel)(GdnWalkParams), int threads, int smem, int items_per_head, GdnWalkParams p, cudaStream_t st) {
@@ -756,13 +794,29 @@ int launch_walk(void (*kernel)(GdnWalkParams), int threads, int smem, int items_
   return check_launch("gdn_chunked_prefill_walk");
 }
 
+// The two launches of a window
+template <bool WINDOWS>
+int prep_and_walk(const GdnWalkParams& p, cudaStream_t st) {
+  gdn_walk_prep_kernel<<<dim3(p.to - p.from, p.heads), GP_THREADS, GP_SMEM, st>>>(p);
+  if (const int rc = check_launch("gdn_chunked_prefill_walk (prep)")) return rc;
+  const int pairs = p.heads * p.batch, sms = sm_count();
+  constexpr int copy = 32 * GW_COPY_WARPS;
+  // What fills the device: four warps per 16 value columns while that leaves SMs free (one sequence of 2048 tokens: 80 us against
+  // 122 on half-head CTAs and 199 on whole heads), two such teams per CTA (2 x 1000..3000: 114 against 135 and 215), half a head
+  // per CTA (4 x 2048: 148 against 214 in teams and 225 on whole heads), whole heads (8 x 1024: 133 against 148).
+  if (pairs * 8 <= sms) return launch_walk(gdn_walk_team_kernel<1, WINDOWS>, 128 + copy, TeamSmem<1>::BYTES, 8, p, st);
+  if (pairs * 4 <= sms) return launch_walk(gdn_walk_team_kernel<2, WINDOWS>, 256 + copy, TeamSmem<2>::BYTES, 4, p, st);
+  if (pairs * 2 <= sms) return launch_walk(gdn_walk_kernel<4, WINDOWS>, 128 + copy, WalkSmem<64>::BYTES, 2, p, st);
+  return launch_walk(gdn_walk_kernel<8, WINDOWS>, 256 + copy, WalkSmem<128>::BYTES, 1, p, st);
+}
+
 }  // namespace
 }  // namespace b200
 
 using namespace b200;
 
 extern "C" int64_t b200_gdn_chunked_prefill_walk_workspace_bytes(int32_t batch, int32_t total_tokens, int32_t num_heads) {
-  return walk_slots(batch, total_tokens) * num_heads * GW_SLOT_BYTES + 16;
+  return window_slots(batch, total_tokens, num_heads) * num_heads * GW_SLOT_BYTES + 16;
 }
 
 extern "C" int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k, int64_t k_stride_t,
@@ -773,6 +827,7 @@ extern "C" int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, 
                                              int32_t num_heads, int32_t key_dim, int32_t value_dim, b200_stream_t stream) {
   B200_REQUIRE(batch > 0 && batch <= 65535 && total_tokens > 0 && num_heads > 0 && num_heads <= 65535,
                "gdn_chunked_prefill_walk: bad shape");
+  B200_REQUIRE(static_cast<int64_t>(batch) * num_heads < (1 << 28), "gdn_chunked_prefill_walk: too many heads and sequences");
   B200_REQUIRE(key_dim == GDN_D && value_dim == GDN_D, "gdn_chunked_prefill_walk: key/value dim must be %d (got %d/%d)", GDN_D, key_dim,
                value_dim);
   B200_REQUIRE(cu_seqlens != nullptr && workspace != nullptr && aligned16(workspace),
@@ -791,19 +846,18 @@ extern "C" int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, 
   p.cu = cu_seqlens, p.ws = static_cast<uint8_t*>(workspace), p.state = state;
   p.out = static_cast<__nv_bfloat16*>(out), p.o_t = out_stride_t, p.o_h = out_stride_h;
   p.heads = num_heads, p.batch = batch, p.slots = static_cast<int>(walk_slots(batch, total_tokens));
-  p.next = reinterpret_cast<int*>(p.ws + walk_slots(batch, total_tokens) * num_heads * GW_SLOT_BYTES);
+  const int window = static_cast<int>(window_slots(batch, total_tokens, num_heads));
+  p.next = reinterpret_cast<int*>(p.ws + static_cast<int64_t>(window) * num_heads * GW_SLOT_BYTES);
   p.err = wait_timeout_flag();
   if (!p.err) return fail(ERR_RUNTIME, "gdn_chunked_prefill_walk: no error flag");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  gdn_walk_prep_kernel<<<dim3(static_cast<unsigned>(walk_slots(batch, total_tokens)), num_heads), GP_THREADS, GP_SMEM, st>>>(p);
-  if (const int rc = check_launch("gdn_chunked_prefill_walk (prep)")) return rc;
-  const int pairs = num_heads * batch, sms = sm_count();
-  constexpr int copy = 32 * GW_COPY_WARPS;
-  // What fills the device: four warps per 16 value columns while that leaves SMs free (one sequence of 2048 tokens: 80 us against
-  // 122 on half-head CTAs and 199 on whole heads), two such teams per CTA (2 x 1000..3000: 114 against 135 and 215), half a head
-  // per CTA (4 x 2048: 148 against 214 in teams and 225 on whole heads), whole heads (8 x 1024: 133 against 148).
-  if (pairs * 8 <= sms) return launch_walk(gdn_walk_team_kernel<1>, 128 + copy, TeamSmem<1>::BYTES, 8, p, st);
-  if (pairs * 4 <= sms) return launch_walk(gdn_walk_team_kernel<2>, 256 + copy, TeamSmem<2>::BYTES, 4, p, st);
-  if (pairs * 2 <= sms) return launch_walk(gdn_walk_kernel<4>, 128 + copy, WalkSmem<64>::BYTES, 2, p, st);
-  return launch_walk(gdn_walk_kernel<8>, 256 + copy, WalkSmem<128>::BYTES, 1, p, st);
+  if (window == p.slots) {
+    p.from = 0, p.to = p.slots;
+    return prep_and_walk<false>(p, st);
+  }
+  for (p.from = 0; p.from < p.slots; p.from = p.to) {
+    p.to = p.slots - p.from < window ? p.slots : p.from + window;
+    if (const int rc = prep_and_walk<true>(p, st)) return rc;
+  }
+  return OK;
 }

@@ -157,6 +157,29 @@ def test_walk_forms(ops, heads, lengths):
     assert torch.equal(state2[others], state[others])
 
 
+@pytest.mark.parametrize("heads,part,lengths", [(18, 9, [190001]), (18, 10, [100000, 90001]), (37, 21, [50001, 45000]),
+                                                (40, 20, [0, 40000, 100, 45001, 64, 0])])
+def test_walk_in_windows(ops, heads, part, lengths):
+    """Batches whose chunks would take more than 1 GiB go through a window of chunks at a time: the same bits as parts of the heads,
+    which fit (in the same form of the walk), give; sequences cut by a window, empty ones at either end."""
+    from b200attn import _lib
+    total, gen = sum(lengths), torch.Generator(device=DEV).manual_seed(heads)
+    assert total // 64 * heads * 20992 > 1 << 30
+    assert _lib.load().b200_gdn_chunked_prefill_walk_workspace_bytes(len(lengths), total, heads) <= (1 << 30) + 16
+    assert (total // 64 + len(lengths)) * part * 20992 <= 1 << 30
+    q, k, v = (torch.randn(total, heads, 128, generator=gen, device=DEV, dtype=torch.bfloat16) for _ in range(3))
+    q, k = (torch.nn.functional.normalize(t, dim=-1) for t in (q, k))
+    beta = torch.rand(total, heads, generator=gen, device=DEV)
+    g = -0.2 * torch.rand(total, heads, generator=gen, device=DEV)
+    cu = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    out, state = ops.gdn_chunked_prefill_packed(q, k, v, beta, g, cu)
+    for lo in (0, heads - part):
+        want, last = ops.gdn_chunked_prefill_packed(*(t[:, lo: lo + part] for t in (q, k, v, beta, g)), cu)
+        assert torch.equal(out[:, lo: lo + part], want) and torch.equal(state[:, lo: lo + part], last)
+    assert torch.isfinite(state).all() and (state.flatten(1).abs().amax(1) > 0).tolist() == [n > 0 for n in lengths]
+    assert _lib.load().b200_wait_timed_out() == 0
+
+
 def test_one_launch_entry(ops):
     """The entry point without a workspace (tcgen05, one CTA per head) gives what the walk gives."""
     from b200attn import _lib
