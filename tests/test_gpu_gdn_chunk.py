@@ -19,6 +19,18 @@ def ops():
     return _ops
 
 
+def packed(ops, form, q, k, v, beta, g, cu, longest):
+    """Packed prefill by the walk, by the one-launch C entry (tcgen05, a CTA per sequence and head), or in three stages."""
+    if form != "one-launch":
+        return ops.gdn_chunked_prefill_packed(q, k, v, beta, g, cu, longest, fused=form == "walk")
+    from b200attn import _lib
+    out, state = torch.empty(v.shape, dtype=v.dtype, device=DEV), torch.empty(cu.numel() - 1, v.shape[1], 128, 128, device=DEV)
+    _lib.call("b200_gdn_chunked_prefill_fused", *(a for t in (q, k, v, beta, g) for a in (t.data_ptr(), t.stride(0), t.stride(1))), cu.data_ptr(),
+              cu.numel() - 1, q.shape[0], state.data_ptr(), out.data_ptr(), out.stride(0), out.stride(1), q.shape[1], 128, 128,
+              torch.cuda.current_stream().cuda_stream)
+    return out, state
+
+
 def test_chunk_ops_golden(ops, golden):
     g = golden("gdn_chunked")
     d = {k: v.to(DEV) for k, v in g.items()}
@@ -67,12 +79,12 @@ def test_prepare_wy_vs_oracle(ops):
     assert maxabs(w, rw) < 2e-4 and maxabs(u, ru) < 2e-4
 
 
-@pytest.mark.parametrize("fused", [True, False], ids=["tcgen05", "three-stage"])
+@pytest.mark.parametrize("form", ["walk", "one-launch", "three-stage"])
 @pytest.mark.parametrize("lengths", [[128] * 4, [5, 64, 65, 1, 200], [130], [63, 300, 17]])
-def test_chunked_prefill_packed(ops, lengths, fused):
-    """Packed chunk-64 prefill (32 prompts in one call, which the reference cannot run in one call), as the single
-    tcgen05 kernel and as the three reference-shaped stages: pinned by (i) the token-serial kernel with cu_seqlens
-    and (ii) the oracle's per-sequence chunk pipeline."""
+def test_chunked_prefill_packed(ops, lengths, form):
+    """Packed chunk-64 prefill (32 prompts in one call, which the reference cannot run in one call), as preparation and
+    walk, as the single tcgen05 kernel and as the three reference-shaped stages: pinned by (i) the token-serial kernel
+    with cu_seqlens and (ii) the oracle's per-sequence chunk pipeline."""
     gen = torch.Generator().manual_seed(1200 + sum(lengths))
     heads, total = 16, sum(lengths)
     q, k, v, beta, g = gdn_inputs(total, heads, gen, v_row_stride=3 * heads * 128)
@@ -81,7 +93,7 @@ def test_chunked_prefill_packed(ops, lengths, fused):
     storage[:, 2 * heads * 128:] = v.to(DEV).reshape(total, -1)
     vd = storage[:, 2 * heads * 128:].view(total, heads, 128)
     qd, kd, bd, gd, cud = q.to(DEV), k.to(DEV), beta.to(DEV), g.to(DEV), cu.to(DEV)
-    out_c, state_c = ops.gdn_chunked_prefill_packed(qd, kd, vd, bd, gd, cud, max(lengths), fused=fused)
+    out_c, state_c = packed(ops, form, qd, kd, vd, bd, gd, cud, max(lengths))
     out_s, state_s = ops.gdn_recurrent_prefill_sequential(qd, kd, vd, bd, gd, cud)
     assert out_c.shape == out_s.shape and state_c.shape == state_s.shape == (len(lengths), heads, 128, 128)
     assert torch.isfinite(out_c.float()).all() and torch.isfinite(state_c).all()
@@ -91,17 +103,19 @@ def test_chunked_prefill_packed(ops, lengths, fused):
         assert maxabs(out_c, ref_out) <= 1e-2 and maxabs(state_c, ref_state) <= 5e-4
 
 
+@pytest.mark.parametrize("form", ["walk", "one-launch"])
 @pytest.mark.parametrize("lengths", [[128] * 32, [1000, 513, 64, 2048]])
-def test_fused_chunk_prefill_long(ops, lengths):
-    """The tcgen05 chunk kernel at the batched-prompt size (32 x 128) and over many chunks per sequence (the state is
-    carried in tensor memory for up to 32 chunks) against the token-serial kernel; no bounded wait may run out."""
+def test_fused_chunk_prefill_long(ops, lengths, form):
+    """The walk and the tcgen05 kernel at the batched-prompt size (32 x 128) and over many chunks per sequence (the state
+    is carried in registers, or in tensor memory, for up to 32 chunks) against the token-serial kernel; no bounded wait
+    may run out."""
     from b200attn import _lib
     gen = torch.Generator().manual_seed(4242 + len(lengths))
     heads, total = 16, sum(lengths)
     q, k, v, beta, g = gdn_inputs(total, heads, gen)
     cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32)
     qd, kd, vd, bd, gd, cud = (x.to(DEV) for x in (q, k, v, beta, g, cu))
-    out_c, state_c = ops.gdn_chunked_prefill_packed(qd, kd, vd, bd, gd, cud)
+    out_c, state_c = packed(ops, form, qd, kd, vd, bd, gd, cud, max(lengths))
     out_s, state_s = ops.gdn_recurrent_prefill_sequential(qd, kd, vd, bd, gd, cud)
     torch.cuda.synchronize()
     assert _lib.load().b200_wait_timed_out() == 0
@@ -155,6 +169,17 @@ def test_walk_forms(ops, heads, lengths):
     assert torch.equal(out2[:lo], out[:lo]) and torch.equal(out2[hi:], out[hi:])
     others = [i for i in range(len(lengths)) if i != 4]
     assert torch.equal(state2[others], state[others])
+
+
+@pytest.mark.parametrize("heads", [1, 3])
+def test_walk_of_many_sequences(ops, heads):
+    """More sequences than a CTA of the preparation looks through at once, twice over."""
+    lengths = [70] + [1, 0, 2, 65, 17] * 120
+    q, k, v, beta, g = (x.to(DEV) for x in gdn_inputs(sum(lengths), heads, torch.Generator().manual_seed(heads)))
+    cu = torch.tensor([0] + torch.tensor(lengths).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    out, state = ops.gdn_chunked_prefill_packed(q, k, v, beta, g, cu)
+    ref_out, ref_state = ops.gdn_recurrent_prefill_sequential(q, k, v, beta, g, cu)
+    assert maxabs(out, ref_out) <= 1e-2 and maxabs(state, ref_state) <= 5e-4
 
 
 @pytest.mark.parametrize("heads,part,lengths", [(18, 9, [190001]), (18, 10, [100000, 90001]), (37, 21, [50001, 45000]),
