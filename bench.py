@@ -700,7 +700,7 @@ def reference_triton_legs(args, sweep, model, value):
         for row in sweep:
             op = alias.get(row["op"], row["op"])
             us = by_key.get((op, row.get("B"), row.get("ctx"), row.get("shape")))
-            if us is None and op.startswith("gdn_chunked_prefill_fused"):
+            if us is None and op.startswith("gdn_chunked_prefill_walk"):
                 us = by_key.get(("gdn_recurrent_prefill_sequential", None, None, row.get("shape")))   # its only packed route
             if us is not None:
                 row["triton_us"] = us
@@ -1015,13 +1015,13 @@ def run_prefill_sweep(ops, device, steps, only=None):
     ms = time_steps(lambda i: ops.gdn_chunked_prefill_packed(gq, gk, gv, beta, g, cu), steps, 3)
     cflops = 12.1e6 * 2 * len(lengths) * heads
     cbytes = total * heads * (4 * 128 * 2 + 8) + len(lengths) * heads * 128 * 128 * 4
-    rows.append({"op": "gdn_chunked_prefill_fused (tcgen05, 1 launch)", "shape": "cfg4 B=32 x 128", "tokens": total,
+    rows.append({"op": "gdn_chunked_prefill_walk (mma.sync, 2 launches)", "shape": "cfg4 B=32 x 128", "tokens": total,
                  "us": ms * 1e3, "tflops": cflops / (ms * 1e-3) / 1e12, "frac_tensor": cflops / (ms * 1e-3) / 1e12 / tf_peak,
                  "gbs": cbytes / (ms * 1e-3) / 1e9, "frac_hbm": cbytes / (ms * 1e-3) / 1e9 / hbm})
     ms = time_steps(lambda i: ops.gdn_chunked_prefill_packed(gq, gk, gv, beta, g, cu, 128, fused=False), steps, 3)
     rows.append({"op": "gdn_chunked_prefill_packed (3 launches)", "shape": "cfg4 B=32 x 128", "tokens": total,
                  "us": ms * 1e3, "tflops": cflops / (ms * 1e-3) / 1e12, "frac_tensor": cflops / (ms * 1e-3) / 1e12 / tf_peak})
-    # the same kernel where every SM has work for many chunks: 32 prompts x 1024 tokens (512 CTAs x 16 chunks)
+    # the same kernels where every SM has work for many chunks: 32 prompts x 1024 tokens (512 heads x 16 chunks)
     long_len = [1024] * 32
     lt = sum(long_len)
     gen2 = torch.Generator().manual_seed(11)
@@ -1036,7 +1036,7 @@ def run_prefill_sweep(ops, device, steps, only=None):
     ms = time_steps(lambda i: ops.gdn_chunked_prefill_packed(lq, lk, lv, lbeta, lg, lcu), steps, 3)
     lflops = 12.1e6 * (lt // 64) * heads
     lbytes = lt * heads * (4 * 128 * 2 + 8) + len(long_len) * heads * 128 * 128 * 4
-    rows.append({"op": "gdn_chunked_prefill_fused (tcgen05, 1 launch)", "shape": "B=32 x 1024", "tokens": lt,
+    rows.append({"op": "gdn_chunked_prefill_walk (mma.sync, 2 launches)", "shape": "B=32 x 1024", "tokens": lt,
                  "us": ms * 1e3, "tflops": lflops / (ms * 1e-3) / 1e12, "frac_tensor": lflops / (ms * 1e-3) / 1e12 / tf_peak,
                  "gbs": lbytes / (ms * 1e-3) / 1e9, "frac_hbm": lbytes / (ms * 1e-3) / 1e9 / hbm})
     del lq, lk, lv, lbeta, lg

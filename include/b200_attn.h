@@ -296,6 +296,8 @@ int b200_gdn_chunked_prefill_packed(const void* q, int64_t q_stride_t, int64_t q
 
 /* The same packed chunk-64 prefill as ONE kernel on the tcgen05 tensor cores: one CTA per (sequence, head) keeps the
  * state in tensor memory and walks the chunks; Q/K/V chunks arrive by tensor-map TMA, no workspace, no max_seqlen.
+ * NaN or infinity in the first rows of a sequence can reach the one in front of it, whose last chunk's tile covers them
+ * (b200_gdn_chunked_prefill_walk keeps sequences apart).
  * q, k, v must be 16-byte aligned with token and head strides that are multiples of 8 elements.  No reference
  * counterpart as a single call (it fuses triton_kernels/gdn_recurrent_prefill.py:703-784, :825-909, :935-1006 for a
  * packed batch); results equal wy_lib::gdn_recurrent_prefill_sequential(..., cu_seqlens) within the reference's
@@ -311,7 +313,9 @@ int b200_gdn_chunked_prefill_fused(const void* q, int64_t q_stride_t, int64_t q_
 /* The same packed chunk-64 prefill in two launches: the chunks' own matrices, all at once, then a walk over every sequence's
  * chunks with the state in registers.  Same arguments and rules, plus `workspace`:
  * b200_gdn_chunked_prefill_walk_workspace_bytes(batch, total_tokens, num_heads) bytes of caller-owned device memory, 16-byte
- * aligned (contents undefined afterwards). */
+ * aligned (contents undefined afterwards): 328 bytes a token and head and 20992 a sequence and head, at most 1 GiB - beyond it
+ * the two launches go through the batch in windows, with the same result.  A sequence that ends behind total_tokens keeps
+ * its state and output, and b200_wait_timed_out() reports the call. */
 int64_t b200_gdn_chunked_prefill_walk_workspace_bytes(int32_t batch, int32_t total_tokens, int32_t num_heads);
 int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k,
                                   int64_t k_stride_t, int64_t k_stride_h, const void* v, int64_t v_stride_t,
@@ -515,7 +519,8 @@ int b200_hgrn2_prefill(const void* qfv, int64_t stride, const float* lower, cons
                        b200_stream_t stream);
 /* b200_hgrn2_prefill (b200_gla_prefill) with a workspace of b200_outer_walk_workspace_bytes() for what every chunk needs of
  * itself: computed for all chunks at once, then walked (64 < dim <= 128; other shapes do not use it).  The size is 0 where
- * the shape does not, or where it would be more than 1 GiB; a NULL workspace is the form without. */
+ * the shape does not, or where it would be more than 1 GiB; a NULL workspace is the form without.  A sequence that ends
+ * behind `tokens` keeps its state and output, and b200_wait_timed_out() reports the call. */
 int64_t b200_outer_walk_workspace_bytes(int32_t tokens, int32_t batch, int32_t heads, int32_t dim, int32_t vdim);
 int b200_hgrn2_prefill_walk(const void* qfv, int64_t stride, const float* lower, const float* bias, const float* norm, float* state,
                             const int32_t* cu_seqlens, const int32_t* slots, const int32_t* start, float* o_scratch, void* out,

@@ -17,7 +17,9 @@
 // reference's 3xTF32 products.  P = (I + L)^-1 is formed in fp32 on the CUDA cores by a blocked inverse (16 x 16 diagonal
 // blocks by forward substitution, two levels of P21 = -P22 L21 P11 with register tiles); the classical
 // delta = P beta (v - e^G k S) then needs P only as the right-hand operand of one tensor-core product, so w never exists.
-// Q/K/V chunks arrive by tensor-map TMA (128-byte swizzle) straight from the strided [T, H, 128] activations.
+// Q/K/V chunks arrive by tensor-map TMA (128-byte swizzle) straight from the strided [T, H, 128] activations.  A chunk's boxes
+// may reach into the next sequence's rows: they are multiplied by zeros, so that NaN or infinity there does reach the sequence
+// in front (the walk of gdn_chunk_walk.cu, which the packed operator runs, reads no such rows).
 #include "b200_attn.h"
 #include "gdn_inverse.cuh"
 #include "umma.cuh"
