@@ -131,10 +131,23 @@ def _chunk_workspace(size: str, x, batch, heads: int, dim: int, vdim: int, takes
     return torch.empty(nbytes, dtype=torch.uint8, device=x.device) if nbytes else None
 
 
-def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool):
+def mostly_one_chunk(tokens: int, count: int, longest: int, groups: int, sms: int, chunk: int, per_sm: int, limit: int) -> bool:
+    """Batches that the one-launch forms serve better: several heads of 128 columns per SM, a chunk or less a sequence on average
+    but for the longest, and that one done (`per_sm` tokens for every head of an SM, at most `limit`) before the others are.  There the
+    walks pay for a preparation and a CTA per SM without a chain of chunks to shorten.  Microseconds in one launch and in two,
+    16 heads, 31 sequences of 16 tokens and one of 33: HGRN2 24.7 and 27.6, gated linear attention 27.3 and 28.9, state space 20.5 and
+    22.4; with one of 1024: 335 and 119, 420 and 142, 139 and 56; 32 of 33: 49.8 and 44.8, 55.5 and 47.5, 31.5 and 29.0; 15 of 16
+    and one of 33: 22.1 and 18.4, 24.8 and 19.2, 14.7 and 13.5."""
+    return groups > 2 * sms and tokens - longest <= (count - 1) * chunk and longest <= min(limit, per_sm * groups // sms)
+
+
+def _outer_chunks(x, batch, heads: int, dim: int, vdim: int, chunked: bool, dense: float = float("inf")):
     """Two launches pay from the third chunk of 16 tokens on: 32 sequences of 16 tokens take 31 us in one launch and 39 in two,
-    one of 64 tokens 28.7 and 24.6, 8 of 256 to 1024 tokens 336 and 158 (16 heads of 128 x 128)."""
-    return _chunk_workspace("b200_outer_walk_workspace_bytes", x, batch, heads, dim, vdim, chunked and batch.max_len >= OUTER_WALK_FROM)
+    one of 64 tokens 28.7 and 24.6, 8 of 256 to 1024 tokens 336 and 158 (16 heads of 128 x 128).  dense: heads per SM from which they
+    pay for any such batch."""
+    groups, sms = batch.count * heads * -(-vdim // 128), sm_count(x.device)
+    few = groups <= dense * sms and mostly_one_chunk(x.shape[0], batch.count, batch.max_len, groups, sms, 16, 16, 64)
+    return _chunk_workspace("b200_outer_walk_workspace_bytes", x, batch, heads, dim, vdim, chunked and batch.max_len >= OUTER_WALK_FROM and not few)
 
 
 def outer_walk_segments(max_len: int, groups: int, sm_count: int, chunk: int = 16) -> tuple[int, int]:
@@ -452,8 +465,10 @@ def ssd_prefill(xbc, dt, dt_bias, a_log, skip, state, groups: int, batch, serial
     _require_cuda(xbc, dt, dt_bias, a_log, skip, state)
     tokens = xbc.shape[0]
     chunked = xbc.dtype == torch.bfloat16 and not serial and bool(_lib.load().b200_ssd_chunked(dim, vdim))
-    chunks = _chunk_workspace("b200_ssd_walk_workspace_bytes", xbc, batch, heads, dim, vdim, chunked and batch.max_len >= SSD_WALK_FROM)
     size = (batch.max_len, batch.count * max(1, heads * vdim // 128), sm_count(xbc.device))
+    few = mostly_one_chunk(tokens, batch.count, *size, 32, 28, batch.max_len)
+    chunks = _chunk_workspace("b200_ssd_walk_workspace_bytes", xbc, batch, heads, dim, vdim,
+                              chunked and batch.max_len >= SSD_WALK_FROM and not few)
     segment, count = (batch.max_len, 1) if not chunked else segments or (ssd_segments(*size) if chunks is None else outer_walk_segments(*size, 32))
     ws = None
     if count > 1:
@@ -508,7 +523,9 @@ def gla_prefill(qkv, z, bias, norm, gate, state, out, batch, true_vdim: int, q_s
     tokens = qkv.shape[0]
     assert z.dtype == torch.float32 and _rows(z) and z.shape == (tokens, heads * dim)
     chunked = qkv.dtype == torch.bfloat16 and dim <= 128 and not serial
-    chunks = _outer_chunks(qkv, batch, heads, dim, vdim, chunked)
+    # with many heads an SM the gates of the one-launch form cost more than a second launch: 127 sequences of 8 tokens and one of 48
+    # take 88.7 us in one and 81.0 in two
+    chunks = _outer_chunks(qkv, batch, heads, dim, vdim, chunked, dense=5.5)
     rule = hgrn2_segments if chunks is None else outer_walk_segments
     segment, count = (batch.max_len, 1) if not chunked else segments or rule(
         batch.max_len, batch.count * heads * -(-vdim // 128), sm_count(qkv.device))

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("heads,dim,vdim", [(5, 128, 128), (2, 72, 8), (3, 96, 136)])
-@pytest.mark.parametrize("lengths", [[33], [64, 1, 65, 16], [49] + [1, 2, 17] * 44])
+@pytest.mark.parametrize("lengths", [[33], [64, 1, 65, 16], [81] + [1, 2, 17] * 44])
 def test_hgrn2_walk(hops, heads, dim, vdim, lengths):  # noqa: F811
     """One sequence, several, and more of them than a CTA looks through at once; states carried in every second one."""
     n, eps = len(lengths), 1e-5
@@ -56,7 +56,7 @@ def test_gla_walk(hops, heads, dim, vdim, true, segments):  # noqa: F811
 
 
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(9, 1, 128, 64), (18, 2, 72, 48), (2, 2, 96, 112)])
-@pytest.mark.parametrize("lengths,segments", [([33], None), ([64, 31, 65, 128, 1], None), ([100] + [1, 32, 40] * 90, None), ([257, 32, 200], (64, 5))])
+@pytest.mark.parametrize("lengths,segments", [([33], None), ([64, 31, 65, 128, 1], None), ([401] + [1, 32, 40] * 90, None), ([257, 32, 200], (64, 5))])
 def test_state_space_walk(hops, heads, groups, dim, vdim, lengths, segments):  # noqa: F811
     """Groups of more heads than a prep CTA takes, whole and part columns, more sequences than a CTA looks through at once."""
     n = len(lengths)
