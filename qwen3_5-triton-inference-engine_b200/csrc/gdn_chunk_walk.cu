@@ -432,7 +432,8 @@ __device__ __forceinline__ void walk_chunk(float (&S)[GDN_D / 8][4], const uint8
 }
 
 // A warp = 16 value columns of one head, alone with its 16 x 128 state; the tensor pipe bounds it (504 products of 2048
-// multiply-adds per full chunk; two warps per scheduler keep the pipe 84 % busy).
+// multiply-adds per full chunk).  32 x 128 tokens, 16 heads: 50 us, the pipe active 58 % of the time on average and 67 % on the
+// busiest SM, where every second chunk is a sequence's first and waits for its loads.
 template <int WARPS, bool WINDOWS>
 __global__ void __launch_bounds__(32 * (WARPS + GW_COPY_WARPS), 1) gdn_walk_kernel(const __grid_constant__ GdnWalkParams p) {
   using L = WalkSmem<16 * WARPS>;
