@@ -78,6 +78,43 @@ __device__ __forceinline__ float ex2_fast(float x) {
   return y;
 }
 
+__device__ __forceinline__ float tanh_fast(float x) {
+  float t;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(x));
+  return t;
+}
+
+// ----------------------------------------------------------------------------- two fp32 values per instruction
+// Each half rounds as the scalar instruction does.
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ uint64_t f32x2(uint32_t lo, uint32_t hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ float f32x2_lo(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float f32x2_hi(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t f32x2_mul(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t pack_bf16x2(uint64_t v) { return pack_bf16(f32x2_lo(v), f32x2_hi(v)); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -148,6 +185,15 @@ __device__ __forceinline__ void bulk_s2g(void* dst_gmem, const void* src_smem, u
 }
 // Wait until the issuing thread's bulk stores have finished READING shared memory (it may then be reused or freed).
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// 16 bytes global -> shared, no registers in between.
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// The same, all but the newest N of them.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read_but() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 // Barrier among `count` threads (a multiple of 32) that all name the same id (1..15; 0 is __syncthreads).
 __device__ __forceinline__ void named_barrier(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
@@ -257,6 +303,46 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t ran
 }
 __device__ __forceinline__ void st_cluster_f32x4(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// Barriers that the other CTA of a cluster arrives on: the arrival (`addr` from cluster_map) and the wait of a whole warp (see
+// warp_wait_bounded), at cluster scope.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// The arrival for what is ordered by other means (tensor memory by tcgen05 fences): the cluster-wide release above first waits for the
+// thread's memory operations, a microsecond where stores are in flight.
+__device__ __forceinline__ void mbar_arrive_cluster_plain(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool warp_wait_cluster(uint64_t* bar, uint32_t parity, bool ok = true) {
+  bool done = false;
+  if (ok) {
+    const uint64_t t0 = global_timer_ns();
+    do {
+      for (int i = 0; i < 64 && !done; ++i) done = mbar_try_wait_cluster(bar, parity);
+    } while (!done && global_timer_ns() - t0 < 1000000000ull);
+  }
+  return __all_sync(0xffffffffu, done) != 0;
+}
+// Registers per thread of the calling warpgroup, which was launched with LAUNCHED of them.  `inc` below what a warpgroup has, or `dec`
+// above it, is an illegal instruction.
+template <int N, int LAUNCHED>
+__device__ __forceinline__ void set_registers() {
+  static_assert(N % 8 == 0 && N >= 24 && N <= 256, "setmaxnreg takes multiples of 8 in [24, 256]");
+  if constexpr (N > LAUNCHED) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+  if constexpr (N < LAUNCHED) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
 // ----------------------------------------------------------------------------- warp-level MMA (bf16, fp32 accumulate)

@@ -195,11 +195,6 @@ __device__ __forceinline__ void stage_q(__nv_bfloat16* buf, const FusedDecodePar
                                         int h, int pos_b, int tid) {
   stage_q_row(buf, p, tb, load_q_row(p, b, h, tid), pos_b, tid);
 }
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Asks the L2 for the q rows and the gate row of a segment ahead of their use (one 16-byte piece per thread of warps
 // 0-3 and 8 bytes of gate per thread: the lines they touch cover both rows).
 __device__ __forceinline__ void prefetch_l2(const void* ptr) {

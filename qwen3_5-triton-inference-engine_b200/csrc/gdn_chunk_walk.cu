@@ -60,7 +60,6 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool on) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // `cols` bf16 columns of 64 rows of one head, rows from `rows` on as zeros
 template <int THREADS>

@@ -268,9 +268,6 @@ __global__ void __launch_bounds__(128) latent_absorb_f32_kernel(const __grid_con
 // (head, 64 columns, 16 slots), a warp per 16 columns.  The whole [K x 64] slice of W is requested at once (cp.async,
 // before the predecessor has finished), the slots' rows after it: one memory round trip.
 // K_ROWS: W_h is stored [K, N] (absorb), else [N, K] (value).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 constexpr int HG_PITCH = 144;                              // bytes of a 64-element row plus 16
 constexpr int HG_STEP = (64 + 16) * HG_PITCH;              // bytes of one 64-wide step of K: W tile, then the slots' tile
 

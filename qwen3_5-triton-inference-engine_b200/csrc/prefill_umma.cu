@@ -3,21 +3,27 @@
 //   b200_fused_prefill_attention <-> the chain of engine/runner.py:339-384: partial_rope(q), partial_rope(k),
 //                                    gqa_attention_varlen_causal, attention_gate_pack, paged_kv_fill_varlen
 //
-// One CTA = one (sequence, kv head, block of 32 query tokens).  The 4 Q heads of the group are stacked into the 128
-// rows of one MMA tile (row = token*4 + head, the stacking idea of gqa_attention_varlen_causal.py:151-160), so every
-// K/V tile is fetched once per group.  Per 128-token KV tile:
-//     S[128 x 128]  = Q[128 x 256] . K^T          tcgen05.mma, both operands K-major in shared memory, D in TMEM
-//     P = exp2(S*scale*log2e - m)                  two softmax threads per row (64 columns each), TMEM -> TMEM
-//     O[128 x 256] += P[128 x 128] . V[128 x 256]  tcgen05.mma, P from TMEM, V as an MN-major operand, O stays in TMEM
-// The tile is 128 tokens wide because a tcgen05.mma with M=128 costs at least ~64 cycles whatever its N (measured:
-// N=64 and N=128 both ~69 cycles per instruction, N=256 128 cycles), so N=64 score tiles ran the tensor pipe at half
-// rate.  Roles: warps 0-7 softmax/epilogue (TMEM lane quarter = warp % 4, column half = warp / 4), warp 8 issues the
-// MMAs (the whole warp walks the loop, lane 0 issues), warps 9 and 10 issue the K and V TMA loads (64 KiB per tile,
-// 128-byte swizzle, no multicast; two independent chains so that K of tile j+1 is requested the moment S of tile j
-// is done).  S is double-buffered in TMEM (2 x 128 columns + 256 for O = all 512) and P never touches shared memory:
-// the softmax threads store it as packed bf16 over the first 64 columns of the S buffer they just read, and the PV
-// product takes its A operand from tensor memory.  Q, K and V are single-buffered in shared memory.  O is rescaled in TMEM only when a row maximum grows by more than 2^8 (the
-// running reference maximum may lag; p then stays <= 256, exact for bf16 and fp32 l).
+// Two CTAs of a cluster work on one item after another: (sequence, kv head, block of 64 query tokens), 32 tokens each.  The 4 Q heads
+// of the group are stacked into the 128 rows of a CTA's half of an M=256 tile (row = token*4 + head, the stacking idea of
+// gqa_attention_varlen_causal.py:151-160).  Per 128-token KV tile, cta_group::2, operands split over the pair:
+//     S[256 x 128]  = Q[256 x 256] . K^T          tcgen05.mma, both operands K-major in shared memory, D in TMEM
+//     P = exp2(S*scale*log2e - m)                  a thread per row, TMEM -> TMEM
+//     O[256 x 256] += P[256 x 128] . V[128 x 256]  tcgen05.mma, P from TMEM, V as an MN-major operand, O stays in TMEM
+// Each CTA holds 64 tokens of a K tile and 128 columns of a V tile, so a pair fetches a tile once (one CTA per tile fetched twice as
+// much, 35 bytes a cycle and SM, and had room for one K and one V tile only; now two of each).  Why not more rows per CTA: O and two
+// buffers of S fill the 512 columns of tensor memory.  Roles of the 16 warps:
+//   0-3, 4-7  exponentials of the even and of the odd tiles, a thread per row; the row's reference maximum goes from one to the other
+//             through shared memory.  (Two threads per row of every tile: the exponential units idle while S, the row maximum and the
+//             store of P are waited for, 2950 cycles a tile; now 2430 with another tile's under them.)
+//   8-11      rotate the next item's Q in shared memory, then take O of this one through gate and copy engine to the output
+//   12, 15    issue S and PV (even CTA only), 13 loads K, 14 deals the items and loads Q and V
+// P is stored as packed bf16 over the first 64 columns of the S buffer just read; S of tile j+2 waits for PV of tile j to complete.  O is
+// rescaled in TMEM only when a row maximum grows by more than 2^8 (the running reference maximum may lag; p then stays <= 256, exact
+// for bf16 and fp32 l).
+// Bound: the tensor pipe, 2137 of 2765 cycles a tile; the rest is the completion of PV that S of the buffer waits for.  The chip's power cap
+// comes before it in long runs (1560 MHz).  8 x 4096 tokens with rope and gate: 630 -> 599 us, in bursts 543 -> 506; 64 x 512 without:
+// 380 -> 333; 32 of 16 to 512: 67.3 -> 59.6.  Short prompts are bound by what comes first: loads from HBM by all SMs at once and the fetch of
+// instructions, some 200 cycles for every eight (therefore loops where unrolled code would run once).
 // The reference's rounding points are kept where they matter for the 2e-2 bar: p is rounded to bf16 for the PV
 // product while l sums the fp32 p; scores are scaled in fp32 (the reference pre-scales q and re-rounds it to bf16).
 // Every mbarrier wait is bounded; on expiry the role sets the device error flag and the CTA drains and exits.
@@ -26,21 +32,26 @@
 
 namespace b200 {
 
-constexpr int PU_BQ = 32;
+constexpr int PU_BQ = 32;                           // query tokens per CTA
+constexpr int PU_PAIR_Q = 2 * PU_BQ;
 constexpr int PU_TKV = 128;
-constexpr int PU_SOFTMAX_THREADS = 256;
-constexpr int PU_THREADS = 352;                     // 8 softmax warps + MMA issuer + K producer + V producer
+constexpr int PU_SOFTMAX_WARPS = 8;
+constexpr int PU_OUT_WARPS = 4;
+constexpr int PU_THREADS = 512;
 constexpr int PU_Q_BYTES = 128 * HEAD_DIM * 2;      // 64 KiB: 4 column blocks of [128 rows][64]
-constexpr int PU_KV_BYTES = PU_TKV * HEAD_DIM * 2;  // 64 KiB: 4 column blocks of [128 rows][64]
-constexpr int PU_SMEM = PU_Q_BYTES + 2 * PU_KV_BYTES;  // 192 KiB; tiles need 1024-byte alignment: the kernel checks
-constexpr int PU_OUT_PITCH = HEAD_DIM * 2 + 16;     // staging pitch of the epilogue (bytes)
-static_assert(128 * PU_OUT_PITCH <= PU_Q_BYTES + PU_KV_BYTES, "output staging must fit in the Q + K region");
+constexpr int PU_KV_BYTES = PU_TKV * HEAD_DIM;      // 32 KiB: half a tile, K 64 tokens, V 128 columns
+constexpr int PU_STAGE = 3, PU_STAGE_BYTES = 32 * 64;  // buffers of an output warp: 32 columns of its 32 rows, first the gates, then the output
+constexpr int PU_SMEM = PU_Q_BYTES + 4 * PU_KV_BYTES + PU_OUT_WARPS * PU_STAGE * PU_STAGE_BYTES;
+constexpr int PU_ITEMS = 4;                         // work items in flight per pair
+constexpr int PU_REGS_SOFTMAX = 160, PU_REGS_OUT = 120, PU_REGS_ISSUE = 64;
+constexpr int PU_REGS = 65536 / PU_THREADS;         // what __launch_bounds__ leaves a thread, and ptxas gives (the host checks)
+static_assert(2 * PU_REGS_SOFTMAX + PU_REGS_OUT + PU_REGS_ISSUE <= PU_THREADS / 128 * PU_REGS, "shares of the registers the CTA is launched with");
 constexpr uint32_t PU_TMEM_COLS = 512;              // S0 [0,128) S1 [128,256) (P over their first 64) O [256,512)
 constexpr float PU_TAU = 8.0f;                      // lazy-rescale threshold (log2 domain)
 constexpr float PU_LOG2E = 1.4426950408889634f;
 
 struct PrefillUmmaParams {
-  int num_kv_heads, batch_wide_order;
+  int num_kv_heads, batch, max_seqlen;
   __nv_bfloat16* out;
   int64_t out_t, out_h;
   const int32_t* cu_seqlens;
@@ -130,192 +141,284 @@ rope_scatter_kernel(const __nv_bfloat16* __restrict__ k, int64_t k_t, int64_t k_
 
 
 
+// ---- the pair's ring of work items: what every role of a CTA reads, written by its last warp
+struct PrefillItem {
+  int start, len, q0, h, tiles;  // first packed row and length of the sequence, the pair's first query, kv head, kv tiles (0: no more)
+};
+
 template <bool FUSED>
 __global__ void __launch_bounds__(PU_THREADS, 1)
-varlen_causal_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                          const __grid_constant__ CUtensorMap map_v, const __grid_constant__ PrefillUmmaParams p) {
+prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_gate,
+                    const __grid_constant__ CUtensorMap map_out, const __grid_constant__ PrefillUmmaParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ uint64_t bar_q, bar_qr, bar_k, bar_v, bar_s[2], bar_p[2], bar_pv;
+  // `lead_*`: waited for by the issuer, the even CTA of the pair; the others are each CTA's own
+  __shared__ uint64_t lead_k[2], lead_v[2], lead_q, lead_p[2][2], lead_o, lead_s[2], bar_q, bar_s[2], bar_pv[2], bar_m[4][2][2], bar_g[PU_OUT_WARPS][PU_STAGE], bar_l[PU_ITEMS], item_full[PU_ITEMS], item_free[PU_ITEMS];
   __shared__ uint32_t tmem_slot;
-  __shared__ float xm[2][2][128];  // [tile parity][column half][row]: row maxima (at the end: row sums) exchanged
-                                   // between the two threads of a row
+  __shared__ PrefillItem items[PU_ITEMS];
+  __shared__ float row_ref[2][2][128];                // [tile parity][item parity][row]: the reference of the last tile of that parity
+  __shared__ float row_end[PU_ITEMS][2][2][128];      // [item][tile parity][reference, sum][row]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Two block orders (blocks are scheduled x-fastest).  Batch-wide: grid = (sequences x kv heads, query blocks), so the
-  // whole batch's last (heaviest) query blocks run first, then the ones before them, ... and the one-tile blocks at
-  // the start of every sequence fill the tail: longest-processing-time-first over the launch.  Taken when the K/V of
-  // the whole batch fits the L2 several times over.  Per sequence: grid = (query blocks, kv heads, sequences), heaviest
-  // block of a sequence first; the CTAs that run together then share one or two sequences' K/V tiles in the L2.
-  const bool batch_wide = p.batch_wide_order != 0;
-  const int qb = batch_wide ? gridDim.y - 1 - blockIdx.y : gridDim.x - 1 - blockIdx.x;
-  const int h = batch_wide ? blockIdx.x % p.num_kv_heads : blockIdx.y;
-  const int b = batch_wide ? blockIdx.x / p.num_kv_heads : blockIdx.z;
-  const int seq_start = p.cu_seqlens[b];
-  const int seq_len = p.cu_seqlens[b + 1] - seq_start;
-  const int q0 = qb * PU_BQ;
-  if (q0 >= seq_len) {
-    if (FUSED) pdl_wait();  // every CTA orders the grid after the kernel in front of it
-    return;
-  }
-  const int kv_end = min(q0 + PU_BQ, seq_len);
-  const int n_tiles = (kv_end + PU_TKV - 1) / PU_TKV;
+  const uint32_t rank = cluster_ctarank();
+  uint8_t* q_s = smem_raw;
+  uint8_t* k_s = q_s + PU_Q_BYTES;
+  uint8_t* v_s = k_s + 2 * PU_KV_BYTES;
+  uint8_t* out_s = v_s + 2 * PU_KV_BYTES;
+  const bool aligned = (smem_u32(smem_raw) & 1023u) == 0;  // swizzled tiles need it; always so with __align__(1024)
 
-  uint8_t* smem = smem_raw;
-  if ((smem_u32(smem) & 1023u) != 0) {  // swizzled tiles need 1024-byte alignment; never taken with __align__(1024)
-    if (tid == 0) atomicExch(p.err, 1);
-    return;
-  }
-  uint8_t* q_s = smem;
-  uint8_t* k_s = smem + PU_Q_BYTES;
-  uint8_t* v_s = k_s + PU_KV_BYTES;
-
-  if (warp == 0) tmem_alloc(&tmem_slot, PU_TMEM_COLS);
-  // The loads that wait for nobody leave before the CTA has met: Q and the first V tile (and, where no kernel in front writes
-  // it, the first K tile) travel while tensor memory is allocated and the other barriers are set up.
-  // A one-tile CTA is a chain of such latencies, 8 us: 32 prompts of 16 to 512 tokens 69.2 -> 67.4 us, without rope and gate
-  // 42.2 -> 41.0; long prompts are as they were (627 us for 8 of 4096).
-  if (tid == 9 * 32) {
-    mbar_init(&bar_q, 1);
-    mbar_init(&bar_k, 1);
-    mbar_init(&bar_v, 1);
-    mbar_fence_init();
-    mbar_expect_tx(&bar_q, PU_Q_BYTES);
-    tma_load_5d(q_s, &map_q, 0, 0, h, seq_start + q0, 0, &bar_q);
-    if (!FUSED) {
-      mbar_expect_tx(&bar_k, PU_KV_BYTES);
-      tma_load_4d(k_s, &map_k, 0, seq_start, 0, h, &bar_k);
-    }
-    mbar_expect_tx(&bar_v, PU_KV_BYTES);
-    tma_load_4d(v_s, &map_v, 0, seq_start, 0, h, &bar_v);
-  }
-  // the gate rows are the epilogue's: asked into the L2 now, 128 rows of four lines
-  if (FUSED && tid < PU_SOFTMAX_THREADS) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int line = tid + i * PU_SOFTMAX_THREADS, r = line >> 2, tok = q0 + (r >> 2);
-      if (tok < seq_len)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gate + static_cast<int64_t>(seq_start + tok) * p.gate_t + (h * GROUP + (r & 3)) * HEAD_DIM + (line & 3) * 64));
-    }
-  }
   if (tid == 0) {
-    mbar_init(&bar_qr, 128);
-    mbar_init(&bar_s[0], 1);
-    mbar_init(&bar_s[1], 1);
-    mbar_init(&bar_p[0], PU_SOFTMAX_THREADS);  // one per S/P buffer: a warp may be a tile ahead of another
-    mbar_init(&bar_p[1], PU_SOFTMAX_THREADS);
-    mbar_init(&bar_pv, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&lead_k[i], 1);
+      mbar_init(&lead_v[i], 1);
+      mbar_init(&lead_p[i][0], PU_SOFTMAX_WARPS);
+      mbar_init(&lead_p[i][1], PU_SOFTMAX_WARPS);  // the warps of one parity in both CTAs
+      mbar_init(&bar_s[i], 1);
+      mbar_init(&bar_pv[i], 1);
+    }
+    mbar_init(&lead_q, FUSED ? 2 * PU_OUT_WARPS : 1);
+    mbar_init(&lead_o, 2 * PU_OUT_WARPS);
+    mbar_init(&lead_s[0], 1);
+    mbar_init(&lead_s[1], 1);
+    mbar_init(&bar_q, 1);
+    for (int i = 0; i < 4; ++i) {
+      for (int n = 0; n < 4; ++n) mbar_init(&bar_m[i][n >> 1][n & 1], 1);
+      for (int n = 0; n < PU_STAGE; ++n) mbar_init(&bar_g[i][n], 1);
+    }
+    for (int i = 0; i < PU_ITEMS; ++i) {
+      mbar_init(&bar_l[i], PU_SOFTMAX_WARPS);
+      mbar_init(&item_full[i], 1);
+      mbar_init(&item_free[i], PU_SOFTMAX_WARPS + PU_OUT_WARPS + 1 + (rank == 0 ? 2 : 0));
+    }
     mbar_fence_init();
+  }
+  if (warp == 12) tmem_alloc_pair(&tmem_slot, PU_TMEM_COLS);
+  if (warp == 13 && lane == 0) {
+    prefetch_tensormap(&map_q);
+    prefetch_tensormap(&map_k);
+    prefetch_tensormap(&map_v);
   }
   tc_fence_before_sync();
-  __syncthreads();
+  cluster_sync();  // barriers of both CTAs are set up, tensor memory is there
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
   const uint32_t tmem_o = tmem + 2 * PU_TKV;
+  bool ok = aligned;
 
-  if (warp == 9) {
-    // ------------------------------------------------------------------ TMA producer: the K tiles
-    if (lane == 0) {
-      bool ok = true;
-      // fused form: started while the rope + scatter kernel still runs (programmatic dependent launch).  Everything up
-      // to here - tensor-memory allocation, barriers, the Q tile, and the V tiles of the other producer - overlaps with
-      // it; the rotated K it writes is read only after it has completed.
-      if (FUSED) pdl_wait();
-      for (int j = FUSED ? 0 : 1; j < n_tiles && ok; ++j) {
-        if (j >= 1) ok = mbar_wait_bounded(&bar_s[(j - 1) & 1], ((j - 1) >> 1) & 1);  // S of tile j-1 done: K free
-        if (!ok) break;
-        mbar_expect_tx(&bar_k, PU_KV_BYTES);
-        tma_load_4d(k_s, &map_k, 0, seq_start + j * PU_TKV, 0, h, &bar_k);
-      }
-      if (!ok) atomicExch(p.err, 1);
-    }
-  } else if (warp == 10) {
-    // ------------------------------------------------------------------ TMA producer: the V tiles
-    if (lane == 0) {
-      bool ok = true;
-      for (int j = 1; j < n_tiles && ok; ++j) {
-        ok = mbar_wait_bounded(&bar_pv, (j - 1) & 1);  // PV of tile j-1 done: V free
-        if (!ok) break;
-        mbar_expect_tx(&bar_v, PU_KV_BYTES);
-        tma_load_4d(v_s, &map_v, 0, seq_start + j * PU_TKV, 0, h, &bar_v);
-      }
-      if (!ok) atomicExch(p.err, 1);
-    }
-  } else if (warp == 8) {
-    // ------------------------------------------------------------------ MMA issuer
-    {
-      // the whole warp walks the loop (uniform control flow), lane 0 issues
-      const bool leader = lane == 0;
-      const uint32_t idesc_s = idesc_bf16_f32(128, PU_TKV, false, false);
-      const uint32_t idesc_o = idesc_bf16_f32(128, HEAD_DIM, false, true);
-      const uint32_t q_addr = smem_u32(q_s), k_addr = smem_u32(k_s), v_addr = smem_u32(v_s);
-      bool ok = FUSED ? mbar_wait_bounded(&bar_qr, 0) : mbar_wait_bounded(&bar_q, 0);
-      auto issue_pv = [&](int jj) {
-        ok = ok && mbar_wait_bounded(&bar_p[jj & 1], (jj >> 1) & 1);
-        ok = ok && mbar_wait_bounded(&bar_v, jj & 1);
-        if (!ok) return;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int kt = 0; kt < PU_TKV / 16; ++kt)
-          umma_ts_leader(tmem_o, tmem + (jj & 1) * PU_TKV + kt * 8,  // P: 16 tokens = 8 packed columns per step
-                         smem_desc_sw128(v_addr + kt * 2048, PU_TKV * 128, 1024), idesc_o, (jj > 0) || (kt > 0), leader);
-        umma_commit_leader(&bar_pv, leader);
-      };
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j & 1;
-        ok = mbar_wait_bounded(&bar_k, j & 1);
-        // S(j) overwrites the buffer whose first columns hold P(j-2): the PV product that reads them from tensor
-        // memory must have COMPLETED, issue order alone does not protect an operand in tensor memory
-        if (ok && j >= 2) ok = mbar_wait_bounded(&bar_pv, (j - 2) & 1);
-        if (!ok) break;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int ks = 0; ks < HEAD_DIM / 16; ++ks) {
-          const uint32_t o = (ks >> 2) * (128 * 128) + (ks & 3) * 32;
-          umma_ss_leader(tmem + s * PU_TKV, smem_desc_sw128(q_addr + o, 16, 1024), smem_desc_sw128(k_addr + o, 16, 1024),
-                         idesc_s, ks > 0, leader);
+  // item i of this pair; the whole warp
+  auto release = [&](int i) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&item_free[i & (PU_ITEMS - 1)]);
+  };
+  auto fetch = [&](int i, PrefillItem& it, bool keep = false) {
+    ok = warp_wait_bounded(&item_full[i & (PU_ITEMS - 1)], (i / PU_ITEMS) & 1, ok);
+    it.tiles = 0;
+    if (ok) it = items[i & (PU_ITEMS - 1)];
+    if (!keep) release(i);
+    return ok && it.tiles > 0;
+  };
+
+  if (warp >= 12) {
+    set_registers<PU_REGS_ISSUE, PU_REGS>();
+    PrefillItem it;
+    if (warp == 14) {
+      // ---------------------------------------------------------------- the items; TMA producer: Q, and this CTA's 128 columns of every V tile
+      // Items come longest first and are dealt to the pairs forth and back.  One is made while the one in front of it is loaded.
+      const int pairs = gridDim.x >> 1, me = blockIdx.x >> 1, heads = p.num_kv_heads;
+      const bool one_read = p.batch <= 32;
+      int len = 0;
+      if (one_read && lane < p.batch) len = p.cu_seqlens[lane + 1] - p.cu_seqlens[lane];
+      int level = (p.max_seqlen - 1) / PU_PAIR_Q, chunk = 0;
+      int64_t base = 0;
+      auto make = [&](int i, PrefillItem& to) {
+        const int64_t target = static_cast<int64_t>(i) * pairs + ((i & 1) ? pairs - 1 - me : me);
+        to.tiles = 0;
+        while (level >= 0) {
+          if (!one_read) len = chunk + lane < p.batch ? p.cu_seqlens[chunk + lane + 1] - p.cu_seqlens[chunk + lane] : 0;
+          const uint32_t has = __ballot_sync(0xffffffffu, len > level * PU_PAIR_Q);
+          const int here = __popc(has) * heads;
+          if (target < base + here) {
+            const int at = static_cast<int>(target - base), nth = at / heads;
+            const bool mine = ((has >> lane) & 1) != 0 && __popc(has & ((1u << lane) - 1)) == nth;
+            const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+            to.len = __shfl_sync(0xffffffffu, len, src);
+            to.start = p.cu_seqlens[chunk + src];
+            to.q0 = level * PU_PAIR_Q;
+            to.h = at - nth * heads;
+            to.tiles = (min(to.q0 + PU_PAIR_Q, to.len) + PU_TKV - 1) / PU_TKV;
+            break;
+          }
+          base += here;
+          chunk += 32;
+          if (chunk >= p.batch) {
+            chunk = 0;
+            --level;
+          }
         }
-        umma_commit_leader(&bar_s[s], leader);
-        if (j >= 1) issue_pv(j - 1);
+        if (i >= PU_ITEMS) ok = warp_wait_bounded(&item_free[i & (PU_ITEMS - 1)], (i / PU_ITEMS - 1) & 1, ok);
+        if (ok && lane == 0) {
+          items[i & (PU_ITEMS - 1)] = to;
+          mbar_arrive(&item_full[i & (PU_ITEMS - 1)]);
+        }
+        return ok && to.tiles > 0;
+      };
+      const uint32_t full[2] = {cluster_map(smem_u32(&lead_v[0]), 0), cluster_map(smem_u32(&lead_v[1]), 0)};
+      const uint32_t full_q = cluster_map(smem_u32(&lead_q), 0);
+      const int q_off = static_cast<int>(rank) * PU_BQ;
+      PrefillItem next;
+      bool more = ok && make(0, it);
+      for (int i = 0, g = 0; more; ++i, it = next) {
+        // the last S of the item in front read Q; the V tile of that S was asked for behind PV of two tiles before it, so this
+        // barrier's phase in front of it is over
+        if (g >= 1) ok = warp_wait_bounded(&bar_s[(g - 1) & 1], ((g - 1) >> 1) & 1, ok);
+        if (!ok) break;
+        if (lane == 0) {
+          if (FUSED) {
+            mbar_expect_tx(&bar_q, PU_Q_BYTES);
+            tma_load_5d(q_s, &map_q, 0, 0, it.h, it.start + it.q0 + q_off, 0, &bar_q);
+          } else {
+            if (rank == 0) mbar_expect_tx(&lead_q, 2 * PU_Q_BYTES);
+            tma_load_5d_pair(q_s, &map_q, 0, 0, it.h, it.start + it.q0 + q_off, 0, full_q);
+          }
+        }
+        for (int j = 0; j < it.tiles; ++j, ++g) {
+          const int s = g & 1;
+          if (g >= 2) ok = warp_wait_bounded(&bar_pv[s], ((g >> 1) - 1) & 1, ok);  // PV of tile g-2 done: its V is free
+          if (!ok) break;
+          if (lane == 0) {
+            if (rank == 0) mbar_expect_tx(&lead_v[s], 2 * PU_KV_BYTES);
+            tma_load_4d_pair(v_s + s * PU_KV_BYTES, &map_v, 0, it.start + j * PU_TKV, 2 * static_cast<int>(rank), it.h, full[s]);
+          }
+          if (j == 0) {
+            more = make(i + 1, next);
+            if (more && lane == 0) tma_prefetch_5d(&map_q, 0, 0, next.h, next.start + next.q0 + q_off, 0);
+          }
+        }
       }
-      if (ok) issue_pv(n_tiles - 1);
-      if (!ok && leader) atomicExch(p.err, 1);
+    } else if (warp == 13) {
+      // ---------------------------------------------------------------- TMA producer: this CTA's 64 tokens of every K tile
+      // Fused form: started while the rope + scatter kernel still runs (programmatic dependent launch).  Everything else of the
+      // prologue, Q and V overlap with it; the rotated K it writes is read only after it has completed.
+      if (FUSED) pdl_wait();
+      const uint32_t full[2] = {cluster_map(smem_u32(&lead_k[0]), 0), cluster_map(smem_u32(&lead_k[1]), 0)};
+      for (int i = 0, g = 0; fetch(i, it); ++i) {
+        for (int j = 0; j < it.tiles; ++j, ++g) {
+          const int s = g & 1;
+          if (g >= 2) ok = warp_wait_bounded(&bar_s[s], ((g >> 1) - 1) & 1, ok);  // S of tile g-2 done: its K is free
+          if (!ok) break;
+          if (lane == 0) {
+            if (rank == 0) mbar_expect_tx(&lead_k[s], 2 * PU_KV_BYTES);
+            tma_load_4d_pair(k_s + s * PU_KV_BYTES, &map_k, 0, it.start + j * PU_TKV + static_cast<int>(rank) * (PU_TKV / 2), 0, it.h, full[s]);
+          }
+        }
+      }
+    } else if (warp == 12 && rank == 0) {
+      // ---------------------------------------------------------------- issuer of S for the pair (the whole warp walks, lane 0 issues)
+      const bool leader = lane == 0;
+      const uint32_t idesc_s = idesc_bf16_f32(256, PU_TKV, false, false);
+      const uint32_t q_addr = smem_u32(q_s), k_addr = smem_u32(k_s);
+      for (int i = 0, g = 0; fetch(i, it); ++i) {
+        ok = warp_wait_cluster(&lead_q, i & 1, ok);
+        for (int j = 0; j < it.tiles; ++j, ++g) {
+          const int s = g & 1;
+          ok = ok && mbar_wait_bounded(&lead_k[s], (g >> 1) & 1);
+          // S(g) overwrites the buffer whose first columns hold P(g-2): the PV product that reads them from tensor
+          // memory must have COMPLETED, issue order alone does not protect an operand in tensor memory
+          if (g >= 2) ok = ok && mbar_wait_bounded(&bar_pv[s], ((g >> 1) - 1) & 1);
+          if (!ok) break;
+          tc_fence_after_sync();
+#pragma unroll
+          for (int ks = 0; ks < HEAD_DIM / 16; ++ks)
+            umma_ss_pair(tmem + s * PU_TKV, smem_desc_sw128(q_addr + (ks >> 2) * (128 * 128) + (ks & 3) * 32, 16, 1024),
+                         smem_desc_sw128(k_addr + s * PU_KV_BYTES + (ks >> 2) * (PU_TKV / 2 * 128) + (ks & 3) * 32, 16, 1024), idesc_s, ks > 0,
+                         leader);
+          umma_commit_pair(&bar_s[s], leader);
+          if (leader) mbar_arrive(&lead_s[s]);
+        }
+      }
+    } else if (rank == 0) {
+      // ---------------------------------------------------------------- issuer of PV for the pair
+      // Inside an item S of the tile behind goes into the pipe first: PV has its operand later anyway, and free to overtake one another
+      // the two issuers end in two tiles' S, then both PV (3025 cycles a tile of 4096-token prompts, 2765 in this order).  From one item to the next
+      // nobody waits: the next S may need a Q that is still on its way.
+      const bool leader = lane == 0;
+      const uint32_t idesc_o = idesc_bf16_f32(256, HEAD_DIM, false, true);
+      const uint32_t v_addr = smem_u32(v_s);
+      for (int i = 0, g = 0; fetch(i, it); ++i) {
+        for (int j = 0; j < it.tiles; ++j, ++g) {
+          const int s = g & 1;
+          ok = ok && mbar_wait_bounded(&lead_s[s], (g >> 1) & 1);
+          if (j + 1 < it.tiles) ok = ok && mbar_wait_bounded(&lead_s[s ^ 1], ((g + 1) >> 1) & 1);
+          ok = ok && mbar_wait_bounded(&lead_v[s], (g >> 1) & 1);
+          if (j == 0 && i > 0) ok = ok && mbar_wait_bounded(&lead_o, (i - 1) & 1);  // O of the item in front has been read
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {  // the second 64 tokens' exponentials are computed under the first 64's product
+            ok = ok && mbar_wait_bounded(&lead_p[s][half], (g >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int kt = half * 4; kt < half * 4 + 4; ++kt)
+              umma_ts_pair(tmem_o, tmem + s * PU_TKV + kt * 8,  // P: 16 tokens = 8 packed columns per step
+                           smem_desc_sw128(v_addr + s * PU_KV_BYTES + kt * 2048, PU_TKV * 128, 1024), idesc_o, j > 0 || kt > 0, leader);
+          }
+          if (!ok) break;
+          umma_commit_pair(&bar_pv[s], leader);
+        }
+      }
     }
-  } else {
-    // ------------------------------------------------------------------ softmax + epilogue
-    const int row = 32 * (warp & 3) + lane;    // TMEM lane; row = token*4 + head
-    const int half = warp >> 2;                // this thread's 64 of the tile's 128 columns
-    const int q_tok = q0 + (row >> 2);
-    const uint32_t lane_base = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-    const int pair_bar = 1 + (warp & 3);       // named barrier of the two warps that share these rows
-    float m_ref = -INFINITY, l_run = 0.f;
-    bool ok = true;
-    if (FUSED && half == 0) {
+    if (!ok) {
+      if (lane == 0) atomicExch(p.err, 1);
+      // copies in flight signal barriers that may be the other CTA's: give them their time before the shared memory goes away
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 100000) __nanosleep(1000);
+    }
+  } else if (warp >= 8) {
+    // ------------------------------------------------------------------ rope of the next item's Q, output of this one
+    set_registers<PU_REGS_OUT, PU_REGS>();
+    
+    const int row = tid - 8 * 32;              // TMEM lane; row = token*4 + head
+    const uint32_t lane_base = static_cast<uint32_t>(row & ~31) << 16;
+    const uint32_t ready_q = cluster_map(smem_u32(&lead_q), 0), read_o = cluster_map(smem_u32(&lead_o), 0);
+    uint8_t* stage = out_s + (warp - 8) * (PU_STAGE * PU_STAGE_BYTES);  // of [32 rows][32 columns], 64-byte swizzle
+    auto rope = [&](const PrefillItem& it, int i) {
       // rotary embedding of this row's q in place (dims [0,32) and [32,64) live in column block 0, chunks c, c+4)
-      const int64_t t = seq_start + min(q_tok, seq_len - 1);
+      const int q_tok = it.q0 + static_cast<int>(rank) * PU_BQ + (row >> 2);
+      const int64_t t = it.start + min(q_tok, it.len - 1);
       const int64_t pid = p.ids_are_int64 ? static_cast<const int64_t*>(p.position_ids)[t]
                                           : static_cast<int64_t>(static_cast<const int32_t*>(p.position_ids)[t]);
       const float posf = static_cast<float>(pid);
       // the four rows of a token share their angles: each lane of a quad computes 8 of the 32 (sin, cos) pairs
-      float sn[8], cs[8];
+      // the gate row is the output's: asked into the L2 now
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sincosf(posf * p.inv_freq[(lane & 3) * 8 + i], &sn[i], &cs[i]);
-      ok = mbar_wait_bounded(&bar_q, 0);
+      for (int n = 0; n < 4; ++n)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gate + t * p.gate_t + (it.h * GROUP + (row & 3)) * HEAD_DIM + n * 64));
+      // (sin, cos) of the warp's eight tokens, one frequency per lane, while Q travels; in loops: code that runs once per item is
+      // fetched as slowly as it is long
+      const float freq = p.inv_freq[lane];
+      float2* angles = reinterpret_cast<float2*>(stage);  // [8 tokens][32]
+#pragma unroll 1
+      for (int n = 0; n < 8; ++n) {
+        float2 sc;
+        sincosf(__shfl_sync(0xffffffffu, posf, n * 4) * freq, &sc.x, &sc.y);
+        angles[n * 32 + lane] = sc;
+      }
+      __syncwarp();
+      ok = warp_wait_bounded(&bar_q, i & 1, ok);
+      if (!ok) return;
       uint8_t* qrow = q_s + row * 128;
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < 4; ++c) {  // chunk c holds dims [8c, 8c+8), chunk c+4 their partners [32+8c, 40+8c)
         uint4* pa = reinterpret_cast<uint4*>(qrow + ((c ^ (row & 7)) << 4));
         uint4* pb = reinterpret_cast<uint4*>(qrow + (((c + 4) ^ (row & 7)) << 4));
         const uint4 va = *pa, vb = *pb;
         uint32_t wa[4] = {va.x, va.y, va.z, va.w}, wb[4] = {vb.x, vb.y, vb.z, vb.w};
+        const float4* at = reinterpret_cast<const float4*>(angles + (lane >> 2) * 32 + c * 8);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          // angle index 8c + 2k (+1) lives in lane (quad base + c), register 2k (+1)
-          const int src = (lane & ~3) + c;
-          const float c0 = __shfl_sync(0xffffffffu, cs[2 * k], src), s0 = __shfl_sync(0xffffffffu, sn[2 * k], src);
-          const float c1 = __shfl_sync(0xffffffffu, cs[2 * k + 1], src), s1 = __shfl_sync(0xffffffffu, sn[2 * k + 1], src);
+          const float4 sc = at[k];  // sin, cos of angle 8c + 2k and of the next
           float f0, g0, f1, g1;
-          rope_pair(bf16_lo(wa[k]), bf16_lo(wb[k]), s0, c0, f0, g0);
-          rope_pair(bf16_hi(wa[k]), bf16_hi(wb[k]), s1, c1, f1, g1);
+          rope_pair(bf16_lo(wa[k]), bf16_lo(wb[k]), sc.x, sc.y, f0, g0);
+          rope_pair(bf16_hi(wa[k]), bf16_hi(wb[k]), sc.z, sc.w, f1, g1);
           wa[k] = pack_bf16(f0, f1);
           wb[k] = pack_bf16(g0, g1);
         }
@@ -323,163 +426,229 @@ varlen_causal_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         *pb = make_uint4(wb[0], wb[1], wb[2], wb[3]);
       }
       fence_proxy_async();  // the rotated rows must be visible to the tensor core's reads
-      mbar_arrive(&bar_qr);
-    }
-    // A failed (timed-out) wait clears `ok`; the loop then keeps only its barriers and arrivals, so that the partner
-    // warp and the MMA issuer are never left waiting for this thread.
-    for (int j = 0; j < n_tiles; ++j) {
-      const int s = j & 1;
-      if (ok) ok = mbar_wait_bounded(&bar_s[s], (j >> 1) & 1);
-      uint32_t r0[32], r1[32];
-      float m_half = 0.f;
-      if (ok) {
-        tc_fence_after_sync();
-        tmem_ld32(tmem + lane_base + s * PU_TKV + half * 64, r0);
-        tmem_ld32(tmem + lane_base + s * PU_TKV + half * 64 + 32, r1);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster_plain(ready_q);
+    };
+    PrefillItem it, next;
+    bool more = fetch(0, it, true);
+    if (FUSED && more) rope(it, 0);
+    for (int i = 0, g = 0, n = 0; more; ++i, it = next) {  // n: 32-column pieces so far
+      g += it.tiles;
+      more = fetch(i + 1, next, true);
+      if (lane == 0) bulk_wait_read();  // the buffers of the item in front
+      __syncwarp();
+      if (FUSED && more) rope(next, i + 1);
+      const int q_tok0 = it.q0 + static_cast<int>(rank) * PU_BQ + (warp - 8) * 8, tok0 = it.start + q_tok0;
+      const bool whole = q_tok0 + 8 <= it.len;  // eight tokens of the sequence: a tile for the copy engine; else row by row
+      auto load_gate = [&](int c) {
+        uint64_t* bar = &bar_g[warp - 8][(n + c) % PU_STAGE];
+        mbar_expect_tx(bar, PU_STAGE_BYTES);
+        tma_load_5d(stage + (n + c) % PU_STAGE * PU_STAGE_BYTES, &map_gate, 0, 0, it.h, tok0, c, bar);
+      };
+      if (FUSED && lane == 0) {
+        load_gate(0);
+        load_gate(1);
+      }
+      const int slot = i & (PU_ITEMS - 1);
+      ok = warp_wait_bounded(&bar_l[slot], (i / PU_ITEMS) & 1, ok);
+      // bar_l is behind S of the item's last tile, S behind PV of two tiles before it: the phase in front of this one is over
+      ok = warp_wait_bounded(&bar_pv[(g - 1) & 1], ((g - 1) >> 1) & 1, ok);
+      tc_fence_after_sync();
+      // even and odd tiles summed against references of their own; O stands at the larger, the last tile's
+      const float m0 = row_end[slot][0][0][row], m1 = row_end[slot][1][0][row], m = fmaxf(m0, m1);
+      const float inv_l = 1.f / (row_end[slot][0][1][row] * ex2_fast(m0 - m) + row_end[slot][1][1][row] * ex2_fast(m1 - m));
+      // o sigmoid(g) = o/2 tanh(g/2) + o/2
+      const uint64_t inv2 = FUSED ? f32x2(0.5f * inv_l, 0.5f * inv_l) : f32x2(inv_l, inv_l);
+      const __nv_bfloat162 half = __floats2bfloat162_rn(0.5f, 0.5f);
+#pragma unroll 1
+      for (int c = 0; c < HEAD_DIM / 32 && ok; ++c) {
+        uint8_t* buf = stage + (n + c) % PU_STAGE * PU_STAGE_BYTES;
+        uint4* mine = reinterpret_cast<uint4*>(buf + lane * 64);  // chunk k of this row at k ^ (row / 2 % 4)
+        uint32_t o[32];
+        tmem_ld32(tmem_o + lane_base + c * 32, o);
+        if (FUSED) {
+          ok = warp_wait_bounded(&bar_g[warp - 8][(n + c) % PU_STAGE], ((n + c) / PU_STAGE) & 1, ok);
+        } else {
+          if (lane == 0) bulk_wait_read_but<PU_STAGE - 1>();
+          __syncwarp();
+        }
         tmem_ld_wait();
-        // mask (causal and inside the sequence; only tiles on the diagonal or at the sequence end need it) and take
-        // the row maximum of the raw scores; the scale (> 0) is folded into the exponent below
-        const int lim = min(q_tok, seq_len - 1) - j * PU_TKV - half * 64;  // last valid column of this half
-        if (lim < 63) {
+        if (c == HEAD_DIM / 32 - 1) {  // O is read: the next item's first product may overwrite it
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_plain(read_o);
+        }
+        uint4 v[4];
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            if (c > lim) r0[c] = 0xff800000u;       // -inf
-            if (c + 32 > lim) r1[c] = 0xff800000u;
+        for (int k = 0; k < 4; ++k) {
+          uint32_t gs[4] = {}, w[4];
+          if (FUSED) {
+            const uint4 gv = mine[k ^ ((lane >> 1) & 3)];
+            gs[0] = gv.x; gs[1] = gv.y; gs[2] = gv.z; gs[3] = gv.w;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint64_t x = f32x2_mul(f32x2(o[k * 8 + e * 2], o[k * 8 + e * 2 + 1]), inv2);
+            if (FUSED) {
+              const __nv_bfloat162 h2 = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&gs[e]), half);
+              const uint32_t hw = *reinterpret_cast<const uint32_t*>(&h2);
+              x = f32x2_fma(x, f32x2(tanh_fast(bf16_lo(hw)), tanh_fast(bf16_hi(hw))), x);
+            }
+            w[e] = pack_bf16x2(x);
+          }
+          v[k] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        if (whole) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mine[k ^ ((lane >> 1) & 3)] = v[k];
+          fence_proxy_async();
+        } else if (q_tok0 + (lane >> 2) < it.len) {
+          __nv_bfloat16* out = p.out + static_cast<int64_t>(tok0 + (lane >> 2)) * p.out_t + (it.h * GROUP + (lane & 3)) * p.out_h + c * 32;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(out)[k] = v[k];
+        }
+        __syncwarp();
+        if (lane == 0) {
+          if (whole) tma_store_5d(&map_out, 0, 0, it.h, tok0, c, buf);
+          if (FUSED && c + 2 < HEAD_DIM / 32) {
+            bulk_wait_read_but<1>();  // the piece in front has left the buffer that the one after the next comes to
+            load_gate(c + 2);
           }
         }
-        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          mx0 = fmaxf(mx0, __uint_as_float(r0[c]));
-          mx1 = fmaxf(mx1, __uint_as_float(r0[c + 1]));
-          mx2 = fmaxf(mx2, __uint_as_float(r1[c]));
-          mx3 = fmaxf(mx3, __uint_as_float(r1[c + 1]));
-        }
-        m_half = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
       }
-      xm[s][half][row] = m_half;
-      named_barrier(pair_bar, 64);
-      // after this barrier both threads of the row hold their scores in registers: the S buffer may take P
-      if (ok) {
-        const float m_tile = fmaxf(m_half, xm[s][half ^ 1][row]) * p.scale_log2;
-        const float m_new = fmaxf(m_ref, m_tile);  // both threads of a row compute the same value
-        if (j == 0) {
-          m_ref = m_new;
-        } else {
-          const bool need = (m_new - m_ref) > PU_TAU;
-          if (__any_sync(__activemask(), need)) {
-            // O must be at rest before it is rescaled: wait for the PV product of tile j-1
-            ok = mbar_wait_bounded(&bar_pv, (j - 1) & 1);
-            tc_fence_after_sync();
-            const float alpha = need ? ex2_fast(m_ref - m_new) : 1.f;
+      if (!ok) break;
+      n += HEAD_DIM / 32;
+      // only now: the item's place in the ring is also that of its sums
+      release(i);
+    }
+    if (lane == 0) bulk_wait_read();
+    if (!ok && lane == 0) {
+      atomicExch(p.err, 1);
+      for (int i = 0; i < PU_STAGE; ++i) mbar_wait_bounded(&bar_g[warp - 8][i], 0, 1u << 12);  // gates in flight
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax
+    set_registers<PU_REGS_SOFTMAX, PU_REGS>();
+    // Warps 0-3 take the even tiles of the pair's stream, warps 4-7 the odd ones, one thread per row: while one of the two warps of a
+    // scheduler waits for its scores, its row's reference or the store of P, the other has its exponentials computed.
+    const int quarter = warp & 3, par = warp >> 2;
+    const int row = 32 * quarter + lane;       // TMEM lane; row = token*4 + head
+    const uint32_t lane_base = static_cast<uint32_t>(32 * quarter) << 16;
+    const uint32_t tmem_s = tmem + lane_base + par * PU_TKV;
+    const uint32_t ready_p = cluster_map(smem_u32(&lead_p[par][0]), 0);
+    const float scale = p.scale_log2;
+    uint32_t refs[2] = {0, 0};                 // references taken over from the other warp so far, in even and odd items
+    PrefillItem it;
+    for (int i = 0, g0 = 0; fetch(i, it); ++i) {
+      const int q_last = min(it.q0 + static_cast<int>(rank) * PU_BQ + (row >> 2), it.len - 1);
+      float m_ref = -INFINITY, l_run = 0.f;
+      for (int j = (g0 ^ par) & 1; j < it.tiles; j += 2) {
+        const int g = g0 + j;
+        ok = warp_wait_bounded(&bar_s[par], (g >> 1) & 1, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
+        // causal and inside the sequence; only tiles on the diagonal or at the sequence end have columns to mask
+        const int lim = q_last - j * PU_TKV;   // last valid column
+        const bool edge = __any_sync(0xffffffffu, lim < PU_TKV - 1);
+        // the row maximum of the raw scores; the scale (> 0) is folded into the exponent below
+        float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll 1
-            for (int c0 = 0; c0 < HEAD_DIM / 2; c0 += 32) {  // this thread's 128 columns of O
+        for (int c0 = 0; c0 < PU_TKV; c0 += 64) {
+          uint32_t r[2][32];
+          tmem_ld32(tmem_s + c0, r[0]);
+          tmem_ld32(tmem_s + c0 + 32, r[1]);
+          tmem_ld_wait();
+          if (edge) {  // back into tensor memory, where the second pass finds it
+#pragma unroll
+            for (int c = 0; c < 64; ++c)
+              if (c0 + c > lim) r[c >> 5][c & 31] = 0xff800000u;  // -inf
+            tmem_st32(tmem_s + c0, r[0]);
+            tmem_st32(tmem_s + c0 + 32, r[1]);
+          }
+#pragma unroll
+          for (int c = 0; c < 32; c += 2) {
+            mx0 = fmaxf(mx0, fmaxf(__uint_as_float(r[0][c]), __uint_as_float(r[0][c + 1])));
+            mx1 = fmaxf(mx1, fmaxf(__uint_as_float(r[1][c]), __uint_as_float(r[1][c + 1])));
+          }
+        }
+        if (edge) tmem_st_wait();
+        const float m_tile = fmaxf(mx0, mx1) * scale;
+        float m_use = m_tile;
+        if (j > 0) {
+          ok = warp_wait_bounded(&bar_m[quarter][par ^ 1][i & 1], ((i & 1) ? refs[1]++ : refs[0]++) & 1, ok);
+          if (!ok) break;
+          const float m_prev = row_ref[par ^ 1][i & 1][row], m_new = fmaxf(m_prev, m_tile);
+          const bool need = m_new - m_prev > PU_TAU;
+          m_use = need ? m_new : m_prev;
+          if (j + 1 < it.tiles) {
+            row_ref[par][i & 1][row] = m_use;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_m[quarter][par][i & 1]);
+          }
+          if (__any_sync(0xffffffffu, need)) {
+            // O must be at rest before it is rescaled: wait for the PV product of the tile in front
+            ok = warp_wait_bounded(&bar_pv[par ^ 1], ((g - 1) >> 1) & 1, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const float alpha = need ? ex2_fast(m_prev - m_new) : 1.f;
+#pragma unroll 1
+            for (int c0 = 0; c0 < HEAD_DIM; c0 += 32) {
               uint32_t o[32];
-              tmem_ld32(tmem_o + lane_base + half * (HEAD_DIM / 2) + c0, o);
+              tmem_ld32(tmem_o + lane_base + c0, o);
               tmem_ld_wait();
 #pragma unroll
               for (int c = 0; c < 32; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * alpha);
-              tmem_st32(tmem_o + lane_base + half * (HEAD_DIM / 2) + c0, o);
+              tmem_st32(tmem_o + lane_base + c0, o);
             }
-            tmem_st_wait();
-            l_run *= alpha;
-            if (need) m_ref = m_new;
           }
+        } else if (it.tiles > 1) {
+          row_ref[par][i & 1][row] = m_use;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_m[quarter][par][i & 1]);
         }
-        // p = 2^(s*scale - m_ref): fp32 for l, bf16 for the PV product, stored as this thread's 32 packed columns of
-        // the P tile (tokens 2c, 2c+1 in column c) over the S buffer
-        float sum0 = 0.f, sum1 = 0.f;
-        const float neg_m = -m_ref, sc = p.scale_log2;
-        uint32_t w[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const float x0 = ex2_fast(fmaf(__uint_as_float(c < 16 ? r0[2 * c] : r1[2 * c - 32]), sc, neg_m));
-          const float x1 = ex2_fast(fmaf(__uint_as_float(c < 16 ? r0[2 * c + 1] : r1[2 * c - 31]), sc, neg_m));
-          sum0 += x0;
-          sum1 += x1;
-          w[c] = pack_bf16(x0, x1);
-        }
-        l_run += sum0 + sum1;
-        tmem_st32(tmem + lane_base + s * PU_TKV + half * 32, w);
-        tmem_st_wait();
-      }
-      tc_fence_before_sync();   // this thread's TMEM loads/stores before the arrive
-      mbar_arrive(&bar_p[s]);
-    }
-    // ---- epilogue: O / l -> bf16 -> staged in shared memory (Q and K are dead) -> coalesced global stores
-    // A parity wait only tells the two most recent phases apart, and this thread may not have seen the PV product of
-    // tile n-2 complete yet: wait for it first, then for the last one.
-    if (ok && n_tiles >= 2) ok = mbar_wait_bounded(&bar_pv, (n_tiles - 2) & 1);
-    if (ok) ok = mbar_wait_bounded(&bar_pv, (n_tiles - 1) & 1);
-    float* xl = &xm[n_tiles & 1][0][0];  // the parity slot the last tile did not use
-    xl[half * 128 + row] = l_run;
-    named_barrier(pair_bar, 64);
-    if (ok) {
-      tc_fence_after_sync();
-      const float inv_l = 1.f / (l_run + xl[(half ^ 1) * 128 + row]);
-      uint8_t* orow = smem + row * PU_OUT_PITCH + half * HEAD_DIM;  // this half's 128 columns = 256 bytes
+        l_run *= ex2_fast(m_ref - m_use);      // this parity's sum so far, against the reference of its last tile
+        m_ref = m_use;
+        // p = 2^(s*scale - m_ref): fp32 for l, bf16 for the PV product, stored as packed columns of the P tile (tokens 2c, 2c+1 in
+        // column c) over the columns of S that have been read
+        const uint64_t sc2 = f32x2(scale, scale), neg2 = f32x2(-m_use, -m_use);
+        uint64_t sum0 = 0, sum1 = 0;
 #pragma unroll 1
-      for (int c0 = 0; c0 < HEAD_DIM / 2; c0 += 64) {
-        uint32_t o[2][32];                         // two loads in flight
-        tmem_ld32(tmem_o + lane_base + half * (HEAD_DIM / 2) + c0, o[0]);
-        tmem_ld32(tmem_o + lane_base + half * (HEAD_DIM / 2) + c0 + 32, o[1]);
-        tmem_ld_wait();
+        for (int c0 = 0; c0 < PU_TKV; c0 += 64) {
+          uint32_t r[2][32];
+          tmem_ld32(tmem_s + c0, r[0]);
+          tmem_ld32(tmem_s + c0 + 32, r[1]);
+          tmem_ld_wait();
+          uint32_t w[32];
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const uint32_t(&x)[32] = o[g >> 2];
-          uint32_t w[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            w[k] = pack_bf16(__uint_as_float(x[(g & 3) * 8 + k * 2]) * inv_l, __uint_as_float(x[(g & 3) * 8 + k * 2 + 1]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + (c0 + g * 8) * 2) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-      }
-    } else {
-      atomicExch(p.err, 1);
-    }
-    named_barrier(9, PU_SOFTMAX_THREADS);  // the eight softmax warps only
-    if (ok) {
-      // 128 rows x 32 sixteen-byte chunks; a warp covers one 512-byte row per step.  The gate rows are fetched
-      // eight steps at a time so that their latency is paid once per batch, not once per chunk.
-      constexpr int STEPS = 128 * (HEAD_DIM / 8) / PU_SOFTMAX_THREADS;  // 16 iterations of 256 threads
-#pragma unroll 1
-      for (int i0 = 0; i0 < STEPS; i0 += 8) {
-        uint4 gv[8];
-        if (FUSED) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int i = (i0 + u) * PU_SOFTMAX_THREADS + tid, r = i >> 5, ch = i & 31;
-            const int tok = min(q0 + (r >> 2), seq_len - 1);
-            gv[u] = *reinterpret_cast<const uint4*>(p.gate + static_cast<int64_t>(seq_start + tok) * p.gate_t +
-                                                    (h * GROUP + (r & 3)) * HEAD_DIM + ch * 8);
+          for (int c = 0; c < 32; ++c) {
+            const uint64_t x = f32x2_fma(f32x2(r[c >> 4][(2 * c) & 31], r[c >> 4][(2 * c + 1) & 31]), sc2, neg2);
+            const uint64_t e = f32x2(ex2_fast(f32x2_lo(x)), ex2_fast(f32x2_hi(x)));
+            if (c & 1) sum1 = f32x2_add(sum1, e);
+            else sum0 = f32x2_add(sum0, e);
+            w[c] = pack_bf16x2(e);
           }
+          tmem_st32(tmem_s + (c0 >> 1), w);
+          tmem_st_wait();
+          tc_fence_before_sync();              // this warp's TMEM loads/stores before the arrive
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_plain(ready_p + (c0 >> 6) * 8);
         }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int i = (i0 + u) * PU_SOFTMAX_THREADS + tid, r = i >> 5, ch = i & 31;
-          const int tok = q0 + (r >> 2);
-          if (tok < seq_len) {
-            uint4 v = *reinterpret_cast<const uint4*>(smem + r * PU_OUT_PITCH + ch * 16);
-            if (FUSED) {
-              uint32_t xs[4] = {v.x, v.y, v.z, v.w};
-              const uint32_t gs[4] = {gv[u].x, gv[u].y, gv[u].z, gv[u].w};
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                xs[k] = pack_bf16(bf16_lo(xs[k]) * sigmoid_fast(bf16_lo(gs[k])),
-                                  bf16_hi(xs[k]) * sigmoid_fast(bf16_hi(gs[k])));
-              }
-              v = make_uint4(xs[0], xs[1], xs[2], xs[3]);
-            }
-            *reinterpret_cast<uint4*>(p.out + static_cast<int64_t>(seq_start + tok) * p.out_t +
-                                      (h * GROUP + (r & 3)) * p.out_h + ch * 8) = v;
-          }
-        }
+        sum0 = f32x2_add(sum0, sum1);
+        l_run += f32x2_lo(sum0) + f32x2_hi(sum0);
       }
+      if (!ok) break;
+      g0 += it.tiles;
+      const int slot = i & (PU_ITEMS - 1);
+      row_end[slot][par][0][row] = m_ref;
+      row_end[slot][par][1][row] = l_run;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_l[slot]);
     }
+    if (!ok && lane == 0) atomicExch(p.err, 1);
   }
   tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, PU_TMEM_COLS);
+  cluster_sync();  // nobody reads or signals the other CTA any more
+  if (warp == 12) tmem_dealloc_pair(tmem, PU_TMEM_COLS);
 }
 
 }  // namespace b200
@@ -494,7 +663,7 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
                                int64_t k_stride_h, const void* v, int64_t v_stride_t, int64_t v_stride_h,
                                PrefillUmmaParams p, int batch, int total_tokens, int max_seqlen, int num_kv_heads,
                                cudaStream_t stream, const char* what) {
-  CUtensorMap map_q, map_k, map_v;
+  CUtensorMap map_q, map_k, map_v, map_gate = {}, map_out;
   const uint64_t T = static_cast<uint64_t>(total_tokens), H = static_cast<uint64_t>(num_kv_heads);
   {
     // q as {64 cols, 4 heads of a group, groups, tokens, 4 column blocks}; one load = 32 tokens of one group
@@ -506,21 +675,33 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
       return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of q", what);
   }
   {
-    // k, v as {64 cols, tokens, 4 column blocks, kv heads}; one load = 64 tokens of one head
+    // k, v as {64 cols, tokens, 4 column blocks, kv heads}; one load = 64 tokens, or 128 columns of 128 tokens, of one head
     const uint64_t dims[4] = {64, T, HEAD_DIM / 64, H};
-    const uint32_t box[4] = {64, PU_TKV, HEAD_DIM / 64, 1};
+    const uint32_t kbox[4] = {64, PU_TKV / 2, HEAD_DIM / 64, 1}, vbox[4] = {64, PU_TKV, HEAD_DIM / 128, 1};
     const uint64_t ks[3] = {static_cast<uint64_t>(k_stride_t) * 2, 128, static_cast<uint64_t>(k_stride_h) * 2};
     const uint64_t vs[3] = {static_cast<uint64_t>(v_stride_t) * 2, 128, static_cast<uint64_t>(v_stride_h) * 2};
-    if (!encode_map_bf16_sw128(&map_k, k, 4, dims, ks, box) || !encode_map_bf16_sw128(&map_v, v, 4, dims, vs, box))
+    if (!encode_map_bf16_sw128(&map_k, k, 4, dims, ks, kbox) || !encode_map_bf16_sw128(&map_v, v, 4, dims, vs, vbox))
       return fail(ERR_RUNTIME, "%s: cannot encode the tensor maps of k / v", what);
+  }
+  {
+    // gates and output as {32 cols, 4 heads of a group, groups, tokens, 8 column blocks}; one copy = 8 tokens of one group
+    const uint64_t dims[5] = {32, GROUP, H, T, HEAD_DIM / 32};
+    const uint64_t gs[4] = {HEAD_DIM * 2, HEAD_DIM * 2 * GROUP, static_cast<uint64_t>(p.gate_t) * 2, 64};
+    const uint64_t os[4] = {static_cast<uint64_t>(p.out_h) * 2, static_cast<uint64_t>(p.out_h) * 2 * GROUP, static_cast<uint64_t>(p.out_t) * 2, 64};
+    const uint32_t box[5] = {32, GROUP, 1, 8, 1};
+    if ((FUSED && !encode_map_bf16_sw64(&map_gate, p.gate, 5, dims, gs, box)) || !encode_map_bf16_sw64(&map_out, p.out, 5, dims, os, box))
+      return fail(ERR_RUNTIME, "%s: cannot encode the tensor maps of gate / out", what);
   }
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(varlen_causal_umma_kernel<FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PU_SMEM) !=
+    if (cudaFuncSetAttribute(prefill_pair_kernel<FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PU_SMEM) !=
         cudaSuccess)
       return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, PU_SMEM);
+    cudaFuncAttributes attr;  // its warpgroups exchange registers: with fewer at the launch than they share out they would wait for good
+    if (cudaFuncGetAttributes(&attr, prefill_pair_kernel<FUSED>) != cudaSuccess || attr.numRegs != PU_REGS)
+      return fail(ERR_RUNTIME, "%s: the kernel was not built with %d registers per thread", what, PU_REGS);
     configured[dev] = true;
   }
   p.err = wait_timeout_flag();
@@ -529,14 +710,14 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
   B200_REQUIRE((max_seqlen + PU_BQ - 1) / PU_BQ <= 65535 && batch <= 65535 && num_kv_heads <= 65535,
                "%s: max_seqlen must be at most %d, batch and heads at most 65535 (got %d, %d, %d)", what, 65535 * PU_BQ,
                max_seqlen, batch, num_kv_heads);
-  const int q_blocks = (max_seqlen + PU_BQ - 1) / PU_BQ;
-  // K and V of the batch (bf16): below a quarter of the 126 MB L2 every running CTA finds its tiles there whatever the order
-  p.batch_wide_order = static_cast<int64_t>(total_tokens) * num_kv_heads * HEAD_DIM * 4 <= (32ll << 20) ? 1 : 0;
   p.num_kv_heads = num_kv_heads;
-  const dim3 grid = p.batch_wide_order ? dim3(static_cast<unsigned>(num_kv_heads) * batch, q_blocks, 1)
-                                       : dim3(q_blocks, num_kv_heads, batch);
+  p.batch = batch;
+  p.max_seqlen = max_seqlen;
+  const int64_t most = static_cast<int64_t>((max_seqlen + PU_PAIR_Q - 1) / PU_PAIR_Q) * num_kv_heads * batch;
+  const int sms = sm_count(), pairs = static_cast<int>(most < sms / 2 ? most : sms / 2);
   // the fused form starts behind its own rope + scatter kernel while that one still runs (see the K producer)
-  if (launch_pdl(FUSED, varlen_causal_umma_kernel<FUSED>, grid, dim3(PU_THREADS), PU_SMEM, stream, map_q, map_k, map_v, p) !=
+  if (launch_pdl_cluster(FUSED, 2, prefill_pair_kernel<FUSED>, dim3(2 * pairs), dim3(PU_THREADS), PU_SMEM, stream, map_q, map_k, map_v, map_gate,
+                         map_out, p) !=
       cudaSuccess)
     return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
   return check_launch(what);

@@ -1,10 +1,10 @@
-// Host side of the tensor-map TMA loads: encoders over row-major bf16 data with the 128-byte swizzle (umma.cuh).
+// Host side of the tensor-map TMA loads: encoders over row-major bf16 data with the 128- or 64-byte swizzle (umma.cuh).
 #include "umma.cuh"
 
 namespace b200 {
 
-bool encode_map_bf16_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                           const uint64_t* strides_bytes, const uint32_t* box) {
+static bool encode_map_bf16(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                            const uint32_t* box, CUtensorMapSwizzle swizzle, uint64_t inner) {
   typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -19,7 +19,7 @@ bool encode_map_bf16_sw128(CUtensorMap* map, const void* base, int rank, const u
     }
     encode = reinterpret_cast<EncodeFn>(fn);
   }
-  if (rank < 3 || rank > 5 || dims[0] != 64 || box[0] != 64 || (reinterpret_cast<uintptr_t>(base) & 15) != 0) return false;
+  if (rank < 3 || rank > 5 || dims[0] != inner || box[0] != inner || (reinterpret_cast<uintptr_t>(base) & 15) != 0) return false;
   cuuint64_t d[5], st[4];
   cuuint32_t bx[5], es[5];
   for (int i = 0; i < rank; ++i) {
@@ -32,8 +32,18 @@ bool encode_map_bf16_sw128(CUtensorMap* map, const void* base, int rank, const u
     }
   }
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(base), d, st, bx,
-                es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool encode_map_bf16_sw128(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
+                           const uint64_t* strides_bytes, const uint32_t* box) {
+  return encode_map_bf16(map, base, rank, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_128B, 64);
+}
+
+bool encode_map_bf16_sw64(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                          const uint32_t* box) {
+  return encode_map_bf16(map, base, rank, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_64B, 32);
 }
 
 bool encode_tile_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t row_stride_bytes,

@@ -1,0 +1,86 @@
+"""The CTA-pair prefill attention where its tiles, pairs and items can go wrong: sequences around 8 (output tile), 32 (CTA), 64 (pair)
+and 128 (key tile) tokens, more sequences than one read of their lengths covers, more items than a pair's ring holds, row maxima
+that grow from tile to tile, and rows behind a sequence that must not be touched.
+
+Bound: p is rounded to bf16 (2^-9 of each weight) and the output is (2^-9 of a value no larger than the largest |v|), so an output is
+off by at most 2^-8 max|v|; sums and scores in fp32 add some 1e-5.  The gated form rounds once, the chain twice more.
+"""
+import pytest
+import torch
+
+from helpers import bf16_randn, cdiv, rope_inv_freq
+from oracle import reference_ops as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _qkv(lengths, seed, kv_heads=2):
+    gen, total = torch.Generator().manual_seed(seed), sum(lengths)
+    cu = torch.tensor([0, *torch.tensor(lengths).cumsum(0).tolist()], dtype=torch.int32)
+    return [bf16_randn(total, n, 256, gen=gen) for n in (4 * kv_heads, kv_heads, kv_heads)] + [cu, gen]
+
+
+def _check(out, exact, v):
+    import b200attn
+    torch.cuda.synchronize()
+    assert b200attn.load().b200_wait_timed_out() == 0
+    assert (out.float().cpu() - exact.float()).abs().max().item() <= 2 ** -8 * v.float().abs().max().item() + 1e-3
+
+
+RAGGED = [int(x) for x in torch.randint(1, 200, (130,), generator=torch.Generator().manual_seed(9))]
+
+
+@pytest.mark.parametrize("lengths", [[1], [8, 7, 9], [31, 32, 33, 40], [63, 64, 65, 72], [96, 97, 127, 128, 129], [191, 192, 193, 256, 257],
+                                     RAGGED, [5] * 33, [640, 1, 320]])
+@pytest.mark.parametrize("kv_heads", [2, 1])
+def test_pairs_vs_oracle(lengths, kv_heads):
+    from b200attn import ops
+    q, k, v, cu, _ = _qkv(lengths, 11 + len(lengths), kv_heads)
+    out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), max(lengths))
+    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+
+
+def test_row_maxima_that_grow():
+    """Every later key tile outweighs the ones before it by far more than the 2^8 a reference maximum may lag: O is rescaled, by both
+    parities, and the sums of even and odd tiles stand against different references."""
+    from b200attn import ops
+    q, k, v, cu, _ = _qkv([700, 300], 5)
+    q = q.abs()
+    k = (k.abs() * (1 + 2 * (torch.arange(1000) // 128)).view(-1, 1, 1)).to(torch.bfloat16)
+    out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), 700)
+    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+
+
+@pytest.mark.parametrize("lengths", [[3], [64, 33, 8, 129], RAGGED[:70]])
+def test_gated_form_vs_chain(lengths):
+    from b200attn import ops
+    q, k, v, cu, gen = _qkv(lengths, 21)
+    gate = bf16_randn(sum(lengths), 2048, gen=gen).to(DEV)
+    q, k, v, cu = (t.to(DEV) for t in (q, k, v, cu))
+    batch, pps = len(lengths), cdiv(max(lengths), 16)
+    table = torch.randperm(batch * pps, generator=gen).view(batch, pps).to(torch.int32).to(DEV)
+    ids = torch.cat([torch.arange(n) for n in lengths]).to(torch.int32).unsqueeze(0).to(DEV)
+    inv = rope_inv_freq().to(DEV)
+    caches = ops.allocate_paged_kv_cache(batch * pps, 2, 256, device=DEV)
+    fused = ops.fused_prefill_attention(q, k, v, gate, *caches, table, cu, ids, inv, 64, max(lengths))
+    qr, kr = (ops.partial_rope(t.unsqueeze(0).permute(0, 2, 1, 3), ids, inv, 64)[0].permute(1, 0, 2).contiguous() for t in (q, k))
+    ctx = ops.gqa_attention_varlen_causal(qr, kr, v, cu, max(lengths)).permute(1, 0, 2).unsqueeze(0)
+    chain = ops.attention_gate_pack(ctx, gate.view(1, -1, 8, 256).permute(0, 2, 1, 3))
+    assert (fused.float() - chain.float()).abs().max().item() <= 2 ** -7 * v.float().abs().max().item()
+
+
+def test_rows_behind_a_sequence_stay():
+    """Sequences that end before the packed rows do: the output rows behind them are left alone (no tile of eight tokens is stored over
+    a sequence's end)."""
+    from b200attn import _lib, ops
+    q, k, v, cu, _ = _qkv([13, 70], 31)
+    q, k, v, cu = (t.to(DEV) for t in (q, k, v, cu))
+    for ends in ([0, 13, 83], [0, 5, 60]):
+        cu = torch.tensor(ends, dtype=torch.int32, device=DEV)
+        out = torch.full_like(q, 7.0)
+        _lib.call("b200_gqa_varlen_causal", q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
+                  v.stride(1), out.data_ptr(), out.stride(0), out.stride(1), cu.data_ptr(), 2, 83, 70, 8, 2, 256, torch.cuda.current_stream().cuda_stream)
+        exact = O.varlen_causal_exact(q[: ends[-1]].cpu(), k[: ends[-1]].cpu(), v[: ends[-1]].cpu(), cu.cpu())
+        _check(out[: ends[-1]], exact, v)
+        assert bool((out[ends[-1]:] == 7.0).all())
