@@ -33,7 +33,6 @@ constexpr int SG_KSPLIT = 2;                      // K = 1280 or less: warps per
 constexpr int SG_STD_WARPS = SG_WARPS * SG_KSPLIT;
 constexpr int SG_STD_THREADS = SG_STD_WARPS * 32;
 constexpr int SG_STD_RING = SG_RING / SG_KSPLIT;  // the same bytes in flight per CTA
-constexpr int SG_PART_BYTES = 16 * SG_WARPS * 32 * 4;
 constexpr int SG_MAX_M = 32;
 constexpr int SG_MAX_K = 1280;           // X staging: 32 x (K*2 + 16) bytes next to 128 KiB of weight rings
 
@@ -49,13 +48,113 @@ struct SkinnyGemmParams {
   int* counter;
 };
 
-template <bool SWIGLU, bool ARGMAX>
+// Which m16n8k16 products a step of 16 k takes for NT groups of eight batch rows, and the sums they go to.  A warp's k steps are a
+// chain: with fewer than four groups the steps take turns among the four accumulators, joined at the end by `join_steps`.
+// One step costs 16 cycles of a scheduler per group: 32 rows of zeros behind a single one were 2.2 us of a 6 us launch.
+template <int NT>
+struct StepProducts;
+template <>
+struct StepProducts<4> {
+  // ldmatrix lane address of X: row = (lane & 7) + 8 * (lane >> 4) inside a 16-row pair, k half = (lane >> 3) & 1
+  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
+    return static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * x_pitch + ((lane >> 3) & 1) * 16);
+  }
+  template <int KS>
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
+    uint32_t b01[4], b23[4];
+    ldmatrix_x4(b01, xk);                   // batch rows 0-15: (b0, b1) of n8 tiles 0 and 1
+    ldmatrix_x4(b23, xk + 16 * x_pitch);    // batch rows 16-31
+    mma_bf16_16816(acc[0], a, b01[0], b01[1]);
+    mma_bf16_16816(acc[1], a, b01[2], b01[3]);
+    mma_bf16_16816(acc[2], a, b23[0], b23[1]);
+    mma_bf16_16816(acc[3], a, b23[2], b23[3]);
+  }
+};
+template <>
+struct StepProducts<2> {
+  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) { return StepProducts<4>::lane_offset(lane, x_pitch); }
+  template <int KS>
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
+    uint32_t b01[4];
+    ldmatrix_x4(b01, xk);
+    mma_bf16_16816(acc[(KS & 1) * 2], a, b01[0], b01[1]);
+    mma_bf16_16816(acc[(KS & 1) * 2 + 1], a, b01[2], b01[3]);
+  }
+};
+template <>
+struct StepProducts<1> {
+  // eight rows, four k groups of eight: one load serves two steps
+  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
+    return static_cast<uint32_t>((lane & 7) * x_pitch + (lane >> 3) * 16);
+  }
+  template <int KS>
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
+    uint32_t (&b4)[4] = *reinterpret_cast<uint32_t (*)[4]>(b);
+    if constexpr ((KS & 1) == 0) ldmatrix_x4(b4, xk);
+    mma_bf16_16816(acc[KS & 3], a, b[(KS & 1) * 2], b[(KS & 1) * 2 + 1]);
+  }
+};
+template <int NT>
+__device__ __forceinline__ void join_steps(float (&acc)[4][4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if constexpr (NT == 1) acc[0][j] = (acc[0][j] + acc[1][j]) + (acc[2][j] + acc[3][j]);
+    if constexpr (NT == 2) {
+      acc[0][j] += acc[2][j];
+      acc[1][j] += acc[3][j];
+    }
+  }
+}
+// The eight steps of a tile of 128 k: A (W tile) by ldmatrix from `tile` + offset(step), X from `xk` on.
+template <int NT, int KS, typename Offset>
+__device__ __forceinline__ void tile_steps(float (&acc)[4][4], uint32_t (&b)[8], uint32_t tile, uint32_t xk, int x_pitch, const Offset& offset) {
+  if constexpr (KS < SG_TILE_K / 16) {
+    uint32_t a[4];
+    ldmatrix_x4(a, tile + offset(KS));
+    StepProducts<NT>::template run<KS>(acc, a, b, xk + KS * 32, x_pitch);
+    tile_steps<NT, KS + 1>(acc, b, tile, xk, x_pitch, offset);
+  }
+}
+// `chunks` 16-byte pieces of each of m rows -> shared memory, by all THREADS threads, thread t starting at piece c of row r
+// (t = r * chunks + c); every load of a round is under way before its first store.  (For few rows: a bulk copy per row takes
+// longer to arrive.)
+template <int THREADS>
+__device__ __forceinline__ void stage_rows(uint8_t* xs, int x_pitch, const __nv_bfloat16* x, int64_t x_stride, int m, int chunks, int r, int c) {
+  constexpr int ROUND = 4;
+  while (r < m) {
+    uint4 v[ROUND];
+    uint8_t* to[ROUND];
+#pragma unroll
+    for (int u = 0; u < ROUND; ++u) {
+      to[u] = nullptr;
+      if (r < m) {
+        v[u] = *reinterpret_cast<const uint4*>(x + r * x_stride + c * 8);
+        to[u] = xs + r * x_pitch + c * 16;
+      }
+      c += THREADS;
+      while (c >= chunks) {
+        c -= chunks;
+        ++r;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < ROUND; ++u)
+      if (to[u] != nullptr) *reinterpret_cast<uint4*>(to[u]) = v[u];
+  }
+}
+constexpr int skinny_smem(int nt, int k) {  // rings, output staging, odd-tile sums, X
+  return SG_WARPS * SG_RING_BYTES + nt * 8 * SG_ROWS * 2 + nt * 4 * SG_WARPS * 32 * 4 + nt * 8 * (k * 2 + 16) + 1024;
+}
+
+// NT: groups of eight batch rows that are staged and multiplied (M <= 8, 16 or 32 rows)
+template <bool SWIGLU, bool ARGMAX, int NT>
 __global__ void __launch_bounds__(SG_STD_THREADS, 1)
 skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_constant__ CUtensorMap map_w) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int SLOT_BYTES = SG_TILE_BYTES;
   constexpr int RING = SG_STD_RING;
   constexpr int OUT = SWIGLU ? 8 * SG_WARPS : SG_ROWS;  // outputs per CTA step
+  constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_STD_WARPS][RING];
   __shared__ uint64_t bar_x;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -64,9 +163,9 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   // dependent ldmatrix + MMA, so two short chains per row group finish in half the time of one long one
   const int wr = warp & (SG_WARPS - 1), kh = warp / SG_WARPS;
   uint8_t* ring = smem + warp * (RING * SLOT_BYTES);
-  uint8_t* stage = smem + SG_WARPS * SG_RING_BYTES;                    // [32 batch][OUT] bf16 output staging, <= 4 KiB
-  float* part = reinterpret_cast<float*>(stage + SG_MAX_M * SG_ROWS * 2);  // [16][4 groups x 32 lanes]: odd-tile sums
-  uint8_t* xs = reinterpret_cast<uint8_t*>(part) + SG_PART_BYTES;      // [32][x_pitch] bf16
+  uint8_t* stage = smem + SG_WARPS * SG_RING_BYTES;                    // [ROWS][OUT] bf16 output staging, <= 4 KiB
+  float* part = reinterpret_cast<float*>(stage + ROWS * SG_ROWS * 2);  // [4 NT][4 groups x 32 lanes]: odd-tile sums
+  uint8_t* xs = reinterpret_cast<uint8_t*>(part + 4 * NT * SG_WARPS * 32);  // [ROWS][x_pitch] bf16
   const int x_pitch = p.k * 2 + 16;                                    // bytes; the 16 shift the banks row by row
   const int k_tiles = p.k / SG_TILE_K;
 
@@ -99,31 +198,37 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   };
   // Started early, the weights are requested while the predecessor runs and X after it.  In plain stream order X goes
   // first: requested behind 128 KiB of weight tiles it would arrive behind them.
-  const bool early = (p.overlap & OVERLAP_START) != 0;
+  const bool early = (p.overlap & OVERLAP_START) != 0, by_threads = early && NT < 4;
   if (p.overlap & OVERLAP_TRIGGER) pdl_trigger();
   if (!early && warp == 0) stage_x();
   if (lane == 0) {
     for (int t = 0; t < RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
-  pdl_wait();  // X is the predecessor's output
-  if (early && warp == 0) stage_x();
-  for (int i = tid; i < (SG_MAX_M - p.m) * (p.k >> 3); i += SG_STD_THREADS) {  // rows beyond M are zero
+  for (int i = tid; i < (ROWS - p.m) * (p.k >> 3); i += SG_STD_THREADS) {  // rows beyond M are zero
     const int r = p.m + i / (p.k >> 3), c = i % (p.k >> 3);
     *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
   }
-  __syncthreads();  // bar_x is initialised for everybody, the zero rows are in place
-  bool ok = mbar_wait_bounded(&bar_x, 0);
+  const int x_row = tid / (p.k >> 3), x_piece = tid % (p.k >> 3);
+  pdl_wait();  // X is the predecessor's output
+  if (by_threads) stage_rows<SG_STD_THREADS>(xs, x_pitch, p.x, p.x_stride, p.m, p.k >> 3, x_row, x_piece);
+  else if (early && warp == 0) stage_x();
+  __syncthreads();  // bar_x is initialised for everybody, the rows that threads wrote are in place
+  bool ok = by_threads || mbar_wait_bounded(&bar_x, 0);
 
   const uint32_t xs_base = smem_u32(xs);
-  // ldmatrix lane addresses: A (W tile) row = lane % 16, chunk parity = lane / 16;
-  //                          B (X) row = (lane & 7) + 8 * (lane >> 4) inside a 16-row pair, k half = (lane >> 3) & 1
+  // ldmatrix lane address of A (W tile): row = lane % 16, chunk parity = lane / 16
   const int a_row = lane & 15, a_par = lane >> 4;
-  const uint32_t b_lane = static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * x_pitch + ((lane >> 3) & 1) * 16);
-  // arg-max form: this thread's running best over its rows, per batch column (8 columns: nt * 2 + (j & 1))
-  float best_v[8];
-  uint32_t best_i[8];
+  const uint32_t xs_lane = xs_base + StepProducts<NT>::lane_offset(lane, x_pitch);
+  const auto a_offset = [&](int ks) -> uint32_t {
+    // plain: [k-block][16 rows][128 B]; SwiGLU: [gate | up][k-block][8 rows][128 B]; 16-byte chunks XOR-swizzled by row
+    return (SWIGLU ? (a_row >> 3) * (SG_TILE_BYTES / 2) + (ks >> 2) * (8 * 128) + (a_row & 7) * 128 : (ks >> 2) * (16 * 128) + a_row * 128) +
+           ((((ks & 3) * 2 + a_par) ^ (a_row & 7)) << 4);
+  };
+  // arg-max form: this thread's running best over its rows, per batch column (nt * 2 + (j & 1))
+  float best_v[2 * NT];
+  uint32_t best_i[2 * NT];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < 2 * NT; ++c) {
     best_v[c] = -INFINITY;
     best_i[c] = 0xffffffffu;
   }
@@ -139,43 +244,29 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
         ok = false;
         break;
       }
-      const uint32_t tile = smem_u32(ring + slot * SLOT_BYTES);
-#pragma unroll
-      for (int ks = 0; ks < SG_TILE_K / 16; ++ks) {
-        uint32_t a[4], b01[4], b23[4];
-        // plain: [k-block][16 rows][128 B]; SwiGLU: [gate | up][k-block][8 rows][128 B]; 16-byte chunks XOR-swizzled by row
-        const uint32_t a_off = (SWIGLU ? (a_row >> 3) * (SG_TILE_BYTES / 2) + (ks >> 2) * (8 * 128) + (a_row & 7) * 128
-                                       : (ks >> 2) * (16 * 128) + a_row * 128) +
-                               ((((ks & 3) * 2 + a_par) ^ (a_row & 7)) << 4);
-        const uint32_t xk = xs_base + b_lane + (kt * SG_TILE_K + ks * 16) * 2;
-        ldmatrix_x4(b01, xk);                   // batch rows 0-15: (b0, b1) of n8 tiles 0 and 1
-        ldmatrix_x4(b23, xk + 16 * x_pitch);    // batch rows 16-31
-        ldmatrix_x4(a, tile + a_off);
-        mma_bf16_16816(acc[0], a, b01[0], b01[1]);
-        mma_bf16_16816(acc[1], a, b01[2], b01[3]);
-        mma_bf16_16816(acc[2], a, b23[0], b23[1]);
-        mma_bf16_16816(acc[3], a, b23[2], b23[3]);
-      }
+      uint32_t b[8];
+      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xs_lane + kt * SG_TILE_K * 2, x_pitch, a_offset);
       __syncwarp();  // every lane has read the tile: its slot can take the tile RING ahead
       if (lane == 0 && t + RING < total_tiles) issue(t + RING);
     }
+    join_steps<NT>(acc);
     // the odd-tile warps hand their sums to the even-tile warps of the same row group
     if (kh == 1) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) part[i * (SG_WARPS * 32) + wr * 32 + lane] = acc[i >> 2][i & 3];
+      for (int i = 0; i < 4 * NT; ++i) part[i * (SG_WARPS * 32) + wr * 32 + lane] = acc[i >> 2][i & 3];
     }
     __syncthreads();  // (also: the previous block's staging has been written out)
     // acc[nt]: rows (tile row = lane/4, +8), cols (batch = nt*8 + (lane%4)*2, +1)  ->  stage[batch][output] -> Y
     if (kh == 0) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i >> 2][i & 3] += part[i * (SG_WARPS * 32) + wr * 32 + lane];
+      for (int i = 0; i < 4 * NT; ++i) acc[i >> 2][i & 3] += part[i * (SG_WARPS * 32) + wr * 32 + lane];
     }
     if (ARGMAX) {
       if (kh == 0) {
         // rows ascend with the row block and, inside it, from fragment row r to r + 8: strict > keeps the lowest index
         const uint32_t n_lo = static_cast<uint32_t>(rb * OUT + wr * 16 + (lane >> 2));
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int c = nt * 2 + (j & 1);
@@ -193,7 +284,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
       __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
       const int bc = (lane & 3) * 2;
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
+      for (int nt = 0; nt < NT; ++nt) {
         if (SWIGLU) {
           // rows r and r + 8 of the tile are gate_j and up_j; the projection is a bf16 tensor in the reference
           const int j = wr * 8 + (lane >> 2);
@@ -211,7 +302,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
       }
     }
     __syncthreads();
-    for (int i = tid; i < SG_MAX_M * (OUT / 8); i += SG_STD_THREADS) {
+    for (int i = tid; i < ROWS * (OUT / 8); i += SG_STD_THREADS) {
       const int r = i / (OUT / 8), c = i % (OUT / 8);
       const int n0 = rb * OUT + c * 8;
       if (r < p.m && n0 < p.n)  // N is a multiple of 8: a 16-byte chunk is inside or outside as a whole
@@ -224,7 +315,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
     unsigned long long* keybuf = reinterpret_cast<unsigned long long*>(part);  // [4 row groups][32 batch]
     if (kh == 0) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < 2 * NT; ++c) {
         unsigned long long key = best_i[c] == 0xffffffffu ? 0ull : argmax_key(best_v[c], best_i[c]);
 #pragma unroll
         for (int o = 4; o <= 16; o <<= 1) {
@@ -446,13 +537,16 @@ skinny_gemm_widek_kernel(const __grid_constant__ WideKParams p, const __grid_con
 // one cluster barrier, rank 0 adds, rounds and writes).  No cluster multicast is used; every CTA loads its own tiles.
 constexpr int PK_RING = 3;                 // W tiles in flight per warp (a warp has K / 1024 tiles per row block)
 constexpr int PK_MAX_K = 4096;
-constexpr int PK_SMEM = SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * SG_MAX_M * 4 +
-                        SG_MAX_M * (PK_MAX_K + 16) + 1024;
-static_assert(PK_SMEM <= 227 * 1024, "weight rings + half of X must fit the 227 KiB a CTA may use");
+constexpr int pairk_smem(int nt, int k) {  // rings, sums of the warps and the peer, half of X
+  return SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * nt * 8 * 4 + nt * 8 * (k + 16) + 1024;
+}
+static_assert(pairk_smem(4, PK_MAX_K) <= 227 * 1024, "weight rings + half of X must fit the 227 KiB a CTA may use");
 
+template <int NT>
 __global__ void __launch_bounds__(SG_THREADS, 1)
 skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_constant__ CUtensorMap map_w) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_WARPS][PK_RING];
   __shared__ uint64_t bar_x;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -460,9 +554,9 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   uint8_t* ring = smem + warp * PK_RING * SG_TILE_BYTES;
-  float* red = reinterpret_cast<float*>(smem + SG_WARPS * PK_RING * SG_TILE_BYTES);  // [4 warps + peer][32 batch][16 rows]
-  float* peer = red + SG_WARPS * WK_ROWS * SG_MAX_M;                                 // written by rank 1 into rank 0
-  uint8_t* xs = reinterpret_cast<uint8_t*>(peer + WK_ROWS * SG_MAX_M);               // [32][x_pitch]: this CTA's half of X
+  float* red = reinterpret_cast<float*>(smem + SG_WARPS * PK_RING * SG_TILE_BYTES);  // [4 warps + peer][ROWS][16]
+  float* peer = red + SG_WARPS * WK_ROWS * ROWS;                                 // written by rank 1 into rank 0
+  uint8_t* xs = reinterpret_cast<uint8_t*>(peer + WK_ROWS * ROWS);               // [ROWS][x_pitch]: this CTA's half of X
   const int half_k = p.k >> 1;
   const int x_pitch = half_k * 2 + 16;
   const int half_tiles = half_k / SG_TILE_K;
@@ -487,22 +581,26 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   if (lane == 0) {
     for (int t = 0; t < PK_RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
+  for (int i = tid; i < (ROWS - p.m) * (half_k >> 3); i += SG_THREADS) {  // rows beyond M are zero
+    const int r = p.m + i / (half_k >> 3), c = i % (half_k >> 3);
+    *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
+  }
+  const int x_row = tid / (half_k >> 3), x_piece = tid % (half_k >> 3);
   pdl_wait();  // X is the predecessor's output
-  if (warp == 0) {
+  if (NT < 4) {
+    stage_rows<SG_THREADS>(xs, x_pitch, p.x + rank * half_k, p.x_stride, p.m, half_k >> 3, x_row, x_piece);
+  } else if (warp == 0) {
     if (lane == 0) mbar_expect_tx(&bar_x, static_cast<uint32_t>(p.m) * half_k * 2);
     __syncwarp();
     if (lane < p.m)
       bulk_g2s(xs + lane * x_pitch, p.x + static_cast<int64_t>(lane) * p.x_stride + rank * half_k, half_k * 2, &bar_x);
   }
-  for (int i = tid; i < (SG_MAX_M - p.m) * (half_k >> 3); i += SG_THREADS) {  // rows beyond M are zero
-    const int r = p.m + i / (half_k >> 3), c = i % (half_k >> 3);
-    *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
-  }
   __syncthreads();
-  bool ok = mbar_wait_bounded(&bar_x, 0);
+  bool ok = NT < 4 || mbar_wait_bounded(&bar_x, 0);
 
   const int a_row = lane & 15, a_par = lane >> 4;
-  const uint32_t xs_base = smem_u32(xs) + static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * x_pitch + ((lane >> 3) & 1) * 16);
+  const uint32_t xs_base = smem_u32(xs) + StepProducts<NT>::lane_offset(lane, x_pitch);
+  const auto a_offset = [&](int ks) -> uint32_t { return (ks >> 2) * (16 * 128) + a_row * 128 + ((((ks & 3) * 2 + a_par) ^ (a_row & 7)) << 4); };
   const uint32_t peer_remote = cluster_map(smem_u32(peer), 0);
   int t = 0;
   for (int blk = 0; blk < my_blocks; ++blk) {
@@ -514,30 +612,19 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
       const int slot = t % PK_RING;
       if (ok && !mbar_wait_bounded(&bars[warp][slot], (t / PK_RING) & 1)) ok = false;
       if (ok) {
-        const uint32_t tile = smem_u32(ring + slot * SG_TILE_BYTES);
-        const uint32_t xk0 = xs_base + kl * SG_TILE_K * 2;
-#pragma unroll
-        for (int ks = 0; ks < SG_TILE_K / 16; ++ks) {
-          uint32_t a[4], b01[4], b23[4];
-          const uint32_t a_off = (ks >> 2) * (16 * 128) + a_row * 128 + ((((ks & 3) * 2 + a_par) ^ (a_row & 7)) << 4);
-          ldmatrix_x4(b01, xk0 + ks * 32);
-          ldmatrix_x4(b23, xk0 + ks * 32 + 16 * x_pitch);
-          ldmatrix_x4(a, tile + a_off);
-          mma_bf16_16816(acc[0], a, b01[0], b01[1]);
-          mma_bf16_16816(acc[1], a, b01[2], b01[3]);
-          mma_bf16_16816(acc[2], a, b23[0], b23[1]);
-          mma_bf16_16816(acc[3], a, b23[2], b23[3]);
-        }
+        uint32_t b[8];
+        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xs_base + kl * SG_TILE_K * 2, x_pitch, a_offset);
       }
       __syncwarp();  // every lane has read the tile: its slot can take the tile PK_RING ahead
       if (ok && lane == 0 && t + PK_RING < total_tiles) issue(t + PK_RING);
     }
     // ---- the warps' partial [16 x 32] sums meet in shared memory: red[warp][batch][row]
+    join_steps<NT>(acc);
     {
-      float* mine = red + warp * (WK_ROWS * SG_MAX_M);
+      float* mine = red + warp * (WK_ROWS * ROWS);
       const int r0 = lane >> 2, bc = (lane & 3) * 2;
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
+      for (int nt = 0; nt < NT; ++nt) {
         mine[(nt * 8 + bc) * WK_ROWS + r0] = acc[nt][0];
         mine[(nt * 8 + bc + 1) * WK_ROWS + r0] = acc[nt][1];
         mine[(nt * 8 + bc) * WK_ROWS + r0 + 8] = acc[nt][2];
@@ -547,16 +634,18 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
     __syncthreads();
     // thread -> batch row tid / 4, outputs (tid % 4) * 4 .. + 4
     const int b = tid >> 2, r = (tid & 3) * 4;
-    float o[4];
+    const bool mine = NT == 4 || b < ROWS;
+    float o[4] = {};
+    if (mine) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int idx = b * WK_ROWS + r + j;
-      o[j] = ((red[idx] + red[WK_ROWS * SG_MAX_M + idx]) + red[2 * WK_ROWS * SG_MAX_M + idx]) +
-             red[3 * WK_ROWS * SG_MAX_M + idx];
+      for (int j = 0; j < 4; ++j) {
+        const int idx = b * WK_ROWS + r + j;
+        o[j] = ((red[idx] + red[WK_ROWS * ROWS + idx]) + red[2 * WK_ROWS * ROWS + idx]) + red[3 * WK_ROWS * ROWS + idx];
+      }
+      if (rank == 1) st_cluster_f32x4(peer_remote + (b * WK_ROWS + r) * 4, o[0], o[1], o[2], o[3]);
     }
-    if (rank == 1) st_cluster_f32x4(peer_remote + (b * WK_ROWS + r) * 4, o[0], o[1], o[2], o[3]);
     cluster_sync();  // rank 1's sum is in rank 0's shared memory; red is free again in both CTAs
-    if (rank == 0) {
+    if (rank == 0 && mine) {
       const float4 other = *reinterpret_cast<const float4*>(peer + b * WK_ROWS + r);
       const int n0 = rb * WK_ROWS + r;
       if (b < p.m && n0 < p.n)  // N is a multiple of 8 and r of 4: the four outputs are inside or outside together
@@ -614,34 +703,38 @@ static bool cache_weight_map(const void* base, int64_t n, int64_t k, int64_t str
 
 using namespace b200;
 
-template <bool SWIGLU, bool ARGMAX = false>
-static int launch_skinny(SkinnyGemmParams p, const void* weight, int64_t w_stride, int w_rows, cudaStream_t stream, const char* what) {
-  CUtensorMap map;
-  if (!cache_weight_map(weight, w_rows, p.k, w_stride, SWIGLU ? 8 : 16, &map)) return fail(ERR_RUNTIME, "%s: cannot encode the weight tensor map", what);
-  constexpr int smem_max =
-      SG_WARPS * SG_RING_BYTES + SG_MAX_M * SG_ROWS * 2 + SG_PART_BYTES + SG_MAX_M * (SG_MAX_K * 2 + 16) + 1024;
+template <bool SWIGLU, bool ARGMAX, int NT>
+static int launch_skinny_rows(SkinnyGemmParams p, const CUtensorMap& map, cudaStream_t stream, const char* what) {
+  constexpr int smem_max = skinny_smem(NT, SG_MAX_K);
   static_assert(smem_max <= 227 * 1024, "weight rings + X staging must fit the 227 KiB a CTA may use");
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(skinny_gemm_kernel<SWIGLU, ARGMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) !=
+    if (cudaFuncSetAttribute(skinny_gemm_kernel<SWIGLU, ARGMAX, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) !=
         cudaSuccess)
       return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, smem_max);
     configured[dev] = true;
   }
+  const int sms = sm_count();
+  if (launch_pdl((p.overlap & OVERLAP_START) != 0, skinny_gemm_kernel<SWIGLU, ARGMAX, NT>, dim3(p.row_blocks < sms ? p.row_blocks : sms),
+                 dim3(SG_STD_THREADS), skinny_smem(NT, p.k), stream, p, map) != cudaSuccess)
+    return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+  return check_launch(what);
+}
+
+template <bool SWIGLU, bool ARGMAX = false>
+static int launch_skinny(SkinnyGemmParams p, const void* weight, int64_t w_stride, int w_rows, cudaStream_t stream, const char* what) {
+  CUtensorMap map;
+  if (!cache_weight_map(weight, w_rows, p.k, w_stride, SWIGLU ? 8 : 16, &map)) return fail(ERR_RUNTIME, "%s: cannot encode the weight tensor map", what);
   p.err = wait_timeout_flag();
   if (!p.err) return fail(ERR_RUNTIME, "%s: no error flag", what);
   constexpr int out_per_cta = SWIGLU ? 8 * SG_WARPS : SG_ROWS;
   p.row_blocks = (p.n + out_per_cta - 1) / out_per_cta;
-  int grid = p.row_blocks;
-  const int sms = sm_count();
-  if (grid > sms) grid = sms;
-  const int dyn = SG_WARPS * SG_RING_BYTES + SG_MAX_M * SG_ROWS * 2 + SG_PART_BYTES + SG_MAX_M * (p.k * 2 + 16) + 1024;
-  if (launch_pdl((p.overlap & OVERLAP_START) != 0, skinny_gemm_kernel<SWIGLU, ARGMAX>, dim3(grid), dim3(SG_STD_THREADS), dyn, stream,
-                 p, map) != cudaSuccess)
-    return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
-  return check_launch(what);
+  // as few groups of eight rows as hold the batch
+  if (p.m <= 8) return launch_skinny_rows<SWIGLU, ARGMAX, 1>(p, map, stream, what);
+  if (p.m <= 16) return launch_skinny_rows<SWIGLU, ARGMAX, 2>(p, map, stream, what);
+  return launch_skinny_rows<SWIGLU, ARGMAX, 4>(p, map, stream, what);
 }
 
 // Chunking of K for the wide-K form: the fewest equal chunks of whole 128-k tiles that are at most WK_CHUNK_MAX long.
@@ -680,30 +773,35 @@ static int launch_widek(WideKParams p, const void* weight, int64_t w_stride, cud
   return check_launch(what);
 }
 
-static int launch_pairk(WideKParams p, const void* weight, int64_t w_stride, cudaStream_t stream) {
+template <int NT>
+static int launch_pairk_rows(WideKParams p, const CUtensorMap& map, cudaStream_t stream) {
   const char* what = "skinny_gemm";
-  CUtensorMap map;
-  if (!cache_weight_map(weight, p.n, p.k, w_stride, 16, &map)) return fail(ERR_RUNTIME, "%s: cannot encode the weight tensor map", what);
+  constexpr int smem_max = pairk_smem(NT, PK_MAX_K);
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(skinny_gemm_pairk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_SMEM) != cudaSuccess)
-      return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, PK_SMEM);
+    if (cudaFuncSetAttribute(skinny_gemm_pairk_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) != cudaSuccess)
+      return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, smem_max);
     configured[dev] = true;
   }
+  const int sms = sm_count(), pairs = p.row_blocks < sms / 2 ? p.row_blocks : sms / 2;
+  if (launch_pdl_cluster((p.overlap & OVERLAP_START) != 0, 2, skinny_gemm_pairk_kernel<NT>, dim3(2 * pairs), dim3(SG_THREADS),
+                         pairk_smem(NT, p.k), stream, p, map) != cudaSuccess)
+    return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+  return check_launch(what);
+}
+
+static int launch_pairk(WideKParams p, const void* weight, int64_t w_stride, cudaStream_t stream) {
+  const char* what = "skinny_gemm";
+  CUtensorMap map;
+  if (!cache_weight_map(weight, p.n, p.k, w_stride, 16, &map)) return fail(ERR_RUNTIME, "%s: cannot encode the weight tensor map", what);
   p.err = wait_timeout_flag();
   if (!p.err) return fail(ERR_RUNTIME, "%s: no error flag", what);
   p.row_blocks = (p.n + WK_ROWS - 1) / WK_ROWS;
-  int pairs = p.row_blocks;
-  const int sms = sm_count();
-  if (pairs > sms / 2) pairs = sms / 2;
-  const int dyn = SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * SG_MAX_M * 4 +
-                  SG_MAX_M * (p.k + 16) + 1024;
-  if (launch_pdl_cluster((p.overlap & OVERLAP_START) != 0, 2, skinny_gemm_pairk_kernel, dim3(2 * pairs), dim3(SG_THREADS),
-                         dyn, stream, p, map) != cudaSuccess)
-    return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
-  return check_launch(what);
+  if (p.m <= 8) return launch_pairk_rows<1>(p, map, stream);
+  if (p.m <= 16) return launch_pairk_rows<2>(p, map, stream);
+  return launch_pairk_rows<4>(p, map, stream);
 }
 
 static int check_skinny_shape(const char* what, int m, int n, int k) {
