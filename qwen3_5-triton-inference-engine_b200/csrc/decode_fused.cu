@@ -36,7 +36,7 @@ namespace b200 {
 constexpr int FD_WARPS = 8;
 constexpr int FD_THREADS = FD_WARPS * 32;
 constexpr int FD_RING = 3;                             // K/V tiles per warp
-constexpr int FD_MERGE_SLOTS = 4;                      // warps merge in two rounds of four
+constexpr int FD_MERGE_SLOTS = 4;                      // warps merge four at a time (in cluster mode all at once)
 constexpr int FD_MAX_BATCH = 512;                      // prefix table and positions live in shared memory
 constexpr int FD_MAX_SEGMENTS = 2048;                  // counters in the workspace
 constexpr int FD_MAX_CTAS = 256;                       // partial slots in the workspace
@@ -46,7 +46,7 @@ constexpr int64_t FD_COUNTER_BYTES = FD_MAX_SEGMENTS * 4;
 constexpr int64_t FD_WORKSPACE_BYTES = FD_COUNTER_BYTES + int64_t(FD_MAX_CTAS) * 2 * FD_PARTIAL_FLOATS * 4;
 
 constexpr int FD_SMEM_RING = FD_WARPS * FD_RING * TILE_BYTES_SW;
-constexpr int FD_SMEM_MERGE = FD_MERGE_SLOTS * FD_PARTIAL_FLOATS * 4;
+constexpr int FD_SMEM_MERGE = FD_MERGE_SLOTS * FD_TILE_FLOATS * 4;
 constexpr int FD_SMEM_CUM = ((FD_MAX_BATCH + 1) * 4 + 15) / 16 * 16;   // exclusive prefix of units
 constexpr int FD_SMEM_POS = FD_MAX_BATCH * 4;                           // pos[] as int32
 constexpr int FD_Q_PITCH = HEAD_DIM + 8;                                // bf16 elements per staged Q row
@@ -75,7 +75,7 @@ struct FusedDecodeParams {
   int batch, num_kv_heads, rotary_half, overlap;
   int partition;  // 0 = the time models below choose, 1 = stream-K, 2 = one whole segment per CTA, 3 = one segment
                   // per thread-block cluster
-  int cluster_size;  // CTAs per cluster of this launch (1 = launched without clusters)
+  int cluster_size, cluster_log2;  // CTAs per cluster of this launch, a power of two (1 = launched without clusters)
   float scale, eps;
 };
 
@@ -117,8 +117,7 @@ __device__ __forceinline__ void segment_advance(Segment& s, const int* cum, int 
 // Optional Qwen RMSNorm over the 256 dims, x * rsqrt(mean(x^2) + eps) * (1 + weight), rounded to bf16 as the
 // reference's q_norm / k_norm output is a bf16 tensor (triton_kernels/qwen_rmsnorm.py:70-73, applied at
 // engine/runner.py:476-489); the summation order is the one of add_rmsnorm_kernel, so both give the same bytes.
-__device__ __forceinline__ void norm_row8(uint32_t (&w)[4], const __nv_bfloat16* weight, float eps, int lane) {
-  const uint4 wraw = *reinterpret_cast<const uint4*>(weight + lane * 8);
+__device__ __forceinline__ void norm_row8(uint32_t (&w)[4], const uint4& wraw, float eps) {
   const uint32_t ww[4] = {wraw.x, wraw.y, wraw.z, wraw.w};
   float v[8];
 #pragma unroll
@@ -138,12 +137,12 @@ __device__ __forceinline__ void norm_row8(uint32_t (&w)[4], const __nv_bfloat16*
 // Partial RoPE of the row at position pos: dims [0, half) pair with [half, 2*half), angles = float(pos) * inv_freq[d] in
 // fp32, full-range sincosf, result rounded to bf16 -- the arithmetic of triton_kernels/partial_rope.py:65-113.  Lanes
 // [0, half/8) hold the first halves, the next half/8 lanes their partners; the other lanes pass through.
-__device__ __forceinline__ void rope_row8(uint32_t (&w)[4], int half, const float* inv_freq, int64_t pos, int lane) {
-  // half <= 32: one angle per lane; inv_freq may be a shared-memory copy
+__device__ __forceinline__ void rope_row8(uint32_t (&w)[4], int half, float inv_freq, int64_t pos, int lane) {
+  // half <= 32: one angle per lane, of frequency `inv_freq`
   if (half == 0) return;
   // the warp computes the `half` angles once, one sincosf per lane, and hands them round by shuffles
   float sn = 0.f, cs = 1.f;
-  if (lane < half) sincosf(static_cast<float>(pos) * inv_freq[lane], &sn, &cs);
+  if (lane < half) sincosf(static_cast<float>(pos) * inv_freq, &sn, &cs);
   const int lanes_half = half / 8;
   const bool in_rot = lane < 2 * lanes_half;
   const bool first = lane < lanes_half;
@@ -182,18 +181,19 @@ __device__ __forceinline__ uint4 load_q_row(const FusedDecodeParams& p, int b, i
   const int head = tid >> 5, lane = tid & 31;
   return *reinterpret_cast<const uint4*>(p.q + b * p.q_b + (h * GROUP + head) * p.q_h + lane * 8);
 }
-__device__ __forceinline__ void stage_q_row(__nv_bfloat16* buf, const FusedDecodeParams& p, const FusedDecodeTables& tb,
+__device__ __forceinline__ void stage_q_row(__nv_bfloat16* buf, const FusedDecodeParams& p, const uint4& norm_w, float inv_freq,
                                             const uint4& raw, int pos_b, int tid) {
   if (tid >= GROUP * 32) return;
   const int head = tid >> 5, lane = tid & 31;
   uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  if (p.q_norm_w != nullptr) norm_row8(w, tb.q_norm_w, p.eps, lane);
-  rope_row8(w, p.rotary_half, tb.inv_freq, pos_b, lane);
+  if (p.q_norm_w != nullptr) norm_row8(w, norm_w, p.eps);
+  rope_row8(w, p.rotary_half, inv_freq, pos_b, lane);
   *reinterpret_cast<uint4*>(buf + head * FD_Q_PITCH + lane * 8) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 __device__ __forceinline__ void stage_q(__nv_bfloat16* buf, const FusedDecodeParams& p, const FusedDecodeTables& tb, int b,
                                         int h, int pos_b, int tid) {
-  stage_q_row(buf, p, tb, load_q_row(p, b, h, tid), pos_b, tid);
+  const int lane = tid & 31;
+  stage_q_row(buf, p, *reinterpret_cast<const uint4*>(tb.q_norm_w + lane * 8), tb.inv_freq[lane], load_q_row(p, b, h, tid), pos_b, tid);
 }
 // Asks the L2 for the q rows and the gate row of a segment ahead of their use (one 16-byte piece per thread of warps
 // 0-3 and 8 bytes of gate per thread: the lines they touch cover both rows).
@@ -215,8 +215,8 @@ __device__ __forceinline__ void stage_new_k(uint8_t* k_tile, const FusedDecodePa
   __syncwarp();
   const uint4 kraw = *reinterpret_cast<const uint4*>(tb.new_rows + lane * 16);
   uint32_t kw[4] = {kraw.x, kraw.y, kraw.z, kraw.w};
-  if (p.k_norm_w != nullptr) norm_row8(kw, tb.k_norm_w, p.eps, lane);
-  rope_row8(kw, p.rotary_half, tb.inv_freq, pos_b, lane);
+  if (p.k_norm_w != nullptr) norm_row8(kw, *reinterpret_cast<const uint4*>(tb.k_norm_w + lane * 8), p.eps);
+  rope_row8(kw, p.rotary_half, tb.inv_freq[lane], pos_b, lane);
   const uint4 krot = make_uint4(kw[0], kw[1], kw[2], kw[3]);
   *reinterpret_cast<uint4*>(k_tile + tile_offset<true>(0, lane)) = krot;
   *reinterpret_cast<uint4*>(p.k_cache + phys * p.kc_p + h * p.kc_h + (pos_b % PAGE) * p.kc_s + lane * 8) = krot;
@@ -228,10 +228,15 @@ __device__ __forceinline__ void stage_new_v(uint8_t* v_tile, const FusedDecodePa
   *reinterpret_cast<uint4*>(p.v_cache + phys * p.vc_p + h * p.vc_h + (pos_b % PAGE) * p.vc_s + lane * 8) = vraw;
 }
 
-// out = bf16( bf16(acc / l) * sigmoid(gate) ), 4 consecutive dims of one head per thread; without a gate (p.gate NULL)
+__device__ __forceinline__ float4 sigmoid4(uint2 g) {
+  return make_float4(1.f / (1.f + __expf(-bf16_lo(g.x))), 1.f / (1.f + __expf(-bf16_hi(g.x))), 1.f / (1.f + __expf(-bf16_lo(g.y))),
+                     1.f / (1.f + __expf(-bf16_hi(g.y))));
+}
+
+// out = bf16( bf16(acc / l) * factor ), factor = sigmoid(gate), 4 consecutive dims of one head per thread; without a gate (p.gate NULL)
 // out = bf16(acc / l), the output of the reference's combine kernel.
 __device__ __forceinline__ void finish_store(const FusedDecodeParams& p, int b, int hq, int d0, const float (&acc)[4],
-                                             float l, uint2 gv) {
+                                             float l, const float4& factor) {
   const int64_t col = static_cast<int64_t>(hq) * HEAD_DIM + d0;
   if (p.gate == nullptr) {
     const int64_t row = static_cast<int64_t>(p.num_kv_heads) * GROUP * HEAD_DIM;
@@ -241,10 +246,8 @@ __device__ __forceinline__ void finish_store(const FusedDecodeParams& p, int b, 
   const float inv_l = 1.f / l;
   const float x0 = round_bf16(acc[0] * inv_l), x1 = round_bf16(acc[1] * inv_l);
   const float x2 = round_bf16(acc[2] * inv_l), x3 = round_bf16(acc[3] * inv_l);
-  const float g0 = 1.f / (1.f + __expf(-bf16_lo(gv.x))), g1 = 1.f / (1.f + __expf(-bf16_hi(gv.x)));
-  const float g2 = 1.f / (1.f + __expf(-bf16_lo(gv.y))), g3 = 1.f / (1.f + __expf(-bf16_hi(gv.y)));
   const int64_t row = static_cast<int64_t>(p.num_kv_heads) * GROUP * HEAD_DIM;
-  *reinterpret_cast<uint2*>(p.out + b * row + col) = make_uint2(pack_bf16(x0 * g0, x1 * g1), pack_bf16(x2 * g2, x3 * g3));
+  *reinterpret_cast<uint2*>(p.out + b * row + col) = make_uint2(pack_bf16(x0 * factor.x, x1 * factor.y), pack_bf16(x2 * factor.z, x3 * factor.w));
 }
 
 // Fold one exported state (m, l, acc) into a running one with the usual max-rescaling.
@@ -262,6 +265,16 @@ __device__ __forceinline__ void merge_state(float& m_run, float& l_run, float (&
   m_run = m_new;
 }
 
+// a / b for 0 <= a < 2^21, b > 0: a third of an integer division's instructions.
+__device__ __forceinline__ int small_div(int a, int b) { return static_cast<int>(__fdividef(static_cast<float>(a) + 0.5f, static_cast<float>(b))); }
+
+// What a short launch (few sequences, a page or two per warp) takes is the chain in front of the first copy and behind the last:
+// positions -> shares -> page ids -> pages, warps' states -> cluster -> output.  One sequence of 1926 tokens, cycles of 19100: shares
+// known 3900 after entry, first page there at 8200, merge of eight warps' states 3000, exchange 2200, merge of sixteen CTAs' states and
+// output 3300.  With the lengths of up to 32 sequences in registers instead of shared memory behind two barriers, and with all weights of
+// a merge taken at once, one per lane, instead of state by state: shares 2400, merges 2100 and 1800.  Six such layers 61.6 -> 54.9 us, of 32
+// sequences of 512 to 4096 tokens 194.9 -> 190.6, of 256 the same (195).  Not kept: rolled merges (65.7 us: a chain per state), the appended token
+// in front of the pages in cluster mode (its CTA then is the last, 55.4).
 __global__ void __launch_bounds__(FD_THREADS, 1)
 fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v) {
@@ -269,6 +282,7 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
   __shared__ uint64_t bars[FD_WARPS][FD_RING];
   __shared__ int s_last;
   __shared__ int s_max_units;
+  __shared__ float s_ml[FD_WARPS][8];  // (m[4], l[4]) of every warp
   __shared__ FusedDecodeTables tb;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* merge = reinterpret_cast<float*>(smem + FD_SMEM_RING);
@@ -295,41 +309,71 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
   // caches); q, k_new, v_new and gate are the predecessor's output and are read only after the wait further down.
   if (!(p.overlap & OVERLAP_PREFETCH)) pdl_wait();
 
-  // weights and frequencies are nobody's output: staged before anything else, published by the barrier below
-  if (warp == 7) tb.inv_freq[lane] = lane < p.rotary_half ? p.inv_freq[lane] : 0.f;
-  if (warp == 6 && p.q_norm_w != nullptr)
-    *reinterpret_cast<uint4*>(tb.q_norm_w + lane * 8) = *reinterpret_cast<const uint4*>(p.q_norm_w + lane * 8);
-  if (warp == 5 && p.k_norm_w != nullptr)
-    *reinterpret_cast<uint4*>(tb.k_norm_w + lane * 8) = *reinterpret_cast<const uint4*>(p.k_norm_w + lane * 8);
+  // weights and frequencies are nobody's output: asked for before anything else.  The warps that rotate the first Q keep theirs; the
+  // copies in shared memory are published by the barrier behind that Q.
+  float q_freq = 0.f;
+  uint4 q_weight = make_uint4(0, 0, 0, 0);
+  if (warp < GROUP) {
+    if (lane < p.rotary_half) q_freq = p.inv_freq[lane];
+    if (p.q_norm_w != nullptr) q_weight = *reinterpret_cast<const uint4*>(p.q_norm_w + lane * 8);
+  }
+  if (warp == 7 && lane < p.rotary_half)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(tb.inv_freq + lane)), "l"(p.inv_freq + lane) : "memory");
+  if (warp == 6 && p.q_norm_w != nullptr) cp_async16(tb.q_norm_w + lane * 8, p.q_norm_w + lane * 8);
+  if (warp == 5 && p.k_norm_w != nullptr) cp_async16(tb.k_norm_w + lane * 8, p.k_norm_w + lane * 8);
   // ---- exclusive prefix of units per sequence: units_b = cdiv(pos[b], 16) + 1
-  for (int b = tid; b < batch; b += FD_THREADS) {
-    const int pb = static_cast<int>(p.pos[b]);
-    pos_s[b] = pb;
-    cum[b + 1] = (pb + PAGE - 1) / PAGE + 1 + gap;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    int carry = 0, longest = 0;
-    for (int base = 0; base < batch; base += 32) {
-      const int idx = base + lane;
-      int v = (idx < batch) ? cum[idx + 1] : 0;
-      longest = max(longest, v);
+  auto prefix = [&](int spans, int carry) {  // inclusive over the lanes of a warp
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += n;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, spans, o);
+      if (lane >= o) spans += n;
+    }
+    return spans + carry;
+  };
+  const bool few = batch <= 32;  // then every warp has all lengths in its lanes, and no barrier is needed to share the work
+  int my_pos = 0, my_span = 0, line, longest;
+  if (few) {
+    if (lane < batch) {
+      my_pos = static_cast<int>(p.pos[lane]);
+      my_span = (my_pos + PAGE - 1) / PAGE + 1 + gap;
+    }
+    longest = __reduce_max_sync(0xffffffffu, my_span) - gap;
+    line = __reduce_add_sync(0xffffffffu, my_span);
+    if (warp == 0) {
+      const int sum = prefix(my_span, 0);
+      if (lane < batch) {
+        pos_s[lane] = my_pos;
+        cum[lane + 1] = sum;
       }
-      if (idx < batch) cum[idx + 1] = v + carry;
-      carry += __shfl_sync(0xffffffffu, v, 31);
+      if (lane == 0) cum[0] = 0;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-    if (lane == 0) {
-      cum[0] = 0;
-      s_max_units = longest - gap;
+  } else {
+    for (int b = tid; b < batch; b += FD_THREADS) {
+      const int pb = static_cast<int>(p.pos[b]);
+      pos_s[b] = pb;
+      cum[b + 1] = (pb + PAGE - 1) / PAGE + 1 + gap;
     }
+    __syncthreads();
+    if (warp == 0) {
+      int carry = 0, most = 0;
+      for (int base = 0; base < batch; base += 32) {
+        const int idx = base + lane;
+        const int v = (idx < batch) ? cum[idx + 1] : 0;
+        most = max(most, v);
+        const int sum = prefix(v, carry);
+        if (idx < batch) cum[idx + 1] = sum;
+        carry = __shfl_sync(0xffffffffu, sum, 31);
+      }
+      most = __reduce_max_sync(0xffffffffu, most);
+      if (lane == 0) {
+        cum[0] = 0;
+        s_max_units = most - gap;
+      }
+    }
+    __syncthreads();
+    longest = s_max_units;
+    line = cum[batch];
   }
-  __syncthreads();
 
   // Three ways to cut the work.
   //  - Stream-K: equal ranges of the unit line per CTA (never less than one position per warp: tiny problems use fewer
@@ -347,14 +391,15 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
   //    whole     max(165 u_longest, 2.64 u_total) + 8500
   //    cluster   max(190 u_longest / cluster_size, 2.64 u_total) + 8500
   // A form is taken over stream-K when its model wins by 5 %.
-  const int total = heads * cum[batch];  // length of the line, gaps included
+  const int total = heads * line;  // length of the line, gaps included
   const int grid = static_cast<int>(gridDim.x), nseg = batch * heads;
   const int chunk = max((total + grid - 1) / grid, FD_WARPS);
   const int csize = p.cluster_size;
   const int dram = (total - nseg * gap) * 66 / 25;  // 2.64 ns per unit
-  const int t_stream = max(300 * chunk, dram) + 8000 + 180 * s_max_units / chunk;
-  const int t_whole = max(165 * s_max_units, dram) + 8500;
-  const int t_cluster = max(190 * ((s_max_units + csize - 1) / csize), dram) + 8500;
+  const int clog = p.cluster_log2;
+  const int t_stream = max(300 * chunk, dram) + 8000 + static_cast<int>(__fdividef(180.f * static_cast<float>(longest), static_cast<float>(chunk)));
+  const int t_whole = max(165 * longest, dram) + 8500;
+  const int t_cluster = max(190 * ((longest + csize - 1) >> clog), dram) + 8500;
   const bool cluster_fits = csize > 1 && nseg * csize <= grid;
   const bool whole_fits = nseg <= grid;
   int form = 1;  // 1 stream-K, 2 whole segments, 3 cluster per segment
@@ -371,24 +416,27 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
   const bool cluster_mode = form == 3, whole_segments = form == 2;
   int r0, r1;
   Segment cseg = {0, 0, 0, 0};  // cluster mode: the segment of this CTA's cluster
-  const int rank = csize > 1 ? static_cast<int>(blockIdx.x) % csize : 0;  // == %cluster_ctarank of a 1-D cluster
+  const int rank = static_cast<int>(blockIdx.x) & (csize - 1);  // == %cluster_ctarank of a 1-D cluster
   if (cluster_mode) {
-    const int cl = static_cast<int>(blockIdx.x) / csize;
+    const int cl = static_cast<int>(blockIdx.x) >> clog;
     if (cl < nseg) {
-      const int sb = cl / heads, sh = cl % heads;
-      const int span = cum[sb + 1] - cum[sb], units = span - gap;
-      const int per = (units + csize - 1) / csize;
-      const int start = heads * cum[sb] + sh * span;
-      cseg.b = sb;
+      const int sb = small_div(cl, heads), sh = cl - sb * heads;
+      const int units = (few ? __shfl_sync(0xffffffffu, my_span, sb) : cum[sb + 1] - cum[sb]) - gap;
+      const int per = (units + csize - 1) >> clog;
+      cseg.b = sb;  // (where on the line it lies does not matter here)
       cseg.h = sh;
-      cseg.start = start;
-      cseg.end = start + units;
-      r0 = min(start + rank * per, start + units);
-      r1 = min(r0 + per, start + units);
+      cseg.start = 0;
+      cseg.end = units;
+      r0 = min(rank * per, units);
+      r1 = min(r0 + per, units);
     } else {
       pdl_wait();  // a cluster without a segment: all its CTAs leave together, nobody waits for them
       return;
     }
+  } else if (few) {
+    __syncthreads();  // cum
+  }
+  if (cluster_mode) {
   } else if (whole_segments) {
     if (static_cast<int>(blockIdx.x) < nseg) {
       const int sb = blockIdx.x / heads, sh = blockIdx.x % heads;
@@ -499,6 +547,7 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
     segment_advance(nxt, cum, batch, heads, gap);
     prefetch_l2(p.q + nxt.b * p.q_b + (nxt.h * GROUP + warp) * p.q_h + lane * 8);
   }
+#pragma unroll 1
   for (int s = 0; s < FD_RING; ++s) issue_next();
 
   // ---- consumer: CTA-uniform loop over the pieces of this range
@@ -530,11 +579,12 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
       for (int i = 0; i < 8; ++i)
         if (c0 + i <= c_last) merge_state(m_fin, l_fin, a4, mm[i], ll[i], xx[i]);
     }
-    finish_store(p, sg.b, sg.h * GROUP + hh, d0, a4, l_fin, gate_bits);
+    finish_store(p, sg.b, sg.h * GROUP + hh, d0, a4, l_fin, sigmoid4(gate_bits));
   };
   pdl_wait();  // from here on the predecessor's q / k_new / v_new / gate are read and global memory is written
   if (!q_early) q_raw = load_q_row(p, seg.b, seg.h, tid);
-  stage_q_row(q_s, p, tb, q_raw, pos_s[seg.b], tid);
+  stage_q_row(q_s, p, q_weight, q_freq, q_raw, few ? __shfl_sync(0xffffffffu, my_pos, seg.b) : pos_s[seg.b], tid);
+  if (warp >= 5) cp_async_wait_all();  // weights and frequencies
   __syncthreads();
   while (seg.start < r1 || (cluster_mode && piece == 0)) {  // in cluster mode exactly once, also without units
     const int lo = max(seg.start, r0), hi = min(seg.end, r1);
@@ -562,6 +612,8 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
       fetch_new_rows(tb, p, seg.b, seg.h, lane);
       new_phys = p.block_table[seg.b * p.bt_b + pos_b / PAGE];
     }
+    // (a cluster's only piece: under the wait for its first page)
+    const float4 factor = cluster_mode ? sigmoid4(gate_pf) : make_float4(0.f, 0.f, 0.f, 0.f);
     DecodeWarpState st;
     decode_state_init(st);
     if (lo + warp < hi) decode_load_q(st, q_s + (piece & 1) * GROUP * FD_Q_PITCH, FD_Q_PITCH, lane);
@@ -605,30 +657,47 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
     }
     decode_reduce_l(st);
 
-    // ---- merge the eight warps' states, four at a time
+    // ---- merge the eight warps' states.  Their (m, l) come first, so that the eight weights are taken at once; the accumulators four at
+    // a time, or, in cluster mode, whose only piece leaves the rings idle, all together (the upper four in their own rings)
     float m_all = -INFINITY, l_all = 0.f;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int round = 0; round < FD_WARPS / FD_MERGE_SLOTS; ++round) {
-      if ((warp / FD_MERGE_SLOTS) == round) {
-        float* mine = merge + (warp % FD_MERGE_SLOTS) * FD_PARTIAL_FLOATS;
-        if (lane < 2) {
-          mine[lane * 2] = st.m[0];
-          mine[lane * 2 + 1] = st.m[1];
-          mine[4 + lane * 2] = st.l[0];
-          mine[4 + lane * 2 + 1] = st.l[1];
-        }
-        decode_store_acc_smem(st, mine + 8, lane);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int w = 0; w < FD_MERGE_SLOTS; ++w) {
-        const float* src = merge + w * FD_PARTIAL_FLOATS;
-        merge_state(m_all, l_all, acc, src[hh], src[4 + hh],
-                    *reinterpret_cast<const float4*>(src + 8 + hh * HEAD_DIM + d0));
-      }
-      __syncthreads();  // merge buffer free again
+    if (lane < 2) {
+      s_ml[warp][lane * 2] = st.m[0];
+      s_ml[warp][lane * 2 + 1] = st.m[1];
+      s_ml[warp][4 + lane * 2] = st.l[0];
+      s_ml[warp][4 + lane * 2 + 1] = st.l[1];
     }
+    float* mine = warp < FD_MERGE_SLOTS ? merge + warp * FD_TILE_FLOATS
+                  : cluster_mode        ? reinterpret_cast<float*>(ring)
+                                        : merge + (warp - FD_MERGE_SLOTS) * FD_TILE_FLOATS;
+    if (cluster_mode || warp < FD_MERGE_SLOTS) decode_store_acc_smem(st, mine, lane);
+    __syncthreads();
+    const float m_w = s_ml[lane & (FD_WARPS - 1)][hh];  // a warp's threads belong to one head: lane w takes the weight of warp w
+    m_all = m_w;
+#pragma unroll
+    for (int o = 1; o < FD_WARPS; o <<= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, o));
+    const float weights = m_w == -INFINITY ? 0.f : __expf(m_w - m_all);  // 0: a warp without units
+    l_all = s_ml[lane & (FD_WARPS - 1)][4 + hh] * weights;
+#pragma unroll
+    for (int o = 1; o < FD_WARPS; o <<= 1) l_all += __shfl_xor_sync(0xffffffffu, l_all, o);
+#pragma unroll
+    for (int w = 0; w < FD_WARPS; ++w) {
+      if (w == FD_MERGE_SLOTS && !cluster_mode) {
+        __syncthreads();
+        if (warp >= FD_MERGE_SLOTS) decode_store_acc_smem(st, mine, lane);
+        __syncthreads();
+      }
+      const float* src = w < FD_MERGE_SLOTS ? merge + w * FD_TILE_FLOATS
+                         : cluster_mode     ? reinterpret_cast<const float*>(smem + w * FD_RING * TILE_BYTES_SW)
+                                            : merge + (w - FD_MERGE_SLOTS) * FD_TILE_FLOATS;
+      const float weight = __shfl_sync(0xffffffffu, weights, w);
+      const float4 x = *reinterpret_cast<const float4*>(src + hh * HEAD_DIM + d0);
+      acc[0] = fmaf(x.x, weight, acc[0]);
+      acc[1] = fmaf(x.y, weight, acc[1]);
+      acc[2] = fmaf(x.z, weight, acc[2]);
+      acc[3] = fmaf(x.w, weight, acc[3]);
+    }
+    if (!cluster_mode) __syncthreads();  // merge buffer and (m, l) free again
 
     // a partial left by the previous piece: its arrival ticket was taken by thread 0 while this piece streamed
     if (have_pending) {
@@ -640,27 +709,38 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
       // ---- exchange through distributed shared memory.  Output element e = tid (4 dims of one head) is finished by
       // the CTA of rank e / tpr; every CTA sends each of its 1024 accumulators to the rank that finishes it (slot
       // [own rank][e % tpr] of that CTA's receive buffer) and its (m, l) to everybody, then all meet at the barrier.
-      const int tpr = FD_THREADS / csize;
-      const uint32_t slot = smem_u32(recv + (rank * tpr + (tid % tpr)) * 4);
-      st_cluster_f32x4(cluster_map(slot, static_cast<uint32_t>(tid / tpr)), acc[0], acc[1], acc[2], acc[3]);
-      if ((tid & 63) == 0) {
-        for (int dst = 0; dst < csize; ++dst) {
-          const uint32_t ml = cluster_map(smem_u32(recv_ml + rank * 8), static_cast<uint32_t>(dst));
-          asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ml + hh * 4), "f"(m_all) : "memory");
-          asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ml + 16 + hh * 4), "f"(l_all) : "memory");
-        }
+      const int tpr = FD_THREADS >> clog, to = tid >> (8 - clog), piece_of = tid & (tpr - 1);
+      st_cluster_f32x4(cluster_map(smem_u32(recv + (rank * tpr + piece_of) * 4), static_cast<uint32_t>(to)), acc[0], acc[1], acc[2], acc[3]);
+      if ((tid & 63) < csize) {  // every thread of a head has the head's (m, l): one of them per rank sends it
+        const uint32_t ml = cluster_map(smem_u32(recv_ml + rank * 8), static_cast<uint32_t>(tid & 63));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ml + hh * 4), "f"(m_all) : "memory");
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ml + 16 + hh * 4), "f"(l_all) : "memory");
       }
       cluster_sync();  // release / acquire: every CTA's slices and (m, l) have landed
-      if (tid / tpr == rank) {
-        float m_fin = -INFINITY, l_fin = 0.f;
-        float a4[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int src = 0; src < csize; ++src)
-          merge_state(m_fin, l_fin, a4, recv_ml[src * 8 + hh], recv_ml[src * 8 + 4 + hh],
-                      *reinterpret_cast<const float4*>(recv + (src * tpr + (tid % tpr)) * 4));
-        finish_store(p, seg.b, seg.h * GROUP + hh, d0, a4, l_fin, gate_pf);
+      // lane i takes the weight of source i (a warp's threads belong to one head); every thread goes along, the rank's own store
+      const float m_src = recv_ml[(lane & (csize - 1)) * 8 + hh];
+      float m_fin = m_src;
+#pragma unroll
+      for (int o = 1; o < FD_MAX_CLUSTER; o <<= 1)
+        if (o < csize) m_fin = fmaxf(m_fin, __shfl_xor_sync(0xffffffffu, m_fin, o));
+      const float weights_src = m_src == -INFINITY ? 0.f : __expf(m_src - m_fin);  // 0: a CTA without units
+      float l_fin = recv_ml[(lane & (csize - 1)) * 8 + 4 + hh] * weights_src;
+#pragma unroll
+      for (int o = 1; o < FD_MAX_CLUSTER; o <<= 1)
+        if (o < csize) l_fin += __shfl_xor_sync(0xffffffffu, l_fin, o);
+      float a4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int src = 0; src < csize; ++src) {
+        const float weight = __shfl_sync(0xffffffffu, weights_src, src);
+        const float4 x = *reinterpret_cast<const float4*>(recv + (src * tpr + piece_of) * 4);
+        a4[0] = fmaf(x.x, weight, a4[0]);
+        a4[1] = fmaf(x.y, weight, a4[1]);
+        a4[2] = fmaf(x.z, weight, a4[2]);
+        a4[3] = fmaf(x.w, weight, a4[3]);
       }
+      if (to == rank) finish_store(p, seg.b, seg.h * GROUP + hh, d0, a4, l_fin, factor);
     } else if (whole) {
-      finish_store(p, seg.b, seg.h * GROUP + hh, d0, acc, l_all, gate_pf);
+      finish_store(p, seg.b, seg.h * GROUP + hh, d0, acc, l_all, sigmoid4(gate_pf));
     } else {
       // ---- leave a partial; the last CTA to arrive on this segment merges all of them.  Nobody waits for the
       // ticket here: the result is looked at after the next piece's merge barriers (or after the loop).
@@ -875,6 +955,8 @@ static int fused_decode_impl(const void* q, int64_t q_stride_b, int64_t q_stride
   p.partition = partition;
   p.gap = FD_GAP;
   p.cluster_size = csize;
+  p.cluster_log2 = 0;
+  while ((1 << p.cluster_log2) < csize) ++p.cluster_log2;
   cudaError_t launched;
   // Also a call without flags is launched with the attribute: the kernel then waits for its predecessor before it reads
   // anything, but its launch does not.  Six layers of 32 sequences 198.7 -> 195.1 us, of one 64.6 -> 64.2 (graph replays).
