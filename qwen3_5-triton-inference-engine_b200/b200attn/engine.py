@@ -16,6 +16,7 @@ import numpy as np
 import torch
 
 from . import glue, glue_ops, ops
+from .host import token_array, upload
 from .slots import SlotEngine
 
 
@@ -159,26 +160,26 @@ class Engine(SlotEngine):
         cfg = self.cfg
         assert all(0 < len(p) <= self.max_context for p in prompts)
         lengths = [len(p) for p in prompts]
-        if slots is not None:
-            slots = torch.tensor(slots, dtype=torch.int64, device=self.device)
-        table = self.block_table if slots is None else self.block_table.index_select(0, slots)
 
         def put(dst, src):          # write a per-sequence result into all slots, or into the chosen ones
             if slots is None:
                 dst.copy_(src)
             else:
                 dst.index_copy_(0, slots, src.to(dst.dtype))
-        # ids, position inside the sequence and first packed row of the sequence (runner.py:136) for every token, built
-        # on the host and sent as one int32 [3, T] array
+        # ids, position inside the sequence and first packed row of the sequence (runner.py:136) for every token, then cumulative
+        # lengths, lengths, last rows and slots of the sequences: built on the host and sent as one int32 array, without waiting
         lens = np.asarray(lengths, dtype=np.int64)
-        first_row = np.repeat(np.cumsum(lens) - lens, lens)
-        host = np.empty((3, int(lens.sum())), dtype=np.int32)
-        host[0] = np.fromiter((t for p in prompts for t in p), dtype=np.int64, count=host.shape[1])
-        host[1] = np.arange(host.shape[1]) - first_row
-        host[2] = first_row
-        ids, pos_in_seq, seq_start = torch.from_numpy(host).to(self.device).unbind(0)
-        cu, max_len = ops.build_cu_seqlens(lengths, device=self.device)
-        total, heads, dim = ids.numel(), cfg.gdn_heads, cfg.gdn_dim
+        total, count, max_len = int(lens.sum()), len(lengths), max(lengths)
+        ends = np.cumsum(lens)
+        first_row = np.repeat(ends - lens, lens)
+        host = np.concatenate((token_array(prompts, np.int64), np.arange(total) - first_row, first_row, [0], ends, lens, ends - 1,
+                               np.asarray([] if slots is None else slots, dtype=np.int64))).astype(np.int32)
+        ids, pos_in_seq, seq_start, cu, sent_lens, last_rows, sent_slots = upload(host, self.device).split(
+            [total, total, total, count + 1, count, count, host.size - 3 * total - 3 * count - 1])
+        if slots is not None:
+            slots = sent_slots.long()
+        table = self.block_table if slots is None else self.block_table.index_select(0, slots)
+        heads, dim = cfg.gdn_heads, cfg.gdn_dim
         if not self.fused_glue:
             assert slots is None, "slot-wise prefill runs on the single-launch operators only"
             return self._prefill_eager_glue(ids, cu, max_len, pos_in_seq, seq_start, lengths)
@@ -221,9 +222,8 @@ class Engine(SlotEngine):
             gate_up = glue.gemm_2d(h, layer["gate_up"])
             pending = glue.gemm_2d(_swiglu(gate_up[:, : cfg.intermediate], gate_up[:, cfg.intermediate:]), layer["down"])
         x = glue.residual_add(pending, x)
-        last = x.index_select(0, cu[1:].long() - 1)
-        first = self._head(last)
-        put(self.pos, torch.tensor(lengths, dtype=torch.int64, device=self.device))
+        first = self._head(x.index_select(0, last_rows))
+        put(self.pos, sent_lens)
         put(self.tok, first)
         return first.clone()
 

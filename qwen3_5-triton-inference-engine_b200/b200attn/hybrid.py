@@ -19,6 +19,7 @@ from . import hybrid_ops as hops
 from . import ops
 from . import cores
 from .cores import CoreMixer, FusedUnit, GatedMLP
+from .host import token_array, upload
 from .mixers import FEED_FORWARDS, MIXERS, padded, round_up
 from .slots import SlotEngine
 
@@ -234,12 +235,12 @@ class PackedBatch:
         ends = np.cumsum(lens, dtype=np.int32)
         n, total = self.count, self.tokens
         host = np.empty(3 * total + 3 * n + 1, dtype=np.int32)
-        host[:total] = np.fromiter((t for p in portions for t in p), dtype=np.int32, count=total)
+        host[:total] = token_array(portions)
         host[total: 2 * total] = np.arange(total) - np.repeat(ends - lens - np.asarray(starts, dtype=np.int32), lens)
         host[2 * total: 3 * total] = np.repeat(np.asarray(slots, dtype=np.int32), lens)
         tail = host[3 * total:]
         tail[:n], tail[n: 2 * n], tail[2 * n], tail[2 * n + 1:] = slots, starts, 0, ends
-        self.ids, self.pos, self.slot_of, rest = torch.from_numpy(host).to(device).split([total, total, total, 3 * n + 1])
+        self.ids, self.pos, self.slot_of, rest = upload(host, device).split([total, total, total, 3 * n + 1])
         self.slots, self.start, self.cu = rest.split([n, n, n + 1])
         self.kept: dict = {}              # gathered contexts: layers that share a latent and a window share the rows too
         self._spans: dict[int, KeySpan] = {}
@@ -253,7 +254,7 @@ class PackedBatch:
             old = [s - f for s, f in zip(self.starts, first)]
             ends = np.cumsum(self.lengths)
             rows = np.arange(self.tokens) + np.repeat(cu[:-1] + old - (ends - self.lengths), self.lengths)
-            host = torch.from_numpy(np.concatenate((cu, first, rows)).astype(np.int32)).to(self.device)
+            host = upload(np.concatenate((cu, first, rows)).astype(np.int32), self.device)
             cu, pos, rows = host.split([self.count + 1, self.count, self.tokens])
             span = self._spans[window] = KeySpan(cu, pos, rows, sum(counts), max(counts), max(old))
         return span
@@ -370,7 +371,7 @@ class HybridEngine(SlotEngine):
         return h
 
     def _set_pos(self, slots, ends) -> None:
-        at = torch.tensor([slots, ends], dtype=torch.int64, device=self.device)
+        at = upload([slots, ends], self.device, torch.int64)
         self.pos.index_copy_(0, at[0], at[1])
 
     @torch.no_grad()
@@ -398,13 +399,13 @@ class HybridEngine(SlotEngine):
             first += len(p)
         if not rows:
             return torch.empty(0, self.cfg.vocab, device=self.device)
-        return self.logits(h.index_select(0, torch.tensor(rows, device=self.device)))[:, : self.cfg.vocab]
+        return self.logits(h.index_select(0, upload(rows, self.device)))[:, : self.cfg.vocab]
 
     def _extend_by_one(self, slots, starts, portions, want) -> torch.Tensor:
         """One token for some slots through the decode step; the other slots are masked out."""
         others = self.active.clone()
         self.set_active([b in slots for b in range(self.batch)])
-        at = torch.tensor([slots, starts, [p[0] for p in portions]], dtype=torch.int64, device=self.device)
+        at = upload([slots, starts, [p[0] for p in portions]], self.device, torch.int64)
         self.pos.index_copy_(0, at[0], at[1])
         tok = self.tok.index_copy(0, at[0], at[2])
         h = self._decode_hidden(tok, False)
@@ -413,7 +414,7 @@ class HybridEngine(SlotEngine):
         rows = [s for s, w in zip(slots, want) for _ in w]
         if not rows:
             return torch.empty(0, self.cfg.vocab, device=self.device)
-        return self.logits(h.index_select(0, torch.tensor(rows, device=self.device)))[:, : self.cfg.vocab]
+        return self.logits(h.index_select(0, upload(rows, self.device)))[:, : self.cfg.vocab]
 
     def _prefill(self, prompts, slots):
         slots = list(range(self.batch)) if slots is None else slots
@@ -427,11 +428,11 @@ class HybridEngine(SlotEngine):
             h = self._forward(batch)
             done = [k for k, i in enumerate(live) if len(prompts[i]) <= start + cut]
             if done:
-                rows = batch.cu[1:].long()[torch.tensor(done, device=self.device)] - 1
+                rows = batch.cu[1:].long()[upload(done, self.device)] - 1
                 ids = ops.argmax_rows(self.logits(h.index_select(0, rows), cap=False), self.argmax_ws)
-                first[torch.tensor([live[k] for k in done], device=self.device)] = ids
+                first[upload([live[k] for k in done], self.device)] = ids
         self._set_pos(slots, [len(p) for p in prompts])
-        self.tok.index_copy_(0, torch.tensor(slots, dtype=torch.int64, device=self.device), first)
+        self.tok.index_copy_(0, upload(slots, self.device, torch.int64), first)
         return first.clone()
 
     # ------------------------------------------------------------------------------------------------------- decode

@@ -24,6 +24,8 @@ from dataclasses import dataclass, field
 
 import torch
 
+from .host import upload
+
 PAGE_SIZE = 16
 
 
@@ -71,7 +73,7 @@ class PageAllocator:
             raise PoolExhausted(f"{missing} pages wanted for slot {slot}, {len(self._free)} free of {self.num_pages - 1}")
         new = self._free[-missing:]
         del self._free[-missing:]
-        self.block_table[slot, len(held): need] = torch.tensor(new, dtype=torch.int32, device=self.block_table.device)
+        self.block_table[slot, len(held): need] = upload(new, self.block_table.device, torch.int32)
         held.extend(new)
         return missing
 
