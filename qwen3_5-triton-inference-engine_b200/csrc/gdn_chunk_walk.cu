@@ -511,14 +511,21 @@ __global__ void __launch_bounds__(32 * (WARPS + GW_COPY_WARPS), 1) gdn_walk_kern
 // Few heads leave the warps above alone on their schedulers, where the chain of a chunk's products sets the time (3.4 us per
 // chunk).  Here four warps share 16 value columns: a warp computes 16 of the chunk's tokens in k S, q S, delta and o, and keeps
 // 32 of the state's key dims; S, R and delta go round as left-operand fragments in shared memory, a lane's four registers being
-// 16 consecutive bytes, so that nothing is rearranged.  Three meetings per chunk, each through an mbarrier; what nobody waits for (q S, A
-// delta) comes behind the last one.
-constexpr int GT_S = 0, GT_R = GT_S + 8 * 1024, GT_D = GT_R + 4 * 1024, GT_E = GT_D + 4 * 1024, GT_BYTES = GT_E + 4 * 1024;   // hi, lo: 512 bytes each
-
+// 16 consecutive bytes, so that nothing is rearranged.  Three meetings per chunk, each through an mbarrier.  What nobody waits for, the
+// output q S + A delta, comes behind the last one; or, with one team per CTA, four more warps compute it one chunk behind (APART),
+// which takes it off the chain that the chunks are: one sequence of 2048 tokens 80.7 -> 77.8 us (with prep), of 8192 298 -> 286; without any
+// output it would be 73 and 268.  S and delta then have two places and two barriers each, by turns: the team in front may be a chunk ahead, and
+// must not come round to a place, or a phase, that is still waited for.  Not kept: bulk copies of rows instead of 16-byte pieces (60 cycles
+// each, 216 us), three stages (no change), the output's first read behind R (79), rolled products (79 to 82).
 template <int TEAMS>
 struct TeamSmem {
   using L = WalkSmem<16 * TEAMS>;
-  static constexpr int EX = (L::BYTES + 127) / 128 * 128, BARS = EX + TEAMS * GT_BYTES, BYTES = BARS + TEAMS * 32;
+  static constexpr bool APART = TEAMS == 1;
+  static constexpr int PLACES = APART ? 2 : 1;
+  static constexpr int S = 0, S_STEP = 8 * 1024, R = S + PLACES * S_STEP, E = R + 4 * 1024, D = E + 4 * 1024, D_STEP = 4 * 1024;   // hi, lo: 512 bytes each
+  static constexpr int EX = (L::BYTES + 127) / 128 * 128, EX_BYTES = D + PLACES * D_STEP, BARS = EX + TEAMS * EX_BYTES, BYTES = BARS + TEAMS * 64;
+  static constexpr int BAR_S = 0, BAR_R = 2, BAR_D = 3, BAR_OUT = 5;   // two each where there are two places, but for R
+  static constexpr int WARPS = (APART ? 8 : 4) * TEAMS, THREADS = 32 * (WARPS + GW_COPY_WARPS);
 };
 
 __device__ __forceinline__ void put_frag(uint8_t* to, const uint32_t (&hi)[4], const uint32_t (&lo)[4], int lane) {
@@ -557,39 +564,152 @@ __device__ __forceinline__ bool team_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// o^T of a warp's 16 tokens: e^G (q S)^T, and A delta from its own fragments (dh, dl) and those of the tokens before, at `d`
+__device__ __forceinline__ void query_state(float (&O)[2][4], const uint32_t (&sh)[8][4], const uint32_t (&sl)[8][4], uint32_t q, const float* eg, int c2) {
+  float m[2][2][4] = {};
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    uint32_t b[4];
+    ldmatrix_x4(b, q + ks * 32);
+    mma_bf16_16816(m[0][0], sh[ks], b[0], b[1]);
+    mma_bf16_16816(m[1][0], sh[ks], b[2], b[3]);
+    mma_bf16_16816(m[0][1], sl[ks], b[0], b[1]);
+    mma_bf16_16816(m[1][1], sl[ks], b[2], b[3]);
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    const float2 e = *reinterpret_cast<const float2*>(eg + n * 8 + c2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) O[n][j] = (m[n][0][j] + m[n][1][j]) * ((j & 1) ? e.y : e.x);
+  }
+}
+__device__ __forceinline__ void add_within(float (&O)[2][4], const uint32_t (&dh)[4], const uint32_t (&dl)[4], const uint8_t* d, const uint8_t* fa, int w, int lane) {
+  float x[2][3][4] = {};
+  pair_products(x, dh, dl, *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w) + w) * 512 + lane * 16),
+                *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w + 1) + w) * 512 + lane * 16));
+#pragma unroll
+  for (int ks = 0; ks < 3; ++ks) {
+    if (ks >= w) break;
+    uint32_t xh[4], xl[4];
+    get_frag(d + ks * 1024, xh, xl, lane);
+    pair_products(x, xh, xl, *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w) + ks) * 512 + lane * 16),
+                  *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w + 1) + ks) * 512 + lane * 16));
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) O[n][j] += x[n][0][j] + x[n][1][j] + x[n][2][j];
+}
+// ... through the own rows of the value tile, 32 bytes per token
+__device__ __forceinline__ void store_tokens(const float (&O)[2][4], uint32_t tile, const uint8_t* rows, int pitch, __nv_bfloat16* out, int64_t o_t, int tokens, int lane) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(tile), "r"(pack_bf16(O[0][0], O[0][1])),
+               "r"(pack_bf16(O[0][2], O[0][3])), "r"(pack_bf16(O[1][0], O[1][1])), "r"(pack_bf16(O[1][2], O[1][3]))
+               : "memory");
+  __syncwarp();
+  const int t = lane >> 1, c = (lane & 1) * 8;
+  if (t < tokens) *reinterpret_cast<uint4*>(out + t * o_t + c) = *reinterpret_cast<const uint4*>(rows + (t * pitch + c) * 2);
+}
+
 template <int TEAMS, bool WINDOWS>
-__global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_team_kernel(const __grid_constant__ GdnWalkParams p) {
+__global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_kernel(const __grid_constant__ GdnWalkParams p) {
   using L = WalkSmem<16 * TEAMS>;
   using T = TeamSmem<TEAMS>;
   constexpr int SPLIT = 8 / TEAMS;
   extern __shared__ __align__(16) uint8_t smem[];
-  const int tid = threadIdx.x, lane = tid & 31, team = tid >> 7, w = (tid >> 5) & 3;
+  const int tid = threadIdx.x, lane = tid & 31, w = (tid >> 5) & 3;
   uint64_t *full = reinterpret_cast<uint64_t*>(smem + L::BARS), *empty = full + GW_STAGES;
   if (tid == 0) {
-    init_stages<16 * TEAMS>(smem, 4 * TEAMS);
-    for (int i = 0; i < TEAMS * 4; ++i) mbar_init(reinterpret_cast<uint64_t*>(smem + T::BARS) + i, 4);
+    init_stages<16 * TEAMS>(smem, T::WARPS);
+    for (int i = 0; i < TEAMS * 8; ++i) mbar_init(reinterpret_cast<uint64_t*>(smem + T::BARS) + i, 4);
     mbar_fence_init();
   }
   __syncthreads();
-  if (team == TEAMS) {
-    copy_chunks<16 * TEAMS, WINDOWS>(p, smem, tid - 128 * TEAMS);
+  if (tid >= 32 * T::WARPS) {
+    copy_chunks<16 * TEAMS, WINDOWS>(p, smem, tid - 32 * T::WARPS);
     return;
   }
-  uint8_t* ex = smem + T::EX + team * GT_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::BARS) + team * 4;   // S, R, delta
-  uint32_t parity_s = 0, parity = 0, full_parity = 0;
+  const bool output_team = T::APART && tid >= 128;
+  const int team = T::APART ? 0 : tid >> 7;
+  uint8_t* ex = smem + T::EX + team * T::EX_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::BARS) + team * 8;
+  uint32_t states = 0, chunks = 0, outputs = 0, full_parity = 0;   // states taken over, chunks begun, outputs waited for, so far
   auto arrive = [&](int i) {
     __syncwarp();
     if (lane == 0) mbar_arrive(&bars[i]);
   };
-  // S^T: value column lane / 4 (+ 8) of the team's 16, key dims 32 w + 8 n + (lane % 4) * 2 (+ 1)
-  float S[4][4] = {};
   const int gr = lane >> 2, c2 = (lane & 3) * 2;
   const uint32_t nk_off = ((w * 16 + (lane >> 4) * 8 + (lane & 7)) * GW_PITCH + ((lane >> 3) & 1) * 8) * 2;
-  const uint32_t kn_off = ((((lane >> 3) & 1) * 8 + (lane & 7)) * GW_PITCH + w * 32 + (lane >> 4) * 8) * 2;
   const uint32_t v_off = ((w * 16 + (lane >> 4) * 8 + (lane & 7)) * L::VP + team * 16 + ((lane >> 3) & 1) * 8) * 2;
+  const int v_rows = L::V + (w * 16 * L::VP + team * 16) * 2;
   int stage = 0, bh = 0, h = 0, col = 0;
   bool ok = true;
+  auto place = [&](uint32_t n) { return T::APART ? n & 1 : 0; };
+  // barrier and phase of the n-th state, delta or output
+  auto bar_of = [&](int first, uint32_t n) { return first + place(n); };
+  auto phase_of = [&](uint32_t n) { return T::APART ? (n >> 1) & 1 : n & 1; };
+
+  if (output_team) {
+    for (;;) {
+      ok = warp_wait_bounded(&full[stage], full_parity, ok);
+      if (!ok) break;
+      const int4 info = *reinterpret_cast<const int4*>(smem + L::INFO + stage * 16);
+      if (info.x < 0) return;
+      if (info.w & (WINDOWS ? 6 : 2)) bh = info.x / SPLIT, h = bh % p.heads, col = info.x % SPLIT * 16;
+      if (info.z > 0) {
+        const uint8_t* st = smem + stage * L::STAGE;
+        const uint8_t* fa = st + L::P + GW_MAT_BYTES;
+        const float* eg = reinterpret_cast<const float*>(fa + GW_MAT_BYTES) + w * 16;
+        const bool mine = info.z > 16 * w;
+        float O[2][4] = {};
+        if (!(info.w & 2)) {
+          ok = ok && team_wait(&bars[bar_of(T::BAR_S, states)], phase_of(states));
+          if (mine) {
+            uint32_t sh[8][4], sl[8][4];
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) get_frag(ex + T::S + place(states) * T::S_STEP + ks * 1024, sh[ks], sl[ks], lane);
+            query_state(O, sh, sl, smem_u32(st) + L::Q + nk_off, eg, c2);
+          }
+          ++states;
+        }
+        ok = ok && team_wait(&bars[bar_of(T::BAR_D, chunks)], phase_of(chunks));
+        if (mine) {
+          const uint8_t* d = ex + T::D + place(chunks) * T::D_STEP;
+          uint32_t dh[4], dl[4];
+          get_frag(d + w * 1024, dh, dl, lane);
+          add_within(O, dh, dl, d, fa, w, lane);
+          store_tokens(O, smem_u32(st) + L::V + v_off, st + v_rows, L::VP, p.out + (static_cast<int64_t>(info.y) + w * 16) * p.o_t + h * p.o_h + col,
+                       p.o_t, ok ? info.z - w * 16 : 0, lane);
+        }
+        arrive(bar_of(T::BAR_OUT, chunks));
+        ++chunks;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[stage]);
+      if (++stage == GW_STAGES) stage = 0, full_parity ^= 1;
+    }
+    if (lane == 0) atomicExch(p.err, 1);
+    return;
+  }
+
+  // S^T: value column lane / 4 (+ 8) of the team's 16, key dims 32 w + 8 n + (lane % 4) * 2 (+ 1)
+  float S[4][4] = {};
+  const uint32_t kn_off = ((((lane >> 3) & 1) * 8 + (lane & 7)) * GW_PITCH + w * 32 + (lane >> 4) * 8) * 2;
+  uint32_t published = 0;
+  // the other team has done with every chunk before this one (their places may be written again, their phases are over)
+  auto outputs_done = [&]() {
+    if constexpr (T::APART)
+      for (; outputs < chunks; ++outputs) ok = ok && team_wait(&bars[bar_of(T::BAR_OUT, outputs)], phase_of(outputs));
+  };
+  auto publish = [&]() {
+    uint8_t* to = ex + T::S + place(published) * T::S_STEP + 2 * w * 1024;
+    uint32_t hi[4], lo[4];
+    split_frag(S[0], S[1], hi, lo);
+    put_frag(to, hi, lo, lane);
+    split_frag(S[2], S[3], hi, lo);
+    put_frag(to + 1024, hi, lo, lane);
+    arrive(bar_of(T::BAR_S, published));
+    ++published;
+  };
   for (;;) {
     ok = warp_wait_bounded(&full[stage], full_parity, ok);
     if (!ok) break;
@@ -602,12 +722,8 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
       for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j) S[n][j] = from[(n * 8 + c2 + (j & 1)) * GDN_D + gr + (j >> 1) * 8];
-      uint32_t hi[4], lo[4];
-      split_frag(S[0], S[1], hi, lo);
-      put_frag(ex + GT_S + 2 * w * 1024, hi, lo, lane);
-      split_frag(S[2], S[3], hi, lo);
-      put_frag(ex + GT_S + (2 * w + 1) * 1024, hi, lo, lane);
-      arrive(0);
+      outputs_done();
+      publish();
     }
     if (info.z > 0) {
       const uint8_t* st = smem + stage * L::STAGE;
@@ -619,15 +735,15 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
       uint32_t rh[4], rl[4], sh[8][4], sl[8][4];
       float O[2][4] = {}, D[2][4] = {};
       if (carry) {
-        ok = ok && team_wait(&bars[0], parity_s);
-        parity_s ^= 1;
+        ok = ok && team_wait(&bars[bar_of(T::BAR_S, states)], phase_of(states));
+        ++states;
       }
       if (mine) {
         // ---- k S of the own tokens, R
         float m[2][2][4] = {};
         if (carry) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) get_frag(ex + GT_S + ks * 1024, sh[ks], sl[ks], lane);
+          for (int ks = 0; ks < 8; ++ks) get_frag(ex + T::S + place(states - 1) * T::S_STEP + ks * 1024, sh[ks], sl[ks], lane);
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
             uint32_t b[4];
@@ -650,9 +766,9 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
           R[n][3] = fmaf(-e.y, m[n][0][3] + m[n][1][3], bf16_hi(v[2 * n + 1]));
         }
         split_frag(R[0], R[1], rh, rl);
-        put_frag(ex + GT_R + w * 1024, rh, rl, lane);
+        put_frag(ex + T::R + w * 1024, rh, rl, lane);
       }
-      arrive(1);
+      arrive(T::BAR_R);
       const float keep = eg[CHUNK - 1];
 #pragma unroll
       for (int n = 0; n < 4; ++n) S[n][0] *= keep, S[n][1] *= keep, S[n][2] *= keep, S[n][3] *= keep;
@@ -660,14 +776,15 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
       if (mine)                                         // the own tokens' part of delta
         pair_products(s, rh, rl, *reinterpret_cast<const uint4*>(fp + (frag_row(2 * w) + w) * 512 + lane * 16),
                       *reinterpret_cast<const uint4*>(fp + (frag_row(2 * w + 1) + w) * 512 + lane * 16));
-      ok = ok && team_wait(&bars[1], parity);
+      ok = ok && team_wait(&bars[T::BAR_R], chunks & 1);
+      uint8_t* d = ex + T::D + place(chunks) * T::D_STEP;
       uint32_t dh[4], dl[4], eh[4], el[4];
       if (mine) {
 #pragma unroll
         for (int ks = 0; ks < 3; ++ks) {
           if (ks >= w) break;
           uint32_t xh[4], xl[4];
-          get_frag(ex + GT_R + ks * 1024, xh, xl, lane);
+          get_frag(ex + T::R + ks * 1024, xh, xl, lane);
           pair_products(s, xh, xl, *reinterpret_cast<const uint4*>(fp + (frag_row(2 * w) + ks) * 512 + lane * 16),
                         *reinterpret_cast<const uint4*>(fp + (frag_row(2 * w + 1) + ks) * 512 + lane * 16));
         }
@@ -682,19 +799,18 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
           }
         }
         split_frag(x[0], x[1], eh, el);
-        put_frag(ex + GT_E + w * 1024, eh, el, lane);
+        put_frag(ex + T::E + w * 1024, eh, el, lane);
         split_frag(D[0], D[1], dh, dl);
-        put_frag(ex + GT_D + w * 1024, dh, dl, lane);
+        put_frag(d + w * 1024, dh, dl, lane);
       }
-      arrive(2);
-      ok = ok && team_wait(&bars[2], parity);
-      parity ^= 1;
+      arrive(bar_of(T::BAR_D, chunks));
+      ok = ok && team_wait(&bars[bar_of(T::BAR_D, chunks)], phase_of(chunks));
       // ---- the own key dims of the state
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         if (ks >= groups) break;
         uint32_t xh[4], xl[4], a[4], b[4];
-        get_frag(ex + GT_E + ks * 1024, xh, xl, lane);
+        get_frag(ex + T::E + ks * 1024, xh, xl, lane);
         ldmatrix_x4_trans(a, at + L::K + kn_off + ks * 16 * GW_PITCH * 2);
         ldmatrix_x4_trans(b, at + L::K + kn_off + ks * 16 * GW_PITCH * 2 + 32);
         mma_bf16_16816(S[0], xh, a[0], a[1]);
@@ -706,58 +822,14 @@ __global__ void __launch_bounds__(32 * (4 * TEAMS + GW_COPY_WARPS), 1) gdn_walk_
         mma_bf16_16816(S[2], xl, b[0], b[1]);
         mma_bf16_16816(S[3], xl, b[2], b[3]);
       }
-      if (!last) {
-        uint32_t hi[4], lo[4];
-        split_frag(S[0], S[1], hi, lo);
-        put_frag(ex + GT_S + 2 * w * 1024, hi, lo, lane);
-        split_frag(S[2], S[3], hi, lo);
-        put_frag(ex + GT_S + (2 * w + 1) * 1024, hi, lo, lane);
-        arrive(0);
-      }
-      if (mine && carry) {                              // q S of the own tokens, where nobody waits for it any more
-        float m[2][2][4] = {};
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          uint32_t b[4];
-          ldmatrix_x4(b, at + L::Q + nk_off + ks * 32);
-          mma_bf16_16816(m[0][0], sh[ks], b[0], b[1]);
-          mma_bf16_16816(m[1][0], sh[ks], b[2], b[3]);
-          mma_bf16_16816(m[0][1], sl[ks], b[0], b[1]);
-          mma_bf16_16816(m[1][1], sl[ks], b[2], b[3]);
-        }
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          const float2 e = *reinterpret_cast<const float2*>(eg + w * 16 + n * 8 + c2);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) O[n][j] = (m[n][0][j] + m[n][1][j]) * ((j & 1) ? e.y : e.x);
-        }
-      }
-      // ---- o of the own tokens: A delta, then out through the own rows of the value tile
-      if (mine) {
-        float x[2][3][4] = {};
-        pair_products(x, dh, dl, *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w) + w) * 512 + lane * 16),
-                      *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w + 1) + w) * 512 + lane * 16));
-#pragma unroll
-        for (int ks = 0; ks < 3; ++ks) {
-          if (ks >= w) break;
-          uint32_t xh[4], xl[4];
-          get_frag(ex + GT_D + ks * 1024, xh, xl, lane);
-          pair_products(x, xh, xl, *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w) + ks) * 512 + lane * 16),
-                        *reinterpret_cast<const uint4*>(fa + (frag_row(2 * w + 1) + ks) * 512 + lane * 16));
-        }
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) O[n][j] += x[n][0][j] + x[n][1][j] + x[n][2][j];
-        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(at + L::V + v_off),
-                     "r"(pack_bf16(O[0][0], O[0][1])), "r"(pack_bf16(O[0][2], O[0][3])), "r"(pack_bf16(O[1][0], O[1][1])),
-                     "r"(pack_bf16(O[1][2], O[1][3]))
-                     : "memory");
-        __syncwarp();
-        const int t = w * 16 + (lane >> 1), c = (lane & 1) * 8;
-        if (t < info.z && ok)
-          *reinterpret_cast<uint4*>(p.out + (static_cast<int64_t>(info.y) + t) * p.o_t + h * p.o_h + col + c) =
-              *reinterpret_cast<const uint4*>(st + L::V + (t * L::VP + team * 16 + c) * 2);
+      outputs_done();
+      if (!last) publish();
+      ++chunks;
+      if (!T::APART && mine) {                          // the output, where nobody waits for it any more
+        if (carry) query_state(O, sh, sl, at + L::Q + nk_off, eg + w * 16, c2);
+        add_within(O, dh, dl, d, fa, w, lane);
+        store_tokens(O, at + L::V + v_off, st + v_rows, L::VP, p.out + (static_cast<int64_t>(info.y) + w * 16) * p.o_t + h * p.o_h + col, p.o_t,
+                     ok ? info.z - w * 16 : 0, lane);
       }
     }
     __syncwarp();
@@ -801,11 +873,11 @@ int prep_and_walk(const GdnWalkParams& p, cudaStream_t st) {
   if (const int rc = check_launch("gdn_chunked_prefill_walk (prep)")) return rc;
   const int pairs = p.heads * p.batch, sms = sm_count();
   constexpr int copy = 32 * GW_COPY_WARPS;
-  // What fills the device: four warps per 16 value columns while that leaves SMs free (one sequence of 2048 tokens: 80 us against
+  // What fills the device: four warps per 16 value columns while that leaves SMs free (one sequence of 2048 tokens: 77 us against
   // 122 on half-head CTAs and 199 on whole heads), two such teams per CTA (2 x 1000..3000: 114 against 135 and 215), half a head
   // per CTA (4 x 2048: 148 against 214 in teams and 225 on whole heads), whole heads (8 x 1024: 133 against 148).
-  if (pairs * 8 <= sms) return launch_walk(gdn_walk_team_kernel<1, WINDOWS>, 128 + copy, TeamSmem<1>::BYTES, 8, p, st);
-  if (pairs * 4 <= sms) return launch_walk(gdn_walk_team_kernel<2, WINDOWS>, 256 + copy, TeamSmem<2>::BYTES, 4, p, st);
+  if (pairs * 8 <= sms) return launch_walk(gdn_walk_team_kernel<1, WINDOWS>, TeamSmem<1>::THREADS, TeamSmem<1>::BYTES, 8, p, st);
+  if (pairs * 4 <= sms) return launch_walk(gdn_walk_team_kernel<2, WINDOWS>, TeamSmem<2>::THREADS, TeamSmem<2>::BYTES, 4, p, st);
   if (pairs * 2 <= sms) return launch_walk(gdn_walk_kernel<4, WINDOWS>, 128 + copy, WalkSmem<64>::BYTES, 2, p, st);
   return launch_walk(gdn_walk_kernel<8, WINDOWS>, 256 + copy, WalkSmem<128>::BYTES, 1, p, st);
 }
