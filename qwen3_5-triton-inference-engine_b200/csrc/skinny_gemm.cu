@@ -34,6 +34,7 @@ constexpr int SG_STD_WARPS = SG_WARPS * SG_KSPLIT;
 constexpr int SG_STD_THREADS = SG_STD_WARPS * 32;
 constexpr int SG_STD_RING = SG_RING / SG_KSPLIT;  // the same bytes in flight per CTA
 constexpr int SG_MAX_M = 32;
+constexpr int SG_X_TILE_BYTES = SG_MAX_M * SG_TILE_K * 2;   // 128 k of 32 batch rows
 constexpr int SG_MAX_K = 1280;           // X staging: 32 x (K*2 + 16) bytes next to 128 KiB of weight rings
 
 struct SkinnyGemmParams {
@@ -56,15 +57,18 @@ template <int NT>
 struct StepProducts;
 template <>
 struct StepProducts<4> {
-  // ldmatrix lane address of X: row = (lane & 7) + 8 * (lane >> 4) inside a 16-row pair, k half = (lane >> 3) & 1
-  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
-    return static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * x_pitch + ((lane >> 3) & 1) * 16);
+  // X tiles as tensor-map boxes of 128 k: two blocks of [32 rows][64 k] with the 128-byte swizzle.  Lane address: row = (lane & 7) + 8 *
+  // (lane >> 4) inside a 16-row pair, k half = (lane >> 3) & 1; a step's 32 bytes are two bits of the address to turn over
+  static __device__ __forceinline__ uint32_t lane_offset(int lane, int) {
+    return static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * 128 + (((lane >> 3) & 1) ^ (lane & 7)) * 16);
   }
+  static __device__ __forceinline__ uint32_t tile_offset(int kt) { return kt * SG_X_TILE_BYTES; }
   template <int KS>
-  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xt, int) {
     uint32_t b01[4], b23[4];
+    const uint32_t xk = (xt + (KS >> 2) * (SG_X_TILE_BYTES / 2)) ^ ((KS & 3) * 32);
     ldmatrix_x4(b01, xk);                   // batch rows 0-15: (b0, b1) of n8 tiles 0 and 1
-    ldmatrix_x4(b23, xk + 16 * x_pitch);    // batch rows 16-31
+    ldmatrix_x4(b23, xk + 16 * 128);        // batch rows 16-31
     mma_bf16_16816(acc[0], a, b01[0], b01[1]);
     mma_bf16_16816(acc[1], a, b01[2], b01[3]);
     mma_bf16_16816(acc[2], a, b23[0], b23[1]);
@@ -73,11 +77,15 @@ struct StepProducts<4> {
 };
 template <>
 struct StepProducts<2> {
-  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) { return StepProducts<4>::lane_offset(lane, x_pitch); }
+  // rows x_pitch bytes apart: row = (lane & 7) + 8 * (lane >> 4) of sixteen, k half = (lane >> 3) & 1
+  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
+    return static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * x_pitch + ((lane >> 3) & 1) * 16);
+  }
+  static __device__ __forceinline__ uint32_t tile_offset(int kt) { return kt * SG_TILE_K * 2; }
   template <int KS>
   static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
     uint32_t b01[4];
-    ldmatrix_x4(b01, xk);
+    ldmatrix_x4(b01, xk + KS * 32);
     mma_bf16_16816(acc[(KS & 1) * 2], a, b01[0], b01[1]);
     mma_bf16_16816(acc[(KS & 1) * 2 + 1], a, b01[2], b01[3]);
   }
@@ -88,10 +96,11 @@ struct StepProducts<1> {
   static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
     return static_cast<uint32_t>((lane & 7) * x_pitch + (lane >> 3) * 16);
   }
+  static __device__ __forceinline__ uint32_t tile_offset(int kt) { return kt * SG_TILE_K * 2; }
   template <int KS>
   static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
     uint32_t (&b4)[4] = *reinterpret_cast<uint32_t (*)[4]>(b);
-    if constexpr ((KS & 1) == 0) ldmatrix_x4(b4, xk);
+    if constexpr ((KS & 1) == 0) ldmatrix_x4(b4, xk + KS * 32);
     mma_bf16_16816(acc[KS & 3], a, b[(KS & 1) * 2], b[(KS & 1) * 2 + 1]);
   }
 };
@@ -112,7 +121,7 @@ __device__ __forceinline__ void tile_steps(float (&acc)[4][4], uint32_t (&b)[8],
   if constexpr (KS < SG_TILE_K / 16) {
     uint32_t a[4];
     ldmatrix_x4(a, tile + offset(KS));
-    StepProducts<NT>::template run<KS>(acc, a, b, xk + KS * 32, x_pitch);
+    StepProducts<NT>::template run<KS>(acc, a, b, xk, x_pitch);
     tile_steps<NT, KS + 1>(acc, b, tile, xk, x_pitch, offset);
   }
 }
@@ -144,20 +153,20 @@ __device__ __forceinline__ void stage_rows(uint8_t* xs, int x_pitch, const __nv_
   }
 }
 constexpr int skinny_smem(int nt, int k) {  // rings, output staging, odd-tile sums, X
-  return SG_WARPS * SG_RING_BYTES + nt * 8 * SG_ROWS * 2 + nt * 4 * SG_WARPS * 32 * 4 + nt * 8 * (k * 2 + 16) + 1024;
+  return SG_WARPS * SG_RING_BYTES + nt * 8 * SG_ROWS * 2 + nt * 4 * SG_WARPS * 32 * 4 + nt * 8 * (k * 2 + (nt < 4 ? 16 : 0)) + 1024;
 }
 
 // NT: groups of eight batch rows that are staged and multiplied (M <= 8, 16 or 32 rows)
 template <bool SWIGLU, bool ARGMAX, int NT>
 __global__ void __launch_bounds__(SG_STD_THREADS, 1)
-skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_constant__ CUtensorMap map_w) {
+skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int SLOT_BYTES = SG_TILE_BYTES;
   constexpr int RING = SG_STD_RING;
   constexpr int OUT = SWIGLU ? 8 * SG_WARPS : SG_ROWS;  // outputs per CTA step
   constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_STD_WARPS][RING];
-  __shared__ uint64_t bar_x;
+  __shared__ uint64_t bar_x[SG_MAX_K / SG_TILE_K];  // 32 rows: one per k tile; fewer: the first one
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // warps wr and wr + 4 share the rows of group wr and take the even / the odd k tiles: a warp's k steps are a chain of
@@ -172,7 +181,8 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
 
   if (lane == 0) {
     for (int s = 0; s < RING; ++s) mbar_init(&bars[warp][s], 1);
-    if (warp == 0) mbar_init(&bar_x, 1);
+    if (warp == 0)
+      for (int i = 0; i < SG_MAX_K / SG_TILE_K; ++i) mbar_init(&bar_x[i], 1);
     mbar_fence_init();
   }
   // my tiles: row block rb = blockIdx.x, + gridDim.x, ...; tile index t counts (row block, k tile) pairs
@@ -192,10 +202,21 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
       tma_load_3d(ring + slot * SLOT_BYTES, &map_w, 0, rb * OUT + wr * 16, kt * 2, &bars[warp][slot]);
     }
   };
-  auto stage_x = [&]() {  // warp 0: one bulk copy per row of X
-    if (lane == 0) mbar_expect_tx(&bar_x, static_cast<uint32_t>(p.m) * p.k * 2);
-    __syncwarp();
-    if (lane < p.m) bulk_g2s(xs + lane * x_pitch, p.x + static_cast<int64_t>(lane) * p.x_stride, p.k * 2, &bar_x);
+  // warp 0: X by tensor-map boxes of a k tile each, whose products start when it is there, rows beyond M arriving as zeros; or by one
+  // bulk copy per row.  (A copy takes some 60 cycles whatever its size: a decode step of 32 sequences 985 us with copies by rows, 929 by boxes; in four
+  // parts of row copies 1021, by loads of all threads 1047.)
+  auto stage_x = [&]() {
+    if constexpr (NT == 4) {
+      if (lane == 0)
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          mbar_expect_tx(&bar_x[kt], SG_X_TILE_BYTES);
+          tma_load_3d(xs + kt * SG_X_TILE_BYTES, &map_x, 0, 0, kt * 2, &bar_x[kt]);
+        }
+    } else {
+      if (lane == 0) mbar_expect_tx(&bar_x[0], static_cast<uint32_t>(p.m) * p.k * 2);
+      __syncwarp();
+      if (lane < p.m) bulk_g2s(xs + lane * x_pitch, p.x + static_cast<int64_t>(lane) * p.x_stride, p.k * 2, &bar_x[0]);
+    }
   };
   // Started early, the weights are requested while the predecessor runs and X after it.  In plain stream order X goes
   // first: requested behind 128 KiB of weight tiles it would arrive behind them.
@@ -205,16 +226,18 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   if (lane == 0) {
     for (int t = 0; t < RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
-  for (int i = tid; i < (ROWS - p.m) * (p.k >> 3); i += SG_STD_THREADS) {  // rows beyond M are zero
-    const int r = p.m + i / (p.k >> 3), c = i % (p.k >> 3);
-    *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
+  if (NT < 4) {
+    for (int i = tid; i < (ROWS - p.m) * (p.k >> 3); i += SG_STD_THREADS) {  // rows beyond M are zero
+      const int r = p.m + i / (p.k >> 3), c = i % (p.k >> 3);
+      *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
+    }
   }
   const int x_row = tid / (p.k >> 3), x_piece = tid % (p.k >> 3);
   pdl_wait();  // X is the predecessor's output
   if (by_threads) stage_rows<SG_STD_THREADS>(xs, x_pitch, p.x, p.x_stride, p.m, p.k >> 3, x_row, x_piece);
   else if (early && warp == 0) stage_x();
   __syncthreads();  // bar_x is initialised for everybody, the rows that threads wrote are in place
-  bool ok = by_threads || mbar_wait_bounded(&bar_x, 0);
+  bool ok = by_threads || NT == 4 || mbar_wait_bounded(&bar_x[0], 0);
 
   const uint32_t xs_base = smem_u32(xs);
   // ldmatrix lane address of A (W tile): row = lane % 16, chunk parity = lane / 16
@@ -245,8 +268,12 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
         ok = false;
         break;
       }
+      if (NT == 4 && blk == 0 && !mbar_wait_bounded(&bar_x[kt], 0)) {
+        ok = false;
+        break;
+      }
       uint32_t b[8];
-      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xs_lane + kt * SG_TILE_K * 2, x_pitch, a_offset);
+      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xs_lane + StepProducts<NT>::tile_offset(kt), x_pitch, a_offset);
       __syncwarp();  // every lane has read the tile: its slot can take the tile RING ahead
       if (lane == 0 && t + RING < total_tiles) issue(t + RING);
     }
@@ -539,17 +566,17 @@ skinny_gemm_widek_kernel(const __grid_constant__ WideKParams p, const __grid_con
 constexpr int PK_RING = 3;                 // W tiles in flight per warp (a warp has K / 1024 tiles per row block)
 constexpr int PK_MAX_K = 4096;
 constexpr int pairk_smem(int nt, int k) {  // rings, sums of the warps and the peer, half of X
-  return SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * nt * 8 * 4 + nt * 8 * (k + 16) + 1024;
+  return SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * nt * 8 * 4 + nt * 8 * (k + (nt < 4 ? 16 : 0)) + 1024;
 }
 static_assert(pairk_smem(4, PK_MAX_K) <= 227 * 1024, "weight rings + half of X must fit the 227 KiB a CTA may use");
 
 template <int NT>
 __global__ void __launch_bounds__(SG_THREADS, 1)
-skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_constant__ CUtensorMap map_w) {
+skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_WARPS][PK_RING];
-  __shared__ uint64_t bar_x;
+  __shared__ uint64_t bar_x[PK_MAX_K / 2 / SG_TILE_K];  // 32 rows: one per k tile
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -565,7 +592,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   if (tid == 0) {
     for (int w = 0; w < SG_WARPS; ++w)
       for (int s = 0; s < PK_RING; ++s) mbar_init(&bars[w][s], 1);
-    mbar_init(&bar_x, 1);
+    for (int i = 0; i < PK_MAX_K / 2 / SG_TILE_K; ++i) mbar_init(&bar_x[i], 1);
     mbar_fence_init();
   }
   const int my_blocks = (p.row_blocks - pair + pairs - 1) / pairs;
@@ -582,22 +609,24 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   if (lane == 0) {
     for (int t = 0; t < PK_RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
-  for (int i = tid; i < (ROWS - p.m) * (half_k >> 3); i += SG_THREADS) {  // rows beyond M are zero
-    const int r = p.m + i / (half_k >> 3), c = i % (half_k >> 3);
-    *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
+  if (NT < 4) {
+    for (int i = tid; i < (ROWS - p.m) * (half_k >> 3); i += SG_THREADS) {  // rows beyond M are zero
+      const int r = p.m + i / (half_k >> 3), c = i % (half_k >> 3);
+      *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
+    }
   }
   const int x_row = tid / (half_k >> 3), x_piece = tid % (half_k >> 3);
   pdl_wait();  // X is the predecessor's output
   if (NT < 4) {
     stage_rows<SG_THREADS>(xs, x_pitch, p.x + rank * half_k, p.x_stride, p.m, half_k >> 3, x_row, x_piece);
-  } else if (warp == 0) {
-    if (lane == 0) mbar_expect_tx(&bar_x, static_cast<uint32_t>(p.m) * half_k * 2);
-    __syncwarp();
-    if (lane < p.m)
-      bulk_g2s(xs + lane * x_pitch, p.x + static_cast<int64_t>(lane) * p.x_stride + rank * half_k, half_k * 2, &bar_x);
+  } else if (tid == 0) {
+    for (int kl = 0; kl < half_tiles; ++kl) {
+      mbar_expect_tx(&bar_x[kl], SG_X_TILE_BYTES);
+      tma_load_3d(xs + kl * SG_X_TILE_BYTES, &map_x, 0, 0, (static_cast<int>(rank) * half_tiles + kl) * 2, &bar_x[kl]);
+    }
   }
   __syncthreads();
-  bool ok = NT < 4 || mbar_wait_bounded(&bar_x, 0);
+  bool ok = true;
 
   const int a_row = lane & 15, a_par = lane >> 4;
   const uint32_t xs_base = smem_u32(xs) + StepProducts<NT>::lane_offset(lane, x_pitch);
@@ -612,9 +641,10 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
     for (int kl = warp; kl < half_tiles; kl += SG_WARPS, ++t) {
       const int slot = t % PK_RING;
       if (ok && !mbar_wait_bounded(&bars[warp][slot], (t / PK_RING) & 1)) ok = false;
+      if (NT == 4 && blk == 0 && ok && !mbar_wait_bounded(&bar_x[kl], 0)) ok = false;
       if (ok) {
         uint32_t b[8];
-        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xs_base + kl * SG_TILE_K * 2, x_pitch, a_offset);
+        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xs_base + StepProducts<NT>::tile_offset(kl), x_pitch, a_offset);
       }
       __syncwarp();  // every lane has read the tile: its slot can take the tile PK_RING ahead
       if (ok && lane == 0 && t + PK_RING < total_tiles) issue(t + PK_RING);
@@ -659,7 +689,8 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
     if (lane == 0) atomicExch(p.err, 1);
     // let this warp's copies in flight land before the shared memory goes away
     for (int s = 0; s < PK_RING; ++s) mbar_wait_bounded(&bars[warp][s], 0, 1u << 12);
-    if (warp == 0) mbar_wait_bounded(&bar_x, 0, 1u << 12);
+    if (NT == 4)
+      for (int kl = 0; kl < half_tiles; ++kl) mbar_wait_bounded(&bar_x[kl], 0, 1u << 12);
   }
 }
 
@@ -704,8 +735,15 @@ static bool cache_weight_map(const void* base, int64_t n, int64_t k, int64_t str
 
 using namespace b200;
 
+// X [m, k] as boxes of 32 rows and 128 k
+static bool encode_x_map(CUtensorMap* map, const void* x, int m, int k, int64_t stride) {
+  return encode_tile_map(map, x, static_cast<uint64_t>(m), static_cast<uint64_t>(k), static_cast<uint64_t>(stride) * 2, SG_MAX_M, 2);
+}
+
 template <bool SWIGLU, bool ARGMAX, int NT>
 static int launch_skinny_rows(SkinnyGemmParams p, const CUtensorMap& map, cudaStream_t stream, const char* what) {
+  CUtensorMap map_x = {};
+  if (NT == 4 && !encode_x_map(&map_x, p.x, p.m, p.k, p.x_stride)) return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of x", what);
   constexpr int smem_max = skinny_smem(NT, SG_MAX_K);
   static_assert(smem_max <= 227 * 1024, "weight rings + X staging must fit the 227 KiB a CTA may use");
   static bool configured[64] = {false};
@@ -719,7 +757,7 @@ static int launch_skinny_rows(SkinnyGemmParams p, const CUtensorMap& map, cudaSt
   }
   const int sms = sm_count();
   if (launch_pdl((p.overlap & OVERLAP_START) != 0, skinny_gemm_kernel<SWIGLU, ARGMAX, NT>, dim3(p.row_blocks < sms ? p.row_blocks : sms),
-                 dim3(SG_STD_THREADS), skinny_smem(NT, p.k), stream, p, map) != cudaSuccess)
+                 dim3(SG_STD_THREADS), skinny_smem(NT, p.k), stream, p, map, map_x) != cudaSuccess)
     return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
   return check_launch(what);
 }
@@ -777,6 +815,8 @@ static int launch_widek(WideKParams p, const void* weight, int64_t w_stride, cud
 template <int NT>
 static int launch_pairk_rows(WideKParams p, const CUtensorMap& map, cudaStream_t stream) {
   const char* what = "skinny_gemm";
+  CUtensorMap map_x = {};
+  if (NT == 4 && !encode_x_map(&map_x, p.x, p.m, p.k, p.x_stride)) return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of x", what);
   constexpr int smem_max = pairk_smem(NT, PK_MAX_K);
   static bool configured[64] = {false};
   int dev = 0;
@@ -788,7 +828,7 @@ static int launch_pairk_rows(WideKParams p, const CUtensorMap& map, cudaStream_t
   }
   const int sms = sm_count(), pairs = p.row_blocks < sms / 2 ? p.row_blocks : sms / 2;
   if (launch_pdl_cluster((p.overlap & OVERLAP_START) != 0, 2, skinny_gemm_pairk_kernel<NT>, dim3(2 * pairs), dim3(SG_THREADS),
-                         pairk_smem(NT, p.k), stream, p, map) != cudaSuccess)
+                         pairk_smem(NT, p.k), stream, p, map, map_x) != cudaSuccess)
     return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
   return check_launch(what);
 }
