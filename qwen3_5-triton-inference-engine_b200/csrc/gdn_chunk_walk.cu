@@ -526,6 +526,10 @@ struct TeamSmem {
   static constexpr int EX = (L::BYTES + 127) / 128 * 128, EX_BYTES = D + PLACES * D_STEP, BARS = EX + TEAMS * EX_BYTES, BYTES = BARS + TEAMS * 64;
   static constexpr int BAR_S = 0, BAR_R = 2, BAR_D = 3, BAR_OUT = 5;   // two each where there are two places, but for R
   static constexpr int WARPS = (APART ? 8 : 4) * TEAMS, THREADS = 32 * (WARPS + GW_COPY_WARPS);
+  // place, barrier and phase of the n-th state, delta or output
+  static __device__ __forceinline__ int place(uint32_t n) { return APART ? n & 1 : 0; }
+  static __device__ __forceinline__ int bar_of(int first, uint32_t n) { return first + place(n); }
+  static __device__ __forceinline__ uint32_t phase_of(uint32_t n) { return APART ? (n >> 1) & 1 : n & 1; }
 };
 
 __device__ __forceinline__ void put_frag(uint8_t* to, const uint32_t (&hi)[4], const uint32_t (&lo)[4], int lane) {
@@ -610,6 +614,73 @@ __device__ __forceinline__ void store_tokens(const float (&O)[2][4], uint32_t ti
   if (t < tokens) *reinterpret_cast<uint4*>(out + t * o_t + c) = *reinterpret_cast<const uint4*>(rows + (t * pitch + c) * 2);
 }
 
+// The output warps have done with every chunk before this one: their places may be written again, their phases are over
+template <typename T>
+__device__ __forceinline__ bool outputs_done(uint64_t* bars, uint32_t& outputs, uint32_t chunks, bool ok) {
+  if constexpr (T::APART)
+    for (; outputs < chunks; ++outputs) ok = ok && team_wait(&bars[T::bar_of(T::BAR_OUT, outputs)], T::phase_of(outputs));
+  return ok;
+}
+
+// The four warps of the output (APART): what the chunk's other team publishes, one chunk behind it
+template <int TEAMS, bool WINDOWS>
+__device__ __forceinline__ void output_chunks(const GdnWalkParams& p, uint8_t* smem, int tid) {
+  using L = WalkSmem<16 * TEAMS>;
+  using T = TeamSmem<TEAMS>;
+  constexpr int SPLIT = 8 / TEAMS;
+  const int lane = tid & 31, w = (tid >> 5) & 3;
+  uint64_t *full = reinterpret_cast<uint64_t*>(smem + L::BARS), *empty = full + GW_STAGES;
+  const uint8_t* ex = smem + T::EX;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::BARS);
+  uint32_t states = 0, chunks = 0, full_parity = 0;     // states taken over and chunks begun so far
+  const int c2 = (lane & 3) * 2;
+  const uint32_t nk_off = ((w * 16 + (lane >> 4) * 8 + (lane & 7)) * GW_PITCH + ((lane >> 3) & 1) * 8) * 2;
+  const uint32_t v_off = ((w * 16 + (lane >> 4) * 8 + (lane & 7)) * L::VP + ((lane >> 3) & 1) * 8) * 2;
+  const int v_rows = L::V + w * 16 * L::VP * 2;
+  int stage = 0, bh = 0, h = 0, col = 0;
+  bool ok = true;
+  for (;;) {
+    ok = warp_wait_bounded(&full[stage], full_parity, ok);
+    if (!ok) break;
+    const int4 info = *reinterpret_cast<const int4*>(smem + L::INFO + stage * 16);
+    if (info.x < 0) return;
+    if (info.w & (WINDOWS ? 6 : 2)) bh = info.x / SPLIT, h = bh % p.heads, col = info.x % SPLIT * 16;
+    if (info.z > 0) {
+      const uint8_t* st = smem + stage * L::STAGE;
+      const uint8_t* fa = st + L::P + GW_MAT_BYTES;
+      const float* eg = reinterpret_cast<const float*>(fa + GW_MAT_BYTES) + w * 16;
+      const bool mine = info.z > 16 * w;
+      float O[2][4] = {};
+      if (!(info.w & 2)) {
+        ok = ok && team_wait(&bars[T::bar_of(T::BAR_S, states)], T::phase_of(states));
+        if (mine) {
+          uint32_t sh[8][4], sl[8][4];
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) get_frag(ex + T::S + T::place(states) * T::S_STEP + ks * 1024, sh[ks], sl[ks], lane);
+          query_state(O, sh, sl, smem_u32(st) + L::Q + nk_off, eg, c2);
+        }
+        ++states;
+      }
+      ok = ok && team_wait(&bars[T::bar_of(T::BAR_D, chunks)], T::phase_of(chunks));
+      if (mine) {
+        const uint8_t* d = ex + T::D + T::place(chunks) * T::D_STEP;
+        uint32_t dh[4], dl[4];
+        get_frag(d + w * 1024, dh, dl, lane);
+        add_within(O, dh, dl, d, fa, w, lane);
+        store_tokens(O, smem_u32(st) + L::V + v_off, st + v_rows, L::VP, p.out + (static_cast<int64_t>(info.y) + w * 16) * p.o_t + h * p.o_h + col,
+                     p.o_t, ok ? info.z - w * 16 : 0, lane);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[T::bar_of(T::BAR_OUT, chunks)]);
+      ++chunks;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[stage]);
+    if (++stage == GW_STAGES) stage = 0, full_parity ^= 1;
+  }
+  if (lane == 0) atomicExch(p.err, 1);
+}
+
 template <int TEAMS, bool WINDOWS>
 __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_kernel(const __grid_constant__ GdnWalkParams p) {
   using L = WalkSmem<16 * TEAMS>;
@@ -624,12 +695,12 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
     mbar_fence_init();
   }
   __syncthreads();
-  if (tid >= 32 * T::WARPS) {
-    copy_chunks<16 * TEAMS, WINDOWS>(p, smem, tid - 32 * T::WARPS);
+  if (tid >= 128 * TEAMS) {
+    if (tid >= 32 * T::WARPS) copy_chunks<16 * TEAMS, WINDOWS>(p, smem, tid - 32 * T::WARPS);
+    else if constexpr (T::APART) output_chunks<TEAMS, WINDOWS>(p, smem, tid);
     return;
   }
-  const bool output_team = T::APART && tid >= 128;
-  const int team = T::APART ? 0 : tid >> 7;
+  const int team = tid >> 7;
   uint8_t* ex = smem + T::EX + team * T::EX_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::BARS) + team * 8;
   uint32_t states = 0, chunks = 0, outputs = 0, full_parity = 0;   // states taken over, chunks begun, outputs waited for, so far
@@ -643,71 +714,18 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
   const int v_rows = L::V + (w * 16 * L::VP + team * 16) * 2;
   int stage = 0, bh = 0, h = 0, col = 0;
   bool ok = true;
-  auto place = [&](uint32_t n) { return T::APART ? n & 1 : 0; };
-  // barrier and phase of the n-th state, delta or output
-  auto bar_of = [&](int first, uint32_t n) { return first + place(n); };
-  auto phase_of = [&](uint32_t n) { return T::APART ? (n >> 1) & 1 : n & 1; };
-
-  if (output_team) {
-    for (;;) {
-      ok = warp_wait_bounded(&full[stage], full_parity, ok);
-      if (!ok) break;
-      const int4 info = *reinterpret_cast<const int4*>(smem + L::INFO + stage * 16);
-      if (info.x < 0) return;
-      if (info.w & (WINDOWS ? 6 : 2)) bh = info.x / SPLIT, h = bh % p.heads, col = info.x % SPLIT * 16;
-      if (info.z > 0) {
-        const uint8_t* st = smem + stage * L::STAGE;
-        const uint8_t* fa = st + L::P + GW_MAT_BYTES;
-        const float* eg = reinterpret_cast<const float*>(fa + GW_MAT_BYTES) + w * 16;
-        const bool mine = info.z > 16 * w;
-        float O[2][4] = {};
-        if (!(info.w & 2)) {
-          ok = ok && team_wait(&bars[bar_of(T::BAR_S, states)], phase_of(states));
-          if (mine) {
-            uint32_t sh[8][4], sl[8][4];
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) get_frag(ex + T::S + place(states) * T::S_STEP + ks * 1024, sh[ks], sl[ks], lane);
-            query_state(O, sh, sl, smem_u32(st) + L::Q + nk_off, eg, c2);
-          }
-          ++states;
-        }
-        ok = ok && team_wait(&bars[bar_of(T::BAR_D, chunks)], phase_of(chunks));
-        if (mine) {
-          const uint8_t* d = ex + T::D + place(chunks) * T::D_STEP;
-          uint32_t dh[4], dl[4];
-          get_frag(d + w * 1024, dh, dl, lane);
-          add_within(O, dh, dl, d, fa, w, lane);
-          store_tokens(O, smem_u32(st) + L::V + v_off, st + v_rows, L::VP, p.out + (static_cast<int64_t>(info.y) + w * 16) * p.o_t + h * p.o_h + col,
-                       p.o_t, ok ? info.z - w * 16 : 0, lane);
-        }
-        arrive(bar_of(T::BAR_OUT, chunks));
-        ++chunks;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[stage]);
-      if (++stage == GW_STAGES) stage = 0, full_parity ^= 1;
-    }
-    if (lane == 0) atomicExch(p.err, 1);
-    return;
-  }
-
   // S^T: value column lane / 4 (+ 8) of the team's 16, key dims 32 w + 8 n + (lane % 4) * 2 (+ 1)
   float S[4][4] = {};
   const uint32_t kn_off = ((((lane >> 3) & 1) * 8 + (lane & 7)) * GW_PITCH + w * 32 + (lane >> 4) * 8) * 2;
   uint32_t published = 0;
-  // the other team has done with every chunk before this one (their places may be written again, their phases are over)
-  auto outputs_done = [&]() {
-    if constexpr (T::APART)
-      for (; outputs < chunks; ++outputs) ok = ok && team_wait(&bars[bar_of(T::BAR_OUT, outputs)], phase_of(outputs));
-  };
   auto publish = [&]() {
-    uint8_t* to = ex + T::S + place(published) * T::S_STEP + 2 * w * 1024;
+    uint8_t* to = ex + T::S + T::place(published) * T::S_STEP + 2 * w * 1024;
     uint32_t hi[4], lo[4];
     split_frag(S[0], S[1], hi, lo);
     put_frag(to, hi, lo, lane);
     split_frag(S[2], S[3], hi, lo);
     put_frag(to + 1024, hi, lo, lane);
-    arrive(bar_of(T::BAR_S, published));
+    arrive(T::bar_of(T::BAR_S, published));
     ++published;
   };
   for (;;) {
@@ -722,7 +740,7 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
       for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j) S[n][j] = from[(n * 8 + c2 + (j & 1)) * GDN_D + gr + (j >> 1) * 8];
-      outputs_done();
+      ok = outputs_done<T>(bars, outputs, chunks, ok);
       publish();
     }
     if (info.z > 0) {
@@ -735,7 +753,7 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
       uint32_t rh[4], rl[4], sh[8][4], sl[8][4];
       float O[2][4] = {}, D[2][4] = {};
       if (carry) {
-        ok = ok && team_wait(&bars[bar_of(T::BAR_S, states)], phase_of(states));
+        ok = ok && team_wait(&bars[T::bar_of(T::BAR_S, states)], T::phase_of(states));
         ++states;
       }
       if (mine) {
@@ -743,7 +761,7 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
         float m[2][2][4] = {};
         if (carry) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) get_frag(ex + T::S + place(states - 1) * T::S_STEP + ks * 1024, sh[ks], sl[ks], lane);
+          for (int ks = 0; ks < 8; ++ks) get_frag(ex + T::S + T::place(states - 1) * T::S_STEP + ks * 1024, sh[ks], sl[ks], lane);
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
             uint32_t b[4];
@@ -777,7 +795,7 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
         pair_products(s, rh, rl, *reinterpret_cast<const uint4*>(fp + (frag_row(2 * w) + w) * 512 + lane * 16),
                       *reinterpret_cast<const uint4*>(fp + (frag_row(2 * w + 1) + w) * 512 + lane * 16));
       ok = ok && team_wait(&bars[T::BAR_R], chunks & 1);
-      uint8_t* d = ex + T::D + place(chunks) * T::D_STEP;
+      uint8_t* d = ex + T::D + T::place(chunks) * T::D_STEP;
       uint32_t dh[4], dl[4], eh[4], el[4];
       if (mine) {
 #pragma unroll
@@ -803,8 +821,8 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
         split_frag(D[0], D[1], dh, dl);
         put_frag(d + w * 1024, dh, dl, lane);
       }
-      arrive(bar_of(T::BAR_D, chunks));
-      ok = ok && team_wait(&bars[bar_of(T::BAR_D, chunks)], phase_of(chunks));
+      arrive(T::bar_of(T::BAR_D, chunks));
+      ok = ok && team_wait(&bars[T::bar_of(T::BAR_D, chunks)], T::phase_of(chunks));
       // ---- the own key dims of the state
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
@@ -822,7 +840,7 @@ __global__ void __launch_bounds__(TeamSmem<TEAMS>::THREADS, 1) gdn_walk_team_ker
         mma_bf16_16816(S[2], xl, b[0], b[1]);
         mma_bf16_16816(S[3], xl, b[2], b[3]);
       }
-      outputs_done();
+      ok = outputs_done<T>(bars, outputs, chunks, ok);
       if (!last) publish();
       ++chunks;
       if (!T::APART && mine) {                          // the output, where nobody waits for it any more
