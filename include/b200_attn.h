@@ -343,7 +343,7 @@ int b200_gdn_chunked_prefill_walk(const void* q, int64_t q_stride_t, int64_t q_s
  * b200_gdn_gated_rmsnorm: out[r,:] = x[r,:] * rsqrt(mean(x^2) + 1e-6) * weight * silu(z[r,:]) for rows r = (n, head);
  * x and out contiguous [rows, 128], z row (n, head) at z + n * z_stride + head * 128
  * (triton_kernels/gdn_gated_rmsnorm.py:95-140). */
-/* Overlap flags (programmatic dependent launch) of b200_(norm_)skinny_gemm, b200_add_rmsnorm, b200_swiglu and
+/* Overlap flags (programmatic dependent launch) of b200_skinny_gemm (all forms), b200_add_rmsnorm, b200_swiglu and
  * b200_gdn_decode_fused; 0 = nothing is read or written before the kernel in front has completed.
  *   START    the kernel may begin while the kernel in front of it in the stream still runs; it reads that kernel's
  *            output, and writes anything, only after that kernel has completed.
@@ -387,6 +387,20 @@ int b200_skinny_gemm_part(const void* x, int64_t x_stride, const void* weight, i
  * [M, intermediate]; intermediate a multiple of 8; other shapes, alignment and overlap flags as b200_skinny_gemm. */
 int b200_skinny_gemm_swiglu(const void* x, int64_t x_stride, const void* weight, void* y, int64_t y_stride, int32_t m,
                             int32_t intermediate, int32_t k, int32_t overlap, b200_stream_t stream);
+
+/* The same two products around a residual add and RMSNorm (b200_add_rmsnorm) without a launch between them, M <= 32:
+ *   b200_skinny_gemm_join    sum = bf16(residual + bf16(X W^T)), scaled = bf16(sum * (1 + gain)), squares[m][j] = sum of squares of
+ *                            sum[m][16 j .. 16 j + 16) (fp32); 1280 < K <= 4096, K a multiple of 256, N of 16; sum and scaled [M,N]
+ *                            contiguous, squares [M, N / 16].  residual and the outputs must not overlap.
+ *   b200_skinny_gemm_normed  Y = (X W^T) / rms, rms = sqrt(mean of squares over K + eps), for X = scaled [M,K] contiguous of the call above:
+ *                            b200_skinny_gemm (or, swiglu != 0, b200_skinny_gemm_swiglu; n counts outputs) of the normed rows, K <= 1280.
+ *   b200_lm_head_argmax_normed  b200_lm_head_argmax of the normed rows. */
+int b200_skinny_gemm_join(const void* x, int64_t x_stride, const void* weight, const void* residual, int64_t res_stride, const void* gain,
+                          void* sum, void* scaled, float* squares, int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream);
+int b200_skinny_gemm_normed(const void* x, const float* squares, const void* weight, void* y, int64_t y_stride, int32_t m, int32_t n,
+                            int32_t k, float eps, int32_t swiglu, int32_t overlap, b200_stream_t stream);
+int b200_lm_head_argmax_normed(const void* x, const float* squares, float eps, const void* weight, int64_t* ids, void* workspace, int32_t m,
+                               int32_t n, int32_t k, int32_t overlap, b200_stream_t stream);
 
 /* ids[b] = argmax over n of <x[b, :], weight[n, :]> with fp32 accumulation, ties to the lowest n: the LM head with a tied
  * embedding and its greedy sampling in one launch (triton_kernels/vocab_argmax.py:141-200); the logits are never written.

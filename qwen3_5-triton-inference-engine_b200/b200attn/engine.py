@@ -124,6 +124,15 @@ class Engine(SlotEngine):
             return ops.skinny_gemm(x, weight, overlap=overlap)
         return glue.gemm_2d(x, weight)
 
+    def _proj_norm(self, x, weight, residual, gain, consumer, overlap: int, plain: int, swiglu: bool = False):
+        """Projection back to the hidden size, residual add and the norm in front of `consumer`: (sum, rows, None) with normed rows, or,
+        where the weight-streaming kernel takes both products (`overlap`), (sum, rows, sums of squares) for its normed form."""
+        if (self._streams_weight(weight) and self._streams_weight(consumer, swiglu)
+                and ops.skinny_gemm_joins(x.shape[0], weight.shape[0], weight.shape[1])):
+            return ops.skinny_gemm_join(x, weight, residual, gain, overlap=overlap)
+        total, h = ops.add_rmsnorm(self._proj(x, weight, overlap), gain, self.cfg.eps, residual=residual, overlap=plain)
+        return total, h, None
+
     def _norm(self, x, weight):
         if self.fused_glue:
             return ops.add_rmsnorm(x, weight, self.cfg.eps)
@@ -301,9 +310,10 @@ class Engine(SlotEngine):
         return nxt
 
     def _decode_fused(self, tok: torch.Tensor) -> torch.Tensor:
-        """The same step with every row-wise operator as one launch: seven launches per layer (norm, projection, mixer
-        with its head norms inside, output projection, norm, gate/up projection with the SwiGLU as its epilogue, down
-        projection).  The residual add after a layer's MLP is fused into the next layer's input norm.  Kernels of this
+        """The same step in five launches per layer (projection, mixer with its head norms inside, output projection, gate/up
+        projection with the SwiGLU as its epilogue, down projection): the projections back to the hidden size add the residual and
+        prepare the norm, the products behind them apply it.  Where a product is not the weight-streaming kernel's, residual
+        and norm are a launch of their own in between.  Kernels of this
         package that follow one another start early (programmatic dependent launch: weights and states stream in while
         the predecessor finishes); a kernel in front of a cuBLAS or PyTorch kernel never triggers early."""
         cfg = self.cfg
@@ -314,19 +324,26 @@ class Engine(SlotEngine):
         def then(own_next: bool) -> int:                 # flags of a kernel whose successor is (not) one of ours
             return start | trigger if own_next else start
 
-        x = _embedding_gather(tok, self.w["embed"])      # this package's kernel: the norm behind it may start early
-        pending = None                                   # MLP output still to be added to the residual stream
-        for i, layer in enumerate(self.w["layers"]):
+        def project(h, squares, weight, overlap):
+            if squares is None:
+                return self._proj(h, weight, overlap)
+            return ops.skinny_gemm_normed(h, squares, weight, cfg.eps, overlap=overlap)
+
+        embed = self.w["embed"]
+        own_head = (embed.shape[1] <= ops.SKINNY_GEMM_MAX_K
+                    and ops.skinny_gemm_supports(batch, embed.shape[0], embed.shape[1]))
+        layers = self.w["layers"]
+        x = _embedding_gather(tok, embed)                # this package's kernel: the norm behind it may start early
+        h = squares = None                               # rows of the next projection; with squares, not yet divided by their rms
+        for i, layer in enumerate(layers):
             gdn = layer["kind"] == "gdn"
             proj_w = layer["in_proj"] if gdn else layer["qkvg"]
             out_w = layer["out_proj"] if gdn else layer["o_proj"]
             own_proj, own_out = self._streams_weight(proj_w), self._streams_weight(out_w)
             own_mlp, own_down = self._streams_weight(layer["gate_up"], swiglu=True), self._streams_weight(layer["down"])
-            if pending is None:
+            if h is None:
                 h = ops.add_rmsnorm(x, layer["ln1"], cfg.eps, overlap=then(own_proj))
-            else:
-                x, h = ops.add_rmsnorm(pending, layer["ln1"], cfg.eps, residual=x, overlap=then(own_proj))
-            fused = self._proj(h, proj_w, then(True))
+            fused = project(h, squares, proj_w, then(True))
             if gdn:
                 mixed_in = ops.gdn_decode_fused(fused, self.conv_state[i], layer["conv4"], layer["a_log"],
                                                 layer["dt_bias"], layer["norm"], self.rec_state[i], heads,
@@ -342,22 +359,28 @@ class Engine(SlotEngine):
                                                       overlap=then(own_out) | (prefetch if own_proj else 0),
                                                       q_norm_weight=layer["q_norm"], k_norm_weight=layer["k_norm"],
                                                       eps=cfg.eps)
-            mixed = self._proj(mixed_in, out_w, then(True))
-            x, h = ops.add_rmsnorm(mixed, layer["ln2"], cfg.eps, residual=x, overlap=then(own_mlp))
-            if own_mlp:
+            x, h, squares = self._proj_norm(mixed_in, out_w, x, layer["ln2"], layer["gate_up"], then(True), then(own_mlp), swiglu=True)
+            if squares is not None:
+                act = ops.skinny_gemm_normed(h, squares, layer["gate_up"], cfg.eps, overlap=then(own_down), swiglu=True)
+            elif own_mlp:
                 act = ops.skinny_gemm(h, layer["gate_up"], overlap=then(own_down), swiglu=True)
             else:
                 act = ops.swiglu_fused(glue.gemm_2d(h, layer["gate_up"]), cfg.intermediate, overlap=then(own_down))
-            pending = self._proj(act, layer["down"], then(True))
-        embed = self.w["embed"]
-        own_head = (embed.shape[1] <= ops.SKINNY_GEMM_MAX_K
-                    and ops.skinny_gemm_supports(batch, embed.shape[0], embed.shape[1]))
-        _, h = ops.add_rmsnorm(pending, self.w["norm"], cfg.eps, residual=x, overlap=then(own_head))
+            if i + 1 < len(layers):
+                gain, nxt_w = layers[i + 1]["ln1"], layers[i + 1]["in_proj" if layers[i + 1]["kind"] == "gdn" else "qkvg"]
+                own_next = self._streams_weight(nxt_w)
+            else:
+                gain, nxt_w, own_next = self.w["norm"], embed, own_head
+            x, h, squares = self._proj_norm(act, layer["down"], x, gain, nxt_w, then(True), then(own_next))
         if own_head:   # tied LM head and greedy sampling in one launch; the logits are never written
             # the ids go straight into `tok` when it is the engine's own token buffer (read only by the gather at the
             # top of the step): no copy kernel behind the step
             in_place = tok.data_ptr() == self.tok.data_ptr() and tok.dtype == torch.int64 and tok.is_contiguous()
-            nxt = ops.lm_head_argmax(h, embed, self.argmax_ws, out=tok if in_place else None, overlap=start)
+            out = tok if in_place else None
+            if squares is None:
+                nxt = ops.lm_head_argmax(h, embed, self.argmax_ws, out=out, overlap=start)
+            else:
+                nxt = ops.lm_head_argmax_normed(h, squares, embed, cfg.eps, self.argmax_ws, out=out, overlap=start)
         else:          # fp32 logits from cuBLAS, arg-max (lowest index on ties) in one launch
             nxt = glue.lm_head_argmax(h, embed, last_only=False,
                                       argmax=lambda logits: ops.argmax_rows(logits, self.argmax_ws, overlap=start))

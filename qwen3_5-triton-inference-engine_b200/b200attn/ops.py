@@ -905,6 +905,59 @@ def skinny_gemm(x, weight, overlap: int = 0, swiglu: bool = False):
     return y
 
 
+def skinny_gemm_joins(m: int, n: int, k: int) -> bool:
+    """Whether `skinny_gemm_join` takes an [m, k] x [n, k]^T product and `skinny_gemm_normed` its rows."""
+    return (0 < m <= SKINNY_GEMM_MAX_M and n % 128 == 0 and 0 < n <= SKINNY_GEMM_MAX_K
+            and SKINNY_GEMM_MAX_K < k <= SKINNY_GEMM_PAIR_MAX_K and k % 256 == 0)
+
+
+def skinny_gemm_join(x, weight, residual, gain, overlap: int = 0):
+    """`skinny_gemm` of a projection back to the hidden size, the residual added and the RMSNorm behind it prepared: returns the sum
+    s = residual + x @ weight^T [M, N], the rows s * (1 + gain) and the sums of squares of every 16 columns of s [M, N / 16] fp32.
+    `skinny_gemm_normed` and `lm_head_argmax_normed` take the last two."""
+    m, k = x.shape
+    n = weight.shape[0]
+    assert skinny_gemm_joins(m, n, k) and weight.shape[1] == k and residual.shape == (m, n) and gain.shape == (n,)
+    assert all(t.dtype == torch.bfloat16 for t in (x, weight, residual, gain)) and weight.is_contiguous() and gain.is_contiguous()
+    assert x.stride(1) == 1 and residual.stride(1) == 1
+    _require_cuda(x, weight, residual, gain)
+    total, scaled = (torch.empty((m, n), dtype=torch.bfloat16, device=x.device) for _ in range(2))
+    squares = torch.empty((m, n // 16), dtype=torch.float32, device=x.device)
+    _lib.call("b200_skinny_gemm_join", _ptr(x), x.stride(0), _ptr(weight), _ptr(residual), residual.stride(0), _ptr(gain), _ptr(total),
+              _ptr(scaled), _ptr(squares), m, n, k, int(overlap), _stream())
+    return total, scaled, squares
+
+
+def skinny_gemm_normed(scaled, squares, weight, eps: float, overlap: int = 0, swiglu: bool = False):
+    """`skinny_gemm` of the RMS-normed rows that `skinny_gemm_join` prepared."""
+    m, k = scaled.shape
+    n = weight.shape[0]
+    assert scaled.dtype == weight.dtype == torch.bfloat16 and scaled.is_contiguous() and weight.is_contiguous() and weight.shape[1] == k
+    assert squares.shape == (m, k // 16) and squares.dtype == torch.float32 and squares.is_contiguous()
+    if swiglu:
+        assert n % 2 == 0
+        n //= 2
+    _require_cuda(scaled, squares, weight)
+    y = torch.empty((m, n), dtype=torch.bfloat16, device=scaled.device)
+    _lib.call("b200_skinny_gemm_normed", _ptr(scaled), _ptr(squares), _ptr(weight), _ptr(y), n, m, n, k, float(eps), int(swiglu), int(overlap),
+              _stream())
+    return y
+
+
+def lm_head_argmax_normed(scaled, squares, table, eps: float, workspace, out=None, overlap: int = 0) -> torch.Tensor:
+    """`lm_head_argmax` of the RMS-normed rows that `skinny_gemm_join` prepared."""
+    m, k = scaled.shape
+    assert scaled.dtype == table.dtype == torch.bfloat16 and scaled.is_contiguous() and table.is_contiguous() and table.shape[1] == k
+    assert squares.shape == (m, k // 16) and squares.dtype == torch.float32 and squares.is_contiguous()
+    _require_cuda(scaled, squares, table, workspace)
+    if out is None:
+        out = torch.empty(m, dtype=torch.int64, device=scaled.device)
+    assert out.dtype == torch.int64 and out.is_contiguous() and out.numel() == m
+    _lib.call("b200_lm_head_argmax_normed", _ptr(scaled), _ptr(squares), float(eps), _ptr(table), _ptr(out), _ptr(workspace), m, table.shape[0], k,
+              int(overlap), _stream())
+    return out
+
+
 def skinny_gemm_part(x, weight, out, overlap: int = 0):
     """out = x @ weight^T where weight is a column range of a wider matrix: one part of a product split along K."""
     assert x.shape[1] == weight.shape[1] and x.stride(1) == weight.stride(1) == 1 and out.shape == (x.shape[0], weight.shape[0])
