@@ -39,7 +39,6 @@ constexpr int SG_STD_WARPS = SG_WARPS * SG_KSPLIT;
 constexpr int SG_STD_THREADS = SG_STD_WARPS * 32;
 constexpr int SG_STD_RING = SG_RING / SG_KSPLIT;  // the same bytes in flight per CTA
 constexpr int SG_MAX_M = 32;
-constexpr int SG_X_TILE_BYTES = SG_MAX_M * SG_TILE_K * 2;   // 128 k of 32 batch rows
 constexpr int SG_MAX_K = 1280;           // X staging: 32 x (K*2 + 16) bytes next to 128 KiB of weight rings
 
 struct SkinnyGemmParams {
@@ -58,22 +57,19 @@ struct SkinnyGemmParams {
 
 // Which m16n8k16 products a step of 16 k takes for NT groups of eight batch rows, and the sums they go to.  A warp's k steps are a
 // chain: with fewer than four groups the steps take turns among the four accumulators, joined at the end by `join_steps`.
-// One step costs eight cycles of a scheduler per group, and two warps share one: 31 rows of zeros behind a single one, and writing them
-// behind the wait for X, were 1.8 us of a 6.3 us launch.
+// One step costs eight cycles of a scheduler per group, and two warps share one: 31 rows of zeros behind a single one were most of 1.8 us
+// of a 6.3 us launch.
 template <int NT>
 struct StepProducts;
 template <>
 struct StepProducts<4> {
-  // X tiles as tensor-map boxes of 128 k: two blocks of [32 rows][64 k] with the 128-byte swizzle.  Lane address: row = (lane & 7) + 8 *
-  // (lane >> 4) inside a 16-row pair, k half = (lane >> 3) & 1; a step's 32 bytes are two bits of the address to turn over
-  static __device__ __forceinline__ uint32_t lane_offset(int lane, int) {
+  // lane address: row = (lane & 7) + 8 * (lane >> 4) of sixteen, k half = (lane >> 3) & 1
+  static __device__ __forceinline__ uint32_t lane_offset(int lane) {
     return static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * 128 + (((lane >> 3) & 1) ^ (lane & 7)) * 16);
   }
-  static __device__ __forceinline__ uint32_t tile_offset(int kt) { return kt * SG_X_TILE_BYTES; }
   template <int KS>
-  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xt, int) {
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk) {
     uint32_t b01[4], b23[4];
-    const uint32_t xk = (xt + (KS >> 2) * (SG_X_TILE_BYTES / 2)) ^ ((KS & 3) * 32);
     ldmatrix_x4(b01, xk);                   // batch rows 0-15: (b0, b1) of n8 tiles 0 and 1
     ldmatrix_x4(b23, xk + 16 * 128);        // batch rows 16-31
     mma_bf16_16816(acc[0], a, b01[0], b01[1]);
@@ -84,15 +80,11 @@ struct StepProducts<4> {
 };
 template <>
 struct StepProducts<2> {
-  // rows x_pitch bytes apart: row = (lane & 7) + 8 * (lane >> 4) of sixteen, k half = (lane >> 3) & 1
-  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
-    return static_cast<uint32_t>(((lane & 7) + ((lane >> 4) << 3)) * x_pitch + ((lane >> 3) & 1) * 16);
-  }
-  static __device__ __forceinline__ uint32_t tile_offset(int kt) { return kt * SG_TILE_K * 2; }
+  static __device__ __forceinline__ uint32_t lane_offset(int lane) { return StepProducts<4>::lane_offset(lane); }
   template <int KS>
-  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk) {
     uint32_t b01[4];
-    ldmatrix_x4(b01, xk + KS * 32);
+    ldmatrix_x4(b01, xk);
     mma_bf16_16816(acc[(KS & 1) * 2], a, b01[0], b01[1]);
     mma_bf16_16816(acc[(KS & 1) * 2 + 1], a, b01[2], b01[3]);
   }
@@ -100,14 +92,11 @@ struct StepProducts<2> {
 template <>
 struct StepProducts<1> {
   // eight rows, four k groups of eight: one load serves two steps
-  static __device__ __forceinline__ uint32_t lane_offset(int lane, int x_pitch) {
-    return static_cast<uint32_t>((lane & 7) * x_pitch + (lane >> 3) * 16);
-  }
-  static __device__ __forceinline__ uint32_t tile_offset(int kt) { return kt * SG_TILE_K * 2; }
+  static __device__ __forceinline__ uint32_t lane_offset(int lane) { return static_cast<uint32_t>((lane & 7) * 128 + ((lane >> 3) ^ (lane & 7)) * 16); }
   template <int KS>
-  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk, int x_pitch) {
+  static __device__ __forceinline__ void run(float (&acc)[4][4], const uint32_t (&a)[4], uint32_t (&b)[8], uint32_t xk) {
     uint32_t (&b4)[4] = *reinterpret_cast<uint32_t (*)[4]>(b);
-    if constexpr ((KS & 1) == 0) ldmatrix_x4(b4, xk + KS * 32);
+    if constexpr ((KS & 1) == 0) ldmatrix_x4(b4, xk);
     mma_bf16_16816(acc[KS & 3], a, b[(KS & 1) * 2], b[(KS & 1) * 2 + 1]);
   }
 };
@@ -122,45 +111,20 @@ __device__ __forceinline__ void join_steps(float (&acc)[4][4]) {
     }
   }
 }
-// The eight steps of a tile of 128 k: A (W tile) by ldmatrix from `tile` + offset(step), X from `xk` on.
+// The eight steps of a tile of 128 k: A (W tile) by ldmatrix from `tile` + offset(step), X from `xt` on (the lane's address in the
+// tensor-map box of the tile: two blocks of [8 NT rows][64 k] with the 128-byte swizzle; a step's 32 bytes are two bits of the address
+// to turn over).
 template <int NT, int KS, typename Offset>
-__device__ __forceinline__ void tile_steps(float (&acc)[4][4], uint32_t (&b)[8], uint32_t tile, uint32_t xk, int x_pitch, const Offset& offset) {
+__device__ __forceinline__ void tile_steps(float (&acc)[4][4], uint32_t (&b)[8], uint32_t tile, uint32_t xt, const Offset& offset) {
   if constexpr (KS < SG_TILE_K / 16) {
     uint32_t a[4];
     ldmatrix_x4(a, tile + offset(KS));
-    StepProducts<NT>::template run<KS>(acc, a, b, xk, x_pitch);
-    tile_steps<NT, KS + 1>(acc, b, tile, xk, x_pitch, offset);
-  }
-}
-// `chunks` 16-byte pieces of each of m rows -> shared memory, by all THREADS threads, thread t starting at piece c of row r
-// (t = r * chunks + c); every load of a round is under way before its first store.  (For few rows: a bulk copy per row takes
-// longer to arrive.)
-template <int THREADS>
-__device__ __forceinline__ void stage_rows(uint8_t* xs, int x_pitch, const __nv_bfloat16* x, int64_t x_stride, int m, int chunks, int r, int c) {
-  constexpr int ROUND = 4;
-  while (r < m) {
-    uint4 v[ROUND];
-    uint8_t* to[ROUND];
-#pragma unroll
-    for (int u = 0; u < ROUND; ++u) {
-      to[u] = nullptr;
-      if (r < m) {
-        v[u] = *reinterpret_cast<const uint4*>(x + r * x_stride + c * 8);
-        to[u] = xs + r * x_pitch + c * 16;
-      }
-      c += THREADS;
-      while (c >= chunks) {
-        c -= chunks;
-        ++r;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < ROUND; ++u)
-      if (to[u] != nullptr) *reinterpret_cast<uint4*>(to[u]) = v[u];
+    StepProducts<NT>::template run<KS>(acc, a, b, (xt + (KS >> 2) * (NT * 8 * 128)) ^ ((KS & 3) * 32));
+    tile_steps<NT, KS + 1>(acc, b, tile, xt, offset);
   }
 }
 constexpr int skinny_smem(int nt, int k) {  // rings, output staging, odd-tile sums, X
-  return SG_WARPS * SG_RING_BYTES + nt * 8 * SG_ROWS * 2 + nt * 4 * SG_WARPS * 32 * 4 + nt * 8 * (k * 2 + (nt < 4 ? 16 : 0)) + 1024;
+  return SG_WARPS * SG_RING_BYTES + nt * 8 * SG_ROWS * 2 + nt * 4 * SG_WARPS * 32 * 4 + nt * 8 * k * 2 + 2048;
 }
 
 // NT: groups of eight batch rows that are staged and multiplied (M <= 8, 16 or 32 rows)
@@ -173,7 +137,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   constexpr int OUT = SWIGLU ? 8 * SG_WARPS : SG_ROWS;  // outputs per CTA step
   constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_STD_WARPS][RING];
-  __shared__ uint64_t bar_x[SG_MAX_K / SG_TILE_K];  // 32 rows: one per k tile; fewer: the first one
+  __shared__ uint64_t bar_x[SG_MAX_K / SG_TILE_K];  // one per k tile
   __shared__ __align__(8) float scale[ROWS];                   // normed form: 1 / rms of the rows
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -183,8 +147,9 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   uint8_t* ring = smem + warp * (RING * SLOT_BYTES);
   uint8_t* stage = smem + SG_WARPS * SG_RING_BYTES;                    // [ROWS][OUT] bf16 output staging, <= 4 KiB
   float* part = reinterpret_cast<float*>(stage + ROWS * SG_ROWS * 2);  // [4 NT][4 groups x 32 lanes]: odd-tile sums
-  uint8_t* xs = reinterpret_cast<uint8_t*>(part + 4 * NT * SG_WARPS * 32);  // [ROWS][x_pitch] bf16
-  const int x_pitch = p.k * 2 + 16;                                    // bytes; the 16 shift the banks row by row
+  constexpr int X_TILE = ROWS * SG_TILE_K * 2;
+  // X, tile by tile; the swizzle counts from 1024-byte boundaries
+  uint8_t* xs = smem + (SG_WARPS * SG_RING_BYTES + ROWS * SG_ROWS * 2 + 4 * NT * SG_WARPS * 32 * 4 + 1023) / 1024 * 1024;
   const int k_tiles = p.k / SG_TILE_K;
 
   if (lane == 0) {
@@ -210,37 +175,25 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
       tma_load_3d(ring + slot * SLOT_BYTES, &map_w, 0, rb * OUT + wr * 16, kt * 2, &bars[warp][slot]);
     }
   };
-  // warp 0: X by tensor-map boxes of a k tile each, whose products start when it is there, rows beyond M arriving as zeros; or by one
-  // bulk copy per row.  (A copy takes some 60 cycles whatever its size: a decode step of 32 sequences 985 us with copies by rows, 929 by boxes; in four
-  // parts of row copies 1021, by loads of all threads 1047.)
+  // X by tensor-map boxes of a k tile each, whose products start when it is there; rows beyond M arrive as zeros.  A copy takes some 60
+  // cycles of the thread that asks for it, whatever its size, so every warp asks for some.  Decode step of 8 / 16 / 32 sequences: rows by
+  // loads of all threads 703 / 882 / 1047 us, a copy per row - / - / 985, boxes from one thread 645 / 717 / 888, from all warps 634 / 709 / 872
+  // (one sequence: 608, -, 614, 597).
   auto stage_x = [&]() {
-    if constexpr (NT == 4) {
-      if (lane == 0)
-        for (int kt = 0; kt < k_tiles; ++kt) {
-          mbar_expect_tx(&bar_x[kt], SG_X_TILE_BYTES);
-          tma_load_3d(xs + kt * SG_X_TILE_BYTES, &map_x, 0, 0, kt * 2, &bar_x[kt]);
-        }
-    } else {
-      if (lane == 0) mbar_expect_tx(&bar_x[0], static_cast<uint32_t>(p.m) * p.k * 2);
-      __syncwarp();
-      if (lane < p.m) bulk_g2s(xs + lane * x_pitch, p.x + static_cast<int64_t>(lane) * p.x_stride, p.k * 2, &bar_x[0]);
+    for (int kt = warp; kt < k_tiles; kt += SG_STD_WARPS) {
+      mbar_expect_tx(&bar_x[kt], X_TILE);
+      tma_load_3d(xs + kt * X_TILE, &map_x, 0, 0, kt * 2, &bar_x[kt]);
     }
   };
   // Started early, the weights are requested while the predecessor runs and X after it.  In plain stream order X goes
   // first: requested behind 128 KiB of weight tiles it would arrive behind them.
-  const bool early = (p.overlap & OVERLAP_START) != 0, by_threads = early && NT < 4;
+  const bool early = (p.overlap & OVERLAP_START) != 0;
   if (p.overlap & OVERLAP_TRIGGER) pdl_trigger();
-  if (!early && warp == 0) stage_x();
+  __syncthreads();  // bar_x is initialised for everybody
+  if (!early && lane == 0) stage_x();
   if (lane == 0) {
     for (int t = 0; t < RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
-  if (NT < 4) {
-    for (int i = tid; i < (ROWS - p.m) * (p.k >> 3); i += SG_STD_THREADS) {  // rows beyond M are zero
-      const int r = p.m + i / (p.k >> 3), c = i % (p.k >> 3);
-      *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
-    }
-  }
-  const int x_row = tid / (p.k >> 3), x_piece = tid % (p.k >> 3);
   pdl_wait();  // X is the predecessor's output
   // normed form: eight threads per row, asked for now and first looked at behind the products
   constexpr int SQUARES = SG_MAX_K / 16 / 8;
@@ -249,15 +202,13 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
 #pragma unroll
   for (int i = 0; i < SQUARES; ++i)
     sq[i] = normed && (tid >> 3) < p.m && i * 8 + (tid & 7) < (p.k >> 4) ? p.squares[(tid >> 3) * (p.k >> 4) + i * 8 + (tid & 7)] : 0.f;
-  if (by_threads) stage_rows<SG_STD_THREADS>(xs, x_pitch, p.x, p.x_stride, p.m, p.k >> 3, x_row, x_piece);
-  else if (early && warp == 0) stage_x();
-  __syncthreads();  // bar_x is initialised for everybody, the rows that threads wrote are in place
-  bool ok = by_threads || NT == 4 || mbar_wait_bounded(&bar_x[0], 0);
+  if (early && lane == 0) stage_x();
+  bool ok = true;
 
   const uint32_t xs_base = smem_u32(xs);
   // ldmatrix lane address of A (W tile): row = lane % 16, chunk parity = lane / 16
   const int a_row = lane & 15, a_par = lane >> 4;
-  const uint32_t xs_lane = xs_base + StepProducts<NT>::lane_offset(lane, x_pitch);
+  const uint32_t xs_lane = xs_base + StepProducts<NT>::lane_offset(lane);
   const auto a_offset = [&](int ks) -> uint32_t {
     // plain: [k-block][16 rows][128 B]; SwiGLU: [gate | up][k-block][8 rows][128 B]; 16-byte chunks XOR-swizzled by row
     return (SWIGLU ? (a_row >> 3) * (SG_TILE_BYTES / 2) + (ks >> 2) * (8 * 128) + (a_row & 7) * 128 : (ks >> 2) * (16 * 128) + a_row * 128) +
@@ -283,12 +234,12 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
         ok = false;
         break;
       }
-      if (NT == 4 && blk == 0 && !mbar_wait_bounded(&bar_x[kt], 0)) {
+      if (blk == 0 && !mbar_wait_bounded(&bar_x[kt], 0)) {
         ok = false;
         break;
       }
       uint32_t b[8];
-      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xs_lane + StepProducts<NT>::tile_offset(kt), x_pitch, a_offset);
+      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xs_lane + kt * X_TILE, a_offset);
       __syncwarp();  // every lane has read the tile: its slot can take the tile RING ahead
       if (lane == 0 && t + RING < total_tiles) issue(t + RING);
     }
@@ -410,6 +361,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
     if (lane == 0) atomicExch(p.err, 1);
     // let this warp's copies in flight land before the shared memory goes away
     for (int s = 0; s < RING; ++s) mbar_wait_bounded(&bars[warp][s], 0, 1u << 12);
+    for (int kt = 0; kt < k_tiles; ++kt) mbar_wait_bounded(&bar_x[kt], 0, 1u << 12);
   }
 }
 
@@ -598,10 +550,10 @@ skinny_gemm_widek_kernel(const __grid_constant__ WideKParams p, const __grid_con
 // as many SMs stream W, a CTA stages only its half of X -- once, whole, so there is no chunk pipeline -- and the two
 // partial [16 x 32] sums meet through distributed shared memory (rank 1 stores its sum into rank 0's shared memory,
 // one cluster barrier, rank 0 adds, rounds and writes).  No cluster multicast is used; every CTA loads its own tiles.
-constexpr int PK_RING = 3;                 // W tiles in flight per warp (a warp has K / 1024 tiles per row block)
+constexpr int PK_RING = 4;                 // W tiles in flight per warp: all of a row block (a decode step of one sequence 597 us with three, 587 with four)
 constexpr int PK_MAX_K = 4096;
 constexpr int pairk_smem(int nt, int k) {  // rings, sums of the warps and the peer, half of X
-  return SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * nt * 8 * 4 + nt * 8 * (k + (nt < 4 ? 16 : 0)) + 1024;
+  return SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * nt * 8 * 4 + nt * 8 * k + 2048;
 }
 static_assert(pairk_smem(4, PK_MAX_K) <= 227 * 1024, "weight rings + half of X must fit the 227 KiB a CTA may use");
 
@@ -611,7 +563,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_WARPS][PK_RING];
-  __shared__ uint64_t bar_x[PK_MAX_K / 2 / SG_TILE_K];  // 32 rows: one per k tile
+  __shared__ uint64_t bar_x[PK_MAX_K / 2 / SG_TILE_K];  // one per k tile
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -619,9 +571,10 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   uint8_t* ring = smem + warp * PK_RING * SG_TILE_BYTES;
   float* red = reinterpret_cast<float*>(smem + SG_WARPS * PK_RING * SG_TILE_BYTES);  // [4 warps + peer][ROWS][16]
   float* peer = red + SG_WARPS * WK_ROWS * ROWS;                                 // written by rank 1 into rank 0
-  uint8_t* xs = reinterpret_cast<uint8_t*>(peer + WK_ROWS * ROWS);               // [ROWS][x_pitch]: this CTA's half of X
+  constexpr int X_TILE = ROWS * SG_TILE_K * 2;
+  // this CTA's half of X, tile by tile; the swizzle counts from 1024-byte boundaries
+  uint8_t* xs = smem + (SG_WARPS * PK_RING * SG_TILE_BYTES + (SG_WARPS + 1) * WK_ROWS * ROWS * 4 + 1023) / 1024 * 1024;
   const int half_k = p.k >> 1;
-  const int x_pitch = half_k * 2 + 16;
   const int half_tiles = half_k / SG_TILE_K;
 
   if (tid == 0) {
@@ -644,51 +597,45 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   if (lane == 0) {
     for (int t = 0; t < PK_RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
-  if (NT < 4) {
-    for (int i = tid; i < (ROWS - p.m) * (half_k >> 3); i += SG_THREADS) {  // rows beyond M are zero
-      const int r = p.m + i / (half_k >> 3), c = i % (half_k >> 3);
-      *reinterpret_cast<uint4*>(xs + r * x_pitch + c * 16) = make_uint4(0, 0, 0, 0);
-    }
-  }
-  const int x_row = tid / (half_k >> 3), x_piece = tid % (half_k >> 3);
+  // thread -> batch row tid / 4, outputs (tid % 4) * 4 .. + 4 of a row block (N is a multiple of 8 and r of 4: inside or outside together)
+  const bool joins = p.scaled != nullptr;
+  const int b = tid >> 2, r = (tid & 3) * 4;
+  const auto writes = [&](int n0) { return rank == 0 && b < p.m && n0 < p.n; };
+  uint2 res = {}, gain = {};
+  if (joins && writes(pair * WK_ROWS + r)) gain = *reinterpret_cast<const uint2*>(p.gain + pair * WK_ROWS + r);
   pdl_wait();  // X is the predecessor's output
-  if (NT < 4) {
-    stage_rows<SG_THREADS>(xs, x_pitch, p.x + rank * half_k, p.x_stride, p.m, half_k >> 3, x_row, x_piece);
-  } else if (tid == 0) {
-    for (int kl = 0; kl < half_tiles; ++kl) {
-      mbar_expect_tx(&bar_x[kl], SG_X_TILE_BYTES);
-      tma_load_3d(xs + kl * SG_X_TILE_BYTES, &map_x, 0, 0, (static_cast<int>(rank) * half_tiles + kl) * 2, &bar_x[kl]);
+  if (lane == 0) {
+    for (int kl = warp; kl < half_tiles; kl += SG_WARPS) {
+      mbar_expect_tx(&bar_x[kl], X_TILE);
+      tma_load_3d(xs + kl * X_TILE, &map_x, 0, 0, (static_cast<int>(rank) * half_tiles + kl) * 2, &bar_x[kl]);
     }
   }
+  if (joins && writes(pair * WK_ROWS + r)) res = *reinterpret_cast<const uint2*>(p.residual + b * p.res_stride + pair * WK_ROWS + r);
   __syncthreads();
   bool ok = true;
 
   const int a_row = lane & 15, a_par = lane >> 4;
-  const uint32_t xs_base = smem_u32(xs) + StepProducts<NT>::lane_offset(lane, x_pitch);
+  const uint32_t xs_base = smem_u32(xs) + StepProducts<NT>::lane_offset(lane);
   const auto a_offset = [&](int ks) -> uint32_t { return (ks >> 2) * (16 * 128) + a_row * 128 + ((((ks & 3) * 2 + a_par) ^ (a_row & 7)) << 4); };
   const uint32_t peer_remote = cluster_map(smem_u32(peer), 0);
-  const bool joins = p.scaled != nullptr;
   int t = 0;
   for (int blk = 0; blk < my_blocks; ++blk) {
     const int rb = pair + blk * pairs;
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    // thread -> batch row tid / 4, outputs (tid % 4) * 4 .. + 4: N is a multiple of 8 and r of 4, so the four are inside or outside together
-    const int b = tid >> 2, r = (tid & 3) * 4, n0 = rb * WK_ROWS + r;
-    const bool writes = rank == 0 && b < p.m && n0 < p.n;
-    uint2 res = {}, gain = {};
-    if (joins && writes) {
+    const int n0 = rb * WK_ROWS + r;
+    if (joins && blk > 0 && writes(n0)) {
       res = *reinterpret_cast<const uint2*>(p.residual + b * p.res_stride + n0);
       gain = *reinterpret_cast<const uint2*>(p.gain + n0);
     }
     for (int kl = warp; kl < half_tiles; kl += SG_WARPS, ++t) {
       const int slot = t % PK_RING;
       if (ok && !mbar_wait_bounded(&bars[warp][slot], (t / PK_RING) & 1)) ok = false;
-      if (NT == 4 && blk == 0 && ok && !mbar_wait_bounded(&bar_x[kl], 0)) ok = false;
+      if (blk == 0 && ok && !mbar_wait_bounded(&bar_x[kl], 0)) ok = false;
       if (ok) {
         uint32_t b[8];
-        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xs_base + StepProducts<NT>::tile_offset(kl), x_pitch, a_offset);
+        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xs_base + kl * X_TILE, a_offset);
       }
       __syncwarp();  // every lane has read the tile: its slot can take the tile PK_RING ahead
       if (ok && lane == 0 && t + PK_RING < total_tiles) issue(t + PK_RING);
@@ -726,16 +673,16 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
         const float v0 = round_bf16(bf16_lo(y.x) + bf16_lo(res.x)), v1 = round_bf16(bf16_hi(y.x) + bf16_hi(res.x));
         const float v2 = round_bf16(bf16_lo(y.y) + bf16_lo(res.y)), v3 = round_bf16(bf16_hi(y.y) + bf16_hi(res.y));
         y = make_uint2(pack_bf16(v0, v1), pack_bf16(v2, v3));
-        if (writes)
+        if (writes(n0))
           *reinterpret_cast<uint2*>(p.scaled + static_cast<int64_t>(b) * p.n + n0) =
               make_uint2(pack_bf16(v0 * (1.f + bf16_lo(gain.x)), v1 * (1.f + bf16_hi(gain.x))),
                          pack_bf16(v2 * (1.f + bf16_lo(gain.y)), v3 * (1.f + bf16_hi(gain.y))));
-        float ss = writes ? fmaf(v0, v0, fmaf(v1, v1, fmaf(v2, v2, v3 * v3))) : 0.f;
+        float ss = writes(n0) ? fmaf(v0, v0, fmaf(v1, v1, fmaf(v2, v2, v3 * v3))) : 0.f;
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
         if (r == 0 && b < p.m) p.squares[b * p.row_blocks + rb] = ss;
       }
-      if (writes) *reinterpret_cast<uint2*>(p.y + static_cast<int64_t>(b) * p.y_stride + n0) = y;
+      if (writes(n0)) *reinterpret_cast<uint2*>(p.y + static_cast<int64_t>(b) * p.y_stride + n0) = y;
     }
     if (blk + 1 < my_blocks) cluster_sync();  // rank 0 has read `peer` before rank 1 writes the next sum
   }
@@ -743,8 +690,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
     if (lane == 0) atomicExch(p.err, 1);
     // let this warp's copies in flight land before the shared memory goes away
     for (int s = 0; s < PK_RING; ++s) mbar_wait_bounded(&bars[warp][s], 0, 1u << 12);
-    if (NT == 4)
-      for (int kl = 0; kl < half_tiles; ++kl) mbar_wait_bounded(&bar_x[kl], 0, 1u << 12);
+    for (int kl = 0; kl < half_tiles; ++kl) mbar_wait_bounded(&bar_x[kl], 0, 1u << 12);
   }
 }
 
@@ -789,15 +735,15 @@ static bool cache_weight_map(const void* base, int64_t n, int64_t k, int64_t str
 
 using namespace b200;
 
-// X [m, k] as boxes of 32 rows and 128 k
-static bool encode_x_map(CUtensorMap* map, const void* x, int m, int k, int64_t stride) {
-  return encode_tile_map(map, x, static_cast<uint64_t>(m), static_cast<uint64_t>(k), static_cast<uint64_t>(stride) * 2, SG_MAX_M, 2);
+// X [m, k] as boxes of `rows` rows and 128 k
+static bool encode_x_map(CUtensorMap* map, const void* x, int m, int k, int64_t stride, int rows) {
+  return encode_tile_map(map, x, static_cast<uint64_t>(m), static_cast<uint64_t>(k), static_cast<uint64_t>(m > 1 ? stride : k) * 2, rows, 2);
 }
 
 template <bool SWIGLU, bool ARGMAX, int NT>
 static int launch_skinny_rows(SkinnyGemmParams p, const CUtensorMap& map, cudaStream_t stream, const char* what) {
   CUtensorMap map_x = {};
-  if (NT == 4 && !encode_x_map(&map_x, p.x, p.m, p.k, p.x_stride)) return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of x", what);
+  if (!encode_x_map(&map_x, p.x, p.m, p.k, p.x_stride, NT * 8)) return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of x", what);
   constexpr int smem_max = skinny_smem(NT, SG_MAX_K);
   static_assert(smem_max <= 227 * 1024, "weight rings + X staging must fit the 227 KiB a CTA may use");
   static bool configured[64] = {false};
@@ -870,7 +816,7 @@ template <int NT>
 static int launch_pairk_rows(WideKParams p, const CUtensorMap& map, cudaStream_t stream) {
   const char* what = "skinny_gemm";
   CUtensorMap map_x = {};
-  if (NT == 4 && !encode_x_map(&map_x, p.x, p.m, p.k, p.x_stride)) return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of x", what);
+  if (!encode_x_map(&map_x, p.x, p.m, p.k, p.x_stride, NT * 8)) return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of x", what);
   constexpr int smem_max = pairk_smem(NT, PK_MAX_K);
   static bool configured[64] = {false};
   int dev = 0;

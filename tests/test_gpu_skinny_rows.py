@@ -36,3 +36,16 @@ def test_rows_swiglu_and_argmax(m):
     logits = x.double() @ w.double().t()
     best = logits.gather(1, ids.view(-1, 1)).squeeze(1)
     assert bool((logits.max(1).values - best <= 1e-4).all())       # fp32 sums: ties up to their rounding
+
+
+@pytest.mark.parametrize("m", [2, 9, 20])
+@pytest.mark.parametrize("k", [256, 2048])
+def test_rows_over_one_another(m, k):
+    """Rows that share their memory, and one row of any stride: X goes through a tensor map of its strides."""
+    from b200attn import ops
+    x, w = _case(1, 72, k)
+    wide = torch.empty(m, 3 * k, dtype=torch.bfloat16, device=DEV).copy_(x.repeat(1, 3))
+    want = ops.skinny_gemm(x.repeat(m, 1), w)
+    for rows in (x.expand(m, k), wide[:, k: 2 * k], torch.as_strided(wide, (m, k), (8 * 3 * k // 8, 1), 2 * k)):
+        assert torch.equal(ops.skinny_gemm(rows, w), want)
+    assert torch.equal(ops.skinny_gemm(torch.as_strided(wide, (1, k), (16, 1), k), w), want[:1])
