@@ -469,6 +469,11 @@ int b200_gdn_conv_norm_gates(const void* x, int64_t x_stride_t, const void* weig
                              int64_t a_stride_t, const void* b, int64_t b_stride_t, const float* a_log, const void* dt_bias,
                              void* q_out, void* k_out, void* v_out, float* beta, float* g, int32_t tokens, int32_t num_heads,
                              int32_t head_dim, b200_stream_t stream);
+/* ... and b200_conv_state_from_packed_prefill of the q, k and v channels in the same launch. */
+int b200_gdn_conv_norm_gates_state(const void* x, int64_t x_stride_t, const void* weight, const int32_t* seq_start, const void* a,
+                                   int64_t a_stride_t, const void* b, int64_t b_stride_t, const float* a_log, const void* dt_bias,
+                                   void* q_out, void* k_out, void* v_out, float* beta, float* g, int32_t tokens, int32_t num_heads,
+                                   int32_t head_dim, const int32_t* cu_seqlens, int32_t batch, void* state, b200_stream_t stream);
 int b200_gdn_qk_norm_gates(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k, int64_t k_stride_t,
                            int64_t k_stride_h, const void* a, int64_t a_stride_t, const void* b, int64_t b_stride_t,
                            const float* a_log, const void* dt_bias, void* q_out, void* k_out, float* beta, float* g,

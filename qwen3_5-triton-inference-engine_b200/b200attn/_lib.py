@@ -62,6 +62,7 @@ SIGNATURES: dict[str, list] = {
     "b200_conv4_decode": [P, I64, P, P, P, I64, I32, I32, P],
     "b200_conv_state_from_packed_prefill": [P, P, I64, P, I32, I32, P],
     "b200_gdn_conv_norm_gates": [P, I64, P, P, P, I64, P, I64, P, P, P, P, P, P, P, I32, I32, I32, P],
+    "b200_gdn_conv_norm_gates_state": [P, I64, P, P, P, I64, P, I64, P, P, P, P, P, P, P, I32, I32, I32, P, I32, P, P],
     "b200_gdn_qk_norm_gates": [P, I64, I64, P, I64, I64, P, I64, P, I64, P, P, P, P, P, P, I32, I32, I32, P],
     "b200_embedding_gather": [P, I32, P, P, I32, I32, P],
     "b200_residual_add": [P, P, P, I64, P],

@@ -203,21 +203,20 @@ class Engine(SlotEngine):
                 x, h = ops.add_rmsnorm(pending, layer["ln1"], cfg.eps, residual=x)
             if layer["kind"] == "gdn":
                 qkv, z, a, b = self._split_gdn(glue.gemm_2d(h, layer["in_proj"]))
-                ready = ops.gdn_conv_norm_gates(qkv, layer["conv"], seq_start, a, b, layer["a_log"], layer["dt_bias"])
+                conv_rows = self.conv_state[i] if slots is None else torch.empty(
+                    (count,) + tuple(self.conv_state[i].shape[1:]), dtype=torch.bfloat16, device=self.device)
+                ready = ops.gdn_conv_norm_gates(qkv, layer["conv"], seq_start, a, b, layer["a_log"], layer["dt_bias"], cu, conv_rows)
                 if ready is None:                        # rows that are no whole vectors
+                    _conv_state_pack(conv_rows, qkv, cu)
                     q, k, v = _conv4_prefill(qkv, layer["conv"], seq_start).view(total, 3, heads, dim).unbind(1)
                     q_n, k_n, beta, g = _qk_norm_gates(q, k, a, b, layer["a_log"], layer["dt_bias"])
                 else:
                     q_n, k_n, v, beta, g = ready
                 if slots is None:                        # every slot: the kernel writes the cache's own states
                     core, _ = ops.gdn_chunked_prefill_packed(q_n, k_n, v, beta, g, cu, state_out=self.rec_state[i])
-                    _conv_state_pack(self.conv_state[i], qkv, cu)
                 else:
                     core, state = ops.gdn_chunked_prefill_packed(q_n, k_n, v, beta, g, cu)
                     put(self.rec_state[i], state)
-                    conv_rows = torch.empty((len(prompts),) + tuple(self.conv_state[i].shape[1:]), dtype=torch.bfloat16,
-                                            device=self.device)
-                    _conv_state_pack(conv_rows, qkv, cu)
                     put(self.conv_state[i], conv_rows)
                 normed = ops.gdn_gated_rmsnorm_fused(core, z, layer["norm"])
                 mixed = glue.gemm_2d(normed, layer["out_proj"])

@@ -788,10 +788,12 @@ def gdn_gated_rmsnorm_fused(x, z, weight):
     return out
 
 
-def gdn_conv_norm_gates(qkv, weight, seq_start, a, b, a_log, dt_bias):
+def gdn_conv_norm_gates(qkv, weight, seq_start, a, b, a_log, dt_bias, cu=None, state=None):
     """Convolution + SiLU, q/k norms and gates of a packed prompt in one pass (the operators depthwise_causal_conv4_prefill and
     gdn_qk_norm_gates, engine/runner.py:255-292): rows [q | k | v], any of them a column range of the projection's ->
-    q_n, k_n, v bf16 [tokens, heads, 128], beta, g fp32 [tokens, heads].  None where rows or taps are not 16-byte vectors."""
+    q_n, k_n, v bf16 [tokens, heads, 128], beta, g fp32 [tokens, heads].  None where rows or taps are not 16-byte vectors.
+    state [sequences, 4, channels] bf16 contiguous, with cu: takes the last four rows of every sequence in the same launch
+    (conv_state_from_packed_prefill)."""
     tokens, heads = a.shape
     assert qkv.shape == (tokens, 3 * heads * GDN_DIM) and weight.numel() == 4 * qkv.shape[1] and b.shape == a.shape
     assert all(t.dtype == torch.bfloat16 for t in (qkv, weight, a, b, dt_bias)) and a_log.dtype == torch.float32
@@ -800,11 +802,16 @@ def gdn_conv_norm_gates(qkv, weight, seq_start, a, b, a_log, dt_bias):
             or a.stride(1) != 1 or b.stride(1) != 1):
         return None
     _require_cuda(qkv, weight, seq_start, a, b, a_log, dt_bias)
+    if state is not None:
+        assert cu.dtype == torch.int32 and cu.is_contiguous() and state.shape == (cu.numel() - 1, 4, qkv.shape[1])
+        assert state.dtype == torch.bfloat16 and state.is_contiguous()
+        _require_cuda(cu, state)
     q, k, v = (torch.empty((tokens, heads, GDN_DIM), dtype=torch.bfloat16, device=qkv.device) for _ in range(3))
     beta, g = (torch.empty((tokens, heads), dtype=torch.float32, device=qkv.device) for _ in range(2))
     a_log, dt_bias = a_log.contiguous(), dt_bias.contiguous()
-    _lib.call("b200_gdn_conv_norm_gates", _ptr(qkv), qkv.stride(0), _ptr(weight), _ptr(seq_start), _ptr(a), a.stride(0), _ptr(b), b.stride(0),
-              _ptr(a_log), _ptr(dt_bias), _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(g), tokens, heads, GDN_DIM, _stream())
+    _lib.call("b200_gdn_conv_norm_gates_state", _ptr(qkv), qkv.stride(0), _ptr(weight), _ptr(seq_start), _ptr(a), a.stride(0), _ptr(b), b.stride(0),
+              _ptr(a_log), _ptr(dt_bias), _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(g), tokens, heads, GDN_DIM,
+              *((None, 0, None) if state is None else (_ptr(cu), state.shape[0], _ptr(state))), _stream())
     return q, k, v, beta, g
 
 

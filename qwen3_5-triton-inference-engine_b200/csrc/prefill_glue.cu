@@ -299,10 +299,22 @@ struct ConvNormParams {
   const __nv_bfloat16* dt_bias;
   __nv_bfloat16 *q, *k, *v;               // [tokens, heads, 128]
   float *beta, *g;                        // [tokens, heads]
-  int tokens, heads;
+  int tokens, heads, token_blocks;
+  const int32_t* cu;                      // CTAs behind the tokens', one per sequence: its last four inputs to state [batch, 4, channels]
+  __nv_bfloat16* state;
 };
 
 __global__ void __launch_bounds__(CONV_THREADS, 4) conv4_norm_gates_kernel(const __grid_constant__ ConvNormParams p) {
+  static_assert(CONV_THREADS == 128, "a warp per row of the state");
+  if (static_cast<int>(blockIdx.x) >= p.token_blocks) {   // as conv_state_pack_kernel; a launch of its own took 2.8 us behind this one
+    const int b = blockIdx.x - p.token_blocks, r = threadIdx.x >> 5, c = (blockIdx.y * 32 + (threadIdx.x & 31)) * 8, channels = 3 * p.heads * GDN_D;
+    if (c >= channels) return;
+    const int t = p.cu[b + 1] - 4 + r;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (t >= p.cu[b]) v = *reinterpret_cast<const uint4*>(p.x + t * p.x_t + c);
+    *reinterpret_cast<uint4*>(p.state + (static_cast<int64_t>(b) * 4 + r) * channels + c) = v;
+    return;
+  }
   const int t0 = (blockIdx.x * (CONV_THREADS / 32) + (threadIdx.x >> 5)) * CN_TPT, lane = threadIdx.x & 31, sub = lane & 15;
   const int unit = blockIdx.y * 2 + (lane >> 4);          // q heads, k heads, v heads
   if (t0 >= p.tokens || blockIdx.y * 2 >= 3 * p.heads) return;
@@ -447,21 +459,34 @@ extern "C" int b200_conv4_prefill(const void* x, int64_t x_stride_t, const void*
   return check_launch("conv4_prefill");
 }
 
-extern "C" int b200_gdn_conv_norm_gates(const void* x, int64_t x_stride_t, const void* weight, const int32_t* seq_start, const void* a,
-                                        int64_t a_stride_t, const void* b, int64_t b_stride_t, const float* a_log,
-                                        const void* dt_bias, void* q_out, void* k_out, void* v_out, float* beta, float* g,
-                                        int32_t tokens, int32_t num_heads, int32_t head_dim, b200_stream_t stream) {
+extern "C" int b200_gdn_conv_norm_gates_state(const void* x, int64_t x_stride_t, const void* weight, const int32_t* seq_start, const void* a,
+                                              int64_t a_stride_t, const void* b, int64_t b_stride_t, const float* a_log,
+                                              const void* dt_bias, void* q_out, void* k_out, void* v_out, float* beta, float* g,
+                                              int32_t tokens, int32_t num_heads, int32_t head_dim, const int32_t* cu_seqlens,
+                                              int32_t batch, void* state, b200_stream_t stream) {
   B200_REQUIRE(tokens > 0 && num_heads > 0 && head_dim == GDN_D, "gdn_conv_norm_gates: head_dim must be %d (got %d)", GDN_D, head_dim);
   B200_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(q_out) && aligned16(k_out) && aligned16(v_out) && x_stride_t % 8 == 0,
                "gdn_conv_norm_gates: rows and taps must be 16-byte aligned, the row stride a multiple of 8 elements");
-  const dim3 grid((tokens + CN_TOKENS - 1) / CN_TOKENS, (3 * num_heads + 1) / 2);
+  B200_REQUIRE(state == nullptr || (batch > 0 && cu_seqlens != nullptr && aligned16(state)),
+               "gdn_conv_norm_gates: the state needs the sequences' bounds and 16-byte alignment");
+  const int token_blocks = (tokens + CN_TOKENS - 1) / CN_TOKENS;
+  const dim3 grid(token_blocks + (state != nullptr ? batch : 0), (3 * num_heads + 1) / 2);
   B200_REQUIRE(grid.y <= 65535, "gdn_conv_norm_gates: too many heads (%d)", num_heads);
   const ConvNormParams p = {static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), x_stride_t, seq_start,
                             static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b), a_stride_t, b_stride_t, a_log,
                             static_cast<const __nv_bfloat16*>(dt_bias), static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_out),
-                            static_cast<__nv_bfloat16*>(v_out), beta, g, tokens, num_heads};
+                            static_cast<__nv_bfloat16*>(v_out), beta, g, tokens, num_heads, token_blocks, cu_seqlens,
+                            static_cast<__nv_bfloat16*>(state)};
   conv4_norm_gates_kernel<<<grid, CONV_THREADS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
   return check_launch("gdn_conv_norm_gates");
+}
+
+extern "C" int b200_gdn_conv_norm_gates(const void* x, int64_t x_stride_t, const void* weight, const int32_t* seq_start, const void* a,
+                                        int64_t a_stride_t, const void* b, int64_t b_stride_t, const float* a_log,
+                                        const void* dt_bias, void* q_out, void* k_out, void* v_out, float* beta, float* g,
+                                        int32_t tokens, int32_t num_heads, int32_t head_dim, b200_stream_t stream) {
+  return b200_gdn_conv_norm_gates_state(x, x_stride_t, weight, seq_start, a, a_stride_t, b, b_stride_t, a_log, dt_bias, q_out, k_out, v_out, beta,
+                                        g, tokens, num_heads, head_dim, nullptr, 0, nullptr, stream);
 }
 
 extern "C" int b200_conv4_decode(const void* x, int64_t x_stride_b, void* state, const void* weight4, void* out,
