@@ -307,11 +307,10 @@ class FusedUnit:
     def prefill(self, h, batch, engine, states):
         fused = engine.linear(h, self.w_in)
         act = torch.empty((h.shape[0], sum(self.outs) + self.pad), dtype=h.dtype, device=h.device)
-        if self.pad:
-            act[:, -self.pad:].zero_()
         for key, (_, core), x, out in self._ranges(fused, act):
             core.prefill(x, out, batch, engine, states[key])
-        return engine.linear(act, self.w_out)
+        used = act.shape[1] - self.pad                   # the padding is the decode step's: no columns that need zeros
+        return engine.linear(act[:, :used], self.w_out[:, :used])
 
     def starts_own(self, engine) -> bool:
         """Whether the product in runs on the weight-streaming kernel: its form for inputs of up to 1280 takes any number of
