@@ -394,13 +394,19 @@ int b200_skinny_gemm_swiglu(const void* x, int64_t x_stride, const void* weight,
  *                            contiguous, squares [M, N / 16].  residual and the outputs must not overlap.
  *   b200_skinny_gemm_normed  Y = (X W^T) / rms, rms = sqrt(mean of squares over K + eps), for X = scaled [M,K] contiguous of the call above:
  *                            b200_skinny_gemm (or, swiglu != 0, b200_skinny_gemm_swiglu; n counts outputs) of the normed rows, K <= 1280.
- *   b200_lm_head_argmax_normed  b200_lm_head_argmax of the normed rows. */
+ *   b200_lm_head_argmax_normed  b200_lm_head_argmax of the normed rows.
+ *   b200_skinny_gemm_hyper_join  b200_hyper_connect in place of add and norm: the streams [M, S <= 4, N] move on in place with the product (and
+ *                            n_parts earlier parts of it, [n_parts][M,N] bf16, summed in front), scaled = bf16(read-out * gain * gains).
+ * true_k: columns that the mean counts. */
 int b200_skinny_gemm_join(const void* x, int64_t x_stride, const void* weight, const void* residual, int64_t res_stride, const void* gain,
                           void* sum, void* scaled, float* squares, int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream);
+int b200_skinny_gemm_hyper_join(const void* x, int64_t x_stride, const void* weight, int64_t w_stride, float* streams, const float* joint,
+                                const float* gains, const void* parts, int32_t n_parts, void* scaled, float* squares, int32_t m, int32_t n,
+                                int32_t k, int32_t s, int32_t overlap, b200_stream_t stream);
 int b200_skinny_gemm_normed(const void* x, const float* squares, const void* weight, void* y, int64_t y_stride, int32_t m, int32_t n,
-                            int32_t k, float eps, int32_t swiglu, int32_t overlap, b200_stream_t stream);
+                            int32_t k, int32_t true_k, float eps, int32_t swiglu, int32_t overlap, b200_stream_t stream);
 int b200_lm_head_argmax_normed(const void* x, const float* squares, float eps, const void* weight, int64_t* ids, void* workspace, int32_t m,
-                               int32_t n, int32_t k, int32_t overlap, b200_stream_t stream);
+                               int32_t n, int32_t k, int32_t true_k, int32_t overlap, b200_stream_t stream);
 
 /* ids[b] = argmax over n of <x[b, :], weight[n, :]> with fp32 accumulation, ties to the lowest n: the LM head with a tied
  * embedding and its greedy sampling in one launch (triton_kernels/vocab_argmax.py:141-200); the logits are never written.

@@ -318,6 +318,9 @@ class FusedUnit:
         n, k = self.w_in.shape
         return engine.streams_weight(self.w_in) and (k <= ops.SKINNY_GEMM_MAX_K or n <= 8192)
 
+    def takes_rows(self, engine) -> bool:
+        return self.starts_own(engine) and self.w_in.shape[1] <= ops.SKINNY_GEMM_MAX_K
+
     def out_parts(self, engine):
         """(weight, first and last column) of the product's parts in a decode step, or None: one library product."""
         if not all(engine.streams_weight(w) for w in self.w_parts):
@@ -343,8 +346,13 @@ class FusedUnit:
             engine.join()
         if not own_out:
             return F.linear(act, self.w_out)
-        y = torch.empty((len(outs), act.shape[0], self.w_out.shape[0]), dtype=act.dtype, device=act.device)
+        joins = engine.joins(nxt, outs[-1][0])           # the last part is the end of the joint
+        y = torch.empty((len(outs) - joins, act.shape[0], self.w_out.shape[0]), dtype=act.dtype, device=act.device)
         for n, (weight, lo, hi) in enumerate(outs):
-            flags = engine.then(nxt or n + 1 < len(outs))
-            ops.skinny_gemm_part(act[:, lo:hi], weight, y[n], overlap=flags & ~ops.OVERLAP_START if side and n == 0 else flags)
+            flags = engine.then(bool(nxt) or n + 1 < len(outs))
+            if side and n == 0:
+                flags &= ~ops.OVERLAP_START
+            if n == len(y):
+                return hops.hyper_join(act[:, lo:hi], weight, *nxt, parts=y if n else None, overlap=flags)
+            ops.skinny_gemm_part(act[:, lo:hi], weight, y[n], overlap=flags)
         return y

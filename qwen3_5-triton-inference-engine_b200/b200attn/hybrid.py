@@ -56,7 +56,9 @@ class HybridConfig:
 
 
 # Units: what runs between two joints.  prefill(h, batch, engine, states) and decode(h, engine, states, nxt) give the
-# sublayer's output; starts_own(engine): whether its first decode-step kernel is one of this package.
+# sublayer's output; nxt: whether a kernel of this package takes it, or the hops.Joint behind it, and then the output may be the next
+# sublayer's hops.Rows.  starts_own(engine): whether its first decode-step kernel is one of this package; takes_rows(engine): whether
+# h may be hops.Rows.
 class MixerUnit:
     def __init__(self, layer: int, mixer):
         self.layer, self.mixer = layer, mixer
@@ -72,6 +74,9 @@ class MixerUnit:
 
     def starts_own(self, engine) -> bool:
         return engine.streams_weight(self.mixer.first_weight())
+
+    def takes_rows(self, engine) -> bool:
+        return self.starts_own(engine) and self.mixer.first_weight().shape[1] <= ops.SKINNY_GEMM_MAX_K
 
     def decode(self, h, engine, states, nxt: bool):
         return self.mixer.decode(h, engine, states, nxt)
@@ -92,6 +97,8 @@ class FeedForwardUnit:
 
     def starts_own(self, engine) -> bool:
         return engine.streams_weight(self.mlp.gate_up, swiglu=True)
+
+    takes_rows = starts_own
 
     def decode(self, h, engine, states, nxt: bool):
         return self.mlp.decode(h, engine, nxt)
@@ -324,10 +331,21 @@ class HybridEngine(SlotEngine):
     def join(self) -> None:
         torch.cuda.current_stream(self.device).wait_stream(self._side)
 
-    def proj(self, x, weight, own_next: bool):
-        """Decode-step projection: the weight-streaming kernel where it takes the shape, cuBLAS otherwise."""
-        if self.streams_weight(weight):
-            return ops.skinny_gemm(x, weight, overlap=self.then(own_next))
+    def joins(self, nxt, weight) -> bool:
+        """Whether the product by this weight can end as the joint `nxt`."""
+        return (isinstance(nxt, hops.Joint) and self.streams_weight(weight) and nxt.streams.shape[1] <= hops.HYPER_JOIN_STREAMS
+                and ops.skinny_gemm_joins(self.batch, weight.shape[0], weight.shape[1]))
+
+    def proj(self, x, weight, own_next, swiglu: bool = False):
+        """Decode-step projection: the weight-streaming kernel where it takes the shape, cuBLAS otherwise.  x may be hops.Rows; own_next
+        a hops.Joint, which the product then is the end of where it can."""
+        overlap = self.then(bool(own_next))
+        if isinstance(x, hops.Rows):
+            return ops.skinny_gemm_normed(x.scaled, x.squares, weight, self.cfg.eps, overlap=overlap, swiglu=swiglu, width=self.cfg.width)
+        if self.joins(own_next, weight):
+            return hops.hyper_join(x, weight, *own_next, overlap=overlap)
+        if self.streams_weight(weight, swiglu):
+            return ops.skinny_gemm(x, weight, overlap=overlap, swiglu=swiglu)
         return F.linear(x, weight)
 
     def fuses_head(self) -> bool:
@@ -447,7 +465,10 @@ class HybridEngine(SlotEngine):
         streams, untraced = self.streams, self.trace is None
         h = self._joint(0, streams, ids=tok, overlap=self.then(first_own(0)))
         for k, unit in enumerate(units, start=1):
-            h = self._joint(k, streams, y=unit.decode(h, self, self.states, True), overlap=self.then(first_own(k) and untraced))
+            takes = untraced and (own_head if k == len(units) else units[k].takes_rows(self))
+            h = unit.decode(h, self, self.states, hops.Joint(streams, self.w.joints[k], self.w.gains[k]) if takes else True)
+            if not isinstance(h, hops.Rows):
+                h = self._joint(k, streams, y=h, overlap=self.then(first_own(k) and untraced))
             if k == len(units) or units[k].layer != unit.layer:          # the layer ends here
                 self._traced(streams)
         return h
@@ -461,7 +482,12 @@ class HybridEngine(SlotEngine):
         h = self._decode_hidden(tok, own_head)
         if own_head:
             in_place = tok.data_ptr() == self.tok.data_ptr()
-            nxt = ops.lm_head_argmax(h, self.w.head, self.argmax_ws, out=tok if in_place else None, overlap=ops.OVERLAP_START)
+            out = tok if in_place else None
+            if isinstance(h, hops.Rows):
+                nxt = ops.lm_head_argmax_normed(h.scaled, h.squares, self.w.head, self.cfg.eps, self.argmax_ws, out=out,
+                                                overlap=ops.OVERLAP_START, width=self.cfg.width)
+            else:
+                nxt = ops.lm_head_argmax(h, self.w.head, self.argmax_ws, out=out, overlap=ops.OVERLAP_START)
         else:
             nxt = ops.argmax_rows(self.logits(h, cap=False), self.argmax_ws)
         self._move_on()

@@ -3,10 +3,12 @@ streams, minGRU, HGRN2 and latent attention.  The element type of activations an
 the tensors; shapes follow the padded layout the weight loader makes (`hybrid.py`)."""
 from __future__ import annotations
 
+from typing import NamedTuple
+
 import torch
 
 from . import _lib
-from .ops import PAGE_SIZE, _ptr, _require_cuda, _stream
+from .ops import PAGE_SIZE, _ptr, _require_cuda, _stream, skinny_gemm_joins
 
 LATENT_MAX_SPLITS = 64
 
@@ -37,6 +39,42 @@ def hyper_connect(streams, weights, true_width: int, eps: float, dtype, y=None, 
               _ptr(y), parts, _ptr(weights), _ptr(gains), _ptr(h), rows, s, width, true_width, float(eps), _f32(h), int(overlap),
               _stream())
     return h
+
+
+HYPER_JOIN_STREAMS = 4
+
+
+class Rows(NamedTuple):
+    """A sublayer's input before its division by the rms."""
+    scaled: torch.Tensor
+    squares: torch.Tensor
+
+
+class Joint(NamedTuple):
+    """What `hyper_join` takes beside the product."""
+    streams: torch.Tensor
+    weights: torch.Tensor
+    gains: torch.Tensor | None
+
+
+def hyper_join(x, weight, streams, weights, gains=None, parts=None, overlap: int = 0) -> Rows:
+    """`hyper_connect` as the end of the product y = x @ weight^T (weight: maybe a column range) whose output it takes, `parts`
+    [P, rows, width] being earlier parts of y: the streams move on in place; returns the next sublayer's input before its division by the
+    rms, and the sums of squares of every 16 columns (`ops.skinny_gemm_normed`)."""
+    rows, s, width = streams.shape
+    assert streams.dtype == weights.dtype == torch.float32 and streams.is_contiguous() and weights.is_contiguous()
+    assert weights.numel() == s * s + 2 * s + 1 and s <= HYPER_JOIN_STREAMS and skinny_gemm_joins(rows, width, x.shape[1])
+    assert x.shape == (rows, weight.shape[1]) and weight.shape[0] == width and x.stride(1) == weight.stride(1) == 1
+    assert x.dtype == weight.dtype == torch.bfloat16
+    assert gains is None or (gains.dtype == torch.float32 and gains.numel() == width and gains.is_contiguous())
+    assert parts is None or (parts.ndim == 3 and parts.shape[1:] == (rows, width) and parts.is_contiguous() and parts.dtype == x.dtype)
+    _require_cuda(x, weight, streams, weights)
+    scaled = torch.empty((rows, width), dtype=x.dtype, device=x.device)
+    squares = torch.empty((rows, width // 16), dtype=torch.float32, device=x.device)
+    _lib.call("b200_skinny_gemm_hyper_join", _ptr(x), x.stride(0), _ptr(weight), weight.stride(0), _ptr(streams), _ptr(weights), _ptr(gains),
+              _ptr(parts), 0 if parts is None else parts.shape[0], _ptr(scaled), _ptr(squares), rows, width, x.shape[1], s, int(overlap),
+              _stream())
+    return Rows(scaled, squares)
 
 
 def swiglu_f32(gate_up, intermediate: int):

@@ -282,11 +282,11 @@ class SwiGLU:
         return engine.linear(self._act(engine.linear(h, self.gate_up)), self.down)
 
     def decode(self, h, engine, nxt: bool):
-        flags = engine.then(engine.streams_weight(self.down))
+        own_down = engine.streams_weight(self.down)
         if engine.streams_weight(self.gate_up, swiglu=True):
-            act = ops.skinny_gemm(h, self.gate_up, swiglu=True, overlap=flags)
+            act = engine.proj(h, self.gate_up, own_down, swiglu=True)
         else:
-            act = self._act(F.linear(h, self.gate_up), overlap=flags)
+            act = self._act(F.linear(h, self.gate_up), overlap=engine.then(own_down))
         return engine.proj(act, self.down, nxt)
 
 

@@ -935,8 +935,8 @@ def skinny_gemm_join(x, weight, residual, gain, overlap: int = 0):
     return total, scaled, squares
 
 
-def skinny_gemm_normed(scaled, squares, weight, eps: float, overlap: int = 0, swiglu: bool = False):
-    """`skinny_gemm` of the RMS-normed rows that `skinny_gemm_join` prepared."""
+def skinny_gemm_normed(scaled, squares, weight, eps: float, overlap: int = 0, swiglu: bool = False, width: int | None = None):
+    """`skinny_gemm` of the RMS-normed rows that `skinny_gemm_join` prepared; width: columns that the mean counts, if not all."""
     m, k = scaled.shape
     n = weight.shape[0]
     assert scaled.dtype == weight.dtype == torch.bfloat16 and scaled.is_contiguous() and weight.is_contiguous() and weight.shape[1] == k
@@ -946,12 +946,12 @@ def skinny_gemm_normed(scaled, squares, weight, eps: float, overlap: int = 0, sw
         n //= 2
     _require_cuda(scaled, squares, weight)
     y = torch.empty((m, n), dtype=torch.bfloat16, device=scaled.device)
-    _lib.call("b200_skinny_gemm_normed", _ptr(scaled), _ptr(squares), _ptr(weight), _ptr(y), n, m, n, k, float(eps), int(swiglu), int(overlap),
-              _stream())
+    _lib.call("b200_skinny_gemm_normed", _ptr(scaled), _ptr(squares), _ptr(weight), _ptr(y), n, m, n, k, width or k, float(eps), int(swiglu),
+              int(overlap), _stream())
     return y
 
 
-def lm_head_argmax_normed(scaled, squares, table, eps: float, workspace, out=None, overlap: int = 0) -> torch.Tensor:
+def lm_head_argmax_normed(scaled, squares, table, eps: float, workspace, out=None, overlap: int = 0, width: int | None = None) -> torch.Tensor:
     """`lm_head_argmax` of the RMS-normed rows that `skinny_gemm_join` prepared."""
     m, k = scaled.shape
     assert scaled.dtype == table.dtype == torch.bfloat16 and scaled.is_contiguous() and table.is_contiguous() and table.shape[1] == k
@@ -961,7 +961,7 @@ def lm_head_argmax_normed(scaled, squares, table, eps: float, workspace, out=Non
         out = torch.empty(m, dtype=torch.int64, device=scaled.device)
     assert out.dtype == torch.int64 and out.is_contiguous() and out.numel() == m
     _lib.call("b200_lm_head_argmax_normed", _ptr(scaled), _ptr(squares), float(eps), _ptr(table), _ptr(out), _ptr(workspace), m, table.shape[0], k,
-              int(overlap), _stream())
+              width or k, int(overlap), _stream())
     return out
 
 

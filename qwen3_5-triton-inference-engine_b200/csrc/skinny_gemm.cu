@@ -49,6 +49,7 @@ struct SkinnyGemmParams {
   int m, n, k, row_blocks, overlap, up_row0;  // n: outputs; up_row0: first W row of the `up` half (SwiGLU form)
   const float* squares;    // normed form: [M, K / 16] sums of squares of 16 columns each; null: X as it is
   float eps;
+  int true_k;              // columns that the mean counts (the others are zeros)
   // arg-max form: ids[b] = argmax_n y[b, n] instead of y (keys / counter: zero-filled workspace, left zero)
   int64_t* ids;
   unsigned long long* keys;
@@ -255,7 +256,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
       for (int i = 0; i < SQUARES; ++i) ss += sq[i];
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      if ((tid & 7) == 0 && (tid >> 3) < ROWS) scale[tid >> 3] = rsqrtf(ss / static_cast<float>(p.k) + p.eps);
+      if ((tid & 7) == 0 && (tid >> 3) < ROWS) scale[tid >> 3] = rsqrtf(ss / static_cast<float>(p.true_k) + p.eps);
     }
     __syncthreads();  // (also: the previous block's staging has been written out)
     // acc[nt]: rows (tile row = lane/4, +8), cols (batch = nt*8 + (lane%4)*2, +1)  ->  stage[batch][output] -> Y
@@ -392,7 +393,14 @@ struct WideKParams {
   int64_t res_stride;
   __nv_bfloat16* scaled;   // [M, N] contiguous
   float* squares;
+  // ... or with S hyper-connected streams [M, S, N] in place of the residual: x_t <- sum_s mix[s, t] x_s + out[t] y with y = earlier parts + X W^T,
+  // s = sum_t in[t] x_t, scaled = s gain gains[n]
+  float* streams;
+  const float *joint, *gains;   // [mix S*S | out S | in S | gain], [N] or null
+  const __nv_bfloat16* parts;   // [n_parts][M, N] contiguous
+  int s, n_parts;
 };
+constexpr int JOINT_STREAMS = 4;
 
 __global__ void __launch_bounds__(SG_THREADS, 1)
 skinny_gemm_widek_kernel(const __grid_constant__ WideKParams p, const __grid_constant__ CUtensorMap map_w) {
@@ -557,13 +565,16 @@ constexpr int pairk_smem(int nt, int k) {  // rings, sums of the warps and the p
 }
 static_assert(pairk_smem(4, PK_MAX_K) <= 227 * 1024, "weight rings + half of X must fit the 227 KiB a CTA may use");
 
-template <int NT>
+// END: what becomes of the product: 0 the output, 1 joined with a residual, 2 with hyper-connected streams (one kernel that decided when it
+// ran cost a decode step of 32 sequences 4 us)
+template <int NT, int END>
 __global__ void __launch_bounds__(SG_THREADS, 1)
 skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr int ROWS = NT * 8;
   __shared__ uint64_t bars[SG_WARPS][PK_RING];
   __shared__ uint64_t bar_x[PK_MAX_K / 2 / SG_TILE_K];  // one per k tile
+  __shared__ float joint[JOINT_STREAMS * JOINT_STREAMS + 2 * JOINT_STREAMS + 1];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -598,11 +609,13 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
     for (int t = 0; t < PK_RING && t < total_tiles; ++t) issue(t);  // weights: independent of the predecessor
   }
   // thread -> batch row tid / 4, outputs (tid % 4) * 4 .. + 4 of a row block (N is a multiple of 8 and r of 4: inside or outside together)
-  const bool joins = p.scaled != nullptr;
+  constexpr bool joins = END > 0, hyper = END == 2;
   const int b = tid >> 2, r = (tid & 3) * 4;
   const auto writes = [&](int n0) { return rank == 0 && b < p.m && n0 < p.n; };
   uint2 res = {}, gain = {};
-  if (joins && writes(pair * WK_ROWS + r)) gain = *reinterpret_cast<const uint2*>(p.gain + pair * WK_ROWS + r);
+  float4 old[JOINT_STREAMS], gains = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (joins && !hyper && writes(pair * WK_ROWS + r)) gain = *reinterpret_cast<const uint2*>(p.gain + pair * WK_ROWS + r);
+  if (hyper && tid < p.s * p.s + 2 * p.s + 1) joint[tid] = p.joint[tid];
   pdl_wait();  // X is the predecessor's output
   if (lane == 0) {
     for (int kl = warp; kl < half_tiles; kl += SG_WARPS) {
@@ -610,7 +623,19 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
       tma_load_3d(xs + kl * X_TILE, &map_x, 0, 0, (static_cast<int>(rank) * half_tiles + kl) * 2, &bar_x[kl]);
     }
   }
-  if (joins && writes(pair * WK_ROWS + r)) res = *reinterpret_cast<const uint2*>(p.residual + b * p.res_stride + pair * WK_ROWS + r);
+  // what the row is joined with, on its way under the products
+  const auto fetch = [&](int n0) {
+    if (!joins || !writes(n0)) return;
+    if (!hyper) {
+      res = *reinterpret_cast<const uint2*>(p.residual + b * p.res_stride + n0);
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < JOINT_STREAMS; ++i)
+      if (i < p.s) old[i] = *reinterpret_cast<const float4*>(p.streams + (static_cast<int64_t>(b) * p.s + i) * p.n + n0);
+    if (p.gains != nullptr) gains = *reinterpret_cast<const float4*>(p.gains + n0);
+  };
+  fetch(pair * WK_ROWS + r);
   __syncthreads();
   bool ok = true;
 
@@ -625,9 +650,9 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     const int n0 = rb * WK_ROWS + r;
-    if (joins && blk > 0 && writes(n0)) {
-      res = *reinterpret_cast<const uint2*>(p.residual + b * p.res_stride + n0);
-      gain = *reinterpret_cast<const uint2*>(p.gain + n0);
+    if (blk > 0) {
+      fetch(n0);
+      if (joins && !hyper && writes(n0)) gain = *reinterpret_cast<const uint2*>(p.gain + n0);
     }
     for (int kl = warp; kl < half_tiles; kl += SG_WARPS, ++t) {
       const int slot = t % PK_RING;
@@ -668,7 +693,44 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
     if (rank == 0 && mine) {
       const float4 other = *reinterpret_cast<const float4*>(peer + b * WK_ROWS + r);
       uint2 y = make_uint2(pack_bf16(o[0] + other.x, o[1] + other.y), pack_bf16(o[2] + other.z, o[3] + other.w));
-      if (joins) {
+      if constexpr (hyper) {
+        float v[4] = {bf16_lo(y.x), bf16_hi(y.x), bf16_lo(y.y), bf16_hi(y.y)}, u[4] = {};
+        if (writes(n0)) {
+          if (p.n_parts > 0) {                          // the parts in their order, this one last
+            float sum[4] = {};
+            for (int i = 0; i < p.n_parts; ++i) {
+              const uint2 part = *reinterpret_cast<const uint2*>(p.parts + (static_cast<int64_t>(i) * p.m + b) * p.n + n0);
+              sum[0] += bf16_lo(part.x), sum[1] += bf16_hi(part.x), sum[2] += bf16_lo(part.y), sum[3] += bf16_hi(part.y);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] += sum[j];
+          }
+          const float *out = joint + p.s * p.s, *in = out + p.s;
+#pragma unroll
+          for (int st = 0; st < JOINT_STREAMS; ++st)
+            if (st < p.s) {
+              float a[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) a[j] = out[st] * v[j];
+#pragma unroll
+              for (int i = 0; i < JOINT_STREAMS; ++i)
+                if (i < p.s) {
+                  const float m = joint[i * p.s + st];
+                  a[0] = fmaf(m, old[i].x, a[0]), a[1] = fmaf(m, old[i].y, a[1]), a[2] = fmaf(m, old[i].z, a[2]), a[3] = fmaf(m, old[i].w, a[3]);
+                }
+              *reinterpret_cast<float4*>(p.streams + (static_cast<int64_t>(b) * p.s + st) * p.n + n0) = make_float4(a[0], a[1], a[2], a[3]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) u[j] = fmaf(in[st], a[j], u[j]);
+            }
+          const float g = in[p.s];
+          *reinterpret_cast<uint2*>(p.scaled + static_cast<int64_t>(b) * p.n + n0) =
+              make_uint2(pack_bf16(u[0] * g * gains.x, u[1] * g * gains.y), pack_bf16(u[2] * g * gains.z, u[3] * g * gains.w));
+        }
+        float ss = u[0] * u[0] + u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (r == 0 && b < p.m) p.squares[b * p.row_blocks + rb] = ss;
+      } else if constexpr (joins) {
         // product and sum are bf16 tensors in the reference
         const float v0 = round_bf16(bf16_lo(y.x) + bf16_lo(res.x)), v1 = round_bf16(bf16_hi(y.x) + bf16_hi(res.x));
         const float v2 = round_bf16(bf16_lo(y.y) + bf16_lo(res.y)), v3 = round_bf16(bf16_hi(y.y) + bf16_hi(res.y));
@@ -682,7 +744,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
         if (r == 0 && b < p.m) p.squares[b * p.row_blocks + rb] = ss;
       }
-      if (writes(n0)) *reinterpret_cast<uint2*>(p.y + static_cast<int64_t>(b) * p.y_stride + n0) = y;
+      if (!hyper && writes(n0)) *reinterpret_cast<uint2*>(p.y + static_cast<int64_t>(b) * p.y_stride + n0) = y;
     }
     if (blk + 1 < my_blocks) cluster_sync();  // rank 0 has read `peer` before rank 1 writes the next sum
   }
@@ -812,7 +874,7 @@ static int launch_widek(WideKParams p, const void* weight, int64_t w_stride, cud
   return check_launch(what);
 }
 
-template <int NT>
+template <int NT, int END>
 static int launch_pairk_rows(WideKParams p, const CUtensorMap& map, cudaStream_t stream) {
   const char* what = "skinny_gemm";
   CUtensorMap map_x = {};
@@ -822,17 +884,18 @@ static int launch_pairk_rows(WideKParams p, const CUtensorMap& map, cudaStream_t
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(skinny_gemm_pairk_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) != cudaSuccess)
+    if (cudaFuncSetAttribute(skinny_gemm_pairk_kernel<NT, END>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max) != cudaSuccess)
       return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, smem_max);
     configured[dev] = true;
   }
   const int sms = sm_count(), pairs = p.row_blocks < sms / 2 ? p.row_blocks : sms / 2;
-  if (launch_pdl_cluster((p.overlap & OVERLAP_START) != 0, 2, skinny_gemm_pairk_kernel<NT>, dim3(2 * pairs), dim3(SG_THREADS),
+  if (launch_pdl_cluster((p.overlap & OVERLAP_START) != 0, 2, skinny_gemm_pairk_kernel<NT, END>, dim3(2 * pairs), dim3(SG_THREADS),
                          pairk_smem(NT, p.k), stream, p, map, map_x) != cudaSuccess)
     return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
   return check_launch(what);
 }
 
+template <int END>
 static int launch_pairk(WideKParams p, const void* weight, int64_t w_stride, cudaStream_t stream) {
   const char* what = "skinny_gemm";
   CUtensorMap map;
@@ -840,9 +903,9 @@ static int launch_pairk(WideKParams p, const void* weight, int64_t w_stride, cud
   p.err = wait_timeout_flag();
   if (!p.err) return fail(ERR_RUNTIME, "%s: no error flag", what);
   p.row_blocks = (p.n + WK_ROWS - 1) / WK_ROWS;
-  if (p.m <= 8) return launch_pairk_rows<1>(p, map, stream);
-  if (p.m <= 16) return launch_pairk_rows<2>(p, map, stream);
-  return launch_pairk_rows<4>(p, map, stream);
+  if (p.m <= 8) return launch_pairk_rows<1, END>(p, map, stream);
+  if (p.m <= 16) return launch_pairk_rows<2, END>(p, map, stream);
+  return launch_pairk_rows<4, END>(p, map, stream);
 }
 
 static int check_skinny_shape(const char* what, int m, int n, int k) {
@@ -876,7 +939,36 @@ extern "C" int b200_skinny_gemm_join(const void* x, int64_t x_stride, const void
   p.gain = static_cast<const __nv_bfloat16*>(gain);
   p.scaled = static_cast<__nv_bfloat16*>(scaled);
   p.squares = squares;
-  return launch_pairk(p, weight, k, reinterpret_cast<cudaStream_t>(stream));
+  return launch_pairk<1>(p, weight, k, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int b200_skinny_gemm_hyper_join(const void* x, int64_t x_stride, const void* weight, int64_t w_stride, float* streams, const float* joint,
+                                           const float* gains, const void* parts, int32_t n_parts, void* scaled, float* squares, int32_t m,
+                                           int32_t n, int32_t k, int32_t s, int32_t overlap, b200_stream_t stream) {
+  B200_REQUIRE(m > 0 && m <= SG_MAX_M && n > 0 && n % WK_ROWS == 0 && k > SG_MAX_K && k <= PK_MAX_K && k % (2 * SG_TILE_K) == 0,
+               "skinny_gemm_hyper_join: M must be in [1, %d], N a multiple of %d, K in (%d, %d] a multiple of %d (got M=%d N=%d K=%d)", SG_MAX_M,
+               WK_ROWS, SG_MAX_K, PK_MAX_K, 2 * SG_TILE_K, m, n, k);
+  B200_REQUIRE(s > 0 && s <= JOINT_STREAMS && n_parts >= 0 && (n_parts == 0 || aligned16(parts)), "skinny_gemm_hyper_join: 1 to %d streams (got %d)",
+               JOINT_STREAMS, s);
+  B200_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(streams) && aligned16(scaled) && joint != nullptr && squares != nullptr &&
+                   (gains == nullptr || aligned16(gains)) && x_stride % 8 == 0 && w_stride >= k && w_stride % 8 == 0,
+               "skinny_gemm_hyper_join: pointers must be 16-byte aligned, row strides multiples of 8 elements");
+  WideKParams p = {};
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.x_stride = x_stride;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.overlap = overlap;
+  p.scaled = static_cast<__nv_bfloat16*>(scaled);
+  p.squares = squares;
+  p.streams = streams;
+  p.joint = joint;
+  p.gains = gains;
+  p.parts = static_cast<const __nv_bfloat16*>(parts);
+  p.s = s;
+  p.n_parts = n_parts;
+  return launch_pairk<2>(p, weight, w_stride, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int b200_skinny_gemm_part(const void* x, int64_t x_stride, const void* weight, int64_t w_stride, void* y,
@@ -897,7 +989,7 @@ extern "C" int b200_skinny_gemm_part(const void* x, int64_t x_stride, const void
     wp.n = n;
     wp.k = k;
     wp.overlap = overlap;
-    if (k <= PK_MAX_K && k % (2 * SG_TILE_K) == 0) return launch_pairk(wp, weight, w_stride, reinterpret_cast<cudaStream_t>(stream));
+    if (k <= PK_MAX_K && k % (2 * SG_TILE_K) == 0) return launch_pairk<0>(wp, weight, w_stride, reinterpret_cast<cudaStream_t>(stream));
     return launch_widek(wp, weight, w_stride, reinterpret_cast<cudaStream_t>(stream));
   }
   int rc = check_skinny_shape("skinny_gemm", m, n, k);
@@ -940,9 +1032,11 @@ extern "C" int b200_skinny_gemm_swiglu(const void* x, int64_t x_stride, const vo
 }
 
 extern "C" int b200_skinny_gemm_normed(const void* x, const float* squares, const void* weight, void* y, int64_t y_stride, int32_t m,
-                                       int32_t n, int32_t k, float eps, int32_t swiglu, int32_t overlap, b200_stream_t stream) {
+                                       int32_t n, int32_t k, int32_t true_k, float eps, int32_t swiglu, int32_t overlap,
+                                       b200_stream_t stream) {
   int rc = check_skinny_shape("skinny_gemm_normed", m, n, k);
   if (rc != OK) return rc;
+  B200_REQUIRE(true_k > 0 && true_k <= k, "skinny_gemm_normed: the mean over %d of %d columns", true_k, k);
   B200_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(y) && squares != nullptr && y_stride % 8 == 0,
                "skinny_gemm_normed: pointers must be 16-byte aligned, the row stride of y a multiple of 8 elements");
   SkinnyGemmParams p = {};
@@ -956,12 +1050,13 @@ extern "C" int b200_skinny_gemm_normed(const void* x, const float* squares, cons
   p.overlap = overlap;
   p.squares = squares;
   p.eps = eps;
+  p.true_k = true_k;
   p.up_row0 = n;
   if (swiglu) return launch_skinny<true>(p, weight, k, 2 * n, reinterpret_cast<cudaStream_t>(stream), "skinny_gemm_normed");
   return launch_skinny<false>(p, weight, k, n, reinterpret_cast<cudaStream_t>(stream), "skinny_gemm_normed");
 }
 
-static int lm_head_argmax(const void* x, int64_t x_stride, const float* squares, float eps, const void* weight, int64_t* ids, void* workspace,
+static int lm_head_argmax(const void* x, int64_t x_stride, const float* squares, int32_t true_k, float eps, const void* weight, int64_t* ids, void* workspace,
                           int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream) {
   int rc = check_skinny_shape("lm_head_argmax", m, n, k);
   if (rc != OK) return rc;
@@ -978,6 +1073,7 @@ static int lm_head_argmax(const void* x, int64_t x_stride, const float* squares,
   p.overlap = overlap;
   p.squares = squares;
   p.eps = eps;
+  p.true_k = true_k;
   p.ids = ids;
   p.keys = static_cast<unsigned long long*>(workspace);  // the layout of b200_argmax_rows: 1024 keys, then counters
   p.counter = reinterpret_cast<int*>(p.keys + 1024);
@@ -986,11 +1082,11 @@ static int lm_head_argmax(const void* x, int64_t x_stride, const float* squares,
 
 extern "C" int b200_lm_head_argmax(const void* x, int64_t x_stride, const void* weight, int64_t* ids, void* workspace,
                                    int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream) {
-  return lm_head_argmax(x, x_stride, nullptr, 0.f, weight, ids, workspace, m, n, k, overlap, stream);
+  return lm_head_argmax(x, x_stride, nullptr, k, 0.f, weight, ids, workspace, m, n, k, overlap, stream);
 }
 
 extern "C" int b200_lm_head_argmax_normed(const void* x, const float* squares, float eps, const void* weight, int64_t* ids, void* workspace,
-                                          int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream) {
-  B200_REQUIRE(squares != nullptr, "lm_head_argmax_normed: no sums of squares");
-  return lm_head_argmax(x, k, squares, eps, weight, ids, workspace, m, n, k, overlap, stream);
+                                          int32_t m, int32_t n, int32_t k, int32_t true_k, int32_t overlap, b200_stream_t stream) {
+  B200_REQUIRE(squares != nullptr && true_k > 0 && true_k <= k, "lm_head_argmax_normed: no sums of squares, or a mean over %d of %d columns", true_k, k);
+  return lm_head_argmax(x, k, squares, true_k, eps, weight, ids, workspace, m, n, k, overlap, stream);
 }

@@ -73,3 +73,37 @@ def test_shapes_refused():
 
     for m, n, k in ((33, 1024, 2048), (8, 1024, 1280), (8, 1024, 4352), (8, 2048, 2048), (8, 1032, 2048), (8, 1024, 2176)):
         assert not ops.skinny_gemm_joins(m, n, k)
+
+
+@pytest.mark.parametrize("m,streams,parts,k", [(1, 2, 0, 2048), (8, 1, 1, 1536), (9, 4, 2, 3584), (32, 2, 1, 4096), (17, 3, 0, 1536)])
+def test_hyper_join(m, streams, parts, k, n=1024):
+    """Against the product and hyper_connect in two launches: the streams are the same bits, the rows times 1 / rms the same values."""
+    from b200attn import hybrid_ops as hops
+    from b200attn import ops
+
+    true_n = n - 40
+    x, w, _, gain = _rows(m, n, 2 * k, m + k)
+    x, w = x[:, k:].contiguous(), w[:, :k]                    # a column range
+    g = torch.Generator().manual_seed(k)
+    state = torch.randn((m, streams, n), generator=g).to("cuda")
+    weights = torch.rand(streams * streams + 2 * streams + 1, generator=g).to("cuda")
+    state[:, :, true_n:], w[true_n:] = 0, 0                   # padding columns
+    earlier = torch.randn((parts, m, n), generator=g).to("cuda", torch.bfloat16) if parts else None
+    gains = gain.float() + 1 if parts else None
+    y = torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+    ops.skinny_gemm_part(x, w, y)
+    if parts:
+        earlier[:, :, true_n:] = 0
+        y = torch.cat((earlier, y[None]))
+    want_state, have_state = state.clone(), state.clone()
+    want = hops.hyper_connect(want_state, weights, true_n, EPS, torch.bfloat16, y=y, gains=gains)
+    rows = hops.hyper_join(x, w, have_state, weights, gains, earlier)
+    assert torch.equal(have_state, want_state)
+    rms = torch.rsqrt(rows.squares.double().sum(-1, keepdim=True) / true_n + EPS)
+    # either is rounded to bf16 once
+    assert ((rows.scaled.double() * rms - want.double()).abs() <= 2.0 ** -7 * want.double().abs() + 1e-30).all()
+    up = torch.randn((64, n), generator=g).to("cuda", torch.bfloat16) * n ** -0.5
+    y64 = (rows.scaled.double() @ up.double().T) * rms
+    bound = ((rows.scaled.double().abs() @ up.double().abs().T) * rms) * (n * 2.0 ** -24)
+    got = ops.skinny_gemm_normed(*rows, up, EPS, width=true_n)
+    assert ((got.double() - y64).abs() <= bound + 2.0 ** -8 * y64.abs()).all()
