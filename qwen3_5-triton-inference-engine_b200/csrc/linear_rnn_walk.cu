@@ -203,7 +203,7 @@ struct WalkSmem {
 // One CTA = one head of one sequence or segment and up to 128 value columns.  LOCAL: only the state from zero and the total
 // decay of every segment.  Eight warps multiply, 16 value columns each, and bring their own values; four others take o from
 // shared memory, a chunk behind: head norm, gate, stores.  Slots come by one bulk copy each, OW_STAGES ahead.
-// What bounds it: the tensor pipe, 84 products per warp and chunk (16 cycles each and scheduler, two warps per scheduler).  The
+// What bounds it: the tensor pipe, 84 products per warp and chunk (8.4 cycles of a scheduler each, two warps per scheduler).  The
 // state's update stands between the products of q and S, so that consecutive ones do not depend on one another, and nothing
 // else is left to the multiplying warps (with norm, gate and stores in their own loop a chunk took 2.2 to 3.0 us, now 1.7; the
 // pipe alone 1.4).  Half heads per CTA, two to a cluster that exchanges the norm's sums, gained on one long sequence and lost on
