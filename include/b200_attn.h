@@ -394,7 +394,7 @@ int b200_skinny_gemm_swiglu(const void* x, int64_t x_stride, const void* weight,
  *                            contiguous, squares [M, N / 16].  residual and the outputs must not overlap.
  *   b200_skinny_gemm_normed  Y = (X W^T) / rms, rms = sqrt(mean of squares over K + eps), for X = scaled [M,K] contiguous of the call above:
  *                            b200_skinny_gemm (or, swiglu != 0, b200_skinny_gemm_swiglu; n counts outputs) of the normed rows, K <= 1280.
- *   b200_lm_head_argmax_normed  b200_lm_head_argmax of the normed rows.
+ *   b200_lm_head_argmax takes the rows as they are: the division does not move an arg-max.
  *   b200_skinny_gemm_hyper_join  b200_hyper_connect in place of add and norm: the streams [M, S <= 4, N] move on in place with the product (and
  *                            n_parts earlier parts of it, [n_parts][M,N] bf16, summed in front), scaled = bf16(read-out * gain * gains).
  * true_k: columns that the mean counts. */
@@ -405,8 +405,6 @@ int b200_skinny_gemm_hyper_join(const void* x, int64_t x_stride, const void* wei
                                 int32_t k, int32_t s, int32_t overlap, b200_stream_t stream);
 int b200_skinny_gemm_normed(const void* x, const float* squares, const void* weight, void* y, int64_t y_stride, int32_t m, int32_t n,
                             int32_t k, int32_t true_k, float eps, int32_t swiglu, int32_t overlap, b200_stream_t stream);
-int b200_lm_head_argmax_normed(const void* x, const float* squares, float eps, const void* weight, int64_t* ids, void* workspace, int32_t m,
-                               int32_t n, int32_t k, int32_t true_k, int32_t overlap, b200_stream_t stream);
 
 /* ids[b] = argmax over n of <x[b, :], weight[n, :]> with fp32 accumulation, ties to the lowest n: the LM head with a tied
  * embedding and its greedy sampling in one launch (triton_kernels/vocab_argmax.py:141-200); the logits are never written.

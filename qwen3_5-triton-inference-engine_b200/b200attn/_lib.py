@@ -51,7 +51,6 @@ SIGNATURES: dict[str, list] = {
     "b200_skinny_gemm_join": [P, I64, P, P, I64, P, P, P, P, I32, I32, I32, I32, P],
     "b200_skinny_gemm_hyper_join": [P, I64, P, I64, P, P, P, P, I32, P, P, I32, I32, I32, I32, I32, P],
     "b200_skinny_gemm_normed": [P, P, P, P, I64, I32, I32, I32, I32, c_float, I32, I32, P],
-    "b200_lm_head_argmax_normed": [P, P, c_float, P, P, P, I32, I32, I32, I32, I32, P],
     "b200_argmax_rows": [P, I64, P, P, I32, I32, I32, P],
     "b200_lm_head_argmax": [P, I64, P, P, P, I32, I32, I32, I32, P],
     "b200_add_rmsnorm": [P, I64, I64, I32, P, I64, P, P, P, I32, I32, c_float, I32, P],

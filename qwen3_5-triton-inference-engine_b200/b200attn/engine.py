@@ -375,11 +375,7 @@ class Engine(SlotEngine):
             # the ids go straight into `tok` when it is the engine's own token buffer (read only by the gather at the
             # top of the step): no copy kernel behind the step
             in_place = tok.data_ptr() == self.tok.data_ptr() and tok.dtype == torch.int64 and tok.is_contiguous()
-            out = tok if in_place else None
-            if squares is None:
-                nxt = ops.lm_head_argmax(h, embed, self.argmax_ws, out=out, overlap=start)
-            else:
-                nxt = ops.lm_head_argmax_normed(h, squares, embed, cfg.eps, self.argmax_ws, out=out, overlap=start)
+            nxt = ops.lm_head_argmax(h, embed, self.argmax_ws, out=tok if in_place else None, overlap=start)
         else:          # fp32 logits from cuBLAS, arg-max (lowest index on ties) in one launch
             nxt = glue.lm_head_argmax(h, embed, last_only=False,
                                       argmax=lambda logits: ops.argmax_rows(logits, self.argmax_ws, overlap=start))

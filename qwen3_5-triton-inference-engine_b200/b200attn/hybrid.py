@@ -482,12 +482,8 @@ class HybridEngine(SlotEngine):
         h = self._decode_hidden(tok, own_head)
         if own_head:
             in_place = tok.data_ptr() == self.tok.data_ptr()
-            out = tok if in_place else None
-            if isinstance(h, hops.Rows):
-                nxt = ops.lm_head_argmax_normed(h.scaled, h.squares, self.w.head, self.cfg.eps, self.argmax_ws, out=out,
-                                                overlap=ops.OVERLAP_START, width=self.cfg.width)
-            else:
-                nxt = ops.lm_head_argmax(h, self.w.head, self.argmax_ws, out=out, overlap=ops.OVERLAP_START)
+            rows = h.scaled if isinstance(h, hops.Rows) else h       # the division by the rms moves no arg-max
+            nxt = ops.lm_head_argmax(rows, self.w.head, self.argmax_ws, out=tok if in_place else None, overlap=ops.OVERLAP_START)
         else:
             nxt = ops.argmax_rows(self.logits(h, cap=False), self.argmax_ws)
         self._move_on()

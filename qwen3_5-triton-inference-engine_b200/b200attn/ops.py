@@ -921,7 +921,7 @@ def skinny_gemm_joins(m: int, n: int, k: int) -> bool:
 def skinny_gemm_join(x, weight, residual, gain, overlap: int = 0):
     """`skinny_gemm` of a projection back to the hidden size, the residual added and the RMSNorm behind it prepared: returns the sum
     s = residual + x @ weight^T [M, N], the rows s * (1 + gain) and the sums of squares of every 16 columns of s [M, N / 16] fp32.
-    `skinny_gemm_normed` and `lm_head_argmax_normed` take the last two."""
+    `skinny_gemm_normed` takes the last two, `lm_head_argmax` the rows (a positive factor moves no arg-max)."""
     m, k = x.shape
     n = weight.shape[0]
     assert skinny_gemm_joins(m, n, k) and weight.shape[1] == k and residual.shape == (m, n) and gain.shape == (n,)
@@ -949,20 +949,6 @@ def skinny_gemm_normed(scaled, squares, weight, eps: float, overlap: int = 0, sw
     _lib.call("b200_skinny_gemm_normed", _ptr(scaled), _ptr(squares), _ptr(weight), _ptr(y), n, m, n, k, width or k, float(eps), int(swiglu),
               int(overlap), _stream())
     return y
-
-
-def lm_head_argmax_normed(scaled, squares, table, eps: float, workspace, out=None, overlap: int = 0, width: int | None = None) -> torch.Tensor:
-    """`lm_head_argmax` of the RMS-normed rows that `skinny_gemm_join` prepared."""
-    m, k = scaled.shape
-    assert scaled.dtype == table.dtype == torch.bfloat16 and scaled.is_contiguous() and table.is_contiguous() and table.shape[1] == k
-    assert squares.shape == (m, k // 16) and squares.dtype == torch.float32 and squares.is_contiguous()
-    _require_cuda(scaled, squares, table, workspace)
-    if out is None:
-        out = torch.empty(m, dtype=torch.int64, device=scaled.device)
-    assert out.dtype == torch.int64 and out.is_contiguous() and out.numel() == m
-    _lib.call("b200_lm_head_argmax_normed", _ptr(scaled), _ptr(squares), float(eps), _ptr(table), _ptr(out), _ptr(workspace), m, table.shape[0], k,
-              width or k, int(overlap), _stream())
-    return out
 
 
 def skinny_gemm_part(x, weight, out, overlap: int = 0):

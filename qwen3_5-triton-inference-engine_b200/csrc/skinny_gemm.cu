@@ -112,16 +112,15 @@ __device__ __forceinline__ void join_steps(float (&acc)[4][4]) {
     }
   }
 }
-// The eight steps of a tile of 128 k: A (W tile) by ldmatrix from `tile` + offset(step), X from `xt` on (the lane's address in the
-// tensor-map box of the tile: two blocks of [8 NT rows][64 k] with the 128-byte swizzle; a step's 32 bytes are two bits of the address
-// to turn over).
+// The eight steps of a tile of 128 k: A (W tile) by ldmatrix from `tile` + offset(step), X from xj[step & 3] + `xt` on: two blocks of
+// [8 NT rows][64 k] with the 128-byte swizzle, where a step's 32 bytes are two bits of the lane's address to turn over.
 template <int NT, int KS, typename Offset>
-__device__ __forceinline__ void tile_steps(float (&acc)[4][4], uint32_t (&b)[8], uint32_t tile, uint32_t xt, const Offset& offset) {
+__device__ __forceinline__ void tile_steps(float (&acc)[4][4], uint32_t (&b)[8], uint32_t tile, const uint32_t (&xj)[4], uint32_t xt, const Offset& offset) {
   if constexpr (KS < SG_TILE_K / 16) {
     uint32_t a[4];
     ldmatrix_x4(a, tile + offset(KS));
-    StepProducts<NT>::template run<KS>(acc, a, b, (xt + (KS >> 2) * (NT * 8 * 128)) ^ ((KS & 3) * 32));
-    tile_steps<NT, KS + 1>(acc, b, tile, xt, offset);
+    StepProducts<NT>::template run<KS>(acc, a, b, xj[KS & 3] + xt + (KS >> 2) * (NT * 8 * 128));
+    tile_steps<NT, KS + 1>(acc, b, tile, xj, xt, offset);
   }
 }
 constexpr int skinny_smem(int nt, int k) {  // rings, output staging, odd-tile sums, X
@@ -198,7 +197,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   pdl_wait();  // X is the predecessor's output
   // normed form: eight threads per row, asked for now and first looked at behind the products
   constexpr int SQUARES = SG_MAX_K / 16 / 8;
-  const bool normed = p.squares != nullptr;
+  const bool normed = !ARGMAX && p.squares != nullptr;   // a positive factor per row moves no arg-max (and cost the LM head of 32 rows 2 of 91 us)
   float sq[SQUARES];
 #pragma unroll
   for (int i = 0; i < SQUARES; ++i)
@@ -210,6 +209,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
   // ldmatrix lane address of A (W tile): row = lane % 16, chunk parity = lane / 16
   const int a_row = lane & 15, a_par = lane >> 4;
   const uint32_t xs_lane = xs_base + StepProducts<NT>::lane_offset(lane);
+  const uint32_t xj[4] = {xs_lane, xs_lane ^ 32, xs_lane ^ 64, xs_lane ^ 96};
   const auto a_offset = [&](int ks) -> uint32_t {
     // plain: [k-block][16 rows][128 B]; SwiGLU: [gate | up][k-block][8 rows][128 B]; 16-byte chunks XOR-swizzled by row
     return (SWIGLU ? (a_row >> 3) * (SG_TILE_BYTES / 2) + (ks >> 2) * (8 * 128) + (a_row & 7) * 128 : (ks >> 2) * (16 * 128) + a_row * 128) +
@@ -240,7 +240,7 @@ skinny_gemm_kernel(const __grid_constant__ SkinnyGemmParams p, const __grid_cons
         break;
       }
       uint32_t b[8];
-      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xs_lane + kt * X_TILE, a_offset);
+      tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SLOT_BYTES), xj, kt * X_TILE, a_offset);
       __syncwarp();  // every lane has read the tile: its slot can take the tile RING ahead
       if (lane == 0 && t + RING < total_tiles) issue(t + RING);
     }
@@ -641,6 +641,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
 
   const int a_row = lane & 15, a_par = lane >> 4;
   const uint32_t xs_base = smem_u32(xs) + StepProducts<NT>::lane_offset(lane);
+  const uint32_t xj[4] = {xs_base, xs_base ^ 32, xs_base ^ 64, xs_base ^ 96};
   const auto a_offset = [&](int ks) -> uint32_t { return (ks >> 2) * (16 * 128) + a_row * 128 + ((((ks & 3) * 2 + a_par) ^ (a_row & 7)) << 4); };
   const uint32_t peer_remote = cluster_map(smem_u32(peer), 0);
   int t = 0;
@@ -660,7 +661,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
       if (blk == 0 && ok && !mbar_wait_bounded(&bar_x[kl], 0)) ok = false;
       if (ok) {
         uint32_t b[8];
-        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xs_base + kl * X_TILE, a_offset);
+        tile_steps<NT, 0>(acc, b, smem_u32(ring + slot * SG_TILE_BYTES), xj, kl * X_TILE, a_offset);
       }
       __syncwarp();  // every lane has read the tile: its slot can take the tile PK_RING ahead
       if (ok && lane == 0 && t + PK_RING < total_tiles) issue(t + PK_RING);
@@ -1056,8 +1057,8 @@ extern "C" int b200_skinny_gemm_normed(const void* x, const float* squares, cons
   return launch_skinny<false>(p, weight, k, n, reinterpret_cast<cudaStream_t>(stream), "skinny_gemm_normed");
 }
 
-static int lm_head_argmax(const void* x, int64_t x_stride, const float* squares, int32_t true_k, float eps, const void* weight, int64_t* ids, void* workspace,
-                          int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream) {
+extern "C" int b200_lm_head_argmax(const void* x, int64_t x_stride, const void* weight, int64_t* ids, void* workspace,
+                                   int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream) {
   int rc = check_skinny_shape("lm_head_argmax", m, n, k);
   if (rc != OK) return rc;
   B200_REQUIRE(aligned16(x) && aligned16(weight) && x_stride % 8 == 0 && ids != nullptr && workspace != nullptr &&
@@ -1071,22 +1072,8 @@ static int lm_head_argmax(const void* x, int64_t x_stride, const float* squares,
   p.n = n;
   p.k = k;
   p.overlap = overlap;
-  p.squares = squares;
-  p.eps = eps;
-  p.true_k = true_k;
   p.ids = ids;
   p.keys = static_cast<unsigned long long*>(workspace);  // the layout of b200_argmax_rows: 1024 keys, then counters
   p.counter = reinterpret_cast<int*>(p.keys + 1024);
   return launch_skinny<false, true>(p, weight, k, n, reinterpret_cast<cudaStream_t>(stream), "lm_head_argmax");
-}
-
-extern "C" int b200_lm_head_argmax(const void* x, int64_t x_stride, const void* weight, int64_t* ids, void* workspace,
-                                   int32_t m, int32_t n, int32_t k, int32_t overlap, b200_stream_t stream) {
-  return lm_head_argmax(x, x_stride, nullptr, k, 0.f, weight, ids, workspace, m, n, k, overlap, stream);
-}
-
-extern "C" int b200_lm_head_argmax_normed(const void* x, const float* squares, float eps, const void* weight, int64_t* ids, void* workspace,
-                                          int32_t m, int32_t n, int32_t k, int32_t true_k, int32_t overlap, b200_stream_t stream) {
-  B200_REQUIRE(squares != nullptr && true_k > 0 && true_k <= k, "lm_head_argmax_normed: no sums of squares, or a mean over %d of %d columns", true_k, k);
-  return lm_head_argmax(x, k, squares, true_k, eps, weight, ids, workspace, m, n, k, overlap, stream);
 }

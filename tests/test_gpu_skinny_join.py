@@ -1,5 +1,5 @@
 """Products around a residual add and RMSNorm without a launch between them: skinny_gemm_join, then skinny_gemm_normed (plain, SwiGLU) or
-lm_head_argmax_normed, against skinny_gemm and 64 bits."""
+lm_head_argmax, against skinny_gemm and 64 bits."""
 import pytest
 import torch
 
@@ -44,7 +44,7 @@ def test_join_and_normed(m, n, k):
     assert ((act.double() - act64).abs() <= 1.1 * da * b.abs() + torch.nn.functional.silu(a).abs() * db + 1.1 * da * db + 2.0 ** -8 * act64.abs() + 1e-6).all()
 
     table = torch.randn((4096, n), generator=torch.Generator().manual_seed(n)).to("cuda", torch.bfloat16)
-    ids = ops.lm_head_argmax_normed(scaled, squares, table, EPS, ops.argmax_workspace())
+    ids = ops.lm_head_argmax(scaled, table, ops.argmax_workspace())
     logits = (scaled.double() @ table.double().T) * rms
     slack = 2 * (scaled.double().abs() @ table.double().abs().T).amax(-1) * rms[:, 0] * (n * 2.0 ** -24)
     assert (logits.gather(1, ids[:, None])[:, 0] >= logits.amax(-1) - slack).all()
