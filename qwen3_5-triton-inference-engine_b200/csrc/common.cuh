@@ -310,8 +310,8 @@ __device__ __forceinline__ void st_cluster_f32x4(uint32_t addr, float a, float b
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
-// The arrival for what is ordered by other means (tensor memory by tcgen05 fences): the cluster-wide release above first waits for the
-// thread's memory operations, a microsecond where stores are in flight.
+// The arrival for what is ordered by other means (tensor memory by tcgen05 fences; never shared memory): the cluster-wide release above
+// first waits for the thread's memory operations, a microsecond where stores are in flight.
 __device__ __forceinline__ void mbar_arrive_cluster_plain(uint32_t addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }

@@ -16,7 +16,7 @@
 //             through shared memory.  (Two threads per row of every tile: the exponential units idle while S, the row maximum and the
 //             store of P are waited for, 2950 cycles a tile; now 2430 with another tile's under them.)
 //   8-11      rotate the next item's Q in shared memory, then take O of this one through gate and copy engine to the output
-//   12, 15    issue S and PV (even CTA only), 13 loads K, 14 deals the items and loads Q and V
+//   12, 15    issue S and PV (even CTA only; the odd one's 12 passes its rotated Q on), 13 loads K, 14 deals the items and loads Q and V
 // P is stored as packed bf16 over the first 64 columns of the S buffer just read; S of tile j+2 waits for PV of tile j to complete.  O is
 // rescaled in TMEM only when a row maximum grows by more than 2^8 (the running reference maximum may lag; p then stays <= 256, exact
 // for bf16 and fp32 l).
@@ -153,7 +153,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const __grid_constant__ CUtensorMap map_out, const __grid_constant__ PrefillUmmaParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // `lead_*`: waited for by the issuer, the even CTA of the pair; the others are each CTA's own
-  __shared__ uint64_t lead_k[2], lead_v[2], lead_q, lead_p[2][2], lead_o, lead_s[2], bar_q, bar_s[2], bar_pv[2], bar_m[4][2][2], bar_g[PU_OUT_WARPS][PU_STAGE], bar_l[PU_ITEMS], item_full[PU_ITEMS], item_free[PU_ITEMS];
+  __shared__ uint64_t lead_k[2], lead_v[2], lead_q, lead_p[2][2], lead_o, lead_s[2], bar_q, bar_rot, bar_s[2], bar_pv[2], bar_m[4][2][2], bar_g[PU_OUT_WARPS][PU_STAGE], bar_l[PU_ITEMS], item_full[PU_ITEMS], item_free[PU_ITEMS];
   __shared__ uint32_t tmem_slot;
   __shared__ PrefillItem items[PU_ITEMS];
   __shared__ float row_ref[2][2][128];                // [tile parity][item parity][row]: the reference of the last tile of that parity
@@ -176,7 +176,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_init(&bar_s[i], 1);
       mbar_init(&bar_pv[i], 1);
     }
-    mbar_init(&lead_q, FUSED ? 2 * PU_OUT_WARPS : 1);
+    mbar_init(&lead_q, FUSED ? PU_OUT_WARPS + 1 : 1);
+    mbar_init(&bar_rot, PU_OUT_WARPS);
     mbar_init(&lead_o, 2 * PU_OUT_WARPS);
     mbar_init(&lead_s[0], 1);
     mbar_init(&lead_s[1], 1);
@@ -188,7 +189,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     for (int i = 0; i < PU_ITEMS; ++i) {
       mbar_init(&bar_l[i], PU_SOFTMAX_WARPS);
       mbar_init(&item_full[i], 1);
-      mbar_init(&item_free[i], PU_SOFTMAX_WARPS + PU_OUT_WARPS + 1 + (rank == 0 ? 2 : 0));
+      mbar_init(&item_free[i], PU_SOFTMAX_WARPS + PU_OUT_WARPS + 1 + (rank == 0 ? 2 : FUSED ? 1 : 0));
     }
     mbar_fence_init();
   }
@@ -336,7 +337,18 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (leader) mbar_arrive(&lead_s[s]);
         }
       }
-    } else if (rank == 0) {
+    } else if (rank == 1) {
+      // ---------------------------------------------------------------- the odd CTA's rotated Q, handed to the issuer in the even one
+      // The product that reads these rows of shared memory is the other CTA's, so they are released at cluster scope.  By a warp that has no
+      // stores of its own: a release waits for them (by the output warps themselves 32 prompts of 16 to 512 tokens take 63.7 us, so 61.4).
+      if (FUSED && warp == 12) {
+        const uint32_t ready_q = cluster_map(smem_u32(&lead_q), 0);
+        for (int i = 0; fetch(i, it); ++i) {
+          ok = warp_wait_bounded(&bar_rot, i & 1, ok);
+          if (ok && lane == 0) mbar_arrive_cluster(ready_q);
+        }
+      }
+    } else {
       // ---------------------------------------------------------------- issuer of PV for the pair
       // Inside an item S of the tile behind goes into the pipe first: PV has its operand later anyway, and free to overtake one another
       // the two issuers end in two tiles' S, then both PV (3025 cycles a tile of 4096-token prompts, 2765 in this order).  From one item to the next
@@ -378,7 +390,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     
     const int row = tid - 8 * 32;              // TMEM lane; row = token*4 + head
     const uint32_t lane_base = static_cast<uint32_t>(row & ~31) << 16;
-    const uint32_t ready_q = cluster_map(smem_u32(&lead_q), 0), read_o = cluster_map(smem_u32(&lead_o), 0);
+    const uint32_t read_o = cluster_map(smem_u32(&lead_o), 0);
     uint8_t* stage = out_s + (warp - 8) * (PU_STAGE * PU_STAGE_BYTES);  // of [32 rows][32 columns], 64-byte swizzle
     auto rope = [&](const PrefillItem& it, int i) {
       // rotary embedding of this row's q in place (dims [0,32) and [32,64) live in column block 0, chunks c, c+4)
@@ -425,9 +437,10 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         *pa = make_uint4(wa[0], wa[1], wa[2], wa[3]);
         *pb = make_uint4(wb[0], wb[1], wb[2], wb[3]);
       }
-      fence_proxy_async();  // the rotated rows must be visible to the tensor core's reads
+      // The rotated rows are the tensor core's to read: fenced to its proxy, and handed to the issuer of S, in the odd CTA through warp 12
+      fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster_plain(ready_q);
+      if (lane == 0) mbar_arrive(rank == 0 ? &lead_q : &bar_rot);
     };
     PrefillItem it, next;
     bool more = fetch(0, it, true);

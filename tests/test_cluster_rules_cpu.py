@@ -1,0 +1,20 @@
+"""Rules between the CTAs of a cluster that no run can show without a race, read from the sources."""
+import re
+
+from test_launch_rules_cpu import CSRC, body
+
+
+def test_rotated_q_is_released_at_cluster_scope():
+    """Q rotated in the odd CTA's shared memory is read by a product that the even CTA issues: the arrival that hands it over orders the
+    stores for the other CTA.  The plain arrival is left to what tcgen05 fences order: tensor memory, behind a fence of its own."""
+    text = body("prefill_umma", "prefill_pair_kernel")
+    assert re.search(r"fence_proxy_async\(\);\s*__syncwarp\(\);\s*if \(lane == 0\) mbar_arrive\(rank == 0 \? &lead_q : &bar_rot\);", text)
+    assert re.search(r"ready_q = cluster_map\(smem_u32\(&lead_q\), 0\);[^}]*ok = warp_wait_bounded\(&bar_rot, i & 1, ok\);\s*"
+                     r"if \(ok && lane == 0\) mbar_arrive_cluster\(ready_q\);", text)
+    assert "lead_q, FUSED ? PU_OUT_WARPS + 1 : 1" in text and "bar_rot, PU_OUT_WARPS)" in text      # the even CTA's warps and the odd one's 12
+    plain = [m.start() for m in re.finditer(r"mbar_arrive_cluster_plain\(", text)]
+    assert len(plain) == 2
+    for at in plain:
+        assert re.search(r"tc_fence_before_sync\(\);\s*__syncwarp\(\);\s*if \(lane == 0\) $", text[:at])
+    helper = (CSRC / "common.cuh").read_text()
+    assert "mbarrier.arrive.release.cluster.shared::cluster.b64" in helper[helper.index("void mbar_arrive_cluster("):][:160]
