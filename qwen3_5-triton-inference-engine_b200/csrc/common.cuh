@@ -295,6 +295,10 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// A CTA's shared memory may be written by its peers once it is known to run.  All threads say so early, and make sure of it where they
+// wait for something else anyway, in front of their first remote store.
+__device__ __forceinline__ void cluster_started() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_all_started() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 // Address of the same shared-memory location in the CTA of rank `rank` of this cluster.
 __device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t rank) {
   uint32_t out;

@@ -429,6 +429,8 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
       cseg.end = units;
       r0 = min(rank * per, units);
       r1 = min(r0 + per, units);
+      __syncwarp();
+      cluster_started();  // (the form and the segment are the same for all CTAs of the cluster)
     } else {
       pdl_wait();  // a cluster without a segment: all its CTAs leave together, nobody waits for them
       return;
@@ -710,6 +712,7 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
       // the CTA of rank e / tpr; every CTA sends each of its 1024 accumulators to the rank that finishes it (slot
       // [own rank][e % tpr] of that CTA's receive buffer) and its (m, l) to everybody, then all meet at the barrier.
       const int tpr = FD_THREADS >> clog, to = tid >> (8 - clog), piece_of = tid & (tpr - 1);
+      cluster_all_started();
       st_cluster_f32x4(cluster_map(smem_u32(recv + (rank * tpr + piece_of) * 4), static_cast<uint32_t>(to)), acc[0], acc[1], acc[2], acc[3]);
       if ((tid & 63) < csize) {  // every thread of a head has the head's (m, l): one of them per rank sends it
         const uint32_t ml = cluster_map(smem_u32(recv_ml + rank * 8), static_cast<uint32_t>(tid & 63));

@@ -598,6 +598,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   const int my_tiles = half_tiles > warp ? (half_tiles - warp + SG_WARPS - 1) / SG_WARPS : 0;  // per row block, this warp
   const int total_tiles = my_blocks * my_tiles;
   __syncthreads();
+  cluster_started();
   auto issue = [&](int t) {  // lane 0: tile t of this warp
     const int rb = pair + (t / my_tiles) * pairs, kt = static_cast<int>(rank) * half_tiles + warp + SG_WARPS * (t % my_tiles);
     const int slot = t % PK_RING;
@@ -637,6 +638,7 @@ skinny_gemm_pairk_kernel(const __grid_constant__ WideKParams p, const __grid_con
   };
   fetch(pair * WK_ROWS + r);
   __syncthreads();
+  cluster_all_started();  // here, where X is on its way, and not in front of the store to the peer, where everybody waits for it
   bool ok = true;
 
   const int a_row = lane & 15, a_par = lane >> 4;

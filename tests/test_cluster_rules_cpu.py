@@ -1,6 +1,8 @@
 """Rules between the CTAs of a cluster that no run can show without a race, read from the sources."""
 import re
 
+import pytest
+
 from test_launch_rules_cpu import CSRC, body
 
 
@@ -18,3 +20,20 @@ def test_rotated_q_is_released_at_cluster_scope():
         assert re.search(r"tc_fence_before_sync\(\);\s*__syncwarp\(\);\s*if \(lane == 0\) $", text[:at])
     helper = (CSRC / "common.cuh").read_text()
     assert "mbarrier.arrive.release.cluster.shared::cluster.b64" in helper[helper.index("void mbar_arrive_cluster("):][:160]
+
+
+@pytest.mark.parametrize("name,function", [("decode_fused", "fused_decode_kernel"), ("skinny_gemm", "skinny_gemm_pairk_kernel"),
+                                           ("prefill_umma", "prefill_pair_kernel")])
+def test_no_remote_access_before_the_peer_runs(name, function):
+    """A cluster barrier lies between a kernel's start and its first access to a peer's shared memory."""
+    text = body(name, function)
+    remote = r"st_cluster_f32x4\(|st\.shared::cluster|mbar_arrive_cluster(?:_plain)?\(|(?:umma_\w+|tma_load_\dd)_pair\("
+    first = re.search(remote, text).start()
+    before = text[:first]
+    assert "cluster_sync();" in before or 0 < before.find("cluster_started();") < before.find("cluster_all_started();")
+
+
+def test_every_cluster_kernel_is_looked_at():
+    """Kernels that reach into a peer's shared memory are those of the test above."""
+    users = {f.stem for f in CSRC.glob("*.cu") if re.search(r"cluster_map\(|st_cluster", re.sub(r"//[^\n]*", "", f.read_text()))}
+    assert users == {"decode_fused", "skinny_gemm", "prefill_umma"}
