@@ -432,6 +432,7 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
       __syncwarp();
       cluster_started();  // (the form and the segment are the same for all CTAs of the cluster)
     } else {
+      cp_async_wait_all();
       pdl_wait();  // a cluster without a segment: all its CTAs leave together, nobody waits for them
       return;
     }
@@ -453,6 +454,7 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
     r1 = min(r0 + chunk, total);
   }
   if (r0 >= r1 && !cluster_mode) {
+    cp_async_wait_all();  // no copy outlives the shared memory it writes
     pdl_wait();  // an idle CTA still orders the grid after its predecessor
     return;
   }
@@ -462,6 +464,7 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
   if (!cluster_mode) {
     if (r0 >= seg0.end) segment_advance(seg0, cum, batch, heads, gap);  // the range starts inside a gap
     if (seg0.start >= r1) {                                             // ... and ends in it
+      cp_async_wait_all();
       pdl_wait();
       return;
     }

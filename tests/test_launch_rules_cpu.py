@@ -63,3 +63,12 @@ def test_team_lanes_stay():
     assert text.index("warp_wait_bounded(&full[stage], full_parity, ok)") < text.index("team_wait(")
     assert len(re.findall(r"ok = ok && team_wait\(", text)) == text.count("team_wait(")
     assert text.count("return;") == 2                   # the copy warps, and the end of the items
+
+
+def test_idle_decode_ctas_leave_no_copy_behind():
+    """A CTA without work has asked for the tables of norm weights and frequencies: it waits for these copies into its shared memory
+    before it leaves."""
+    text = body("decode_fused", "fused_decode_kernel")
+    asked = text.index("cp_async16(")
+    text = text[asked: text.index("auto issue_next")]
+    assert text.count("return;") == len(re.findall(r"cp_async_wait_all\(\);\s*pdl_wait\(\);\s*return;", text)) == 3
