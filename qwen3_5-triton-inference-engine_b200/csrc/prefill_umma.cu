@@ -43,6 +43,7 @@ constexpr int PU_KV_BYTES = PU_TKV * HEAD_DIM;      // 32 KiB: half a tile, K 64
 constexpr int PU_STAGE = 3, PU_STAGE_BYTES = 32 * 64;  // buffers of an output warp: 32 columns of its 32 rows, first the gates, then the output
 constexpr int PU_SMEM = PU_Q_BYTES + 4 * PU_KV_BYTES + PU_OUT_WARPS * PU_STAGE * PU_STAGE_BYTES;
 constexpr int PU_ITEMS = 4;                         // work items in flight per pair
+constexpr int PU_GROUP = 64;                        // most sequences whose items are dealt together
 constexpr int PU_REGS_SOFTMAX = 160, PU_REGS_OUT = 120, PU_REGS_ISSUE = 64;
 constexpr int PU_REGS = 65536 / PU_THREADS;         // what __launch_bounds__ leaves a thread, and ptxas gives (the host checks)
 static_assert(2 * PU_REGS_SOFTMAX + PU_REGS_OUT + PU_REGS_ISSUE <= PU_THREADS / 128 * PU_REGS, "shares of the registers the CTA is launched with");
@@ -51,7 +52,7 @@ constexpr float PU_TAU = 8.0f;                      // lazy-rescale threshold (l
 constexpr float PU_LOG2E = 1.4426950408889634f;
 
 struct PrefillUmmaParams {
-  int num_kv_heads, batch, max_seqlen;
+  int num_kv_heads, batch, max_seqlen, group;  // group: sequences whose items are dealt together
   __nv_bfloat16* out;
   int64_t out_t, out_h;
   const int32_t* cu_seqlens;
@@ -146,7 +147,8 @@ struct PrefillItem {
   int start, len, q0, h, tiles;  // first packed row and length of the sequence, the pair's first query, kv head, kv tiles (0: no more)
 };
 
-template <bool FUSED>
+// SLOTS: sequences of a group per lane of the warp that deals them
+template <bool FUSED, int SLOTS>
 __global__ void __launch_bounds__(PU_THREADS, 1)
 prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_gate,
@@ -193,6 +195,79 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     mbar_fence_init();
   }
+  // ---- the items (warp 14).  They are dealt to the pairs forth and back, group by group of sequences, in a group longest first: all blocks in
+  // the highest of its levels of 64 queries, then those in the next, and so on.  A group's lengths are read once, and a level is found by
+  // halving: `above(l)` counts the (sequence, level) blocks from level l on.  Walked level by level, 32 lengths read at a time and from the
+  // longest level that the caller names on, the list took 1024 prompts of 16 tokens 371 us where that was 4096, now 105.  The code is kept
+  // short, and the first item found while the pair meets: with four sequences per lane, or loops over shared memory, 8 prompts of 1024 tokens
+  // took 64.4 us (62.5 with one).
+  const int pairs = gridDim.x >> 1, me = blockIdx.x >> 1, heads = p.num_kv_heads;
+  int first = 0, from[SLOTS], to[SLOTS], levels[SLOTS];  // the group's first sequence; bounds and levels of a lane's sequences
+  int blocks = 0, top = 0, over_top = 0;  // blocks of the group; items to come have none of the over_top from level `top` on
+  uint32_t base = 0;  // items of the groups in front (q, k, v and the output of 2^32 of them do not fit the device)
+  auto above = [&](int level) {
+    int n = 0;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) n += max(levels[s] - level, 0);
+    return __reduce_add_sync(0xffffffffu, n);
+  };
+  auto open_group = [&]() {
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int nth = s * 32 + lane, b = first + nth;
+      from[s] = to[s] = 0;
+      if (nth < p.group && b < p.batch) from[s] = p.cu_seqlens[b], to[s] = p.cu_seqlens[b + 1];
+    }
+    top = 0;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      levels[s] = (min(max(to[s] - from[s], 0), p.max_seqlen) + PU_PAIR_Q - 1) / PU_PAIR_Q;
+      top = max(top, levels[s]);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    blocks = above(0);
+    over_top = 0;
+  };
+  auto find = [&](int i, PrefillItem& it) {
+    const uint32_t target = static_cast<uint32_t>(i) * pairs + ((i & 1) ? pairs - 1 - me : me);
+    it.tiles = 0;
+    while (first < p.batch) {
+      const int block = static_cast<int>((target - base) / heads);
+      if (block < blocks) {
+        int level = 0;                               // above(level) > block >= over_top = above(top)
+        while (top - level > 1) {
+          const int mid = (level + top) >> 1, n = above(mid);
+          if (n > block) level = mid;
+          else top = mid, over_top = n;
+        }
+        int nth = block - over_top;
+        it.q0 = level * PU_PAIR_Q;
+        it.h = static_cast<int>(target - base) - block * heads;
+#pragma unroll
+        for (int s = 0; s < SLOTS; ++s) {
+          const uint32_t has = __ballot_sync(0xffffffffu, levels[s] > level);
+          const int here = __popc(has);
+          if (nth >= 0 && nth < here) {
+            const bool mine = ((has >> lane) & 1) != 0 && __popc(has & ((1u << lane) - 1)) == nth;
+            const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+            it.start = __shfl_sync(0xffffffffu, from[s], src);
+            it.len = __shfl_sync(0xffffffffu, to[s], src) - it.start;
+          }
+          nth -= here;
+        }
+        it.tiles = (min(it.q0 + PU_PAIR_Q, it.len) + PU_TKV - 1) / PU_TKV;
+        break;
+      }
+      base += static_cast<uint32_t>(blocks) * heads;
+      first += p.group;
+      if (first < p.batch) open_group();
+    }
+  };
+  PrefillItem it0;
+  if (warp == 14) {  // while the pair meets
+    open_group();
+    find(0, it0);
+  }
   if (warp == 12) tmem_alloc_pair(&tmem_slot, PU_TMEM_COLS);
   if (warp == 13 && lane == 0) {
     prefetch_tensormap(&map_q);
@@ -224,49 +299,21 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     PrefillItem it;
     if (warp == 14) {
       // ---------------------------------------------------------------- the items; TMA producer: Q, and this CTA's 128 columns of every V tile
-      // Items come longest first and are dealt to the pairs forth and back.  One is made while the one in front of it is loaded.
-      const int pairs = gridDim.x >> 1, me = blockIdx.x >> 1, heads = p.num_kv_heads;
-      const bool one_read = p.batch <= 32;
-      int len = 0;
-      if (one_read && lane < p.batch) len = p.cu_seqlens[lane + 1] - p.cu_seqlens[lane];
-      int level = (p.max_seqlen - 1) / PU_PAIR_Q, chunk = 0;
-      int64_t base = 0;
-      auto make = [&](int i, PrefillItem& to) {
-        const int64_t target = static_cast<int64_t>(i) * pairs + ((i & 1) ? pairs - 1 - me : me);
-        to.tiles = 0;
-        while (level >= 0) {
-          if (!one_read) len = chunk + lane < p.batch ? p.cu_seqlens[chunk + lane + 1] - p.cu_seqlens[chunk + lane] : 0;
-          const uint32_t has = __ballot_sync(0xffffffffu, len > level * PU_PAIR_Q);
-          const int here = __popc(has) * heads;
-          if (target < base + here) {
-            const int at = static_cast<int>(target - base), nth = at / heads;
-            const bool mine = ((has >> lane) & 1) != 0 && __popc(has & ((1u << lane) - 1)) == nth;
-            const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
-            to.len = __shfl_sync(0xffffffffu, len, src);
-            to.start = p.cu_seqlens[chunk + src];
-            to.q0 = level * PU_PAIR_Q;
-            to.h = at - nth * heads;
-            to.tiles = (min(to.q0 + PU_PAIR_Q, to.len) + PU_TKV - 1) / PU_TKV;
-            break;
-          }
-          base += here;
-          chunk += 32;
-          if (chunk >= p.batch) {
-            chunk = 0;
-            --level;
-          }
-        }
+      // One item is made while the one in front of it is loaded.
+      auto make = [&](int i, PrefillItem& it) {
+        if (i > 0) find(i, it);
         if (i >= PU_ITEMS) ok = warp_wait_bounded(&item_free[i & (PU_ITEMS - 1)], (i / PU_ITEMS - 1) & 1, ok);
         if (ok && lane == 0) {
-          items[i & (PU_ITEMS - 1)] = to;
+          items[i & (PU_ITEMS - 1)] = it;
           mbar_arrive(&item_full[i & (PU_ITEMS - 1)]);
         }
-        return ok && to.tiles > 0;
+        return ok && it.tiles > 0;
       };
       const uint32_t full[2] = {cluster_map(smem_u32(&lead_v[0]), 0), cluster_map(smem_u32(&lead_v[1]), 0)};
       const uint32_t full_q = cluster_map(smem_u32(&lead_q), 0);
       const int q_off = static_cast<int>(rank) * PU_BQ;
       PrefillItem next;
+      it = it0;
       bool more = ok && make(0, it);
       for (int i = 0, g = 0; more; ++i, it = next) {
         // the last S of the item in front read Q; the V tile of that S was asked for behind PV of two tiles before it, so this
@@ -290,7 +337,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (rank == 0) mbar_expect_tx(&lead_v[s], 2 * PU_KV_BYTES);
             tma_load_4d_pair(v_s + s * PU_KV_BYTES, &map_v, 0, it.start + j * PU_TKV, 2 * static_cast<int>(rank), it.h, full[s]);
           }
-          if (j == 0) {
+          if (j == (i == 0 && it.tiles > 1)) {  // (the first two V tiles wait for nobody)
             more = make(i + 1, next);
             if (more && lane == 0) tma_prefetch_5d(&map_q, 0, 0, next.h, next.start + next.q0 + q_off, 0);
           }
@@ -708,13 +755,15 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
+  const auto one = prefill_pair_kernel<FUSED, 1>, two = prefill_pair_kernel<FUSED, 2>;
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(prefill_pair_kernel<FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PU_SMEM) !=
-        cudaSuccess)
-      return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, PU_SMEM);
-    cudaFuncAttributes attr;  // its warpgroups exchange registers: with fewer at the launch than they share out they would wait for good
-    if (cudaFuncGetAttributes(&attr, prefill_pair_kernel<FUSED>) != cudaSuccess || attr.numRegs != PU_REGS)
-      return fail(ERR_RUNTIME, "%s: the kernel was not built with %d registers per thread", what, PU_REGS);
+    for (const auto k : {one, two}) {
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, PU_SMEM) != cudaSuccess)
+        return fail(ERR_RUNTIME, "%s: cannot raise dynamic shared memory to %d", what, PU_SMEM);
+      cudaFuncAttributes attr;  // its warpgroups exchange registers: with fewer at the launch than they share out they would wait for good
+      if (cudaFuncGetAttributes(&attr, k) != cudaSuccess || attr.numRegs != PU_REGS)
+        return fail(ERR_RUNTIME, "%s: the kernel was not built with %d registers per thread", what, PU_REGS);
+    }
     configured[dev] = true;
   }
   p.err = wait_timeout_flag();
@@ -726,10 +775,11 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
   p.num_kv_heads = num_kv_heads;
   p.batch = batch;
   p.max_seqlen = max_seqlen;
+  p.group = batch < PU_GROUP ? batch : PU_GROUP;
   const int64_t most = static_cast<int64_t>((max_seqlen + PU_PAIR_Q - 1) / PU_PAIR_Q) * num_kv_heads * batch;
   const int sms = sm_count(), pairs = static_cast<int>(most < sms / 2 ? most : sms / 2);
   // the fused form starts behind its own rope + scatter kernel while that one still runs (see the K producer)
-  if (launch_pdl_cluster(FUSED, 2, prefill_pair_kernel<FUSED>, dim3(2 * pairs), dim3(PU_THREADS), PU_SMEM, stream, map_q, map_k, map_v, map_gate,
+  if (launch_pdl_cluster(FUSED, 2, p.group <= 32 ? one : two, dim3(2 * pairs), dim3(PU_THREADS), PU_SMEM, stream, map_q, map_k, map_v, map_gate,
                          map_out, p) !=
       cudaSuccess)
     return fail(ERR_LAUNCH, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));

@@ -84,3 +84,13 @@ def test_rows_behind_a_sequence_stay():
         exact = O.varlen_causal_exact(q[: ends[-1]].cpu(), k[: ends[-1]].cpu(), v[: ends[-1]].cpu(), cu.cpu())
         _check(out[: ends[-1]], exact, v)
         assert bool((out[ends[-1]:] == 7.0).all())
+
+
+@pytest.mark.parametrize("lengths,longest", [([1 + n % 40 for n in range(190)] + [700] + [7] * 230, 5000), ([0] * 200 + [90] + [0] * 191 + [64, 65] + [0] * 33, 4096),
+                                             ([33] * 192 + [129], 129)])
+def test_items_of_many_sequences(lengths, longest):
+    """More sequences than the items are dealt out of at a time, most of them short or empty, and a longest length far above any."""
+    from b200attn import ops
+    q, k, v, cu, _ = _qkv(lengths, 41, 1)
+    out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), longest)
+    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
