@@ -717,6 +717,20 @@ using namespace b200;
 
 static bool mult8(int64_t x) { return (x & 7) == 0; }
 
+// Sequences whose items are dealt together.  All of them balance best.  But the pairs go level by level, and between two levels of a sequence
+// the K and V of all, and a level's rows of q, output and (row_tensors = 3) gate, pass through the L2 of 126 MB: beyond 80 MiB groups of 48.
+// Not with six pairs or more to a (sequence, head): those read the same tiles at about the same time.  us, all together and in groups: 64 x
+// 2048 tokens 1476 and 1260, 64 x 4096 4662 and 4229, 128 x 512 370 and 336, 12 x 4096 880 and 863; on the wrong side of the lines 8 x 4096
+// (70 MiB) 502 and 522, 6 x 8192 1322 and 1345.
+static int prefill_group(int batch, int total_tokens, int num_kv_heads, int row_tensors, int pairs) {
+  const int64_t rows = total_tokens < static_cast<int64_t>(batch) * PU_PAIR_Q ? total_tokens : static_cast<int64_t>(batch) * PU_PAIR_Q;
+  const int64_t pass = (2 * static_cast<int64_t>(total_tokens) + row_tensors * GROUP * rows) * num_kv_heads * HEAD_DIM * 2;
+  int64_t groups = 1;
+  if (pass > (80ll << 20) && static_cast<int64_t>(batch) * num_kv_heads * 6 > pairs) groups = (pass + (48ll << 20) - 1) / (48ll << 20);
+  const int64_t group = (batch + groups - 1) / groups;
+  return static_cast<int>(group < PU_GROUP ? group : PU_GROUP);
+}
+
 // Encodes the tensor maps and launches the attention kernel (FUSED adds rope on q and the output gate).
 template <bool FUSED>
 static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k, int64_t k_stride_t,
@@ -775,7 +789,7 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
   p.num_kv_heads = num_kv_heads;
   p.batch = batch;
   p.max_seqlen = max_seqlen;
-  p.group = batch < PU_GROUP ? batch : PU_GROUP;
+  p.group = prefill_group(batch, total_tokens, num_kv_heads, FUSED ? 3 : 2, sm_count() / 2);
   const int64_t most = static_cast<int64_t>((max_seqlen + PU_PAIR_Q - 1) / PU_PAIR_Q) * num_kv_heads * batch;
   const int sms = sm_count(), pairs = static_cast<int>(most < sms / 2 ? most : sms / 2);
   // the fused form starts behind its own rope + scatter kernel while that one still runs (see the K producer)

@@ -94,3 +94,20 @@ def test_items_of_many_sequences(lengths, longest):
     q, k, v, cu, _ = _qkv(lengths, 41, 1)
     out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), longest)
     _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+
+
+@pytest.mark.parametrize("lengths", [[1000 - 17 * n for n in range(50)], [257] * 130, [2048] * 20])
+def test_groups_beyond_the_l2(lengths):
+    """Batches whose items are dealt in groups of sequences against their halves: an item is computed alike in whatever order it comes."""
+    from b200attn import ops
+    g, half = torch.Generator(device=DEV).manual_seed(3), len(lengths) // 2
+    x = torch.randn((sum(lengths), 12, 256), generator=g, device=DEV, dtype=torch.bfloat16)
+
+    def attend(lengths, x):
+        cu = torch.tensor([0, *torch.tensor(lengths).cumsum(0).tolist()], dtype=torch.int32, device=DEV)
+        return ops.gqa_attention_varlen_causal(x[:, :8], x[:, 8:10], x[:, 10:], cu, max(lengths))
+
+    cut = sum(lengths[:half])
+    out = attend(lengths, x)
+    assert torch.equal(out[:cut], attend(lengths[:half], x[:cut])) and torch.equal(out[cut:], attend(lengths[half:], x[cut:]))
+    assert bool(out.isfinite().all())
