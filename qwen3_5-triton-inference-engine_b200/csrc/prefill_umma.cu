@@ -3,6 +3,7 @@
 //   b200_fused_prefill_attention <-> the chain of engine/runner.py:339-384: partial_rope(q), partial_rope(k),
 //                                    gqa_attention_varlen_causal, attention_gate_pack, paged_kv_fill_varlen
 //
+// Calls that are over in one wave of CTAs run on a kernel without pairs (prefill_short.cu); here is the other one.
 // Two CTAs of a cluster work on one item after another: (sequence, kv head, block of 64 query tokens), 32 tokens each.  The 4 Q heads
 // of the group are stacked into the 128 rows of a CTA's half of an M=256 tile (row = token*4 + head, the stacking idea of
 // gqa_attention_varlen_causal.py:151-160).  Per 128-token KV tile, cta_group::2, operands split over the pair:
@@ -27,14 +28,11 @@
 // The reference's rounding points are kept where they matter for the 2e-2 bar: p is rounded to bf16 for the PV
 // product while l sums the fp32 p; scores are scaled in fp32 (the reference pre-scales q and re-rounds it to bf16).
 // Every mbarrier wait is bounded; on expiry the role sets the device error flag and the CTA drains and exits.
-#include "b200_attn.h"
-#include "umma.cuh"
+#include "prefill.cuh"
 
 namespace b200 {
 
-constexpr int PU_BQ = 32;                           // query tokens per CTA
 constexpr int PU_PAIR_Q = 2 * PU_BQ;
-constexpr int PU_TKV = 128;
 constexpr int PU_SOFTMAX_WARPS = 8;
 constexpr int PU_OUT_WARPS = 4;
 constexpr int PU_THREADS = 512;
@@ -47,24 +45,7 @@ constexpr int PU_GROUP = 64;                        // most sequences whose item
 constexpr int PU_REGS_SOFTMAX = 160, PU_REGS_OUT = 120, PU_REGS_ISSUE = 64;
 constexpr int PU_REGS = 65536 / PU_THREADS;         // what __launch_bounds__ leaves a thread, and ptxas gives (the host checks)
 static_assert(2 * PU_REGS_SOFTMAX + PU_REGS_OUT + PU_REGS_ISSUE <= PU_THREADS / 128 * PU_REGS, "shares of the registers the CTA is launched with");
-constexpr uint32_t PU_TMEM_COLS = 512;              // S0 [0,128) S1 [128,256) (P over their first 64) O [256,512)
-constexpr float PU_TAU = 8.0f;                      // lazy-rescale threshold (log2 domain)
 constexpr float PU_LOG2E = 1.4426950408889634f;
-
-struct PrefillUmmaParams {
-  int num_kv_heads, batch, max_seqlen, group;  // group: sequences whose items are dealt together
-  __nv_bfloat16* out;
-  int64_t out_t, out_h;
-  const int32_t* cu_seqlens;
-  int* err;
-  float scale_log2;
-  // fused form only: rotary embedding of q in shared memory, sigmoid gate in the epilogue
-  const __nv_bfloat16* gate;
-  int64_t gate_t;
-  const void* position_ids;
-  int ids_are_int64;
-  const float* inv_freq;
-};
 
 // Fused path, first kernel: rotate K at its position, scatter K (rotated) and V into the paged cache and keep a
 // packed copy of the rotated K [T, H_kv, 256] for the attention kernel's TMA loads (so the rotation is computed once
@@ -733,33 +714,26 @@ static int prefill_group(int batch, int total_tokens, int num_kv_heads, int row_
 
 // Encodes the tensor maps and launches the attention kernel (FUSED adds rope on q and the output gate).
 template <bool FUSED>
-static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k, int64_t k_stride_t,
-                               int64_t k_stride_h, const void* v, int64_t v_stride_t, int64_t v_stride_h,
-                               PrefillUmmaParams p, int batch, int total_tokens, int max_seqlen, int num_kv_heads,
-                               cudaStream_t stream, const char* what) {
+static int launch_prefill_umma(const PrefillTensors& t, PrefillUmmaParams p, int batch, int max_seqlen, cudaStream_t stream, const char* what) {
+  const int num_kv_heads = t.num_kv_heads, sms = sm_count();
+  B200_REQUIRE((max_seqlen + PU_BQ - 1) / PU_BQ <= 65535 && batch <= 65535 && num_kv_heads <= 65535,
+               "%s: max_seqlen must be at most %d, batch and heads at most 65535 (got %d, %d, %d)", what, 65535 * PU_BQ,
+               max_seqlen, batch, num_kv_heads);
+  p.err = wait_timeout_flag();
+  if (!p.err) return fail(ERR_RUNTIME, "%s: no error flag", what);
+  p.scale_log2 = (1.0f / sqrtf(static_cast<float>(HEAD_DIM))) * PU_LOG2E;
+  p.num_kv_heads = num_kv_heads;
+  p.batch = batch;
+  p.max_seqlen = max_seqlen;
+  if (prefill_takes_short(FUSED, batch, t.tokens, max_seqlen, num_kv_heads)) return launch_prefill_short(FUSED, t, p, stream, what);
   CUtensorMap map_q, map_k, map_v, map_gate = {}, map_out;
-  const uint64_t T = static_cast<uint64_t>(total_tokens), H = static_cast<uint64_t>(num_kv_heads);
-  {
-    // q as {64 cols, 4 heads of a group, groups, tokens, 4 column blocks}; one load = 32 tokens of one group
-    const uint64_t dims[5] = {64, GROUP, H, T, HEAD_DIM / 64};
-    const uint64_t strides[4] = {static_cast<uint64_t>(q_stride_h) * 2, static_cast<uint64_t>(q_stride_h) * 2 * GROUP,
-                                 static_cast<uint64_t>(q_stride_t) * 2, 128};
-    const uint32_t box[5] = {64, GROUP, 1, PU_BQ, HEAD_DIM / 64};
-    if (!encode_map_bf16_sw128(&map_q, q, 5, dims, strides, box))
-      return fail(ERR_RUNTIME, "%s: cannot encode the tensor map of q", what);
-  }
-  {
-    // k, v as {64 cols, tokens, 4 column blocks, kv heads}; one load = 64 tokens, or 128 columns of 128 tokens, of one head
-    const uint64_t dims[4] = {64, T, HEAD_DIM / 64, H};
-    const uint32_t kbox[4] = {64, PU_TKV / 2, HEAD_DIM / 64, 1}, vbox[4] = {64, PU_TKV, HEAD_DIM / 128, 1};
-    const uint64_t ks[3] = {static_cast<uint64_t>(k_stride_t) * 2, 128, static_cast<uint64_t>(k_stride_h) * 2};
-    const uint64_t vs[3] = {static_cast<uint64_t>(v_stride_t) * 2, 128, static_cast<uint64_t>(v_stride_h) * 2};
-    if (!encode_map_bf16_sw128(&map_k, k, 4, dims, ks, kbox) || !encode_map_bf16_sw128(&map_v, v, 4, dims, vs, vbox))
-      return fail(ERR_RUNTIME, "%s: cannot encode the tensor maps of k / v", what);
-  }
+  // of K a CTA loads 64 tokens of a head, of V 128 columns of 128 tokens
+  if (!encode_prefill_q(&map_q, t) || !encode_prefill_kv(&map_k, t, t.k, t.k_t, t.k_h, PU_TKV / 2, HEAD_DIM / 64) ||
+      !encode_prefill_kv(&map_v, t, t.v, t.v_t, t.v_h, PU_TKV, HEAD_DIM / 128))
+    return fail(ERR_RUNTIME, "%s: cannot encode the tensor maps of q / k / v", what);
   {
     // gates and output as {32 cols, 4 heads of a group, groups, tokens, 8 column blocks}; one copy = 8 tokens of one group
-    const uint64_t dims[5] = {32, GROUP, H, T, HEAD_DIM / 32};
+    const uint64_t dims[5] = {32, GROUP, static_cast<uint64_t>(num_kv_heads), static_cast<uint64_t>(t.tokens), HEAD_DIM / 32};
     const uint64_t gs[4] = {HEAD_DIM * 2, HEAD_DIM * 2 * GROUP, static_cast<uint64_t>(p.gate_t) * 2, 64};
     const uint64_t os[4] = {static_cast<uint64_t>(p.out_h) * 2, static_cast<uint64_t>(p.out_h) * 2 * GROUP, static_cast<uint64_t>(p.out_t) * 2, 64};
     const uint32_t box[5] = {32, GROUP, 1, 8, 1};
@@ -780,18 +754,9 @@ static int launch_prefill_umma(const void* q, int64_t q_stride_t, int64_t q_stri
     }
     configured[dev] = true;
   }
-  p.err = wait_timeout_flag();
-  if (!p.err) return fail(ERR_RUNTIME, "%s: no error flag", what);
-  p.scale_log2 = (1.0f / sqrtf(static_cast<float>(HEAD_DIM))) * PU_LOG2E;
-  B200_REQUIRE((max_seqlen + PU_BQ - 1) / PU_BQ <= 65535 && batch <= 65535 && num_kv_heads <= 65535,
-               "%s: max_seqlen must be at most %d, batch and heads at most 65535 (got %d, %d, %d)", what, 65535 * PU_BQ,
-               max_seqlen, batch, num_kv_heads);
-  p.num_kv_heads = num_kv_heads;
-  p.batch = batch;
-  p.max_seqlen = max_seqlen;
-  p.group = prefill_group(batch, total_tokens, num_kv_heads, FUSED ? 3 : 2, sm_count() / 2);
+  p.group = prefill_group(batch, t.tokens, num_kv_heads, FUSED ? 3 : 2, sms / 2);
   const int64_t most = static_cast<int64_t>((max_seqlen + PU_PAIR_Q - 1) / PU_PAIR_Q) * num_kv_heads * batch;
-  const int sms = sm_count(), pairs = static_cast<int>(most < sms / 2 ? most : sms / 2);
+  const int pairs = static_cast<int>(most < sms / 2 ? most : sms / 2);
   // the fused form starts behind its own rope + scatter kernel while that one still runs (see the K producer)
   if (launch_pdl_cluster(FUSED, 2, p.group <= 32 ? one : two, dim3(2 * pairs), dim3(PU_THREADS), PU_SMEM, stream, map_q, map_k, map_v, map_gate,
                          map_out, p) !=
@@ -821,9 +786,8 @@ extern "C" int b200_gqa_varlen_causal(const void* q, int64_t q_stride_t, int64_t
   p.out_t = out_stride_t;
   p.out_h = out_stride_h;
   p.cu_seqlens = cu_seqlens;
-  return launch_prefill_umma<false>(q, q_stride_t, q_stride_h, k, k_stride_t, k_stride_h, v, v_stride_t, v_stride_h, p,
-                                    batch, total_tokens, max_seqlen, num_kv_heads,
-                                    reinterpret_cast<cudaStream_t>(stream), "gqa_varlen_causal");
+  const PrefillTensors t = {q, k, v, q_stride_t, q_stride_h, k_stride_t, k_stride_h, v_stride_t, v_stride_h, total_tokens, num_kv_heads};
+  return launch_prefill_umma<false>(t, p, batch, max_seqlen, reinterpret_cast<cudaStream_t>(stream), "gqa_varlen_causal");
 }
 
 extern "C" int b200_fused_prefill_attention(const void* q, int64_t q_stride_t, int64_t q_stride_h, const void* k,
@@ -871,7 +835,7 @@ extern "C" int b200_fused_prefill_attention(const void* q, int64_t q_stride_t, i
   p.position_ids = position_ids;
   p.ids_are_int64 = ids_are_int64;
   p.inv_freq = inv_freq;
-  return launch_prefill_umma<true>(q, q_stride_t, q_stride_h, k_rot_scratch, static_cast<int64_t>(num_kv_heads) * HEAD_DIM,
-                                   HEAD_DIM, v, v_stride_t, v_stride_h, p, batch, total_tokens, max_seqlen,
-                                   num_kv_heads, st, "fused_prefill_attention");
+  const PrefillTensors t = {q, k_rot_scratch, v, q_stride_t, q_stride_h, static_cast<int64_t>(num_kv_heads) * HEAD_DIM, HEAD_DIM,
+                            v_stride_t, v_stride_h, total_tokens, num_kv_heads};
+  return launch_prefill_umma<true>(t, p, batch, max_seqlen, st, "fused_prefill_attention");
 }

@@ -37,3 +37,14 @@ def test_every_cluster_kernel_is_looked_at():
     """Kernels that reach into a peer's shared memory are those of the test above."""
     users = {f.stem for f in CSRC.glob("*.cu") if re.search(r"cluster_map\(|st_cluster", re.sub(r"//[^\n]*", "", f.read_text()))}
     assert users == {"decode_fused", "skinny_gemm", "prefill_umma"}
+
+
+def test_one_cta_prefill_waits_name_one_phase():
+    """A wait by parity tells two phases apart.  Behind its last P a thread cannot say whether one PV product is still to come or two: the last
+    one has a barrier of its own, and no other wait in the softmax warps follows an arrival that lets a second phase pass."""
+    text = body("prefill_short", "prefill_short_kernel")
+    assert "umma_commit_leader(jj + 1 < n_tiles ? &bar_pv : &bar_o, leader)" in text
+    epilogue = text[text.rindex("mbar_arrive(&bar_p[s])"):]
+    assert "bar_pv" not in epilogue and "warp_wait_bounded(&bar_o, 0, ok)" in epilogue
+    rescale = text[text.index("if (__any_sync("): text.index("mbar_arrive(&bar_p[s])")]
+    assert "warp_wait_bounded(&bar_pv, (j - 1) & 1)" in rescale      # in front of the own P(j), without which PV(j) cannot pass

@@ -111,3 +111,25 @@ def test_groups_beyond_the_l2(lengths):
     out = attend(lengths, x)
     assert torch.equal(out[:cut], attend(lengths[:half], x[:cut])) and torch.equal(out[cut:], attend(lengths[half:], x[cut:]))
     assert bool(out.isfinite().all())
+
+
+# Beside four long sequences, which make a call more than one wave of CTAs, the lengths above meet the pairs' tiles; by themselves they are
+# the one-CTA kernel's.
+@pytest.mark.parametrize("lengths", [[1], [8, 7, 9], [31, 32, 33, 40], [63, 64, 65, 72], [96, 97, 127, 128, 129], [191, 192, 193, 256, 257]])
+@pytest.mark.parametrize("kv_heads", [2, 1])
+def test_edges_on_pairs(lengths, kv_heads):
+    from b200attn import ops
+    lengths = [1100, 1300] + lengths + [1200, 1170]
+    q, k, v, cu, _ = _qkv(lengths, 51 + len(lengths), kv_heads)
+    out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), max(lengths))
+    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+
+
+@pytest.mark.parametrize("lengths", [[1], [32] * 74, [32] * 75, [31, 33], [128] * 16, [129] * 14, [2048], [2960], [2961], [4096], [4145], [1000, 1, 300], [512, 3, 64, 200, 77, 1, 1, 400]])
+@pytest.mark.parametrize("longest", [0, 333])
+def test_short_calls(lengths, longest):
+    """Calls on both sides of the line to the one-CTA kernel: one CTA and one wave of them, one tile and many, longest lengths that say too much."""
+    from b200attn import ops
+    q, k, v, cu, _ = _qkv(lengths, 61 + len(lengths))
+    out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), max(lengths) + longest)
+    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
