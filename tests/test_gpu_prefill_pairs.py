@@ -2,8 +2,10 @@
 and 128 (key tile) tokens, more sequences than one read of their lengths covers, more items than a pair's ring holds, row maxima
 that grow from tile to tile, and rows behind a sequence that must not be touched.
 
-Bound: p is rounded to bf16 (2^-9 of each weight) and the output is (2^-9 of a value no larger than the largest |v|), so an output is
-off by at most 2^-8 max|v|; sums and scores in fp32 add some 1e-5.  The gated form rounds once, the chain twice more.
+Bounds: bf16 keeps eight bits, so that a rounding moves a value by at most 2^-8 of itself.  An output element is off by at most 2^-8 sum p |v|
+(rounding of the weights p) + 2^-8 |out| (its own) and what fp32 sums make of the scores: 2^-12 sum p |v| for products of unit size, where the
+256 terms of a score sum up to some 10 in magnitude.  All elements together stay within 2^-8 max|v|, the gated form, which rounds once, and the
+chain, which rounds twice more, within 2^-7 max|v| of one another.
 """
 import pytest
 import torch
@@ -21,11 +23,20 @@ def _qkv(lengths, seed, kv_heads=2):
     return [bf16_randn(total, n, 256, gen=gen) for n in (4 * kv_heads, kv_heads, kv_heads)] + [cu, gen]
 
 
-def _check(out, exact, v):
+def _bounds(q, k, v, cu, scores=2 ** -12):
+    """The exact output, and what rounding may move each element by."""
+    exact, spread = O.varlen_causal_exact(q, k, v, cu).float(), O.varlen_causal_exact(q, k, v.abs(), cu).float()
+    return exact, 1.01 * ((2 ** -8 + scores) * spread + 2 ** -8 * exact.abs()) + 1e-6
+
+
+def _check(out, q, k, v, cu, scores=2 ** -12):
     import b200attn
     torch.cuda.synchronize()
     assert b200attn.load().b200_wait_timed_out() == 0
-    assert (out.float().cpu() - exact.float()).abs().max().item() <= 2 ** -8 * v.float().abs().max().item() + 1e-3
+    exact, bound = _bounds(q, k, v, cu, scores)
+    off = (out.float().cpu() - exact).abs()
+    assert (off <= bound).all()
+    assert off.max().item() <= 2 ** -8 * v.float().abs().max().item() + 1e-3
 
 
 RAGGED = [int(x) for x in torch.randint(1, 200, (130,), generator=torch.Generator().manual_seed(9))]
@@ -38,7 +49,7 @@ def test_pairs_vs_oracle(lengths, kv_heads):
     from b200attn import ops
     q, k, v, cu, _ = _qkv(lengths, 11 + len(lengths), kv_heads)
     out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), max(lengths))
-    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+    _check(out, q, k, v, cu)
 
 
 def test_row_maxima_that_grow():
@@ -49,7 +60,7 @@ def test_row_maxima_that_grow():
     q = q.abs()
     k = (k.abs() * (1 + 2 * (torch.arange(1000) // 128)).view(-1, 1, 1)).to(torch.bfloat16)
     out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), 700)
-    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+    _check(out, q, k, v, cu, scores=2 ** -9)                                # terms up to eleven times as large
 
 
 @pytest.mark.parametrize("lengths", [[3], [64, 33, 8, 129], RAGGED[:70]])
@@ -81,8 +92,7 @@ def test_rows_behind_a_sequence_stay():
         out = torch.full_like(q, 7.0)
         _lib.call("b200_gqa_varlen_causal", q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
                   v.stride(1), out.data_ptr(), out.stride(0), out.stride(1), cu.data_ptr(), 2, 83, 70, 8, 2, 256, torch.cuda.current_stream().cuda_stream)
-        exact = O.varlen_causal_exact(q[: ends[-1]].cpu(), k[: ends[-1]].cpu(), v[: ends[-1]].cpu(), cu.cpu())
-        _check(out[: ends[-1]], exact, v)
+        _check(out[: ends[-1]], *(t[: ends[-1]].cpu() for t in (q, k, v)), cu.cpu())
         assert bool((out[ends[-1]:] == 7.0).all())
 
 
@@ -93,7 +103,7 @@ def test_items_of_many_sequences(lengths, longest):
     from b200attn import ops
     q, k, v, cu, _ = _qkv(lengths, 41, 1)
     out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), longest)
-    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+    _check(out, q, k, v, cu)
 
 
 @pytest.mark.parametrize("lengths", [[1000 - 17 * n for n in range(50)], [257] * 130, [2048] * 20])
@@ -122,7 +132,7 @@ def test_edges_on_pairs(lengths, kv_heads):
     lengths = [1100, 1300] + lengths + [1200, 1170]
     q, k, v, cu, _ = _qkv(lengths, 51 + len(lengths), kv_heads)
     out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), max(lengths))
-    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+    _check(out, q, k, v, cu)
 
 
 @pytest.mark.parametrize("lengths", [[1], [32] * 74, [32] * 75, [31, 33], [128] * 16, [129] * 14, [2048], [2960], [2961], [4096], [4145], [1000, 1, 300], [512, 3, 64, 200, 77, 1, 1, 400]])
@@ -132,4 +142,37 @@ def test_short_calls(lengths, longest):
     from b200attn import ops
     q, k, v, cu, _ = _qkv(lengths, 61 + len(lengths))
     out = ops.gqa_attention_varlen_causal(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), max(lengths) + longest)
-    _check(out, O.varlen_causal_exact(q, k, v, cu), v)
+    _check(out, q, k, v, cu)
+
+
+@pytest.mark.parametrize("lengths", [[700, 300], [1200, 1100, 900, 700, 650, 600]])
+def test_bounds_catch_a_lost_tile(lengths):
+    """On the CPU: an output without one of the 128-token key tiles, or with a tile counted twice, is outside the bounds in every long row."""
+    q, k, v, cu, _ = _qkv(lengths, 71)
+    exact, bound = _bounds(q, k, v, cu)
+    n, (q, k, v) = lengths[0], (t[: lengths[0]].float() for t in (q, k, v))
+    p = torch.exp((q[n - 1].view(2, 4, 256) @ k.permute(1, 2, 0)) / 16)     # weights of the last row, [kv head, head, token]
+    for tile in range(n // 128):
+        for factor in (0.0, 2.0):
+            w = p.clone()
+            w[:, :, tile * 128: tile * 128 + 128] *= factor
+            out = ((w / w.sum(-1, keepdim=True)) @ v.permute(1, 0, 2)).view(8, 256)
+            assert ((out - exact[n - 1]).abs() > bound[n - 1]).any(1).all()
+
+
+@pytest.mark.parametrize("lengths", [[40, 9], [300, 45], [1100] * 5])
+def test_gates_far_from_zero(lengths):
+    """Gates of -12 to 12 against the exact sigmoid.  o/2 tanh(g/2) + o/2 with the hardware's tanh, off by 2^-11 of itself, is off by 2^-12 |o| at
+    most, however small the sigmoid: an absolute error, of what the gate lets through where it is open."""
+    from b200attn import ops
+    q, k, v, cu, gen = _qkv(lengths, 81)
+    total, batch, pps = sum(lengths), len(lengths), cdiv(max(lengths), 16)
+    gate = ((torch.rand(total, 2048, generator=gen) * 24 - 12)).to(torch.bfloat16)
+    table = torch.randperm(batch * pps, generator=gen).view(batch, pps).to(torch.int32).to(DEV)
+    ids = torch.zeros(1, total, dtype=torch.int32, device=DEV)              # no rotation
+    caches = ops.allocate_paged_kv_cache(batch * pps, 2, 256, device=DEV)
+    out = ops.fused_prefill_attention(q.to(DEV), k.to(DEV), v.to(DEV), gate.to(DEV), *caches, table, cu.to(DEV), ids, rope_inv_freq().to(DEV), 64,
+                                      max(lengths)).float().cpu().view(total, 8, 256)
+    exact, bound = _bounds(q, k, v, cu)
+    factor = torch.sigmoid(gate.double()).float().view(total, 8, 256)
+    assert ((out - exact * factor).abs() <= bound * factor + 2 ** -12 * 1.01 * (exact.abs() + bound) + 1e-6).all()
