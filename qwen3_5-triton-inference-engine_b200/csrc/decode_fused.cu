@@ -272,8 +272,8 @@ __device__ __forceinline__ int small_div(int a, int b) { return static_cast<int>
 // positions -> shares -> page ids -> pages, warps' states -> cluster -> output.  One sequence of 1926 tokens, cycles of 19100: shares
 // known 3900 after entry, first page there at 8200, merge of eight warps' states 3000, exchange 2200, merge of sixteen CTAs' states and
 // output 3300.  With the lengths of up to 32 sequences in registers instead of shared memory behind two barriers, and with all weights of
-// a merge taken at once, one per lane, instead of state by state: shares 2400, merges 2100 and 1800.  Six such layers 61.6 -> 54.9 us, of 32
-// sequences of 512 to 4096 tokens 194.9 -> 190.6, of 256 the same (195).  Not kept: rolled merges (65.7 us: a chain per state), the appended token
+// a merge taken at once, one per lane, instead of state by state: shares 2400, merges 2100 and 1800.  Six such layers 64.5 -> 57.3 us, of 32
+// sequences of 512 to 4096 tokens 195.2 -> 191.6, of 256 the same (200).  Not kept: rolled merges (65.7 us: a chain per state), the appended token
 // in front of the pages in cluster mode (its CTA then is the last, 55.4).
 __global__ void __launch_bounds__(FD_THREADS, 1)
 fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_constant__ CUtensorMap map_k,
@@ -384,22 +384,23 @@ fused_decode_kernel(const __grid_constant__ FusedDecodeParams p, const __grid_co
   //    segment sets the time, and an SM alone streams at about 75 GB/s.
   //  - One segment per CLUSTER (launches with clusters only, when every segment gets a cluster of its own): the CTAs
   //    of a cluster take equal shares of the segment's units and merge through distributed shared memory.
-  // The choice compares time models fitted to measurements of this kernel on B200 (nanoseconds, u = units of 16 KiB;
-  // every form is also bound by the DRAM rate, 2.64 ns per unit):
-  //    stream-K  max(300 line positions per CTA, 2.64 u_total) + 8000 + 180 u_longest / (positions per CTA)
+  // The choice compares models of the time (nanoseconds, u = units of 16 KiB), fitted so that it falls on the fastest form over 1 to 74
+  // sequences of equal lengths from 64 to 32768 tokens and of mixed ones:
+  //    stream-K  max(360 line positions per CTA, 2.64 u_total) + 9500 + 180 u_longest / (positions per CTA)
   //              (the last term: partials the longest segment leaves for its final merge)
-  //    whole     max(165 u_longest, 2.64 u_total) + 8500
-  //    cluster   max(190 u_longest / cluster_size, 2.64 u_total) + 8500
-  // A form is taken over stream-K when its model wins by 5 %.
+  //    whole     max(190 u_longest, 2.64 u_total) + 8000
+  //    cluster   max(250 u_longest / cluster_size, 2.64 u_total) + 8800
+  // A form is taken over stream-K when its model wins by 5 %.  With constants from before the merges were shortened it missed the fastest
+  // form by up to 13 % (us a launch, chosen and fastest: 32 x 2000 tokens 29.9 and 26.4, 16 x 4096 30.3 and 27.1, 64 x 2000 51.2 and 46.6).
   const int total = heads * line;  // length of the line, gaps included
   const int grid = static_cast<int>(gridDim.x), nseg = batch * heads;
   const int chunk = max((total + grid - 1) / grid, FD_WARPS);
   const int csize = p.cluster_size;
   const int dram = (total - nseg * gap) * 66 / 25;  // 2.64 ns per unit
   const int clog = p.cluster_log2;
-  const int t_stream = max(300 * chunk, dram) + 8000 + static_cast<int>(__fdividef(180.f * static_cast<float>(longest), static_cast<float>(chunk)));
-  const int t_whole = max(165 * longest, dram) + 8500;
-  const int t_cluster = max(190 * ((longest + csize - 1) >> clog), dram) + 8500;
+  const int t_stream = max(360 * chunk, dram) + 9500 + static_cast<int>(__fdividef(180.f * static_cast<float>(longest), static_cast<float>(chunk)));
+  const int t_whole = max(190 * longest, dram) + 8000;
+  const int t_cluster = max(250 * ((longest + csize - 1) >> clog), dram) + 8800;
   const bool cluster_fits = csize > 1 && nseg * csize <= grid;
   const bool whole_fits = nseg <= grid;
   int form = 1;  // 1 stream-K, 2 whole segments, 3 cluster per segment
