@@ -63,14 +63,6 @@ __device__ __forceinline__ void rope_pair(float a, float b, float sn, float cs, 
   second = __fmaf_rn(a, sn, __fmul_rn(b, cs));
 }
 
-// sigmoid(x) = 0.5 * tanh(x / 2) + 0.5 with the hardware tanh approximation (relative error ~2^-11, far below
-// one bf16 ulp): three instructions instead of exp + add + divide.  Used where few warps have a lot of gating to do.
-__device__ __forceinline__ float sigmoid_fast(float x) {
-  float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
-  return fmaf(t, 0.5f, 0.5f);
-}
-
 // 2^x with the hardware approximation (one MUFU instruction; -inf gives 0).
 __device__ __forceinline__ float ex2_fast(float x) {
   float y;
@@ -78,6 +70,8 @@ __device__ __forceinline__ float ex2_fast(float x) {
   return y;
 }
 
+// tanh with the hardware approximation, off by up to 2^-11 of itself: o sigmoid(g) = o/2 tanh(g/2) + o/2 is then off by 2^-12 of |o| at most,
+// an absolute error that does not shrink with the sigmoid where the gate is far below zero.
 __device__ __forceinline__ float tanh_fast(float x) {
   float t;
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(x));
@@ -169,7 +163,7 @@ __device__ __forceinline__ bool warp_wait_bounded(uint64_t* bar, uint32_t parity
   return __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar, parity)) != 0;
 }
 // 1-D bulk async copy global -> shared, completion counted in bytes on an mbarrier.  dst, src and
-// bytes must all be multiples of 16.  No cluster multicast is used anywhere in this library.
+// bytes must all be multiples of 16.  No load is multicast to a cluster anywhere in this library.
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst_smem)),

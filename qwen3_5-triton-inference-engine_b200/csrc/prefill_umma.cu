@@ -15,15 +15,15 @@
 // buffers of S fill the 512 columns of tensor memory.  Roles of the 16 warps:
 //   0-3, 4-7  exponentials of the even and of the odd tiles, a thread per row; the row's reference maximum goes from one to the other
 //             through shared memory.  (Two threads per row of every tile: the exponential units idle while S, the row maximum and the
-//             store of P are waited for, 2950 cycles a tile; now 2430 with another tile's under them.)
+//             store of P are waited for, 2950 cycles a tile.)
 //   8-11      rotate the next item's Q in shared memory, then take O of this one through gate and copy engine to the output
 //   12, 15    issue S and PV (even CTA only; the odd one's 12 passes its rotated Q on), 13 loads K, 14 deals the items and loads Q and V
 // P is stored as packed bf16 over the first 64 columns of the S buffer just read; S of tile j+2 waits for PV of tile j to complete.  O is
 // rescaled in TMEM only when a row maximum grows by more than 2^8 (the running reference maximum may lag; p then stays <= 256, exact
 // for bf16 and fp32 l).
 // Bound: the tensor pipe, 2137 of 2765 cycles a tile; the rest is the completion of PV that S of the buffer waits for.  The chip's power cap
-// comes before it in long runs (1560 MHz).  8 x 4096 tokens with rope and gate: 630 -> 599 us, in bursts 543 -> 506; 64 x 512 without:
-// 380 -> 333; 32 of 16 to 512: 67.3 -> 59.6.  Short prompts are bound by what comes first: loads from HBM by all SMs at once and the fetch of
+// comes before it in long runs (1560 MHz).  us with rope and gate, one CTA per 32 queries and pairs: 8 x 4096 tokens 623 -> 575, in bursts 533 ->
+// 497; 64 x 512 227 -> 174; 32 of 16 to 512 67.5 -> 61.4.  Short prompts are bound by what comes first: loads from HBM by all SMs at once and the fetch of
 // instructions, some 200 cycles for every eight (therefore loops where unrolled code would run once).
 // The reference's rounding points are kept where they matter for the 2e-2 bar: p is rounded to bf16 for the PV
 // product while l sums the fp32 p; scores are scaled in fp32 (the reference pre-scales q and re-rounds it to bf16).

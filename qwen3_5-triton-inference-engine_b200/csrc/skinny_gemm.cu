@@ -4,7 +4,7 @@
 // decode step (README-EN.md:116).
 //
 // The product is HBM-bound on W (M is tiny), so the kernel is built like the decode-attention kernels: X is staged once
-// per CTA in shared memory (one bulk copy per row), every warp streams rows of W through a private ring of 4 KiB tiles
+// per CTA in shared memory (a tensor-map box per 128 columns), every warp streams rows of W through a private ring of 4 KiB tiles
 // (tensor-map TMA, 128-byte swizzle -> conflict-free ldmatrix, one mbarrier per tile, no cluster multicast), and
 // multiplies with mma.sync m16n8k16 taking the W rows as the MMA M dimension and the batch as N (M <= 32 is far too
 // thin for a tcgen05 tile).  CTAs walk the row blocks persistently, so X is read once per CTA however large N is.
@@ -39,7 +39,7 @@ constexpr int SG_STD_WARPS = SG_WARPS * SG_KSPLIT;
 constexpr int SG_STD_THREADS = SG_STD_WARPS * 32;
 constexpr int SG_STD_RING = SG_RING / SG_KSPLIT;  // the same bytes in flight per CTA
 constexpr int SG_MAX_M = 32;
-constexpr int SG_MAX_K = 1280;           // X staging: 32 x (K*2 + 16) bytes next to 128 KiB of weight rings
+constexpr int SG_MAX_K = 1280;           // X staging: 32 rows of it next to 128 KiB of weight rings (skinny_smem)
 
 struct SkinnyGemmParams {
   const __nv_bfloat16* x;  // [M, K]

@@ -1,5 +1,6 @@
 // Blackwell (sm_100a) building blocks: TMA tensor-map loads, tcgen05 tensor-core MMA with accumulators in tensor
-// memory (TMEM), and the descriptors both need.  Inline PTX only; no cluster multicast anywhere.
+// memory (TMEM), and the descriptors both need.  Inline PTX only; no load is multicast to a
+// cluster (umma_commit_pair's arrival, which names both CTAs of a pair, is no load).
 //
 // Shared-memory operand tiles use the 128-byte swizzle: a tile is stored as column blocks of 64 bf16 (128 bytes)
 // by R rows, block after block; inside a block row r lives at byte r*128 with its 16-byte chunk c at position
