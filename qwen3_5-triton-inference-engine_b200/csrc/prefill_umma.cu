@@ -21,10 +21,11 @@
 // P is stored as packed bf16 over the first 64 columns of the S buffer just read; S of tile j+2 waits for PV of tile j to complete.  O is
 // rescaled in TMEM only when a row maximum grows by more than 2^8 (the running reference maximum may lag; p then stays <= 256, exact
 // for bf16 and fp32 l).
-// Bound: the tensor pipe, 2137 of 2765 cycles a tile; the rest is the completion of PV that S of the buffer waits for.  The chip's power cap
-// comes before it in long runs (1560 MHz).  us with rope and gate, one CTA per 32 queries and pairs: 8 x 4096 tokens 623 -> 575, in bursts 533 ->
-// 497; 64 x 512 227 -> 174; 32 of 16 to 512 67.5 -> 61.4.  Short prompts are bound by what comes first: loads from HBM by all SMs at once and the fetch of
-// instructions, some 200 cycles for every eight (therefore loops where unrolled code would run once).
+// Bound: the tensor pipe, 2137 of 2765 cycles a tile (68 % of a launch of 8 x 4096 tokens by counter); the rest is the completion of PV that
+// S of the buffer waits for.  The chip's power cap comes before it in long runs (1560 MHz).  us with rope and gate, one CTA per 32 queries and
+// pairs: 8 x 4096 tokens 623 -> 575, in bursts 533 -> 497; 64 x 512 227 -> 174; 32 of 16 to 512 67.5 -> 61.4.  Short prompts are bound by what
+// comes first: loads from HBM by all SMs at once and the fetch of instructions, some 200 cycles for every eight (therefore loops where unrolled
+// code would run once).
 // The reference's rounding points are kept where they matter for the 2e-2 bar: p is rounded to bf16 for the PV
 // product while l sums the fp32 p; scores are scaled in fp32 (the reference pre-scales q and re-rounds it to bf16).
 // Every mbarrier wait is bounded; on expiry the role sets the device error flag and the CTA drains and exits.
